@@ -284,8 +284,8 @@ extern "C" void n2m_context_destroy(n2m_context *c) {
                       &c->tris_raw, &c->pts, &c->tris, &c->ntf, &c->weld, &c->gath, &c->hmesh,
                       &c->mc.words, &c->mc.counts, &c->mc.cand, &c->mc.verts_tmp, &c->mc.tris_tmp, &c->mc.signs, &c->mc.ctr, &c->scan.part,
                       &c->lab.lab, &c->lab.mask, &c->lab.keep, &c->lab.cnt, &c->lab.edge, &c->lab.rc, &c->lab.misc,
-                      &c->deg.flags, &c->deg.tmp, &c->hc.start, &c->hc.refs, &c->hc.fill, &c->hc.P, &c->hc.Q,
-                      &c->hc.B, &c->hc.Lo, &c->hc.border, &c->hc.hasnb, &c->hc.bad, &c->th.buf, &c->th.table,
+                      &c->deg.flags, &c->deg.tmp, &c->hc.zero, &c->hc.adj, &c->hc.meta, &c->hc.P, &c->hc.Q,
+                      &c->hc.B, &c->hc.Lo, &c->th.buf, &c->th.table,
                       &c->stmp2, &c->lubits, &c->od.st, &c->od.unc, &c->od.cmin, &c->od.cmax, &c->od.need_z, &c->od.need_y,
                       &c->od.need_x, &c->od.off, &c->od.list, &c->od.lcnt, &c->od.vsign,
                       &c->wr.mt, &c->wr.mp, &c->wr.pack, &c->wr.pack2, &c->wr.lens, &c->wr.flag, &c->wr.out};
@@ -1157,7 +1157,7 @@ extern "C" n2m_status n2m_meshify_backward(n2m_context *c, const float *d_grad_p
     CKS(c->gs.ensure(nvox * sizeof(float)));
     const float3 *go = (const float3 *)d_grad_pts;
     if (c->fwd.post_smooth > 0) {
-        CKS(mesh_smooth_hc_backward(c->res_tris, np, 0.1, 0.5, c->fwd.post_smooth, true, c->hc, go, c->gA.as<float3>(),
+        CKS(mesh_smooth_hc_backward(np, 0.1, 0.5, c->fwd.post_smooth, true, c->hc, go, c->gA.as<float3>(),
                                     c->stream));
         go = c->gA.as<float3>();
     }

@@ -290,7 +290,10 @@ struct DegWork {
 n2m_status mesh_remove_degenerate(const vec3d *d_pts, const vec3i *d_tris_in, int nt, vec3i *d_tris_out,
                                   unsigned *d_nt_out, DegWork &w, ScanWork &sw, cudaStream_t s);
 struct HcWork {
-    DevBuf start, refs, fill, P, Q, B, Lo, border, hasnb, bad;
+    DevBuf zero;              // degrees / offsets, cursors, the bad-index flag, border flags
+    DevBuf adj, meta;         // neighbour lists and their per-vertex heads
+    DevBuf P, Q, B, Lo;       // displacements
+
 };
 // Triangles with an index outside [0, np) are skipped and flagged; the flag
 // makes the last kernel leave d_pts unchanged.  mesh_smooth_hc_check waits for
@@ -300,9 +303,9 @@ struct HcWork {
 n2m_status mesh_smooth_hc(vec3d *d_pts, const vec3i *d_tris, int np, int nt, double alpha, double beta, int iter,
                           bool lock_edges, HcWork &w, ScanWork &sw, cudaStream_t s);
 n2m_status mesh_smooth_hc_check(HcWork &w, int np, int iter, cudaStream_t s);
-// adjoint of mesh_smooth_hc (uses the CSR and border flags the forward left in w)
-n2m_status mesh_smooth_hc_backward(const vec3i *d_tris, int np, double alpha, double beta, int iter, bool lock_edges,
-                                   HcWork &w, const float3 *d_g, float3 *d_go, cudaStream_t s);
+// adjoint of mesh_smooth_hc (uses the neighbour lists and border flags the forward left in w)
+n2m_status mesh_smooth_hc_backward(int np, double alpha, double beta, int iter, bool lock_edges, HcWork &w,
+                                   const float3 *d_g, float3 *d_go, cudaStream_t s);
 // grad of raw (pre-weld) vertices from grad of welded vertices
 n2m_status mesh_weld_backward(const float3 *d_go, int np_final, int nv_raw, const int *d_removed, int nrem,
                               const int *d_ov_id, const int *d_ov_src, int nov, float3 *d_graw, cudaStream_t s);
