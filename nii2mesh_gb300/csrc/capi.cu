@@ -282,7 +282,7 @@ extern "C" void n2m_context_destroy(n2m_context *c) {
                       &c->aw.pts, &c->aw.pts2, &c->aw.tris, &c->aw.tris2, &c->aw.cand, &c->aw.gath, &c->aw.weld,
                       &c->aw.ranges, &c->alab, &c->lpts, &c->ltris, &c->gA, &c->gB, &c->gs, &c->gtmp, &c->in, &c->raw, &c->vol, &c->stmp, &c->stats, &c->totals, &c->cand, &c->ncand, &c->ocq, &c->pts_raw,
                       &c->tris_raw, &c->pts, &c->tris, &c->ntf, &c->weld, &c->gath, &c->hmesh,
-                      &c->mc.words, &c->mc.counts, &c->mc.cand, &c->mc.verts_tmp, &c->mc.tris_tmp, &c->mc.signs, &c->mc.ctr, &c->scan.part,
+                      &c->mc.signs, &c->mc.words, &c->mc.act, &c->mc.staged, &c->mc.sub, &c->scan.part,
                       &c->lab.lab, &c->lab.mask, &c->lab.keep, &c->lab.cnt, &c->lab.edge, &c->lab.rc, &c->lab.misc,
                       &c->deg.flags, &c->deg.tmp, &c->hc.zero, &c->hc.adj, &c->hc.meta, &c->hc.P, &c->hc.Q,
                       &c->hc.B, &c->hc.Lo, &c->th.buf, &c->th.table,
@@ -512,8 +512,8 @@ n2m_status weld_oc(n2m_context *c, const Prep &P, const int dim[3], int nv, int 
     CKS(c->gath.ensure((size_t)n * (sizeof(vec3d) + sizeof(int))));
     vec3d *dpos = c->gath.as<vec3d>();
     int *dvid = (int *)(dpos + n);
-    CKS(oc_copy_positions(P.vol, dim, P.lo, P.hi, P.iso, P.edge_max, c->mc, c->tris_raw.as<vec3i>(), dq, n, dvid, dpos,
-                          c->stream));
+    CKS(oc_copy_positions(P.vol, dim, P.lo, P.hi, P.iso, P.edge_max, c->mc, c->fwd.mcn.nactive, c->tris_raw.as<vec3i>(), dq, n,
+                          dvid, dpos, c->stream));
     std::vector<unsigned> q(n);
     std::vector<int> vid(n);
     std::vector<vec3d> pos(n);
@@ -723,10 +723,10 @@ n2m_status march(n2m_context *c, const Prep &P, const int dim[3], int cubes, int
         CKS(c->stmp2.ensure(n * sizeof(float)));
         const OdRepair rep{P.src, c->stmp.as<float>(), c->stmp2.as<float>(), (float *)P.vol, {dim[0], dim[1], dim[2]},
                            &c->od, &c->scan, P.post};
-        if (old) CKS(oc_count(P.vol, dim, P.lo, P.hi, P.iso, P.edge_max, c->mc, c->scan, dtot, c->stream, &rep));
-        else CKS(mc_count(g, cubes, c->mc, c->scan, dtot, c->stream, &rep));
-    } else if (old) CKS(oc_count(P.vol, dim, P.lo, P.hi, P.iso, P.edge_max, c->mc, c->scan, dtot, c->stream));
-    else CKS(mc_count(g, cubes, c->mc, c->scan, dtot, c->stream));
+        if (old) CKS(oc_count(P.vol, dim, P.lo, P.hi, P.iso, P.edge_max, c->mc, dtot, c->stream, &rep));
+        else CKS(mc_count(g, cubes, c->mc, dtot, c->stream, &rep));
+    } else if (old) CKS(oc_count(P.vol, dim, P.lo, P.hi, P.iso, P.edge_max, c->mc, dtot, c->stream));
+    else CKS(mc_count(g, cubes, c->mc, dtot, c->stream));
     CK(cudaEventRecord(c->evs[3], c->stream));
     uint4 tot;
     CKS(readback(c, &tot, dtot));

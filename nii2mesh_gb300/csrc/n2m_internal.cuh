@@ -244,7 +244,10 @@ struct McGrid {
     float iso, edge_max, pad_val;   // pad_val = float(min' - iso)
 };
 struct McWork {
-    DevBuf words, counts, cand, verts_tmp, tris_tmp, signs, ctr;
+    DevBuf signs;            // sign words of the grid
+    DevBuf words;            // per active word {x, y, z crossing masks, vertex offset}
+    DevBuf act;              // active words in order {word, triangle offset, c-vertex offset, -}
+    DevBuf staged, sub;      // counting scratch (mcwords.cuh: Out)
 };
 struct McCounts {
     unsigned nv_edge, nt, nc, nactive;
@@ -253,7 +256,7 @@ struct McCounts {
 // after the sign pass and runs od_repair before any value is read (null: none)
 // (with a repair and no labelling, the sign words of grid points strictly inside
 // the volume come from repair->w->vsign instead of the values)
-n2m_status mc_count(const McGrid &g, int variant, McWork &w, ScanWork &sw, uint4 *d_total, cudaStream_t s,
+n2m_status mc_count(const McGrid &g, int variant, McWork &w, uint4 *d_total, cudaStream_t s,
                     const OdRepair *repair = nullptr);
 n2m_status mc_emit(const McGrid &g, int variant, McWork &w, const McCounts &c, vec3d *d_pts, vec3i *d_tris,
                    int *d_cand, unsigned *d_ncand, int cand_cap, cudaStream_t s);
@@ -265,7 +268,7 @@ n2m_status mc_ccand_scan(const vec3d *d_pts, int np, const int *d_ccand, int ncc
 // oldcubes.cu
 // repair: as for mc_count (vsign must then hold od_resolve's at_or_above sign)
 n2m_status oc_count(const float *vol, const int dim[3], const int lo[3], const int hi[3], float iso, float edge_max,
-                    McWork &w, ScanWork &sw, uint4 *d_total, cudaStream_t s, const OdRepair *repair = nullptr);
+                    McWork &w, uint4 *d_total, cudaStream_t s, const OdRepair *repair = nullptr);
 n2m_status oc_emit(const float *vol, const int dim[3], const int lo[3], const int hi[3], float iso, float edge_max,
                     McWork &w, const McCounts &c, vec3d *d_pts, vec3i *d_tris, int *d_cand, unsigned *d_ncand,
                     int cand_cap, cudaStream_t s);
@@ -277,8 +280,8 @@ n2m_status oc_copies(const vec3i *d_tris, int nt, int nv, const int *d_cand, int
 // the vertex id each listed corner names and the position the cube that emitted
 // its triangle interpolates for it (needs oc_count's words of the same grid)
 n2m_status oc_copy_positions(const float *vol, const int dim[3], const int lo[3], const int hi[3], float iso,
-                             float edge_max, const McWork &w, const vec3i *d_tris, const unsigned *d_q, int n, int *d_vid,
-                             vec3d *d_pos, cudaStream_t s);
+                             float edge_max, const McWork &w, unsigned nactive, const vec3i *d_tris, const unsigned *d_q,
+                             int n, int *d_vid, vec3d *d_pos, cudaStream_t s);
 
 // mesh.cu
 n2m_status mesh_apply_weld(vec3d *d_pts, vec3i *d_tris, int np, int nt, const int *d_removed, const int *d_keep,
