@@ -286,7 +286,7 @@ extern "C" void n2m_context_destroy(n2m_context *c) {
                       &c->lab.lab, &c->lab.mask, &c->lab.keep, &c->lab.cnt, &c->lab.edge, &c->lab.rc, &c->lab.misc,
                       &c->deg.flags, &c->deg.tmp, &c->hc.zero, &c->hc.adj, &c->hc.meta, &c->hc.P, &c->hc.Q,
                       &c->hc.B, &c->hc.Lo, &c->th.buf, &c->th.table,
-                      &c->stmp2, &c->lubits, &c->od.st, &c->od.unc, &c->od.cmin, &c->od.cmax, &c->od.need_z, &c->od.need_y,
+                      &c->stmp2, &c->lubits, &c->od.st, &c->od.unc, &c->od.cmin, &c->od.cmax, &c->od.range, &c->od.need_z, &c->od.need_y,
                       &c->od.need_x, &c->od.off, &c->od.list, &c->od.lcnt, &c->od.vsign,
                       &c->wr.mt, &c->wr.mp, &c->wr.pack, &c->wr.pack2, &c->wr.lens, &c->wr.flag, &c->wr.out};
     for (DevBuf *b : bufs) b->release();
@@ -602,19 +602,22 @@ n2m_status prepare(n2m_context *c, const float *d_src, const int dim[3], const n
     // smoothed while it arrives that way (the on-demand repair could only start after
     // the last slab)
     bool od = smooth && (!label || o.only_largest) && !c->stage.host && od_eligible(d_src, nx, ny, nz);
+    OdStats hod;
     if (smooth) {
         CKS(c->stmp.ensure(n * sizeof(float)));
         const StagedInput *stage = c->stage.host ? &c->stage : nullptr;
         if (od) {
-            bool fallback = false;
             CK(cudaEventRecord(c->eva[0], c->stream));
-            CKS(od_approx(d_src, vol, nx, ny, nz, iso, c->od, c->stream, stage));
+            CKS(od_approx(d_src, vol, nx, ny, nz, iso, c->od, c->stream));
             CK(cudaEventRecord(c->eva[1], c->stream));
             c->pass_a = true;
-            CKS(od_resolve(d_src, vol, nx, ny, nz, iso, c->od, dst, c->stream, &fallback, label || o.cubes == N2M_CUBES_OLDCUBES));
-            if (fallback) {   // the input is on the device by now
+            CKS(od_resolve(d_src, vol, nx, ny, nz, iso, c->od, c->stream, label || o.cubes == N2M_CUBES_OLDCUBES));
+            CK(cudaEventRecord(c->evs[1], c->stream));
+            CKS(readback(c, &hod, c->od.st.p));
+            bool fallback = false;
+            CKS(od_check(c->od, hod, &fallback));
+            if (fallback) {
                 od = false;
-                CK(cudaMemcpyAsync(dst, h, sizeof(VolStats), cudaMemcpyHostToDevice, c->stream));
                 CKS(launch_smooth(d_src, vol, c->stmp.as<float>(), nx, ny, nz, iso, dst, c->stream, nullptr));
             }
         } else {
@@ -622,10 +625,11 @@ n2m_status prepare(n2m_context *c, const float *d_src, const int dim[3], const n
         }
     }
     else CKS(launch_stats(label ? vol : d_src, nx, ny, nz, iso, true, dst, c->stream));
-    CK(cudaEventRecord(c->evs[1], c->stream));
+    if (!od) CK(cudaEventRecord(c->evs[1], c->stream));
     const float *v = vol ? vol : d_src;
     VolStats s0;
-    CKS(readback(c, &s0, dst));
+    if (od) s0 = hod.vs;
+    else CKS(readback(c, &s0, dst));
     if (s0.nonfinite) {
         n2m_set_error("%u non-finite voxels in the volume", s0.nonfinite);
         return N2M_ERR_NONFINITE;

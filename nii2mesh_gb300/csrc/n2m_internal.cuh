@@ -88,14 +88,15 @@ n2m_status launch_smooth(const float *in, float *out, float *tmp, int nx, int ny
 bool smooth_can_stage(int nx, int ny, int nz);
 
 // Pre-smooth with exact rounding on demand (smooth.cu): od_approx smooths the
-// whole volume approximately (one fused FP32 pass, rigorous error bound) and
-// lists the voxels whose sign against iso it cannot decide and the candidates
-// for the volume's range; od_resolve gives those their exact values and fills
-// `dst` (exact range, bbox, no non-finite count) unless *fallback (a
-// non-finite or huge input, a list overflow): then the caller runs
-// launch_smooth instead.  Marching cubes marks the corners of the cubes the
-// surface crosses in need_z (mc.cu: mc_count with an OdRepair), and od_repair
-// writes the reference's exact value at every marked voxel of `out`.
+// whole volume approximately (one fused FP32 pass, rigorous error bound), lists
+// the voxels whose sign against iso it cannot decide and leaves the range of each
+// task; od_resolve gives those voxels, and every voxel that can be the volume's
+// minimum or maximum, their exact values, which completes w.st (exact range and
+// bbox in its vs).  Once the host has read w.st, od_check says whether the caller
+// has to run launch_smooth instead (a non-finite or huge input, a list overflow).
+// Marching cubes marks the corners of the cubes the surface crosses in need_z
+// (mc.cu: mc_count with an OdRepair), and od_repair writes the reference's exact
+// value at every marked voxel of `out`.
 enum : unsigned { OD_FALLBACK = 1u, OD_TIMEOUT = 2u };
 struct OdStats {
     VolStats vs;             // bbox of decided voxels >= iso; exact range after od_resolve
@@ -103,20 +104,16 @@ struct OdStats {
     unsigned cnt[3];         // undecided, min candidates, max candidates
     int umin, lmax;          // ordered: smallest task min + B, largest task max - B
 };
-struct OdCand {              // a range candidate: voxel, approximate value, its bound
-    unsigned j;
-    float v, b;
-};
 struct OdLists {
-    unsigned *unc;
-    OdCand *cmin, *cmax;
+    unsigned *unc, *cmin, *cmax;   // voxels
     unsigned *cnt;
     unsigned cap;
     unsigned *vsign;         // sign bitmap of the smoothed volume (see OdWork)
-    unsigned wv, nys;        // its words per row, groups of 8 rows per slice
+    float4 *range;           // per task of pass A {min, max, B, -}
+    unsigned wv, nys;        // the bitmap's words per row, groups of 8 rows per slice
 };
 struct OdWork {
-    DevBuf st, unc, cmin, cmax, need_z, need_y, need_x, off, list, lcnt;
+    DevBuf st, unc, cmin, cmax, range, need_z, need_y, need_x, off, list, lcnt;
     // bit x & 31 of word od_vsign_word(x, y, z): the smoothed value of voxel (x, y, z)
     // minus iso is above -FLT_EPSILON (Lewiner's sign before edge darkening), or with
     // od_resolve's at_or_above, the value is >= iso (the complement of oldcubes'
@@ -161,10 +158,10 @@ __device__ __forceinline__ void od_need_mark(unsigned *need, long long j, unsign
 }
 // whether the on-demand path applies: rows a multiple of 16 bytes (TMA tiles), fewer than 2^32 voxels
 bool od_eligible(const float *in, int nx, int ny, int nz);
-n2m_status od_approx(const float *in, float *out, int nx, int ny, int nz, float iso, OdWork &w, cudaStream_t s,
-                     const StagedInput *stage = nullptr);
-n2m_status od_resolve(const float *in, float *out, int nx, int ny, int nz, float iso, OdWork &w, VolStats *dst,
-                      cudaStream_t s, bool *fallback, bool at_or_above = false);
+n2m_status od_approx(const float *in, float *out, int nx, int ny, int nz, float iso, OdWork &w, cudaStream_t s);
+n2m_status od_resolve(const float *in, float *out, int nx, int ny, int nz, float iso, OdWork &w, cudaStream_t s,
+                      bool at_or_above = false);
+n2m_status od_check(const OdWork &w, const OdStats &h, bool *fallback);
 n2m_status od_repair(const OdRepair &r, cudaStream_t s);
 // transposed pre-smooth: g_img = Sx^T Sy^T Sz^T g (tmp: one volume of scratch)
 n2m_status launch_smooth_adjoint(const float *g, float *tmp, float *out, int nx, int ny, int nz, cudaStream_t s);

@@ -491,9 +491,45 @@ n2m_status launch_stats(const float *vol, int nx, int ny, int nz, float iso, boo
 // 21 * 2^-24 * M < 2^-19 * M, M being any bound on the input magnitudes the
 // voxel depends on.  A warp uses the largest magnitude it has read so far.
 namespace {
-constexpr int OW_Y = 8, OW_Z = 32;   // pass A warp task: 32 x 8 x 32 output voxels
 constexpr float OW0 = 0.45f, OW1 = 0.225f, OW2 = 0.05f;
 
+// two floats in one 64-bit register pair: each instruction works on both halves, rounded as the scalar one rounds
+typedef unsigned long long f2;
+__device__ __forceinline__ f2 pack2(float lo, float hi) {
+    f2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void unpack2(f2 v, float &lo, float &hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
+    f2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
+    f2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f2 add2(f2 a, f2 b) {
+    f2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+// three-input minimum and maximum (a NaN operand is ignored, as by fminf and fmaxf)
+__device__ __forceinline__ float min3(float a, float b, float c) {
+    float r;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+__device__ __forceinline__ f2 tap2(f2 a, f2 b, f2 c, f2 d, f2 e, f2 w0, f2 w1, f2 w2) {
+    return fma2(e, w2, fma2(d, w1, fma2(c, w0, fma2(b, w1, mul2(a, w2)))));
+}
 __device__ __forceinline__ float fma5(float a, float b, float c, float d, float e) {
     return __fmaf_rn(e, OW2, __fmaf_rn(d, OW1, __fmaf_rn(c, OW0, __fmaf_rn(b, OW1, __fmul_rn(a, OW2)))));
 }
@@ -529,33 +565,78 @@ __device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, u
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 // Pass A: the input volume through a TMA tensor map (nx a multiple of 4, so
-// that the rows are 16-byte aligned); boxes of 40 x 12 x 1 floats, x0 - 4 ..
-// x0 + 35 and y0 - 2 .. y0 + 9 of one slice (outside the volume the copy fills
-// zeros).  A warp takes 32 x 8 columns of 32 slices (lane = x): its lane 0
-// keeps OA_S slices in flight in the warp's own ring of shared-memory stages,
-// each completing on its mbarrier; the x pass reads the stage, the y pass runs
-// over the 12 rows in registers, the z pass over a five-slice ring of the
-// eight rows' y values.  Each output is classified on the spot:
-// |v - iso| <= B + 4 eps -> listed as undecided, else v >= iso -> bbox.  At the
-// end of its task the warp lists the outputs within 2.5 B of its minimum
-// (maximum) with their value and B (range candidates) and offers min + B
-// (max - B) as a bound on the volume's exact extreme.  Waits give up after a
-// fixed number of polls (flag OD_TIMEOUT), after waiting, also bounded, for the
-// warp's copies still in flight.
-constexpr int OA_S = 4, OA_BW = 40, OA_BH = 12, OA_WARPS = 4;
+// that the rows are 16-byte aligned); boxes of 72 x 12 x 1 floats, x0 - 4 ..
+// x0 + 67 and y0 - 2 .. y0 + 9 of one slice (outside the volume the copy fills
+// zeros).  A warp takes 64 x 8 columns of `zrun` slices; its lane 0 keeps OA_S
+// slices in flight in the warp's own ring of shared-memory stages, each
+// completing on its mbarrier.  A lane owns 4 consecutive columns (one 16-byte
+// load per row, two register pairs) of 4 rows, lanes 0-15 the tile's upper rows
+// and 16-31 its lower ones.  The passes run y, z, x: the y pass over the 8 loaded
+// rows and the z pass over a five-slice register ring stay inside a lane and use
+// the paired FP32 instructions; only the x pass needs neighbours, two values from
+// each side per row, by shuffle.  The two columns beyond either end of a tile row
+// are 16 (column, row) pairs, one per lane, that take the same y and z passes.
+// The separable filter's axes commute, so the order does not enter the bound.
+// Each output is classified on the spot: |v - iso| <= B + 4 eps -> listed as
+// undecided, else its sign goes to the bitmap and, when positive, the bbox.  A
+// task leaves its minimum, maximum and B for k_od_scan and offers min + B
+// (max - B) as a bound on the volume's exact extreme.  Waits give up after a fixed
+// number of polls (flag OD_TIMEOUT), after waiting, also bounded, for the warp's
+// copies still in flight.
+//
+// 512^3: 1.09 GB (8.1 bytes a voxel) in 268 us = 4.1 TB/s, 38 instructions a voxel at
+// 53 % of the issue slots: the register ring allows 12 warps per SM, and their
+// dependent FP32 chains and the half-rate min/max and shifts bound it.  With one column
+// and 8 rows per lane (x pass first, five shared-memory loads per row, 92
+// instructions a voxel) it took 479 us.  Two rows per lane (more warps, twice the halo
+// rows): 292 us; a fourth CTA per SM (spills): 423 us.
+constexpr int OA_R = 4, OA_S = 4, OA_X = 64, OA_Y = 2 * OA_R, OA_BW = OA_X + 8, OA_BH = OA_Y + 4, OA_WARPS = 4;
 constexpr unsigned OA_BYTES = OA_BW * OA_BH * 4;
 constexpr int OA_POLLS = 1 << 22;
 struct __align__(128) OaStage {
     float v[OA_BH][OA_BW];
 };
 
-__global__ void __launch_bounds__(OA_WARPS * 32) k_od_approx(const __grid_constant__ CUtensorMap tmap, float *out,
-                                                             int nx, int ny, int nz, int z_lo, int z_hi, float iso,
-                                                             OdStats *st, OdLists L) {
+// OR over the eight lanes that share a 32-voxel word, of the lane's four rows' words at once: lane i of the eight
+// ends up with the word of row word_row(i)
+__device__ __forceinline__ int word_row(int lane) { return (lane & 1) * 2 + (lane >> 1 & 1); }
+__device__ __forceinline__ unsigned or_rows(const unsigned (&p)[OA_R], int lane) {
+    const unsigned FULL = 0xffffffffu;
+    const bool b0 = lane & 1, b1 = lane & 2;
+    unsigned k0 = b0 ? p[2] : p[0], k1 = b0 ? p[3] : p[1];
+    k0 |= __shfl_xor_sync(FULL, b0 ? p[0] : p[2], 1);
+    k1 |= __shfl_xor_sync(FULL, b0 ? p[1] : p[3], 1);
+    unsigned k = b1 ? k1 : k0;
+    k |= __shfl_xor_sync(FULL, b1 ? k0 : k1, 2);
+    return k | __shfl_xor_sync(FULL, k, 4);
+}
+
+// lists the lane's undecided voxels (any: it has some), in `rows` rows of 4 from p; returns its row word's bits of them.
+// Out of line: rare, and the kernel's slice loop is unrolled five times.
+__device__ __noinline__ unsigned list_undecided(const float *p, int nx, int rows, unsigned j, bool any, float band, float iso,
+                                                unsigned *cnt, unsigned *list, unsigned cap, int lane) {
+    unsigned uw[OA_R];
+#pragma unroll
+    for (int r = 0; r < OA_R; r++) {
+        unsigned m = 0u;
+        for (int c = 0; any && r < rows && c < 4; c++)
+            if (fabsf(__fsub_rn(p[(size_t)r * nx + c], iso)) <= band) {
+                m |= 1u << (4 * (lane & 7) + c);
+                const unsigned q = atomicAdd(cnt, 1u);
+                if (q < cap) list[q] = j + (unsigned)(r * nx + c);
+            }
+        uw[r] = m;
+    }
+    return or_rows(uw, lane);
+}
+
+__global__ void __launch_bounds__(OA_WARPS * 32, 3) k_od_approx(const __grid_constant__ CUtensorMap tmap, float *out,
+                                                             int nx, int ny, int nz, int zrun, float iso, OdStats *st,
+                                                             OdLists L) {
     const unsigned FULL = 0xffffffffu;
     __shared__ OaStage stage[OA_WARPS][OA_S];
     __shared__ unsigned long long bars[OA_WARPS][OA_S];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, seg = lane >> 4, li = lane & 15;
     OaStage *sg = stage[wid];
     unsigned long long *bw = bars[wid];
     if (lane == 0) {
@@ -564,16 +645,19 @@ __global__ void __launch_bounds__(OA_WARPS * 32) k_od_approx(const __grid_consta
     }
     __syncwarp();
     unsigned issued = 0, used = 0;   // loads issued / consumed by this warp (stage = n % OA_S, parity = n / OA_S)
-    const unsigned nxs = (unsigned)(nx + 31) / 32, nys = (unsigned)(ny + OW_Y - 1) / OW_Y;
-    const unsigned nzs = (unsigned)(z_hi - z_lo + OW_Z - 1) / OW_Z;
-    const unsigned ntask = nxs * nys * nzs;
+    const unsigned nxs = (unsigned)(nx + OA_X - 1) / OA_X, nys = (unsigned)(ny + OA_Y - 1) / OA_Y;
+    const unsigned ntask = nxs * nys * ((unsigned)(nz + zrun - 1) / (unsigned)zrun);
     const size_t nxy = (size_t)nx * ny;
+    const f2 w0 = pack2(OW0, OW0), w1 = pack2(OW1, OW1), w2 = pack2(OW2, OW2), zero2 = pack2(0.f, 0.f), niso2 = pack2(-iso, -iso);
+    // this lane's halo column and row: columns x0-2, x0-1, x0+64, x0+65
+    const int hc = (li / OA_R) & 3, hr = li % OA_R, hcol = hc < 2 ? 2 + hc : OA_X + 2 + hc;
     bool timed_out = false;
     for (unsigned task = blockIdx.x * OA_WARPS + wid; task < ntask && !timed_out; task += gridDim.x * OA_WARPS) {
         const unsigned xs = task % nxs, t2 = task / nxs;
-        const int y0 = (int)(t2 % nys) * OW_Y, zs = z_lo + (int)(t2 / nys) * OW_Z, ze = min(zs + OW_Z, z_hi);
-        const int x0 = (int)xs * 32, x = x0 + lane;
-        const bool ownx = x < nx, xint = x >= 2 && x <= nx - 3;
+        const int x0 = (int)xs * OA_X, y0 = (int)(t2 % nys) * OA_Y, zs = (int)(t2 / nys) * zrun, ze = min(zs + zrun, nz);
+        const int x = x0 + 4 * li, y = y0 + OA_R * seg;   // first column and row of this lane
+        const bool ownx = x < nx;
+        const bool xedge = x0 == 0 || x0 + OA_X >= nx, yedge = y0 < 2 || y0 + OA_Y > ny - 2;
         // every slice zs-2 .. ze+1 is loaded (outside the volume: zeros, read only by outputs that ignore them)
         int znext = zs - 2;
         const int zlast = ze + 1;
@@ -588,162 +672,170 @@ __global__ void __launch_bounds__(OA_WARPS * 32) k_od_approx(const __grid_consta
             znext++;
         };
         while (znext <= zlast && issued - used < (unsigned)OA_S) issue();
-        float zr[5][OW_Y];   // y values of slices z-2 .. z+2 (slot 4 newest)
+        f2 zr[5][OA_R][2];   // y values of five slices
+        float hz[5];
 #pragma unroll
-        for (int a = 0; a < 5; a++)
+        for (int a = 0; a < 5; a++) {
+            hz[a] = 0.f;
 #pragma unroll
-            for (int k = 0; k < OW_Y; k++) zr[a][k] = 0.f;
+            for (int r = 0; r < OA_R; r++) zr[a][r][0] = zr[a][r][1] = zero2;
+        }
         float mrun = 0.f, lmin = INFINITY, lmax = -INFINITY, B = 0.f;
-        float lmin2 = INFINITY, lmax2 = -INFINITY;   // second smallest / largest
-        unsigned jmin = 0, jmax = 0;                 // where lmin / lmax are
         int bzl = INT_MAX, bzh = INT_MIN;
-        unsigned ymask = 0;                          // rows with a decided voxel >= iso
-        unsigned sgn = 0;                            // this slice's sign bits, bit kk = row y0 + kk
-        float nanacc = 0.f;                          // becomes NaN if an output is NaN or infinite
-        for (int zi = zs - 2; zi <= zlast; zi++) {
-            const unsigned k = used % OA_S, par = (used / OA_S) & 1u;
-            bool ok = false;
-            for (int it = 0; it < OA_POLLS && !ok; it++) ok = mbar_try_wait(&bw[k], par);
-            if (!__all_sync(FULL, ok)) {
-                timed_out = true;
-                break;
-            }
+        unsigned orx = 0;      // this lane's row word, over the slices: columns with a decided voxel >= iso
+        f2 nanacc = zero2;     // becomes NaN if an output is NaN or infinite
+        for (int zb = zs - 2; zb <= zlast && !timed_out; zb += 5) {
 #pragma unroll
-            for (int a = 0; a < 4; a++)
-#pragma unroll
-                for (int kk = 0; kk < OW_Y; kk++) zr[a][kk] = zr[a + 1][kk];
-            const OaStage &S = sg[k];
-            float xv[OA_BH];
-#pragma unroll
-            for (int r = 0; r < OA_BH; r++) {
-                const float *q = &S.v[r][lane + 2];   // x - 2 .. x + 2
-                const float a = q[0], b = q[1], c = q[2], d = q[3], e = q[4];
-                mrun = fmaxf(mrun, fmaxf(fabsf(a), fabsf(e)));   // lanes together cover x0-2 .. x0+33
-                xv[r] = xint ? fma5(a, b, c, d, e) : c;
-            }
-#pragma unroll
-            for (int kk = 0; kk < OW_Y; kk++) {
-                const int yy = y0 + kk;
-                zr[4][kk] = (yy >= 2 && yy <= ny - 3) ? fma5(xv[kk], xv[kk + 1], xv[kk + 2], xv[kk + 3], xv[kk + 4])
-                                                      : xv[kk + 2];
-            }
-            __syncwarp();   // every lane is done with the stage
-            used++;
-            if (znext <= zlast) issue();
-            float m = mrun;
-            for (int o = 16; o; o >>= 1) m = fmaxf(m, __shfl_xor_sync(FULL, m, o));
-            B = m * 0x1p-19f;   // bounds every output whose inputs have been read
-            const int z = zi - 2;
-            sgn = 0;
-            if (z >= zs && z < ze && ownx) {
-                const bool zint = z >= 2 && z <= nz - 3;
-                const float band = B + 4.0f * N2M_FLT_EPS;
-                const unsigned j0 = (unsigned)((size_t)z * nxy + (size_t)y0 * nx + x);
-                unsigned ge = 0;
-#pragma unroll
-                for (int kk = 0; kk < OW_Y; kk++) {
-                    if (y0 + kk >= ny) continue;
-                    const float zv = zint ? fma5(zr[0][kk], zr[1][kk], zr[2][kk], zr[3][kk], zr[4][kk]) : zr[2][kk];
-                    const unsigned j = j0 + (unsigned)kk * (unsigned)nx;
-                    out[j] = zv;
-                    nanacc = __fmaf_rn(zv, 0.f, nanacc);
-                    const bool lo = zv < lmin, hi = zv > lmax;
-                    lmin2 = lo ? lmin : fminf(lmin2, zv);
-                    jmin = lo ? j : jmin;
-                    lmin = fminf(lmin, zv);
-                    lmax2 = hi ? lmax : fmaxf(lmax2, zv);
-                    jmax = hi ? j : jmax;
-                    lmax = fmaxf(lmax, zv);
-                    const float dv = __fsub_rn(zv, iso);
-                    sgn |= (unsigned)(dv > -N2M_FLT_EPS) << kk;   // provisional for undecided voxels
-                    const bool und = fabsf(dv) <= band;
-                    if (und) {
-                        const unsigned q = atomicAdd(&L.cnt[0], 1u);
-                        if (q < L.cap) L.unc[q] = j;
-                    }
-                    ge |= (unsigned)(!und && zv >= iso) << kk;
+            for (int u = 0; u < 5; u++) {   // ring slot u takes slice zb + u
+                const int zi = zb + u;
+                if (zi > zlast) break;
+                const unsigned k = used % OA_S, par = (used / OA_S) & 1u;
+                bool ok = false;
+                for (int it = 0; it < OA_POLLS && !ok; it++) ok = mbar_try_wait(&bw[k], par);
+                if (!__all_sync(FULL, ok)) {
+                    timed_out = true;
+                    break;
                 }
-                if (ge) {
-                    ymask |= ge;
+                const OaStage &S = sg[k];
+                f2 in[OA_R + 4][2];
+#pragma unroll
+                for (int r = 0; r < OA_R + 4; r++) {
+                    const ulonglong2 q = *(const ulonglong2 *)&S.v[OA_R * seg + r][4 + 4 * li];
+                    in[r][0] = q.x;
+                    in[r][1] = q.y;
+                    float a, b, c, d;
+                    unpack2(q.x, a, b);
+                    unpack2(q.y, c, d);
+                    mrun = max3(max3(mrun, fabsf(a), fabsf(b)), fabsf(c), fabsf(d));
+                }
+                float hv;
+                {
+                    const float *q = &S.v[OA_R * seg + hr][hcol];
+                    const float a = q[0], b = q[OA_BW], c = q[2 * OA_BW], d = q[3 * OA_BW], e = q[4 * OA_BW];
+                    mrun = fmaxf(max3(max3(mrun, fabsf(a), fabsf(b)), fabsf(c), fabsf(d)), fabsf(e));
+                    hv = fma5(a, b, c, d, e);
+                    if (yedge && (y + hr < 2 || y + hr > ny - 3)) hv = c;
+                }
+#pragma unroll
+                for (int r = 0; r < OA_R; r++)
+#pragma unroll
+                    for (int h = 0; h < 2; h++)
+                        zr[u][r][h] = tap2(in[r][h], in[r + 1][h], in[r + 2][h], in[r + 3][h], in[r + 4][h], w0, w1, w2);
+                if (yedge) {
+#pragma unroll
+                    for (int r = 0; r < OA_R; r++)
+                        if (y + r < 2 || y + r > ny - 3) {
+                            zr[u][r][0] = in[r + 2][0];
+                            zr[u][r][1] = in[r + 2][1];
+                        }
+                }
+                hz[u] = hv;
+                __syncwarp();   // every lane is done with the stage
+                used++;
+                if (znext <= zlast) issue();
+                // bounds every output whose inputs have been read
+                B = __uint_as_float(__reduce_max_sync(FULL, __float_as_uint(mrun))) * 0x1p-19f;
+                const int z = zi - 2;
+                if (z < zs) continue;
+                constexpr int P = 5;
+                const int s0 = (u + 1) % P, s1 = (u + 2) % P, s2 = (u + 3) % P, s3 = (u + 4) % P;   // slices z-2 .. z+1
+                const bool zint = z >= 2 && z <= nz - 3;
+                const float hy = zint ? fma5(hz[s0], hz[s1], hz[s2], hz[s3], hz[u]) : hz[s2];
+                const float band = B + 4.0f * N2M_FLT_EPS;
+                float *op = out + (size_t)z * nxy + (size_t)y * nx + x;
+                unsigned pw[OA_R];
+                float dmin = INFINITY;
+#pragma unroll
+                for (int r = 0; r < OA_R; r++) {
+                    f2 va = zr[s2][r][0], vb = zr[s2][r][1];
+                    if (zint) {
+                        va = tap2(zr[s0][r][0], zr[s1][r][0], va, zr[s3][r][0], zr[u][r][0], w0, w1, w2);
+                        vb = tap2(zr[s0][r][1], zr[s1][r][1], vb, zr[s3][r][1], zr[u][r][1], w0, w1, w2);
+                    }
+                    float v0, v1, v2, v3;
+                    unpack2(va, v0, v1);
+                    unpack2(vb, v2, v3);
+                    const float h1 = __shfl_sync(FULL, hy, li == 0 ? r : 2 * OA_R + r, 16), h2 = __shfl_sync(FULL, hy, li == 0 ? OA_R + r : 3 * OA_R + r, 16);
+                    float l2 = __shfl_up_sync(FULL, v2, 1, 16), l3 = __shfl_up_sync(FULL, v3, 1, 16);
+                    float r0 = __shfl_down_sync(FULL, v0, 1, 16), r1 = __shfl_down_sync(FULL, v1, 1, 16);
+                    l2 = li == 0 ? h1 : l2;
+                    l3 = li == 0 ? h2 : l3;
+                    r0 = li == 15 ? h1 : r0;
+                    r1 = li == 15 ? h2 : r1;
+                    const f2 m1 = pack2(v1, v2);
+                    f2 oa = tap2(pack2(l2, l3), pack2(l3, v0), va, m1, vb, w0, w1, w2);
+                    f2 ob = tap2(va, m1, vb, pack2(v3, r0), pack2(r0, r1), w0, w1, w2);
+                    if (xedge) {   // columns 0, 1 and nx-2, nx-1 keep their value
+                        if (x == 0) oa = va;
+                        if (x + 4 == nx) ob = vb;
+                    }
+                    pw[r] = 0u;
+                    if (ownx && y + r < ny) {
+                        *(ulonglong2 *)(op + (size_t)r * nx) = make_ulonglong2(oa, ob);
+                        nanacc = fma2(oa, zero2, fma2(ob, zero2, nanacc));
+                        float o0, o1, o2, o3;
+                        unpack2(oa, o0, o1);
+                        unpack2(ob, o2, o3);
+                        lmin = min3(min3(lmin, o0, o1), o2, o3);
+                        lmax = max3(max3(lmax, o0, o1), o2, o3);
+                        unpack2(add2(oa, niso2), o0, o1);
+                        unpack2(add2(ob, niso2), o2, o3);
+                        dmin = min3(min3(dmin, fabsf(o0), fabsf(o1)), fabsf(o2), fabsf(o3));
+                        // sign bits (the exact sign of every decided voxel; pass B sets the others)
+                        unsigned n = __float_as_uint(o3) >> 31;
+                        n = __funnelshift_l(__float_as_uint(o2), n, 1);
+                        n = __funnelshift_l(__float_as_uint(o1), n, 1);
+                        n = __funnelshift_l(__float_as_uint(o0), n, 1);
+                        pw[r] = (n ^ 15u) << (4 * (li & 7));
+                    }
+                }
+                const unsigned word = or_rows(pw, lane);
+                unsigned dec = word;
+                if (__any_sync(FULL, dmin <= band)) {   // list the undecided voxels (their values are in `out`)
+                    dec &= ~list_undecided(op, nx, min(OA_R, ny - y), (unsigned)((size_t)z * nxy + (size_t)y * nx + x), dmin <= band,
+                                           band, iso, L.cnt, L.unc, L.cap, lane);
+                }
+                const int row = word_row(lane);
+                if (!(lane & 4) && x0 + (li & 8) * 4 < nx)
+                    L.vsign[od_vsign_word((unsigned)(x0 + (li & 8) * 4), (unsigned)(y + row), (unsigned)z, L.wv, L.nys)] = word;
+                if (dec) {
+                    orx |= dec;
                     bzl = min(bzl, z);
                     bzh = z;
                 }
             }
-            if (z >= zs && z < ze) {   // warp-uniform: the tile's 8 row words, lanes 0-7, one sector
-                unsigned mine = 0;
-#pragma unroll
-                for (int kk = 0; kk < OW_Y; kk++) {
-                    const unsigned b = __ballot_sync(FULL, (sgn >> kk) & 1u);
-                    mine = lane == kk ? b : mine;
-                }
-                if (lane < OW_Y) L.vsign[od_vsign_word((unsigned)x0, (unsigned)(y0 + lane), (unsigned)z, L.wv, L.nys)] = mine;
-            }
         }
         if (timed_out) break;
         // huge, infinite or NaN input (an unbounded B), or a non-finite output
-        const bool bad = !(B < 0x1p+120f * 0x1p-19f) || nanacc != 0.f;
+        float na, nb;
+        unpack2(nanacc, na, nb);
+        const bool bad = !(B < 0x1p+120f * 0x1p-19f) || na != 0.f || nb != 0.f;
         if (__any_sync(FULL, bad)) {   // the exact three-pass path handles the volume
             if (lane == 0) od_flag(st, OD_FALLBACK);
             continue;
         }
-        // bbox of the decided voxels >= iso
-        {
-            const bool any = ymask != 0u;
-            int byl = any ? y0 + __ffs(ymask) - 1 : INT_MAX, byh = any ? y0 + 31 - __clz(ymask) : INT_MIN;
-            int xl = any ? x : INT_MAX, xh = any ? x : INT_MIN;
-            for (int o = 16; o; o >>= 1) {
-                xl = min(xl, __shfl_xor_sync(FULL, xl, o)); xh = max(xh, __shfl_xor_sync(FULL, xh, o));
-                byl = min(byl, __shfl_xor_sync(FULL, byl, o)); byh = max(byh, __shfl_xor_sync(FULL, byh, o));
-                bzl = min(bzl, __shfl_xor_sync(FULL, bzl, o)); bzh = max(bzh, __shfl_xor_sync(FULL, bzh, o));
-            }
-            if (lane == 0 && xl != INT_MAX) {
-                atomicMin(&st->vs.lo[0], xl); atomicMax(&st->vs.hi[0], xh);
-                atomicMin(&st->vs.lo[1], byl); atomicMax(&st->vs.hi[1], byh);
-                atomicMin(&st->vs.lo[2], bzl); atomicMax(&st->vs.hi[2], bzh);
+        // bbox of the decided voxels >= iso; an atomic only where it may still change something
+        if (__any_sync(FULL, orx != 0u)) {
+            const int gx = x0 + (li & 8) * 4, row = y + word_row(lane);
+            const int xl = __reduce_min_sync(FULL, orx ? gx + __ffs(orx) - 1 : INT_MAX);
+            const int xh = __reduce_max_sync(FULL, orx ? gx + 31 - __clz(orx) : INT_MIN);
+            const int yl = __reduce_min_sync(FULL, orx ? row : INT_MAX), yh = __reduce_max_sync(FULL, orx ? row : INT_MIN);
+            const int zl = __reduce_min_sync(FULL, bzl), zh = __reduce_max_sync(FULL, bzh);
+            if (lane < 3) {
+                const int lo = lane == 0 ? xl : (lane == 1 ? yl : zl), hi = lane == 0 ? xh : (lane == 1 ? yh : zh);
+                if (lo < *(volatile int *)&st->vs.lo[lane]) atomicMin(&st->vs.lo[lane], lo);
+                if (hi > *(volatile int *)&st->vs.hi[lane]) atomicMax(&st->vs.hi[lane], hi);
             }
         }
-        // range candidates of this task
-        float wmin = lmin, wmax = lmax;
         for (int o = 16; o; o >>= 1) {
-            wmin = fminf(wmin, __shfl_xor_sync(FULL, wmin, o));
-            wmax = fmaxf(wmax, __shfl_xor_sync(FULL, wmax, o));
+            lmin = fminf(lmin, __shfl_xor_sync(FULL, lmin, o));
+            lmax = fmaxf(lmax, __shfl_xor_sync(FULL, lmax, o));
         }
         if (lane == 0) {
-            atomicMin(&st->umin, f2ord(__fadd_ru(wmin, B)));
-            atomicMax(&st->lmax, f2ord(__fsub_rd(wmax, B)));
-        }
-        const float cmin = __fadd_ru(wmin, 2.5f * B), cmax = __fsub_rd(wmax, 2.5f * B);
-        // a lane with one candidate lists it directly; with more (its second extreme is
-        // close too: plateaus) it re-reads its outputs
-        if (ownx && lmin <= cmin && lmin2 > cmin) {
-            const unsigned q = atomicAdd(&L.cnt[1], 1u);
-            if (q < L.cap) L.cmin[q] = OdCand{jmin, lmin, B};
-        }
-        if (ownx && lmax >= cmax && lmax2 < cmax) {
-            const unsigned q = atomicAdd(&L.cnt[2], 1u);
-            if (q < L.cap) L.cmax[q] = OdCand{jmax, lmax, B};
-        }
-        if (ownx && (lmin2 <= cmin || lmax2 >= cmax)) {
-            const bool wmn = lmin2 <= cmin, wmx = lmax2 >= cmax;
-            for (int z = zs; z < ze; z++) {
-                float v[OW_Y];
-#pragma unroll
-                for (int kk = 0; kk < OW_Y; kk++)
-                    v[kk] = y0 + kk < ny ? out[(size_t)z * nxy + (size_t)(y0 + kk) * nx + x] : 0.f;
-#pragma unroll
-                for (int kk = 0; kk < OW_Y; kk++) {
-                    if (y0 + kk >= ny) continue;
-                    const unsigned j = (unsigned)((size_t)z * nxy + (size_t)(y0 + kk) * nx + x);
-                    if (wmn && v[kk] <= cmin) {
-                        const unsigned q = atomicAdd(&L.cnt[1], 1u);
-                        if (q < L.cap) L.cmin[q] = OdCand{j, v[kk], B};
-                    }
-                    if (wmx && v[kk] >= cmax) {
-                        const unsigned q = atomicAdd(&L.cnt[2], 1u);
-                        if (q < L.cap) L.cmax[q] = OdCand{j, v[kk], B};
-                    }
-                }
-            }
+            L.range[task] = make_float4(lmin, lmax, B, 0.f);
+            const int um = f2ord(__fadd_ru(lmin, B)), lm = f2ord(__fsub_rd(lmax, B));
+            if (um < *(volatile int *)&st->umin) atomicMin(&st->umin, um);
+            if (lm > *(volatile int *)&st->lmax) atomicMax(&st->lmax, lm);
         }
     }
     if (timed_out) {
@@ -758,54 +850,99 @@ __global__ void __launch_bounds__(OA_WARPS * 32) k_od_approx(const __grid_consta
     }
 }
 
-// the reference's smoothed value of voxel (x, y, z), every tap in its double sequence
-__device__ float od_exact_at(const float *__restrict__ in, int x, int y, int z, int nx, int ny, int nz) {
+// The voxels that can still be the volume's extreme: those of a task whose minimum
+// (maximum) can, with a value within B of the bound.  A block looks at OS_T tasks and
+// reads the few that qualify again with all its warps, a slice's 16 loads of a warp in
+// flight at once (a warp per task and one row after another took 246 us for the
+// 512^3 CT volume's handful).  Lists that overflow (plateaus) make the caller fall back.
+constexpr int OS_T = 64;
+__global__ void __launch_bounds__(256) k_od_scan(const float *__restrict__ out, int nx, int ny, int nz, int zrun,
+                                                 OdStats *st, OdLists L) {
+    __shared__ unsigned todo[OS_T], ntodo;
+    if (st->flags) return;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const unsigned nxs = (unsigned)(nx + OA_X - 1) / OA_X, nys = (unsigned)(ny + OA_Y - 1) / OA_Y;
+    const unsigned ntask = nxs * nys * ((unsigned)(nz + zrun - 1) / (unsigned)zrun);
+    const float umin = ord2f(st->umin), lmax = ord2f(st->lmax);
     const size_t nxy = (size_t)nx * ny;
-    auto X = [&](int yy, int zz) -> float {
-        const float *p = in + (size_t)zz * nxy + (size_t)yy * nx + x;
-        return (x < 2 || x > nx - 3) ? p[0] : tap5_double(p[-2], p[-1], p[0], p[1], p[2]);
-    };
-    auto Y = [&](int zz) -> float {
-        return (y < 2 || y > ny - 3) ? X(y, zz) : tap5_double(X(y - 2, zz), X(y - 1, zz), X(y, zz), X(y + 1, zz), X(y + 2, zz));
-    };
-    return (z < 2 || z > nz - 3) ? Y(z) : tap5_double(Y(z - 2), Y(z - 1), Y(z), Y(z + 1), Y(z + 2));
+    if (threadIdx.x == 0) ntodo = 0u;
+    __syncthreads();
+    if (threadIdx.x < OS_T) {
+        const unsigned task = blockIdx.x * OS_T + threadIdx.x;
+        const float4 t = task < ntask ? L.range[task] : make_float4(0.f, 0.f, 0.f, 0.f);
+        if (task < ntask && (__fsub_rd(t.x, t.z) <= umin || __fadd_ru(t.y, t.z) >= lmax)) todo[atomicAdd(&ntodo, 1u)] = task;
+    }
+    __syncthreads();
+    for (unsigned i = 0; i < ntodo; i++) {
+        if (*(volatile unsigned *)&L.cnt[1] > L.cap || *(volatile unsigned *)&L.cnt[2] > L.cap) return;   // falls back anyway
+        const unsigned task = todo[i], xs = task % nxs, t2 = task / nxs;
+        const float4 t = L.range[task];
+        const bool mn = __fsub_rd(t.x, t.z) <= umin, mx = __fadd_ru(t.y, t.z) >= lmax;
+        const int x0 = (int)xs * OA_X, y0 = (int)(t2 % nys) * OA_Y, zs = (int)(t2 / nys) * zrun, ze = min(zs + zrun, nz);
+        for (int z = zs + wid; z < ze; z += 8) {
+            float v[2 * OA_Y];
+#pragma unroll
+            for (int k = 0; k < 2 * OA_Y; k++) {
+                const int x = x0 + 32 * (k & 1) + lane, y = y0 + (k >> 1);
+                v[k] = x < nx && y < ny ? out[(size_t)z * nxy + (size_t)y * nx + x] : NAN;
+            }
+#pragma unroll
+            for (int k = 0; k < 2 * OA_Y; k++) {   // a NaN is in neither list
+                const unsigned j = (unsigned)((size_t)z * nxy + (size_t)(y0 + (k >> 1)) * nx + x0 + 32 * (k & 1) + lane);
+                if (mn && __fsub_rd(v[k], t.z) <= umin) {
+                    const unsigned q = atomicAdd(&L.cnt[1], 1u);
+                    if (q < L.cap) L.cmin[q] = j;
+                }
+                if (mx && __fadd_ru(v[k], t.z) >= lmax) {
+                    const unsigned q = atomicAdd(&L.cnt[2], 1u);
+                    if (q < L.cap) L.cmax[q] = j;
+                }
+            }
+        }
+    }
 }
 
 // Pass B: undecided voxels get their exact value (and join the bbox if >= iso);
-// the range is the exact extreme over the candidates that can still reach it
-// (value - B <= the smallest min + B of any task; the same for the maximum)
-__global__ void k_od_resolve(const float *__restrict__ in, float *out, int nx, int ny, int nz, float iso, OdStats *st,
-                             OdLists L, unsigned nu, unsigned nmin, unsigned nmax, bool at_or_above) {
-    const unsigned n = nu + nmin + nmax;
-    const float umin = ord2f(st->umin), lmax = ord2f(st->lmax);
-    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        unsigned j;
-        int which;
-        if (i < nu) {
-            which = 0;
-            j = L.unc[i];
-        } else if (i < nu + nmin) {
-            const OdCand c = L.cmin[i - nu];
-            if (__fsub_rd(c.v, c.b) > umin) continue;
-            which = 1;
-            j = c.j;
-        } else {
-            const OdCand c = L.cmax[i - nu - nmin];
-            if (__fadd_ru(c.v, c.b) < lmax) continue;
-            which = 2;
-            j = c.j;
+// the range is the exact extreme over the candidates of k_od_scan.  A warp per
+// voxel: 25 lanes take one row's x tap each, five the y taps, then the z tap, all in
+// the reference's double sequence (a thread per voxel walked the 31 taps one after
+// another: 29 us for the 512^3 CT volume's few thousand voxels).
+__global__ void __launch_bounds__(256) k_od_resolve(const float *__restrict__ in, float *out, int nx, int ny, int nz,
+                                                    float iso, OdStats *st, OdLists L, bool at_or_above) {
+    const unsigned FULL = 0xffffffffu;
+    const unsigned nu = st->cnt[0], nmin = st->cnt[1], nmax = st->cnt[2], n = nu + nmin + nmax;
+    if (st->flags || nu > L.cap || nmin > L.cap || nmax > L.cap) return;   // the caller falls back
+    const int lane = threadIdx.x & 31;
+    for (unsigned i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += (gridDim.x * blockDim.x) >> 5) {
+        const int which = i < nu ? 0 : (i < nu + nmin ? 1 : 2);
+        const unsigned j = which == 0 ? L.unc[i] : (which == 1 ? L.cmin[i - nu] : L.cmax[i - nu - nmin]);
+        const unsigned q = j / (unsigned)nx;
+        const int x = (int)(j - q * (unsigned)nx), z = (int)(q / (unsigned)ny), y = (int)(q - (unsigned)z * (unsigned)ny);
+        const bool xi = x >= 2 && x <= nx - 3, yi = y >= 2 && y <= ny - 3, zi = z >= 2 && z <= nz - 3;
+        // lane 5 * dz + dy: the x value of row (y - 2 + dy, z - 2 + dz); rows past the volume are not used
+        const int yy = y - 2 + lane % 5, zz = z - 2 + lane / 5;
+        float X = 0.f;
+        if (lane < 25 && yy >= 0 && yy < ny && zz >= 0 && zz < nz) {
+            const float *p = in + ((size_t)zz * ny + yy) * nx + x;
+            X = xi ? tap5_double(p[-2], p[-1], p[0], p[1], p[2]) : p[0];
         }
-        const unsigned x = j % (unsigned)nx, r = j / (unsigned)nx, y = r % (unsigned)ny, z = r / (unsigned)ny;
-        const float v = od_exact_at(in, (int)x, (int)y, (int)z, nx, ny, nz);
+        const int r = min(lane, 4) * 5;
+        const float a = __shfl_sync(FULL, X, r), b = __shfl_sync(FULL, X, r + 1), c = __shfl_sync(FULL, X, r + 2),
+                    d = __shfl_sync(FULL, X, r + 3), e = __shfl_sync(FULL, X, r + 4);
+        const float Y = lane < 5 && yi ? tap5_double(a, b, c, d, e) : c;
+        const float f = __shfl_sync(FULL, Y, 0), g = __shfl_sync(FULL, Y, 1), h = __shfl_sync(FULL, Y, 2),
+                    k = __shfl_sync(FULL, Y, 3), l = __shfl_sync(FULL, Y, 4);
+        if (lane != 0) continue;
+        const float v = zi ? tap5_double(f, g, h, k, l) : h;
         if (which == 0) {
             out[j] = v;
-            unsigned *sw = L.vsign + od_vsign_word(x, y, z, L.wv, L.nys);
+            unsigned *sw = L.vsign + od_vsign_word((unsigned)x, (unsigned)y, (unsigned)z, L.wv, L.nys);
             if (at_or_above ? v >= iso : __fsub_rn(v, iso) > -N2M_FLT_EPS) atomicOr(sw, 1u << (x & 31));
             else atomicAnd(sw, ~(1u << (x & 31)));
             if (v >= iso) {
-                atomicMin(&st->vs.lo[0], (int)x); atomicMax(&st->vs.hi[0], (int)x);
-                atomicMin(&st->vs.lo[1], (int)y); atomicMax(&st->vs.hi[1], (int)y);
-                atomicMin(&st->vs.lo[2], (int)z); atomicMax(&st->vs.hi[2], (int)z);
+                atomicMin(&st->vs.lo[0], x); atomicMax(&st->vs.hi[0], x);
+                atomicMin(&st->vs.lo[1], y); atomicMax(&st->vs.hi[1], y);
+                atomicMin(&st->vs.lo[2], z); atomicMax(&st->vs.hi[2], z);
             }
         } else if (which == 1) {
             atomicMin(&st->vs.vmin, f2ord(v));
@@ -1007,8 +1144,28 @@ bool od_eligible(const float *in, int nx, int ny, int nz) {
            ny >= 5 && nz >= 5;
 }
 
-n2m_status od_approx(const float *in, float *out, int nx, int ny, int nz, float iso, OdWork &w, cudaStream_t s,
-                     const StagedInput *stage) {
+namespace {
+// slices per task: long runs read few slices twice (zrun + 4 for zrun); a volume too
+// small to give every warp of the GPU a task takes shorter ones instead (64^3: 45 us
+// with 32 slices per task for want of warps)
+int od_zrun(int nx, int ny, int nz) {
+    const long long cols = (long long)((nx + OA_X - 1) / OA_X) * ((ny + OA_Y - 1) / OA_Y);
+    int zrun = 32;
+    while (zrun > 4 && cols * ((nz + zrun - 1) / zrun) < 152 * 8) zrun /= 2;
+    return zrun;
+}
+// warp tasks of pass A
+size_t od_tasks(int nx, int ny, int nz, int zrun) {
+    return (size_t)((nx + OA_X - 1) / OA_X) * ((ny + OA_Y - 1) / OA_Y) * ((nz + zrun - 1) / zrun);
+}
+OdLists od_lists(const OdWork &w, int nx, int ny) {
+    return OdLists{w.unc.as<unsigned>(), w.cmin.as<unsigned>(), w.cmax.as<unsigned>(),
+                   (unsigned *)((char *)w.st.p + offsetof(OdStats, cnt)), w.cap, w.vsign.as<unsigned>(), w.range.as<float4>(),
+                   (unsigned)(nx + 31) / 32, (unsigned)(ny + 7) / 8};
+}
+}  // namespace
+
+n2m_status od_approx(const float *in, float *out, int nx, int ny, int nz, float iso, OdWork &w, cudaStream_t s) {
     const size_t n = (size_t)nx * ny * nz;
     auto encode = tensor_map_encoder();
     if (!encode) {
@@ -1029,77 +1186,43 @@ n2m_status od_approx(const float *in, float *out, int nx, int ny, int nz, float 
         }
     }
     w.cap = (unsigned)std::min<size_t>(n / 64 + 4096, 1u << 22);
+    const int zrun = od_zrun(nx, ny, nz);
+    const size_t nys = (size_t)(ny + 7) / 8, wv = (size_t)(nx + 31) / 32, ntask = od_tasks(nx, ny, nz, zrun);
     CKS(w.st.ensure(sizeof(OdStats)));
     CKS(w.unc.ensure((size_t)w.cap * sizeof(unsigned)));
-    CKS(w.cmin.ensure((size_t)w.cap * sizeof(OdCand)));
-    CKS(w.cmax.ensure((size_t)w.cap * sizeof(OdCand)));
+    CKS(w.cmin.ensure((size_t)w.cap * sizeof(unsigned)));
+    CKS(w.cmax.ensure((size_t)w.cap * sizeof(unsigned)));
+    CKS(w.range.ensure(ntask * sizeof(float4)));
+    CKS(w.vsign.ensure((size_t)nz * nys * wv * 8 * sizeof(unsigned)));
     OdStats h{};
-    stats_init_host(&h.vs);
-    h.vs.vmin = INT_MAX;   // filled by pass B from the candidates
-    h.vs.vmax = INT_MIN;
+    stats_init_host(&h.vs);   // vmin / vmax are filled by pass B from the candidates
     h.umin = INT_MAX;
     h.lmax = INT_MIN;
     CK(cudaMemcpyAsync(w.st.p, &h, sizeof(OdStats), cudaMemcpyHostToDevice, s));
-    const unsigned wv = (unsigned)(nx + 31) / 32, nys = (unsigned)(ny + 7) / 8;
-    CKS(w.vsign.ensure((size_t)nz * nys * wv * 8 * sizeof(unsigned)));
-    OdStats *st = w.st.as<OdStats>();
-    OdLists L{w.unc.as<unsigned>(), w.cmin.as<OdCand>(), w.cmax.as<OdCand>(),
-              (unsigned *)((char *)w.st.p + offsetof(OdStats, cnt)), w.cap, w.vsign.as<unsigned>(), wv, nys};
-    const int grid = od_grid((const void *)k_od_approx, OA_WARPS * 32);
-    auto launch = [&](int z_lo, int z_hi) -> n2m_status {
-        if (z_hi <= z_lo) return N2M_OK;
-        k_od_approx<<<grid, OA_WARPS * 32, 0, s>>>(tmap, out, nx, ny, nz, z_lo, z_hi, iso, st, L);
-        N2M_COUNT();
-        CKL();
-        return N2M_OK;
-    };
-    if (stage && stage->host) {
-        // the copy stream may only overwrite `in` once earlier work on s is done with it
-        CK(cudaEventRecord(stage->ev[N2M_STAGE_SLABS], s));
-        CK(cudaStreamWaitEvent(stage->copy, stage->ev[N2M_STAGE_SLABS], 0));
-        const size_t nxy = (size_t)nx * ny;
-        int zdone = 0;
-        for (int k = 0; k < N2M_STAGE_SLABS; k++) {
-            const int z0 = (int)((long long)nz * k / N2M_STAGE_SLABS), z1 = (int)((long long)nz * (k + 1) / N2M_STAGE_SLABS);
-            if (z1 <= z0) continue;
-            CK(cudaMemcpyAsync((float *)in + (size_t)z0 * nxy, stage->host + (size_t)z0 * nxy,
-                               (size_t)(z1 - z0) * nxy * sizeof(float), cudaMemcpyHostToDevice, stage->copy));
-            CK(cudaEventRecord(stage->ev[k], stage->copy));
-            CK(cudaStreamWaitEvent(s, stage->ev[k], 0));
-            const int zready = z1 == nz ? nz : z1 - 2;   // outputs whose input slices (+-2) have arrived
-            if (zready - zdone >= 32 || zready == nz) {
-                CKS(launch(zdone, zready));
-                zdone = zready;
-            }
-        }
-    } else {
-        CKS(launch(0, nz));
-    }
+    const unsigned grid = (unsigned)std::min<size_t>((ntask + OA_WARPS - 1) / OA_WARPS, (size_t)od_grid((const void *)k_od_approx, OA_WARPS * 32));
+    { k_od_approx<<<grid, OA_WARPS * 32, 0, s>>>(tmap, out, nx, ny, nz, zrun, iso, w.st.as<OdStats>(), od_lists(w, nx, ny)); N2M_COUNT(); }
+    CKL();
     return N2M_OK;
 }
 
-n2m_status od_resolve(const float *in, float *out, int nx, int ny, int nz, float iso, OdWork &w, VolStats *dst,
-                      cudaStream_t s, bool *fallback, bool at_or_above) {
-    OdStats h;
-    CK(cudaMemcpyAsync(&h, w.st.p, sizeof(OdStats), cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
+n2m_status od_resolve(const float *in, float *out, int nx, int ny, int nz, float iso, OdWork &w, cudaStream_t s,
+                      bool at_or_above) {
+    const OdLists L = od_lists(w, nx, ny);
+    const int zrun = od_zrun(nx, ny, nz);
+    const size_t ntask = od_tasks(nx, ny, nz, zrun);
+    { k_od_scan<<<(unsigned)((ntask + OS_T - 1) / OS_T), 256, 0, s>>>(out, nx, ny, nz, zrun, w.st.as<OdStats>(), L); N2M_COUNT(); }
+    { k_od_resolve<<<152 * 8, 256, 0, s>>>(in, out, nx, ny, nz, iso, w.st.as<OdStats>(), L, at_or_above); N2M_COUNT(); }
+    CKL();
+    return N2M_OK;
+}
+
+n2m_status od_check(const OdWork &w, const OdStats &h, bool *fallback) {
     if (h.flags & OD_TIMEOUT) {
         n2m_set_error("pre-smooth: a tile copy did not complete");
         return N2M_ERR_TIMEOUT;
     }
     *fallback = (h.flags & OD_FALLBACK) != 0 || h.cnt[0] > w.cap || h.cnt[1] > w.cap || h.cnt[2] > w.cap ||
                 h.cnt[1] == 0 || h.cnt[2] == 0;
-    if (*fallback) return N2M_OK;
-    OdLists L{w.unc.as<unsigned>(), w.cmin.as<OdCand>(), w.cmax.as<OdCand>(),
-              (unsigned *)((char *)w.st.p + offsetof(OdStats, cnt)), w.cap, w.vsign.as<unsigned>(),
-              (unsigned)(nx + 31) / 32, (unsigned)(ny + 7) / 8};
-    const unsigned tot = h.cnt[0] + h.cnt[1] + h.cnt[2];
-    const unsigned blocks = std::max(1u, std::min((tot + 127) / 128, 152u * 8u));
-    k_od_resolve<<<blocks, 128, 0, s>>>(in, out, nx, ny, nz, iso, w.st.as<OdStats>(), L, h.cnt[0], h.cnt[1], h.cnt[2],
-                                        at_or_above);
-    N2M_COUNT();
-    CKL();
-    CK(cudaMemcpyAsync(dst, w.st.p, sizeof(VolStats), cudaMemcpyDeviceToDevice, s));   // vs is the first member
     return N2M_OK;
 }
 
