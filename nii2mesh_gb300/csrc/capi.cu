@@ -282,12 +282,11 @@ extern "C" void n2m_context_destroy(n2m_context *c) {
                       &c->aw.pts, &c->aw.pts2, &c->aw.tris, &c->aw.tris2, &c->aw.cand, &c->aw.gath, &c->aw.weld,
                       &c->aw.ranges, &c->alab, &c->lpts, &c->ltris, &c->gA, &c->gB, &c->gs, &c->gtmp, &c->in, &c->raw, &c->vol, &c->stmp, &c->stats, &c->totals, &c->cand, &c->ncand, &c->ocq, &c->pts_raw,
                       &c->tris_raw, &c->pts, &c->tris, &c->ntf, &c->weld, &c->gath, &c->hmesh,
-                      &c->mc.signs, &c->mc.words, &c->mc.act, &c->mc.staged, &c->mc.sub, &c->scan.part,
+                      &c->mc.signs, &c->mc.words, &c->mc.act, &c->mc.cnt, &c->mc.staged, &c->mc.sub, &c->scan.part,
                       &c->lab.lab, &c->lab.mask, &c->lab.keep, &c->lab.cnt, &c->lab.edge, &c->lab.rc, &c->lab.misc,
                       &c->deg.flags, &c->deg.tmp, &c->hc.zero, &c->hc.adj, &c->hc.meta, &c->hc.P, &c->hc.Q,
                       &c->hc.B, &c->hc.Lo, &c->th.buf, &c->th.table,
-                      &c->stmp2, &c->lubits, &c->od.st, &c->od.unc, &c->od.cmin, &c->od.cmax, &c->od.range, &c->od.need_z, &c->od.need_y,
-                      &c->od.need_x, &c->od.off, &c->od.list, &c->od.lcnt, &c->od.vsign,
+                      &c->stmp2, &c->lubits, &c->od.st, &c->od.unc, &c->od.cmin, &c->od.cmax, &c->od.range, &c->od.need, &c->od.list, &c->od.lcnt, &c->od.vsign,
                       &c->wr.mt, &c->wr.mp, &c->wr.pack, &c->wr.pack2, &c->wr.lens, &c->wr.flag, &c->wr.out};
     for (DevBuf *b : bufs) b->release();
     deflate_release(c->wr.df);
@@ -726,7 +725,7 @@ n2m_status march(n2m_context *c, const Prep &P, const int dim[3], int cubes, int
         const size_t n = (size_t)dim[0] * dim[1] * dim[2];
         CKS(c->stmp2.ensure(n * sizeof(float)));
         const OdRepair rep{P.src, c->stmp.as<float>(), c->stmp2.as<float>(), (float *)P.vol, {dim[0], dim[1], dim[2]},
-                           &c->od, &c->scan, P.post};
+                           &c->od, P.post};
         if (old) CKS(oc_count(P.vol, dim, P.lo, P.hi, P.iso, P.edge_max, c->mc, dtot, c->stream, &rep));
         else CKS(mc_count(g, cubes, c->mc, dtot, c->stream, &rep));
     } else if (old) CKS(oc_count(P.vol, dim, P.lo, P.hi, P.iso, P.edge_max, c->mc, dtot, c->stream));

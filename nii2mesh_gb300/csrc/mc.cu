@@ -176,34 +176,6 @@ __global__ void __launch_bounds__(256) k_signs_bits(GV g, unsigned nwords, unsig
     }
 }
 
-// Marks for the exact pre-smooth on demand: the voxel behind every corner of
-// every cube whose corner signs differ (the only cubes whose values marching
-// cubes reads), as bits of a linear bitmap over the volume.  A grid point's
-// voxel is gval's linear index j (row wrap included); j past the volume is the
-// padding value, which needs no voxel.
-__global__ void __launch_bounds__(256) k_need(GV g, unsigned nwords, const unsigned *__restrict__ signs, unsigned *need) {
-    const unsigned rowstride = g.WX, slicestride = g.WX * (unsigned)g.NY;
-    for (unsigned w = blockIdx.x * blockDim.x + threadIdx.x; w < nwords; w += gridDim.x * blockDim.x) {
-        const unsigned xw = w % g.WX, row = w / g.WX;
-        mcw::Geo q{0, (int)(row % (unsigned)g.NY), (int)(row / (unsigned)g.NY), rowstride, slicestride, 0u, 0u, false, false, false, 0};
-        q.hy = q.y < g.NY - 1;
-        q.hz = q.z < g.NZ - 1;
-        if (!q.hy || !q.hz) continue;   // no cubes start on the last row / slice
-        q.nx = xw + 1 < g.WX;
-        q.hxm = mcw::bit_range(g.xoff - 32 * (int)xw, g.xoff + g.NX - 1 - 32 * (int)xw);
-        const unsigned mix = mcw::mixed_cubes(mcw::load_corners(signs, w, q), q);
-        if (!mix) continue;
-        const unsigned cm = mix | (mix << 1), carry = mix >> 31;   // corners x and x + 1 of each mixed cube
-#pragma unroll
-        for (int r = 0; r < 4; r++) {
-            const long long j = (long long)(g.lo0 - g.xoff + 32 * (int)xw) + (long long)(q.y + (r & 1) + g.lo1) * g.dx +
-                                (long long)(q.z + (r >> 1) + g.lo2) * g.dxy;
-            od_need_mark(need, j, cm, g.nvox);
-            if (carry) od_need_mark(need, j + 32, 1u, g.nvox);
-        }
-    }
-}
-
 // ---- emit pass -------------------------------------------------------------------
 // grid value at p (strictly inside the volume: no darkening, wrap or padding)
 __device__ __forceinline__ float ival(const GV &g, const float *p) {
@@ -313,6 +285,11 @@ struct Policy {
         q.nx = xw + 1 < g.WX;
         q.tag = 0;
         return true;
+    }
+    __device__ __forceinline__ void voxel_word(const mcw::Geo &q, int &wx, int &vy, int &vz) const {
+        wx = (g.lo0 + q.x0) >> 5;
+        vy = g.lo1 + q.y;
+        vz = g.lo2 + q.z;
     }
     __device__ __forceinline__ void shifts(const mcw::Out &, unsigned, const uint4 &total, unsigned &e, unsigned &c) const {
         e = 0;
@@ -519,16 +496,13 @@ n2m_status mc_count(const McGrid &g, int variant, McWork &w, uint4 *d_total, cud
         k_signs<<<std::min<unsigned>((nrows + 7) / 8, 152u * 16u), 256, 0, s>>>(v, nrows, signs);
         N2M_COUNT();
     }
-    if (repair) {   // exact smoothed values where the cubes below read them
-        const size_t nvw = (size_t)((v.nvox + 31) >> 5);
-        CKS(repair->w->need_z.ensure(nvw * sizeof(unsigned)));
-        CK(cudaMemsetAsync(repair->w->need_z.p, 0, nvw * sizeof(unsigned), s));
-        { k_need<<<blocks, 256, 0, s>>>(v, (unsigned)nwords, signs, repair->w->need_z.as<unsigned>()); N2M_COUNT(); }
-        CKL();
-        CKS(od_repair(*repair, s));
-    }
-    const Policy pol{v, variant == N2M_CUBES_CLASSIC_TABLE, nullptr, nullptr, nullptr, nullptr, nullptr, 0};
-    return mcw::count(pol, signs, w, o, s);
+    const bool classic = variant == N2M_CUBES_CLASSIC_TABLE;
+    const Policy pol{v, classic, nullptr, nullptr, nullptr, nullptr, nullptr, 0};
+    mcw::Marks marks{nullptr, v.dx, v.dy, v.dz, (unsigned)(v.dx + 31) / 32u};
+    if (repair) CKS(od_marks(*repair->w, g.dim, &marks.need, s));
+    CKS(mcw::count_signs(pol, signs, o, marks, s));
+    if (repair) CKS(od_repair(*repair, s));   // exact smoothed values where anything below reads them
+    return mcw::count_values(pol, signs, w, o, !classic, s);
 }
 
 n2m_status mc_emit(const McGrid &g, int variant, McWork &w, const McCounts &c, vec3d *d_pts, vec3i *d_tris,

@@ -5,14 +5,19 @@
 // over words.  A variant supplies a policy (its grid geometry, tilings and vertex
 // arithmetic); this file counts, numbers and emits:
 //
-//   k_words   edge-crossing masks and output counts of every word.  A warp turns
-//             the mixed cubes of its 32 words into one dense list (a cube per
-//             lane), so that neither an empty word nor a full one costs its
-//             neighbours time.  Sub-tiles of 256 words are scanned in the block;
-//             the last block to finish scans the tiles.
+//   k_words   edge-crossing masks of every word and the counts that follow from
+//             signs alone; marks the voxels whose exact values will be read; lists
+//             the words holding ambiguous cubes.  A warp turns the mixed cubes of its
+//             32 words into one dense list (a cube per lane), so that neither an empty
+//             word nor a full one costs its neighbours time.  Sub-tiles of 256 words
+//             are scanned in the block; the last block to finish scans the tiles.
+//   k_amb     the face and interior tests of the listed words' ambiguous cubes, which
+//             need values (so with the exact smoothing on demand they come after the
+//             repair), again a cube per lane: their loads no longer hold up k_words.
+//   k_sum     triangle and c-vertex sums, over active words only.
 //   k_finish  the active words (those that own output) as one list in word order
 //             with their absolute triangle and c-vertex offsets; the words'
-//             vertex offsets become absolute.  Only active words are touched.
+//             vertex offsets become absolute.
 //   k_emit    a warp takes G active words, numbers their vertices and cubes
 //             densely and emits them with all lanes busy; triangles pass through
 //             a small queue because cubes make different numbers of them.
@@ -23,7 +28,7 @@
 //
 // Measured on the 512^3 CT volume (7.1 M triangles, cold caches): emit 474 -> 218 us
 // against one lane per word listing its cubes for the warp and separate mask and
-// offset arrays; masks, scan and active list 240 -> 162 us.  On the brain volume
+// offset arrays; masks, marks, counts, scan and active list 290 -> 178 us.  On the brain volume
 // (0.2 M triangles, 1.7 k groups of 32 words for 5 k resident warps) the emit went
 // from 157 to 23 us.
 #pragma once
@@ -129,27 +134,99 @@ constexpr unsigned TESTS = 0xffu;   // quick(): the tiling depends on corner val
 
 // what the count pass leaves behind (see McWork)
 struct Out {
-    uint4 *words;      // per active word
-    uint2 *staged;     // per sub-tile, its active words in order: {word in the sub-tile | triangle offset << 8, c-vertex offset}
-    uint4 *sub;        // per sub-tile, what precedes it in its tile {vertices, triangles, c-vertices, active | own active << 20}
-    uint4 *part;       // per tile, what precedes it
-    uint4 *total;
-    unsigned *done;    // tiles finished (left at zero)
+    uint4 *words;           // per active word
+    unsigned *cnt;          // per active word, triangles | c-vertices << 16
+    unsigned *amb;          // per active word, its ambiguous cubes
+    unsigned *amblist;      // words with any
+    unsigned char *staged;  // per sub-tile, its active words in order (number within the sub-tile)
+    uint2 *sub;             // per sub-tile, what precedes it in its tile {vertices, active words | own active words << 20}
+    uint2 *subt;            // the same {triangles, c-vertices}
+    uint2 *part, *partt;    // per tile, what precedes it, likewise
+    uint4 *total;           // {vertices, triangles, c-vertices, active words}
+    unsigned *ctr;          // tiles finished (two passes), words in amblist, group counter of the emit
     unsigned nwords, nsub, per;   // per: sub-tiles per tile (tile = block)
 };
 
-__device__ __forceinline__ uint4 add4(uint4 a, uint4 b) { return make_uint4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
+// marks voxels of a volume in a bitmap of row-aligned words (bit x & 31 of word (z*ny + y)*W + x/32): word wx of row
+// (y, z), of which y may be one row and z one slice past the volume, and bit nx of a row its padding column (they wrap
+// into the next row or slice as the padded grid reads them, src/MarchingCubes.c:1097-1115)
+struct Marks {
+    unsigned *need;         // null: none wanted
+    int nx, ny, nz;
+    unsigned W;
+    __device__ __forceinline__ void put(int wx, int y, int z, unsigned bits) const {
+        if (!bits) return;
+        if (y >= ny) {
+            y -= ny;
+            z++;
+        }
+        if (z >= nz) return;
+        const int p = nx - 32 * wx;   // bit of the padding column
+        const unsigned in = bits & bit_range(0, p);
+        if (in) atomicOr(need + ((size_t)z * ny + y) * W + wx, in);
+        if (p >= 0 && p < 32 && (bits >> p & 1u)) {
+            if (++y >= ny) {
+                y -= ny;
+                z++;
+            }
+            if (z < nz) atomicOr(need + ((size_t)z * ny + y) * W, 1u);
+        }
+    }
+};
+
+// turns n per-tile sums into what precedes each, by one block; the total goes to *all
+__device__ __forceinline__ void scan_parts(uint2 *part, unsigned n, uint2 *psum, int tid, uint2 &all) {
+    const int lane = tid & 31, wid = tid >> 5;
+    const unsigned each = (n + SUB - 1) / SUB, p0 = min(n, (unsigned)tid * each), p1 = min(n, p0 + each);
+    uint2 s = make_uint2(0u, 0u);
+    for (unsigned k = p0; k < p1; k++) {
+        const uint2 v = __ldcg(part + k);
+        s.x += v.x;
+        s.y += v.y;
+    }
+    unsigned tx, ty;
+    uint2 before;
+    before.x = warp_excl(s.x, lane, tx);
+    before.y = warp_excl(s.y, lane, ty);
+    if (lane == 0) psum[wid] = make_uint2(tx, ty);
+    __syncthreads();
+    all = make_uint2(0u, 0u);
+    for (int k = 0; k < SUB / 32; k++) {
+        if (k < wid) {
+            before.x += psum[k].x;
+            before.y += psum[k].y;
+        }
+        all.x += psum[k].x;
+        all.y += psum[k].y;
+    }
+    for (unsigned k = p0; k < p1; k++) {
+        const uint2 v = __ldcg(part + k);
+        part[k] = before;
+        before.x += v.x;
+        before.y += v.y;
+    }
+}
+// whether this block is the last to hand in its tile's sums (all threads call it)
+__device__ __forceinline__ bool last_tile(uint2 *part, uint2 sums, unsigned *done, bool &flag) {
+    if (threadIdx.x == 0) {
+        part[blockIdx.x] = sums;
+        __threadfence();
+        flag = atomicAdd(done, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (flag) __threadfence();
+    return flag;
+}
 
 template <class P>
-__global__ void __launch_bounds__(SUB) k_words(P pol, const unsigned *__restrict__ signs, Out o) {
-    __shared__ unsigned qt[256], pre[8][32], cor[8][6][32], cnt[SUB];
+__global__ void __launch_bounds__(SUB) k_words(P pol, const unsigned *__restrict__ signs, Out o, Marks marks) {
+    __shared__ unsigned qt[256], pre[8][32], cor[8][6][32], cnt[SUB], amb[SUB], abase;
     __shared__ uint2 wsum[8];
-    __shared__ uint4 psum[8];
     __shared__ bool last;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     qt[tid] = pol.quick(tid);
     __syncthreads();
-    uint4 run = make_uint4(0u, 0u, 0u, 0u);
+    uint2 run = make_uint2(0u, 0u);   // vertices, active words of the tile so far
     const unsigned s1 = min(o.nsub, (blockIdx.x + 1) * o.per);
     for (unsigned sub = blockIdx.x * o.per; sub < s1; sub++) {
         const unsigned w = sub * SUB + (unsigned)tid;
@@ -161,14 +238,17 @@ __global__ void __launch_bounds__(SUB) k_words(P pol, const unsigned *__restrict
             ym = g.hy ? (q.a ^ q.b) & g.inm : 0u;
             zm = g.hz ? (q.a ^ q.c) & g.inm : 0u;
             mix = mixed_cubes(q, g);
-            cor[wid][0][lane] = q.a;
-            cor[wid][1][lane] = q.b;
-            cor[wid][2][lane] = q.c;
-            cor[wid][3][lane] = q.d;
-            cor[wid][4][lane] = q.nxt;
-            cor[wid][5][lane] = mix;
+            if (mix) {
+                cor[wid][0][lane] = q.a;
+                cor[wid][1][lane] = q.b;
+                cor[wid][2][lane] = q.c;
+                cor[wid][3][lane] = q.d;
+                cor[wid][4][lane] = q.nxt;
+                cor[wid][5][lane] = mix;
+            }
         }
         cnt[tid] = 0u;
+        amb[tid] = 0u;
         unsigned ncube;
         pre[wid][lane] = warp_excl(__popc(mix), lane, ncube);
         __syncwarp();
@@ -176,25 +256,21 @@ __global__ void __launch_bounds__(SUB) k_words(P pol, const unsigned *__restrict
             const int l = find_lane(pre[wid], k);
             const int i = nth_bit(cor[wid][5][l], (int)(k - pre[wid][l]));
             const int lut = cube_index(cor[wid][0][l], cor[wid][1][l], cor[wid][2][l], cor[wid][3][l], cor[wid][4][l], i);
-            const unsigned q = qt[lut];
-            unsigned n = q & 0xffu;
-            if (n == TESTS) {
-                Geo gl;
-                pol.geo(w - (unsigned)lane + (unsigned)l, gl);
-                const CubeTiling T = pol.tests(gl, gl.x0 + i, gl.y, gl.z, lut);
-                n = (unsigned)T.n | (T.cv ? 1u << 16 : 0u);
-            }
-            atomicAdd(&cnt[wid * 32 + l], n);
+            const unsigned n = qt[lut] & 0xffu;
+            if (n == TESTS) atomicOr(&amb[wid * 32 + l], 1u << i);
+            else atomicAdd(&cnt[wid * 32 + l], n);
         }
         __syncwarp();
-        // sums of a sub-tile: at most 24576 vertices, 256 active words; 98304 triangles, 8192 c-vertices
-        const unsigned nv = __popc(xm) + __popc(ym) + __popc(zm), nt = cnt[tid] & 0xffffu, nc = cnt[tid] >> 16;
-        const bool act = (nv | nt) != 0u;
-        const unsigned va = nv | (act ? 1u << 16 : 0u), vb = nt | nc << 18;
-        unsigned ta, tb, ea = warp_excl(va, lane, ta), eb = warp_excl(vb, lane, tb);
+        // a sub-tile has at most 24576 vertices and 256 active words (256 with ambiguous cubes)
+        const unsigned nv = __popc(xm) + __popc(ym) + __popc(zm), am = amb[tid];
+        const bool act = (nv | mix) != 0u;
+        unsigned ta, tb, ea = warp_excl(nv | (act ? 1u << 16 : 0u), lane, ta);
+        const unsigned ab = __ballot_sync(FULL, am != 0u);
+        tb = __popc(ab);
         if (lane == 0) wsum[wid] = make_uint2(ta, tb);
         __syncthreads();
         uint2 all = make_uint2(0u, 0u);
+        unsigned eb = __popc(ab & ((1u << lane) - 1u));
 #pragma unroll
         for (int k = 0; k < SUB / 32; k++) {
             const uint2 t = wsum[k];
@@ -205,74 +281,156 @@ __global__ void __launch_bounds__(SUB) k_words(P pol, const unsigned *__restrict
             all.x += t.x;
             all.y += t.y;
         }
+        if (tid == 0 && all.y) abase = atomicAdd(o.ctr + 2, all.y);
         if (act) {
             o.words[w] = make_uint4(xm, ym, zm, ea & 0xffffu);
-            o.staged[(size_t)sub * SUB + (ea >> 16)] = make_uint2((unsigned)tid | (eb & 0x3ffffu) << 8, eb >> 18);
+            o.staged[(size_t)sub * SUB + (ea >> 16)] = (unsigned char)tid;
+            o.cnt[w] = cnt[tid];
+            if (P::CVERTS) o.amb[w] = am;
+            if (marks.need) {   // both ends of every crossing edge; every corner of the ambiguous cubes
+                int wx, vy, vz;
+                pol.voxel_word(g, wx, vy, vz);
+                const unsigned am2 = am | am << 1;
+                marks.put(wx, vy, vz, xm | xm << 1 | ym | zm | am2);
+                if ((xm | am) >> 31) marks.put(wx + 1, vy, vz, 1u);
+                marks.put(wx, vy + 1, vz, ym | am2);
+                marks.put(wx, vy, vz + 1, zm | am2);
+                if (am) {
+                    marks.put(wx, vy + 1, vz + 1, am2);
+                    if (am >> 31) {
+                        marks.put(wx + 1, vy + 1, vz, 1u);
+                        marks.put(wx + 1, vy, vz + 1, 1u);
+                        marks.put(wx + 1, vy + 1, vz + 1, 1u);
+                    }
+                }
+            }
         }
-        if (tid == 0) o.sub[sub] = make_uint4(run.x, run.y, run.z, run.w | (all.x >> 16) << 20);
-        run = add4(run, make_uint4(all.x & 0xffffu, all.y & 0x3ffffu, all.y >> 18, all.x >> 16));
-        __syncthreads();   // wsum is reused
+        if (tid == 0) o.sub[sub] = make_uint2(run.x, run.y | (all.x >> 16) << 20);
+        run.x += all.x & 0xffffu;
+        run.y += all.x >> 16;
+        __syncthreads();   // abase; wsum is reused
+        if (am) o.amblist[abase + eb] = w;
     }
-    // the last tile to finish turns the tiles' sums into offsets
+    if (!last_tile(o.part, run, o.ctr, last)) return;
+    uint2 all;
+    scan_parts(o.part, gridDim.x, wsum, tid, all);
     if (tid == 0) {
-        o.part[blockIdx.x] = run;
-        __threadfence();
-        last = atomicAdd(o.done, 1u) == gridDim.x - 1;
+        o.total->x = all.x;
+        o.total->w = all.y;
     }
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    const unsigned n = gridDim.x, each = (n + SUB - 1) / SUB, p0 = min(n, (unsigned)tid * each), p1 = min(n, p0 + each);
-    uint4 s = make_uint4(0u, 0u, 0u, 0u);
-    for (unsigned k = p0; k < p1; k++) s = add4(s, __ldcg(o.part + k));
-    uint4 in = s;
-    for (int d = 1; d < 32; d <<= 1) {
-        uint4 t;
-        t.x = __shfl_up_sync(FULL, in.x, d); t.y = __shfl_up_sync(FULL, in.y, d);
-        t.z = __shfl_up_sync(FULL, in.z, d); t.w = __shfl_up_sync(FULL, in.w, d);
-        if (lane >= d) in = add4(in, t);
+}
+
+// the ambiguous cubes of the listed words, a warp per 32 words
+template <class P>
+__global__ void __launch_bounds__(128) k_amb(P pol, const unsigned *__restrict__ signs, Out o) {
+    __shared__ unsigned pre[4][32], cor[4][6][32], words[4][32];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const unsigned n = o.ctr[2];
+    for (unsigned a0 = (blockIdx.x * 4 + (unsigned)wid) * 32; a0 < n; a0 += gridDim.x * 128) {
+        unsigned am = 0;
+        if (a0 + (unsigned)lane < n) {
+            const unsigned w = o.amblist[a0 + lane];
+            Geo g;
+            pol.geo(w, g);
+            const Corners q = load_corners(signs, w, g);
+            am = o.amb[w];
+            words[wid][lane] = w;
+            cor[wid][0][lane] = q.a;
+            cor[wid][1][lane] = q.b;
+            cor[wid][2][lane] = q.c;
+            cor[wid][3][lane] = q.d;
+            cor[wid][4][lane] = q.nxt;
+            cor[wid][5][lane] = am;
+        }
+        unsigned ncube;
+        pre[wid][lane] = warp_excl(__popc(am), lane, ncube);
+        __syncwarp();
+        for (unsigned k = lane; k < ncube; k += 32) {
+            const int l = find_lane(pre[wid], k);
+            const int i = nth_bit(cor[wid][5][l], (int)(k - pre[wid][l]));
+            const int lut = cube_index(cor[wid][0][l], cor[wid][1][l], cor[wid][2][l], cor[wid][3][l], cor[wid][4][l], i);
+            Geo g;
+            pol.geo(words[wid][l], g);
+            const CubeTiling T = pol.tests(g, g.x0 + i, g.y, g.z, lut);
+            atomicAdd(o.cnt + words[wid][l], (unsigned)T.n | (T.cv ? 1u << 16 : 0u));
+        }
+        __syncwarp();
     }
-    if (lane == 31) psum[wid] = in;
-    __syncthreads();
-    uint4 before = make_uint4(in.x - s.x, in.y - s.y, in.z - s.z, in.w - s.w), tot = make_uint4(0u, 0u, 0u, 0u);
-    for (int k = 0; k < SUB / 32; k++) {
-        if (k < wid) before = add4(before, psum[k]);
-        tot = add4(tot, psum[k]);
+}
+
+// triangle and c-vertex sums of the sub-tiles, a warp each, in rounds of 8 (a template only to be emitted once per unit)
+template <class P>
+__global__ void __launch_bounds__(SUB) k_sum(Out o) {
+    __shared__ uint2 wsum[8];
+    __shared__ bool last;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    uint2 run = make_uint2(0u, 0u);
+    const unsigned s0 = blockIdx.x * o.per, s1 = min(o.nsub, s0 + o.per);
+    for (unsigned r = s0; r < s1; r += 8) {
+        const unsigned sub = r + (unsigned)wid;
+        uint2 t = make_uint2(0u, 0u);
+        if (sub < s1) {
+            const unsigned n = o.sub[sub].y >> 20;
+            for (unsigned k = (unsigned)lane; k < n; k += 32) {
+                const unsigned c = o.cnt[sub * SUB + o.staged[(size_t)sub * SUB + k]];
+                t.x += c & 0xffffu;
+                t.y += c >> 16;
+            }
+        }
+        t.x = __reduce_add_sync(FULL, t.x);
+        t.y = __reduce_add_sync(FULL, t.y);
+        if (lane == 0) wsum[wid] = t;
+        __syncthreads();
+        uint2 before = run;
+        for (int k = 0; k < 8; k++) {
+            if (k < wid) {
+                before.x += wsum[k].x;
+                before.y += wsum[k].y;
+            }
+            run.x += wsum[k].x;
+            run.y += wsum[k].y;
+        }
+        if (lane == 0 && sub < s1) o.subt[sub] = before;
+        __syncthreads();
     }
-    for (unsigned k = p0; k < p1; k++) {
-        const uint4 v = __ldcg(o.part + k);
-        o.part[k] = before;
-        before = add4(before, v);
-    }
+    if (!last_tile(o.partt, run, o.ctr + 1, last)) return;
+    uint2 all;
+    scan_parts(o.partt, gridDim.x, wsum, tid, all);
     if (tid == 0) {
-        *o.total = tot;
-        *o.done = 0u;
+        o.total->y = all.x;
+        o.total->z = all.y;
     }
 }
 
 // what precedes sub-tile s: vertices, triangles, c-vertices, active words
 __device__ __forceinline__ uint4 sub_offset(const Out &o, unsigned s) {
-    uint4 b = o.sub[s];
-    b.w &= 0xfffffu;
-    return add4(b, o.part[s / o.per]);
+    const uint2 a = o.sub[s], b = o.subt[s], pa = o.part[s / o.per], pb = o.partt[s / o.per];
+    return make_uint4(a.x + pa.x, b.x + pb.x, b.y + pb.y, (a.y & 0xfffffu) + pa.y);
 }
 
 // a warp per sub-tile
 template <class P>
 __global__ void __launch_bounds__(256) k_finish(P pol, Out o, uint4 *act) {
-    const unsigned lane = threadIdx.x & 31u;
+    const int lane = threadIdx.x & 31;
     const uint4 total = *o.total;
     for (unsigned s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; s < o.nsub; s += (gridDim.x * blockDim.x) >> 5) {
-        const unsigned n = o.sub[s].w >> 20;
+        const unsigned n = o.sub[s].y >> 20;
         if (!n) continue;
-        const uint4 b = sub_offset(o, s);
+        uint4 b = sub_offset(o, s);
         unsigned eshift, cshift;   // added to edge-vertex and c-vertex numbers
         pol.shifts(o, s, total, eshift, cshift);
-        for (unsigned k = lane; k < n; k += 32) {
-            const uint2 e = o.staged[(size_t)s * SUB + k];
-            const unsigned w = s * SUB + (e.x & 0xffu);
-            o.words[w].w += b.x + eshift;
-            act[b.w + k] = make_uint4(w, b.y + (e.x >> 8), b.z + e.y + cshift, 0u);
+        for (unsigned k0 = 0; k0 < n; k0 += 32) {
+            const unsigned k = k0 + (unsigned)lane;
+            const unsigned w = s * SUB + (k < n ? o.staged[(size_t)s * SUB + k] : 0u);
+            const unsigned c = k < n ? o.cnt[w] : 0u;
+            unsigned tt, tc;
+            const unsigned et = warp_excl(c & 0xffffu, lane, tt), ec = warp_excl(c >> 16, lane, tc);
+            if (k < n) {
+                o.words[w].w += b.x + eshift;
+                act[b.w + k] = make_uint4(w, b.y + et, b.z + ec + cshift, 0u);
+            }
+            b.y += tt;
+            b.z += tc;
         }
     }
 }
@@ -466,26 +624,43 @@ inline n2m_status prepare(McWork &w, size_t nwords, uint4 *d_total, Out &o) {
     o.nwords = (unsigned)nwords;
     o.nsub = (unsigned)nsub;
     o.per = subs_per_tile(nsub);
+    const size_t tiles = (nsub + o.per - 1) / o.per;
     CKS(w.words.ensure(nwords * sizeof(uint4)));
     CKS(w.act.ensure(nwords * sizeof(uint4)));
-    CKS(w.staged.ensure(nsub * SUB * sizeof(uint2)));
-    const size_t tiles = (nsub + o.per - 1) / o.per;
-    CKS(w.sub.ensure((nsub + tiles) * sizeof(uint4) + 2 * sizeof(unsigned)));
+    CKS(w.cnt.ensure(3 * nwords * sizeof(unsigned)));
+    CKS(w.staged.ensure(nsub * SUB));
+    CKS(w.sub.ensure(2 * (nsub + tiles) * sizeof(uint2) + 4 * sizeof(unsigned)));
     o.words = w.words.as<uint4>();
-    o.staged = w.staged.as<uint2>();
-    o.sub = w.sub.as<uint4>();
-    o.part = o.sub + nsub;
-    o.done = (unsigned *)(o.part + tiles);
+    o.cnt = w.cnt.as<unsigned>();
+    o.amb = o.cnt + nwords;
+    o.amblist = o.amb + nwords;
+    o.staged = w.staged.as<unsigned char>();
+    o.sub = w.sub.as<uint2>();
+    o.subt = o.sub + nsub;
+    o.part = o.subt + nsub;
+    o.partt = o.part + tiles;
+    o.ctr = (unsigned *)(o.partt + tiles);
     o.total = d_total;
     return N2M_OK;
 }
 
-// count and number; the group counter of the emit is cleared here too
+// what follows from signs alone (and the marks, if wanted); the counters are cleared here
 template <class P>
-n2m_status count(const P &pol, const unsigned *signs, McWork &w, const Out &o, cudaStream_t s) {
-    const unsigned tiles = (o.nsub + o.per - 1) / o.per;
-    CK(cudaMemsetAsync(o.done, 0, 2 * sizeof(unsigned), s));
-    { k_words<P><<<tiles, SUB, 0, s>>>(pol, signs, o); N2M_COUNT(); }
+n2m_status count_signs(const P &pol, const unsigned *signs, const Out &o, const Marks &marks, cudaStream_t s) {
+    CK(cudaMemsetAsync(o.ctr, 0, 4 * sizeof(unsigned), s));
+    { k_words<P><<<(o.nsub + o.per - 1) / o.per, SUB, 0, s>>>(pol, signs, o, marks); N2M_COUNT(); }
+    CKL();
+    return N2M_OK;
+}
+// the rest: values are final
+template <class P>
+n2m_status count_values(const P &pol, const unsigned *signs, McWork &w, const Out &o, bool tests, cudaStream_t s) {
+    if (tests) {
+        const unsigned b = std::max(1u, std::min((o.nwords / 32 + 127) / 128, 152u * 8u));   // 1 word in 32 fills it
+        k_amb<P><<<b, 128, 0, s>>>(pol, signs, o);
+        N2M_COUNT();
+    }
+    { k_sum<P><<<(o.nsub + o.per - 1) / o.per, SUB, 0, s>>>(o); N2M_COUNT(); }
     { k_finish<P><<<std::max(1u, std::min((o.nsub + 7) / 8, 152u * 8u)), 256, 0, s>>>(pol, o, w.act.as<uint4>()); N2M_COUNT(); }
     CKL();
     return N2M_OK;
@@ -511,7 +686,7 @@ n2m_status emit(const P &pol, const unsigned *signs, McWork &w, const Out &o, un
     const unsigned G = nact >= 64u * warps ? 32u : (nact >= 16u * warps ? 16u : 8u);
     const unsigned groups = (nact + G - 1) / G;
     const unsigned blocks = std::min<unsigned>((groups + EW - 1) / EW, (unsigned)resident);
-    { k_emit<P><<<blocks, EW * 32, 0, s>>>(pol, signs, o.words, w.act.as<uint4>(), nact, G, d_tris, o.done + 1); N2M_COUNT(); }
+    { k_emit<P><<<blocks, EW * 32, 0, s>>>(pol, signs, o.words, w.act.as<uint4>(), nact, G, d_tris, o.ctr + 3); N2M_COUNT(); }
     CKL();
     return N2M_OK;
 }

@@ -94,9 +94,10 @@ bool smooth_can_stage(int nx, int ny, int nz);
 // minimum or maximum, their exact values, which completes w.st (exact range and
 // bbox in its vs).  Once the host has read w.st, od_check says whether the caller
 // has to run launch_smooth instead (a non-finite or huge input, a list overflow).
-// Marching cubes marks the corners of the cubes the surface crosses in need_z
-// (mc.cu: mc_count with an OdRepair), and od_repair writes the reference's exact
-// value at every marked voxel of `out`.
+// Marching cubes marks the voxels whose values it reads in `need` (mcwords.cuh:
+// k_words, with an OdRepair): the ends of the edges the surface crosses and the
+// corners of ambiguous cubes; od_repair writes the reference's exact value at every
+// marked voxel of `out`.
 enum : unsigned { OD_FALLBACK = 1u, OD_TIMEOUT = 2u };
 struct OdStats {
     VolStats vs;             // bbox of decided voxels >= iso; exact range after od_resolve
@@ -113,7 +114,7 @@ struct OdLists {
     unsigned wv, nys;        // the bitmap's words per row, groups of 8 rows per slice
 };
 struct OdWork {
-    DevBuf st, unc, cmin, cmax, range, need_z, need_y, need_x, off, list, lcnt;
+    DevBuf st, unc, cmin, cmax, range, need, list, lcnt;
     // bit x & 31 of word od_vsign_word(x, y, z): the smoothed value of voxel (x, y, z)
     // minus iso is above -FLT_EPSILON (Lewiner's sign before edge darkening), or with
     // od_resolve's at_or_above, the value is >= iso (the complement of oldcubes'
@@ -121,7 +122,6 @@ struct OdWork {
     DevBuf vsign;
     unsigned cap = 0;
 };
-struct ScanWork;
 // What meshify's labelling did to each voxel (src/meshify.c:330-342), for the
 // exact values the repair writes afterwards: voxels of K (bit x & 31 of word
 // (z*ny + y)*W + x/32) are raised to iso when fill; with largest, voxels
@@ -138,7 +138,6 @@ struct OdRepair {
     float *out;              // the approximately smoothed volume, exact where marked
     int dim[3];
     OdWork *w;
-    ScanWork *scan;
     const LabelPost *post = nullptr;   // the volume was labelled: the repaired values get the same treatment
 };
 // the sign bitmap's word of voxel (x, y, z): the 8 row words of one 32 x 8 tile of a
@@ -146,22 +145,14 @@ struct OdRepair {
 __host__ __device__ __forceinline__ size_t od_vsign_word(unsigned x, unsigned y, unsigned z, unsigned wv, unsigned nys) {
     return (((size_t)z * nys + (y >> 3)) * wv + (x >> 5)) * 8u + (y & 7u);
 }
-// marks the voxels j .. j+31 whose bits are set in a linear bitmap over nvox voxels
-__device__ __forceinline__ void od_need_mark(unsigned *need, long long j, unsigned bits, long long nvox) {
-    if (j >= nvox || !bits) return;
-    if (nvox - j < 32) bits &= (1u << (unsigned)(nvox - j)) - 1u;
-    const long long w = j >> 5;
-    const int sh = (int)(j & 31);
-    const unsigned p0 = bits << sh, p1 = sh ? bits >> (32 - sh) : 0u;
-    if (p0) atomicOr(need + w, p0);
-    if (p1) atomicOr(need + w + 1, p1);
-}
 // whether the on-demand path applies: rows a multiple of 16 bytes (TMA tiles), fewer than 2^32 voxels
 bool od_eligible(const float *in, int nx, int ny, int nz);
 n2m_status od_approx(const float *in, float *out, int nx, int ny, int nz, float iso, OdWork &w, cudaStream_t s);
 n2m_status od_resolve(const float *in, float *out, int nx, int ny, int nz, float iso, OdWork &w, cudaStream_t s,
                       bool at_or_above = false);
 n2m_status od_check(const OdWork &w, const OdStats &h, bool *fallback);
+// the cleared mark bitmap: bit x & 31 of word (z*ny + y)*ceil(nx/32) + x/32
+n2m_status od_marks(OdWork &w, const int dim[3], unsigned **need, cudaStream_t s);
 n2m_status od_repair(const OdRepair &r, cudaStream_t s);
 // transposed pre-smooth: g_img = Sx^T Sy^T Sz^T g (tmp: one volume of scratch)
 n2m_status launch_smooth_adjoint(const float *g, float *tmp, float *out, int nx, int ny, int nz, cudaStream_t s);
@@ -244,13 +235,13 @@ struct McWork {
     DevBuf signs;            // sign words of the grid
     DevBuf words;            // per active word {x, y, z crossing masks, vertex offset}
     DevBuf act;              // active words in order {word, triangle offset, c-vertex offset, -}
-    DevBuf staged, sub;      // counting scratch (mcwords.cuh: Out)
+    DevBuf cnt, staged, sub; // counting scratch (mcwords.cuh: Out)
 };
 struct McCounts {
     unsigned nv_edge, nt, nc, nactive;
 };
-// repair: marks the corners of the cubes with mixed signs in repair->w->need_z
-// after the sign pass and runs od_repair before any value is read (null: none)
+// repair: marks the voxels whose values are needed after the sign pass and runs
+// od_repair before any value is read (null: none)
 // (with a repair and no labelling, the sign words of grid points strictly inside
 // the volume come from repair->w->vsign instead of the values)
 n2m_status mc_count(const McGrid &g, int variant, McWork &w, uint4 *d_total, cudaStream_t s,

@@ -117,29 +117,6 @@ __device__ __forceinline__ void ogeo(const OV &g, unsigned w, mcw::Geo &q) {
     q.tag = 0;
 }
 
-// Marks for the exact pre-smooth on demand: the voxel of every corner of
-// every cube whose corner signs differ (the only cubes whose values the emit
-// reads), as bits of a linear bitmap over the volume.
-__global__ void __launch_bounds__(256) k_oc_need(OV g, unsigned nwords, const unsigned *__restrict__ signs,
-                                                 unsigned *need) {
-    const long long nvox = g.dxy * g.dz;
-    for (unsigned w = blockIdx.x * blockDim.x + threadIdx.x; w < nwords; w += gridDim.x * blockDim.x) {
-        mcw::Geo q;
-        ogeo(g, w, q);
-        if (!q.hy || !q.hz) continue;   // no cubes start on the last row / slice
-        const unsigned mix = mcw::mixed_cubes(mcw::load_corners(signs, w, q), q);
-        if (!mix) continue;
-        const unsigned cm = mix | (mix << 1), carry = mix >> 31;   // corners x and x + 1 of each mixed cube
-#pragma unroll
-        for (int r = 0; r < 4; r++) {
-            const long long j = (long long)(g.lo0 + q.x0) + (long long)(g.lo1 + q.y + (r & 1)) * g.dx +
-                                (long long)(g.lo2 + q.z + (r >> 1)) * g.dxy;
-            od_need_mark(need, j, cm, nvox);
-            if (carry) od_need_mark(need, j + 32, 1u, nvox);
-        }
-    }
-}
-
 // ---- emit pass -------------------------------------------------------------------
 // VertexInterp (src/oldcubes.c:22-40) along one axis: p = p1 + mu*(p2-p1)
 // with mu = (iso - v1)/(v2 - v1); only the coordinate along the edge moves.
@@ -201,6 +178,11 @@ struct Policy {
     __device__ __forceinline__ bool geo(unsigned w, mcw::Geo &q) const {
         ogeo(g, w, q);
         return true;
+    }
+    __device__ __forceinline__ void voxel_word(const mcw::Geo &q, int &wx, int &vy, int &vz) const {
+        wx = (g.lo0 + q.x0) >> 5;
+        vy = g.lo1 + q.y;
+        vz = g.lo2 + q.z;
     }
     __device__ __forceinline__ void shifts(const mcw::Out &, unsigned, const uint4 &, unsigned &e, unsigned &c) const { e = c = 0; }
     __device__ __forceinline__ mcw::CubeTiling tests(const mcw::Geo &, int, int, int, int) const { return {0, 0, false}; }
@@ -324,15 +306,12 @@ n2m_status oc_count(const float *vol, const int dim[3], const int lo[3], const i
         const unsigned nrows = (unsigned)g.NY * (unsigned)g.NZ;
         { k_oc_signs<<<std::min<unsigned>((nrows + 7) / 8, 152u * 16u), 256, 0, s>>>(g, nrows, signs); N2M_COUNT(); }
     }
-    if (repair) {   // exact smoothed values where the emit reads them
-        const size_t nvw = ((size_t)dim[0] * dim[1] * dim[2] + 31) / 32;
-        CKS(repair->w->need_z.ensure(nvw * sizeof(unsigned)));
-        CK(cudaMemsetAsync(repair->w->need_z.p, 0, nvw * sizeof(unsigned), s));
-        { k_oc_need<<<wblocks, 256, 0, s>>>(g, (unsigned)nwords, signs, repair->w->need_z.as<unsigned>()); N2M_COUNT(); }
-        CKL();
-        CKS(od_repair(*repair, s));
-    }
-    return mcw::count(Policy{g, nullptr, nullptr, nullptr, 0}, signs, w, o, s);
+    const Policy pol{g, nullptr, nullptr, nullptr, 0};
+    mcw::Marks marks{nullptr, g.dx, g.dy, g.dz, (unsigned)(g.dx + 31) / 32u};
+    if (repair) CKS(od_marks(*repair->w, dim, &marks.need, s));
+    CKS(mcw::count_signs(pol, signs, o, marks, s));
+    if (repair) CKS(od_repair(*repair, s));   // exact smoothed values where the emit reads them
+    return mcw::count_values(pol, signs, w, o, false, s);
 }
 
 n2m_status oc_emit(const float *vol, const int dim[3], const int lo[3], const int hi[3], float iso, float edge_max,
