@@ -282,7 +282,7 @@ extern "C" void n2m_context_destroy(n2m_context *c) {
                       &c->aw.pts, &c->aw.pts2, &c->aw.tris, &c->aw.tris2, &c->aw.cand, &c->aw.gath, &c->aw.weld,
                       &c->aw.ranges, &c->alab, &c->lpts, &c->ltris, &c->gA, &c->gB, &c->gs, &c->gtmp, &c->in, &c->raw, &c->vol, &c->stmp, &c->stats, &c->totals, &c->cand, &c->ncand, &c->ocq, &c->pts_raw,
                       &c->tris_raw, &c->pts, &c->tris, &c->ntf, &c->weld, &c->gath, &c->hmesh,
-                      &c->mc.signs, &c->mc.words, &c->mc.act, &c->mc.cnt, &c->mc.staged, &c->mc.sub, &c->scan.part,
+                      &c->mc.signs, &c->mc.words, &c->mc.act, &c->mc.cnt, &c->mc.sub, &c->scan.part,
                       &c->lab.lab, &c->lab.mask, &c->lab.keep, &c->lab.cnt, &c->lab.edge, &c->lab.rc, &c->lab.misc,
                       &c->deg.flags, &c->deg.tmp, &c->hc.zero, &c->hc.adj, &c->hc.meta, &c->hc.P, &c->hc.Q,
                       &c->hc.B, &c->hc.Lo, &c->th.buf, &c->th.table,

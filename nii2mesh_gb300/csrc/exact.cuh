@@ -178,17 +178,19 @@ N2M_HD bool tap5_split(float aH, float aL, float bH, float bL, float cH, float c
     return fabsf(R3) < t25 && (yb & 0x7FFFFFu) != 0u && fabsf(y) >= mth;
 }
 
-// tap5_split on five raw inputs, the group being the window itself
-N2M_HD bool tap5_split_window(float a, float b, float c, float d, float e, float *out) {
+// tap5_split on five raw inputs, the group being the window itself: 1 decided, 0 undecided, -1 not applicable
+N2M_HD int tap5_split_state(float a, float b, float c, float d, float e, float *out) {
     const float mx = fmaxf(fmaxf(fmaxf(fabsf(a), fabsf(b)), fmaxf(fabsf(c), fabsf(d))), fabsf(e));
     const float mn = fminf(fminf(fminf(fabsf(a), fabsf(b)), fminf(fabsf(c), fabsf(d))), fabsf(e));
-    if (!split_group_ok(mn, mx)) return false;
+    if (!split_group_ok(mn, mx)) return -1;
     float aH, aL, bH, bL, cH, cL, dH, dL, eH, eL;
     split12(a, aH, aL);
     split12(b, bH, bL);
     split12(c, cH, cL);
     split12(d, dH, dL);
     split12(e, eH, eL);
-    return tap5_split(aH, aL, bH, bL, cH, cL, dH, dL, eH, eL, FMUL(mx, 0x1p-8f), out);
+    return tap5_split(aH, aL, bH, bL, cH, cL, dH, dL, eH, eL, FMUL(mx, 0x1p-8f), out) ? 1 : 0;
 }
-
+N2M_HD bool tap5_split_window(float a, float b, float c, float d, float e, float *out) {
+    return tap5_split_state(a, b, c, d, e, out) == 1;
+}

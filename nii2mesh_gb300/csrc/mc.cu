@@ -186,25 +186,25 @@ __device__ __forceinline__ float ival(const GV &g, const float *p) {
 // exact float -> double by assembling the bits in integer registers (a
 // conversion instruction would issue on the pipe this part shares with FP64;
 // a predicated one still issues)
-__device__ __forceinline__ double f2d(float f) {
+__device__ __noinline__ double f2d_rare(float f) {   // zero, subnormal, Inf, NaN
     const unsigned u = __float_as_uint(f), e = (u >> 23) & 0xffu, m = u & 0x7fffffu;
     const unsigned long long sign = (unsigned long long)(u & 0x80000000u) << 32;
-    unsigned long long de, dm;
-    if (e == 0xffu) {               // Inf, NaN
+    unsigned long long de = 0, dm = 0;
+    if (e == 0xffu) {
         de = 0x7ffull;
         dm = (unsigned long long)m << 29;
-    } else if (e != 0u) {           // normal
-        de = e + 896u;
-        dm = (unsigned long long)m << 29;
-    } else if (m != 0u) {           // subnormal: m * 2^-149, leading bit p
+    } else if (m != 0u) {           // m * 2^-149, leading bit p
         const int p = 31 - __clz((int)m);
         de = (unsigned long long)(p - 149 + 1023);
         dm = ((unsigned long long)m << (52 - p)) & 0xfffffffffffffull;
-    } else {                        // signed zero
-        de = 0;
-        dm = 0;
     }
     return __longlong_as_double((long long)(sign | (de << 52) | dm));
+}
+__device__ __forceinline__ double f2d(float f) {
+    const unsigned u = __float_as_uint(f);
+    if (((u >> 23) & 0xffu) - 1u < 0xfeu)
+        return __hiloint2double((int)((u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + 0x38000000u)), (int)(u << 29));
+    return u == 0u ? 0.0 : f2d_rare(f);
 }
 
 // exact float of 0 <= v < 2^23 by bit assembly (no I2F conversion)
@@ -260,6 +260,7 @@ __device__ __noinline__ mcw::CubeTiling tested_tiling(const GV &g, int x, int y,
 // mcwords.cuh's policy for the padded Lewiner grid
 struct Policy {
     static constexpr bool MULTI = false, REVERSE = true, CVERTS = true;
+    static constexpr int CTAS = 8, EV = 1;   // of k_emit: CTAs per SM, vertices per lane in flight
     GV g;
     bool classic;
     vec3d *pts;
@@ -303,25 +304,26 @@ struct Policy {
         cube_values(g, x, y, z, c);
         emit_cvertex(c, x, y, z, (float)g.lo0, (float)g.lo1, (float)g.lo2, id, pts, ccand, nccand, cap);
     }
-    __device__ __forceinline__ void vertex(int x, int y, int z, int ax, int, int id) const {
-        const int vx = g.lo0 + x, vy = g.lo1 + y, vz = g.lo2 + z;
+    struct Edge {
         float c0, c1;
+    };
+    __device__ __forceinline__ Edge edge(int x, int y, int z, int ax, int) const {
+        const int vx = g.lo0 + x, vy = g.lo1 + y, vz = g.lo2 + z;
         if (vx >= 1 && vx + 1 <= g.dx - 2 && vy >= 1 && vy + 1 <= g.dy - 2 && vz >= 1 && vz + 1 <= g.dz - 2) {
             const float *q = g.vol + ((long long)vx + (long long)vy * g.dx + (long long)vz * g.dxy);
-            c0 = ival(g, q);
-            c1 = ival(g, q + (ax == 0 ? 1ll : (ax == 1 ? (long long)g.dx : g.dxy)));
-        } else {
-            c0 = gval(g, x, y, z);
-            c1 = gval(g, x + (ax == 0), y + (ax == 1), z + (ax == 2));
+            return Edge{ival(g, q), ival(g, q + (ax == 0 ? 1ll : (ax == 1 ? (long long)g.dx : g.dxy)))};
         }
-        const float u = edge_u(c0, c1), flo0 = (float)g.lo0, flo1 = (float)g.lo1, flo2 = (float)g.lo2;
+        return Edge{gval(g, x, y, z), gval(g, x + (ax == 0), y + (ax == 1), z + (ax == 2))};
+    }
+    __device__ __forceinline__ vec3d vertex(const Edge &c, int x, int y, int z, int ax, int id) const {
+        const float u = edge_u(c.c0, c.c1), flo0 = (float)g.lo0, flo1 = (float)g.lo1, flo2 = (float)g.lo2;
         const float fx = i2f_small(x), fy = i2f_small(y), fz = i2f_small(z);
         float X = __fadd_rn(fx, flo0), Y = __fadd_rn(fy, flo1), Z = __fadd_rn(fz, flo2), axv;
         if (ax == 0) axv = X = __fadd_rn(__fadd_rn(fx, u), flo0);
         else if (ax == 1) axv = Y = __fadd_rn(__fadd_rn(fy, u), flo1);
         else axv = Z = __fadd_rn(__fadd_rn(fz, u), flo2);
-        pts[id] = {f2d(X), f2d(Y), f2d(Z)};
         if (frac_dist(axv) < 1.5e-5f) add_cand(cand, ncand, cap, id);
+        return {f2d(X), f2d(Y), f2d(Z)};
     }
 };
 

@@ -6,15 +6,16 @@
 // arithmetic); this file counts, numbers and emits:
 //
 //   k_words   edge-crossing masks of every word and the counts that follow from
-//             signs alone; marks the voxels whose exact values will be read; lists
-//             the words holding ambiguous cubes.  A warp turns the mixed cubes of its
-//             32 words into one dense list (a cube per lane), so that neither an empty
-//             word nor a full one costs its neighbours time.  Sub-tiles of 256 words
-//             are scanned in the block; the last block to finish scans the tiles.
-//   k_amb     the face and interior tests of the listed words' ambiguous cubes, which
-//             need values (so with the exact smoothing on demand they come after the
-//             repair), again a cube per lane: their loads no longer hold up k_words.
-//   k_sum     triangle and c-vertex sums, over active words only.
+//             signs alone; marks the voxels whose exact values will be read.  A
+//             warp takes 32 words (a sub-tile) and turns their mixed cubes into
+//             one dense list (a cube per lane), so that neither an empty word nor a
+//             full one costs its neighbours time; warps never wait for one another.
+//   k_amb     the face and interior tests of the ambiguous cubes, which need values
+//             (so with the exact smoothing on demand they come after the repair): a
+//             block lists the words of 32 sub-tiles that hold any, then takes them a
+//             cube per lane.
+//   k_sum     sums of the sub-tiles, scanned per tile of 256 in the block; the last
+//             block to finish scans the tiles.
 //   k_finish  the active words (those that own output) as one list in word order
 //             with their absolute triangle and c-vertex offsets; the words'
 //             vertex offsets become absolute.
@@ -26,11 +27,14 @@
 // triangle corner finds its vertex id with one 16-byte load.  Inactive words have
 // no record: nothing refers to them.
 //
-// Measured on the 512^3 CT volume (7.1 M triangles, cold caches): emit 474 -> 218 us
-// against one lane per word listing its cubes for the warp and separate mask and
-// offset arrays; masks, marks, counts, scan and active list 290 -> 178 us.  On the brain volume
+// Measured on the 512^3 CT volume (7.1 M triangles, 4.5 M words, cold caches): masks,
+// marks, counts, scan and active list 290 -> 150 us (k_words 85: a block scan per 256
+// words had cost 120, waiting for the block's fullest warp); emit 474 -> 211 us
+// against one lane per word listing its cubes for the warp, with separate mask and
+// offset arrays and the ambiguous tests repeated.  Two emit kernels (vertices,
+// triangles) took 255, two vertices per lane in flight 250.  On the brain volume
 // (0.2 M triangles, 1.7 k groups of 32 words for 5 k resident warps) the emit went
-// from 157 to 23 us.
+// from 157 to 23 us with smaller groups.
 #pragma once
 #include <algorithm>
 #include <atomic>
@@ -39,7 +43,8 @@
 
 namespace mcw {
 constexpr unsigned FULL = 0xffffffffu;
-constexpr int SUB = 256;          // words per sub-tile
+constexpr int SUB = 32;           // words per sub-tile
+constexpr int TILE = 256;         // sub-tiles per tile
 
 // bits [lo, hi) of a word, clipped to it
 __device__ __forceinline__ unsigned bit_range(int lo, int hi) {
@@ -134,18 +139,20 @@ constexpr unsigned TESTS = 0xffu;   // quick(): the tiling depends on corner val
 
 // what the count pass leaves behind (see McWork)
 struct Out {
-    uint4 *words;           // per active word
-    unsigned *cnt;          // per active word, triangles | c-vertices << 16
-    unsigned *amb;          // per active word, its ambiguous cubes
-    unsigned *amblist;      // words with any
-    unsigned char *staged;  // per sub-tile, its active words in order (number within the sub-tile)
-    uint2 *sub;             // per sub-tile, what precedes it in its tile {vertices, active words | own active words << 20}
-    uint2 *subt;            // the same {triangles, c-vertices}
-    uint2 *part, *partt;    // per tile, what precedes it, likewise
-    uint4 *total;           // {vertices, triangles, c-vertices, active words}
-    unsigned *ctr;          // tiles finished (two passes), words in amblist, group counter of the emit
-    unsigned nwords, nsub, per;   // per: sub-tiles per tile (tile = block)
+    uint4 *words;      // per active word (its vertex offset within the sub-tile until k_finish)
+    unsigned *cnt;     // per active word, triangles | c-vertices << 16
+    unsigned *amb;     // per active word, its ambiguous cubes
+    unsigned *ambat;   // per word with any, its first entry in tilings
+    unsigned *tilings; // of the ambiguous cubes: code offset | triangles << 22 | c-vertex << 26; nwords entries
+    uint4 *sub;        // per sub-tile {vertices, its active words, its words with ambiguous cubes, -}
+    uint4 *pre;        // per sub-tile, what precedes it in its tile {vertices, triangles, c-vertices, active words}
+    uint4 *part;       // per tile, what precedes it, likewise
+    uint4 *total;
+    unsigned *ctr;     // tiles finished, group counter of the emit, tilings
+    unsigned nwords, nsub;
 };
+
+__device__ __forceinline__ uint4 add4(uint4 a, uint4 b) { return make_uint4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
 
 // marks voxels of a volume in a bitmap of row-aligned words (bit x & 31 of word (z*ny + y)*W + x/32): word wx of row
 // (y, z), of which y may be one row and z one slice past the volume, and bit nx of a row its padding column (they wrap
@@ -174,62 +181,14 @@ struct Marks {
     }
 };
 
-// turns n per-tile sums into what precedes each, by one block; the total goes to *all
-__device__ __forceinline__ void scan_parts(uint2 *part, unsigned n, uint2 *psum, int tid, uint2 &all) {
-    const int lane = tid & 31, wid = tid >> 5;
-    const unsigned each = (n + SUB - 1) / SUB, p0 = min(n, (unsigned)tid * each), p1 = min(n, p0 + each);
-    uint2 s = make_uint2(0u, 0u);
-    for (unsigned k = p0; k < p1; k++) {
-        const uint2 v = __ldcg(part + k);
-        s.x += v.x;
-        s.y += v.y;
-    }
-    unsigned tx, ty;
-    uint2 before;
-    before.x = warp_excl(s.x, lane, tx);
-    before.y = warp_excl(s.y, lane, ty);
-    if (lane == 0) psum[wid] = make_uint2(tx, ty);
-    __syncthreads();
-    all = make_uint2(0u, 0u);
-    for (int k = 0; k < SUB / 32; k++) {
-        if (k < wid) {
-            before.x += psum[k].x;
-            before.y += psum[k].y;
-        }
-        all.x += psum[k].x;
-        all.y += psum[k].y;
-    }
-    for (unsigned k = p0; k < p1; k++) {
-        const uint2 v = __ldcg(part + k);
-        part[k] = before;
-        before.x += v.x;
-        before.y += v.y;
-    }
-}
-// whether this block is the last to hand in its tile's sums (all threads call it)
-__device__ __forceinline__ bool last_tile(uint2 *part, uint2 sums, unsigned *done, bool &flag) {
-    if (threadIdx.x == 0) {
-        part[blockIdx.x] = sums;
-        __threadfence();
-        flag = atomicAdd(done, 1u) == gridDim.x - 1;
-    }
-    __syncthreads();
-    if (flag) __threadfence();
-    return flag;
-}
-
 template <class P>
-__global__ void __launch_bounds__(SUB) k_words(P pol, const unsigned *__restrict__ signs, Out o, Marks marks) {
-    __shared__ unsigned qt[256], pre[8][32], cor[8][6][32], cnt[SUB], amb[SUB], abase;
-    __shared__ uint2 wsum[8];
-    __shared__ bool last;
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    qt[tid] = pol.quick(tid);
+__global__ void __launch_bounds__(256) k_words(P pol, const unsigned *__restrict__ signs, Out o, Marks marks) {
+    __shared__ unsigned qt[256], pre[8][32], cor[8][6][32], cnt[8][32], amb[8][32];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    qt[threadIdx.x] = pol.quick(threadIdx.x);
     __syncthreads();
-    uint2 run = make_uint2(0u, 0u);   // vertices, active words of the tile so far
-    const unsigned s1 = min(o.nsub, (blockIdx.x + 1) * o.per);
-    for (unsigned sub = blockIdx.x * o.per; sub < s1; sub++) {
-        const unsigned w = sub * SUB + (unsigned)tid;
+    for (unsigned sub = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; sub < o.nsub; sub += (gridDim.x * blockDim.x) >> 5) {
+        const unsigned w = sub * SUB + (unsigned)lane;
         unsigned xm = 0, ym = 0, zm = 0, mix = 0;
         Geo g;
         if (w < o.nwords && pol.geo(w, g)) {
@@ -247,45 +206,34 @@ __global__ void __launch_bounds__(SUB) k_words(P pol, const unsigned *__restrict
                 cor[wid][5][lane] = mix;
             }
         }
-        cnt[tid] = 0u;
-        amb[tid] = 0u;
-        unsigned ncube;
-        pre[wid][lane] = warp_excl(__popc(mix), lane, ncube);
+        const unsigned nv = __popc(xm) + __popc(ym) + __popc(zm);
+        const bool act = (nv | mix) != 0u;
+        const unsigned acts = __ballot_sync(FULL, act);
+        if (!acts) {
+            if (lane == 0) o.sub[sub] = make_uint4(0u, 0u, 0u, 0u);
+            continue;
+        }
+        cnt[wid][lane] = 0u;
+        amb[wid][lane] = 0u;
+        unsigned both;   // vertices | cubes << 16
+        const unsigned ex = warp_excl(nv | __popc(mix) << 16, lane, both);
+        const unsigned ncube = both >> 16;
+        pre[wid][lane] = ex >> 16;
         __syncwarp();
         for (unsigned k = lane; k < ncube; k += 32) {
             const int l = find_lane(pre[wid], k);
             const int i = nth_bit(cor[wid][5][l], (int)(k - pre[wid][l]));
             const int lut = cube_index(cor[wid][0][l], cor[wid][1][l], cor[wid][2][l], cor[wid][3][l], cor[wid][4][l], i);
             const unsigned n = qt[lut] & 0xffu;
-            if (n == TESTS) atomicOr(&amb[wid * 32 + l], 1u << i);
-            else atomicAdd(&cnt[wid * 32 + l], n);
+            if (n == TESTS) atomicOr(&amb[wid][l], 1u << i);
+            else atomicAdd(&cnt[wid][l], n);
         }
         __syncwarp();
-        // a sub-tile has at most 24576 vertices and 256 active words (256 with ambiguous cubes)
-        const unsigned nv = __popc(xm) + __popc(ym) + __popc(zm), am = amb[tid];
-        const bool act = (nv | mix) != 0u;
-        unsigned ta, tb, ea = warp_excl(nv | (act ? 1u << 16 : 0u), lane, ta);
-        const unsigned ab = __ballot_sync(FULL, am != 0u);
-        tb = __popc(ab);
-        if (lane == 0) wsum[wid] = make_uint2(ta, tb);
-        __syncthreads();
-        uint2 all = make_uint2(0u, 0u);
-        unsigned eb = __popc(ab & ((1u << lane) - 1u));
-#pragma unroll
-        for (int k = 0; k < SUB / 32; k++) {
-            const uint2 t = wsum[k];
-            if (k < wid) {
-                ea += t.x;
-                eb += t.y;
-            }
-            all.x += t.x;
-            all.y += t.y;
-        }
-        if (tid == 0 && all.y) abase = atomicAdd(o.ctr + 2, all.y);
+        const unsigned am = amb[wid][lane], ambs = __ballot_sync(FULL, am != 0u);
+        if (lane == 0) o.sub[sub] = make_uint4(both & 0xffffu, acts, ambs, 0u);
         if (act) {
-            o.words[w] = make_uint4(xm, ym, zm, ea & 0xffffu);
-            o.staged[(size_t)sub * SUB + (ea >> 16)] = (unsigned char)tid;
-            o.cnt[w] = cnt[tid];
+            o.words[w] = make_uint4(xm, ym, zm, ex & 0xffffu);
+            o.cnt[w] = cnt[wid][lane];
             if (P::CVERTS) o.amb[w] = am;
             if (marks.need) {   // both ends of every crossing edge; every corner of the ambiguous cubes
                 int wx, vy, vz;
@@ -305,31 +253,31 @@ __global__ void __launch_bounds__(SUB) k_words(P pol, const unsigned *__restrict
                 }
             }
         }
-        if (tid == 0) o.sub[sub] = make_uint2(run.x, run.y | (all.x >> 16) << 20);
-        run.x += all.x & 0xffffu;
-        run.y += all.x >> 16;
-        __syncthreads();   // abase; wsum is reused
-        if (am) o.amblist[abase + eb] = w;
-    }
-    if (!last_tile(o.part, run, o.ctr, last)) return;
-    uint2 all;
-    scan_parts(o.part, gridDim.x, wsum, tid, all);
-    if (tid == 0) {
-        o.total->x = all.x;
-        o.total->w = all.y;
+        __syncwarp();   // the shared lists are reused
     }
 }
 
-// the ambiguous cubes of the listed words, a warp per 32 words
+constexpr unsigned NO_TILING = 0xffffffffu;
+constexpr int AMB_T = 128, AMB_S = 32, AMB_W = 8;   // threads of k_amb, sub-tiles of a block, words of a warp at a time
 template <class P>
-__global__ void __launch_bounds__(128) k_amb(P pol, const unsigned *__restrict__ signs, Out o) {
-    __shared__ unsigned pre[4][32], cor[4][6][32], words[4][32];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const unsigned n = o.ctr[2];
-    for (unsigned a0 = (blockIdx.x * 4 + (unsigned)wid) * 32; a0 < n; a0 += gridDim.x * 128) {
+__global__ void __launch_bounds__(AMB_T) k_amb(P pol, const unsigned *__restrict__ signs, Out o) {
+    __shared__ unsigned short list[AMB_S * SUB];
+    __shared__ unsigned nlist, pre[4][32], cor[4][6][32], words[4][32];
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    if (tid == 0) nlist = 0u;
+    __syncthreads();
+    const unsigned sub = blockIdx.x * AMB_S + (unsigned)tid, w0 = blockIdx.x * AMB_S * SUB;
+    unsigned m = tid < AMB_S && sub < o.nsub ? o.sub[sub].z : 0u;
+    if (m) {
+        unsigned at = atomicAdd(&nlist, (unsigned)__popc(m));
+        for (; m; m &= m - 1) list[at++] = (unsigned short)(tid * SUB + __ffs(m) - 1);
+    }
+    __syncthreads();
+    const unsigned n = nlist;
+    for (unsigned a0 = (unsigned)wid * AMB_W; a0 < n; a0 += AMB_W * AMB_T / 32) {
         unsigned am = 0;
-        if (a0 + (unsigned)lane < n) {
-            const unsigned w = o.amblist[a0 + lane];
+        if (lane < AMB_W && a0 + (unsigned)lane < n) {
+            const unsigned w = w0 + list[a0 + lane];
             Geo g;
             pol.geo(w, g);
             const Corners q = load_corners(signs, w, g);
@@ -342,8 +290,12 @@ __global__ void __launch_bounds__(128) k_amb(P pol, const unsigned *__restrict__
             cor[wid][4][lane] = q.nxt;
             cor[wid][5][lane] = am;
         }
-        unsigned ncube;
+        unsigned ncube, at = 0;
         pre[wid][lane] = warp_excl(__popc(am), lane, ncube);
+        if (lane == 0) at = atomicAdd(o.ctr + 2, ncube);
+        at = __shfl_sync(FULL, at, 0);
+        const bool room = at + ncube <= o.nwords;          // else the emit repeats the tests
+        if (am) o.ambat[words[wid][lane]] = room ? at + pre[wid][lane] : NO_TILING;
         __syncwarp();
         for (unsigned k = lane; k < ncube; k += 32) {
             const int l = find_lane(pre[wid], k);
@@ -353,84 +305,116 @@ __global__ void __launch_bounds__(128) k_amb(P pol, const unsigned *__restrict__
             pol.geo(words[wid][l], g);
             const CubeTiling T = pol.tests(g, g.x0 + i, g.y, g.z, lut);
             atomicAdd(o.cnt + words[wid][l], (unsigned)T.n | (T.cv ? 1u << 16 : 0u));
+            if (room) o.tilings[at + k] = (unsigned)T.off | (unsigned)T.n << 22 | (T.cv ? 1u << 26 : 0u);
         }
         __syncwarp();
     }
 }
 
-// triangle and c-vertex sums of the sub-tiles, a warp each, in rounds of 8 (a template only to be emitted once per unit)
+__device__ __forceinline__ uint4 warp_incl4(uint4 v, int lane) {
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        uint4 t;
+        t.x = __shfl_up_sync(FULL, v.x, d); t.y = __shfl_up_sync(FULL, v.y, d);
+        t.z = __shfl_up_sync(FULL, v.z, d); t.w = __shfl_up_sync(FULL, v.w, d);
+        if (lane >= d) v = add4(v, t);
+    }
+    return v;
+}
+// exclusive scan over a block of 256, *all: its total
+__device__ __forceinline__ uint4 block_excl4(uint4 v, uint4 *wsum, int lane, int wid, uint4 *all) {
+    const uint4 in = warp_incl4(v, lane);
+    if (lane == 31) wsum[wid] = in;
+    __syncthreads();
+    uint4 before = make_uint4(in.x - v.x, in.y - v.y, in.z - v.z, in.w - v.w), t = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        if (k < wid) before = add4(before, wsum[k]);
+        t = add4(t, wsum[k]);
+    }
+    *all = t;
+    return before;
+}
+
+// (a template only so that each unit has its own)
 template <class P>
-__global__ void __launch_bounds__(SUB) k_sum(Out o) {
-    __shared__ uint2 wsum[8];
+__global__ void __launch_bounds__(TILE) k_sum(Out o) {
+    __shared__ uint4 wsum[8];
     __shared__ bool last;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    uint2 run = make_uint2(0u, 0u);
-    const unsigned s0 = blockIdx.x * o.per, s1 = min(o.nsub, s0 + o.per);
-    for (unsigned r = s0; r < s1; r += 8) {
-        const unsigned sub = r + (unsigned)wid;
-        uint2 t = make_uint2(0u, 0u);
-        if (sub < s1) {
-            const unsigned n = o.sub[sub].y >> 20;
-            for (unsigned k = (unsigned)lane; k < n; k += 32) {
-                const unsigned c = o.cnt[sub * SUB + o.staged[(size_t)sub * SUB + k]];
-                t.x += c & 0xffffu;
-                t.y += c >> 16;
-            }
+    const unsigned s = blockIdx.x * TILE + (unsigned)tid;
+    const uint4 rec = s < o.nsub ? o.sub[s] : make_uint4(0u, 0u, 0u, 0u);
+    unsigned mine = 0;   // this lane's sub-tile: triangles (at most 12288) | c-vertices << 16
+    if (rec.y) {         // its 32 counts at once (only those of active words are set)
+        const uint4 *c4 = (const uint4 *)(o.cnt + (size_t)s * SUB);
+        uint4 c[SUB / 4];
+#pragma unroll
+        for (int q = 0; q < SUB / 4; q++) c[q] = __ldg(c4 + q);
+#pragma unroll
+        for (int q = 0; q < SUB / 4; q++) {
+            const unsigned m = rec.y >> (4 * q);
+            mine += (m & 1u ? c[q].x : 0u) + (m & 2u ? c[q].y : 0u) + (m & 4u ? c[q].z : 0u) + (m & 8u ? c[q].w : 0u);
         }
-        t.x = __reduce_add_sync(FULL, t.x);
-        t.y = __reduce_add_sync(FULL, t.y);
-        if (lane == 0) wsum[wid] = t;
-        __syncthreads();
-        uint2 before = run;
-        for (int k = 0; k < 8; k++) {
-            if (k < wid) {
-                before.x += wsum[k].x;
-                before.y += wsum[k].y;
-            }
-            run.x += wsum[k].x;
-            run.y += wsum[k].y;
-        }
-        if (lane == 0 && sub < s1) o.subt[sub] = before;
-        __syncthreads();
     }
-    if (!last_tile(o.partt, run, o.ctr + 1, last)) return;
-    uint2 all;
-    scan_parts(o.partt, gridDim.x, wsum, tid, all);
+    uint4 all;
+    const uint4 before = block_excl4(make_uint4(rec.x, mine & 0xffffu, mine >> 16, (unsigned)__popc(rec.y)), wsum, lane, wid, &all);
+    if (s < o.nsub) o.pre[s] = before;
     if (tid == 0) {
-        o.total->y = all.x;
-        o.total->z = all.y;
+        o.part[blockIdx.x] = all;
+        __threadfence();
+        last = atomicAdd(o.ctr, 1u) == gridDim.x - 1;
     }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    const unsigned n = gridDim.x, each = (n + TILE - 1) / TILE, p0 = min(n, (unsigned)tid * each), p1 = min(n, p0 + each);
+    uint4 sum = make_uint4(0u, 0u, 0u, 0u);
+    for (unsigned k = p0; k < p1; k++) sum = add4(sum, __ldcg(o.part + k));
+    uint4 at = block_excl4(sum, wsum, lane, wid, &all);
+    for (unsigned k = p0; k < p1; k++) {
+        const uint4 v = __ldcg(o.part + k);
+        o.part[k] = at;
+        at = add4(at, v);
+    }
+    if (tid == 0) *o.total = all;
 }
 
 // what precedes sub-tile s: vertices, triangles, c-vertices, active words
-__device__ __forceinline__ uint4 sub_offset(const Out &o, unsigned s) {
-    const uint2 a = o.sub[s], b = o.subt[s], pa = o.part[s / o.per], pb = o.partt[s / o.per];
-    return make_uint4(a.x + pa.x, b.x + pb.x, b.y + pb.y, (a.y & 0xfffffu) + pa.y);
-}
+__device__ __forceinline__ uint4 sub_offset(const Out &o, unsigned s) { return add4(o.pre[s], o.part[s / TILE]); }
 
-// a warp per sub-tile
+// a warp takes FIN sub-tiles at once, a lane per word
+constexpr int FIN = 4;
 template <class P>
 __global__ void __launch_bounds__(256) k_finish(P pol, Out o, uint4 *act) {
     const int lane = threadIdx.x & 31;
     const uint4 total = *o.total;
-    for (unsigned s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; s < o.nsub; s += (gridDim.x * blockDim.x) >> 5) {
-        const unsigned n = o.sub[s].y >> 20;
-        if (!n) continue;
-        uint4 b = sub_offset(o, s);
-        unsigned eshift, cshift;   // added to edge-vertex and c-vertex numbers
-        pol.shifts(o, s, total, eshift, cshift);
-        for (unsigned k0 = 0; k0 < n; k0 += 32) {
-            const unsigned k = k0 + (unsigned)lane;
-            const unsigned w = s * SUB + (k < n ? o.staged[(size_t)s * SUB + k] : 0u);
-            const unsigned c = k < n ? o.cnt[w] : 0u;
-            unsigned tt, tc;
-            const unsigned et = warp_excl(c & 0xffffu, lane, tt), ec = warp_excl(c >> 16, lane, tc);
-            if (k < n) {
-                o.words[w].w += b.x + eshift;
-                act[b.w + k] = make_uint4(w, b.y + et, b.z + ec + cshift, 0u);
+    for (unsigned s0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * FIN; s0 < o.nsub; s0 += ((gridDim.x * blockDim.x) >> 5) * FIN) {
+        unsigned m[FIN], c[FIN];
+        uint4 b[FIN];
+#pragma unroll
+        for (int u = 0; u < FIN; u++) m[u] = s0 + u < o.nsub ? o.sub[s0 + u].y : 0u;
+#pragma unroll
+        for (int u = 0; u < FIN; u++) {
+            const unsigned w = (s0 + u) * SUB + (unsigned)lane;
+            c[u] = m[u] >> lane & 1u ? __ldg(o.cnt + w) : 0u;
+            b[u] = make_uint4(0u, 0u, 0u, 0u);
+            if (m[u]) {
+                b[u] = sub_offset(o, s0 + u);
+                unsigned eshift, cshift;   // added to edge-vertex and c-vertex numbers
+                pol.shifts(o, s0 + u, total, eshift, cshift);
+                b[u].x += eshift;
+                b[u].z += cshift;
             }
-            b.y += tt;
-            b.z += tc;
+        }
+#pragma unroll
+        for (int u = 0; u < FIN; u++) {
+            if (!m[u]) continue;
+            unsigned t;
+            const unsigned w = (s0 + u) * SUB + (unsigned)lane, e = warp_excl(c[u], lane, t);
+            if (m[u] >> lane & 1u) {
+                o.words[w].w += b[u].x;
+                act[b[u].w + __popc(m[u] & ((1u << lane) - 1u))] = make_uint4(w, b[u].y + (e & 0xffffu), b[u].z + (e >> 16), 0u);
+            }
         }
     }
 }
@@ -455,19 +439,26 @@ __device__ __forceinline__ unsigned edge_code(int code) {
 constexpr int EW = 4;              // warps per CTA of k_emit
 constexpr int TQ = 32 + 32 * 12;   // queued triangles: fewer than 32 left over, 32 cubes of at most 12
 
+// next: a zeroed group counter (groups are handed out one at a time: their work varies); G active words per group
+__device__ __forceinline__ unsigned next_group(unsigned *next, int lane) {
+    unsigned grp = 0;
+    if (lane == 0) grp = atomicAdd(next, 1u);
+    return __shfl_sync(FULL, grp, 0);
+}
+
 struct EmitShared {
-    unsigned prev[32], prec[32];   // first vertex / cube of each lane's word
+    unsigned prev[32], pre[32];    // first vertex / cube of each lane's word
     unsigned cor[6][32];
-    unsigned first_c[32];          // c-vertices of the group before each word's
-    unsigned tri[TQ];              // lane << 27 | bit << 22 | code offset
+    unsigned first_c[32], amb[32]; // c-vertices of the group before each word's; ambiguous cubes
+    __align__(8) unsigned tri[TQ]; // lane << 27 | bit << 22 | code offset; before that, 32 vertices on their way out
     int cvert[TQ];                 // the cube's c-vertex
+    int out[96];                   // 32 triangles on their way out
 };
 
-// next: a zeroed group counter (groups are handed out one at a time: their work varies); G active words per group
 template <class P>
-__global__ void __launch_bounds__(EW * 32) k_emit(P pol, const unsigned *__restrict__ signs, const uint4 *__restrict__ words,
-                                                  const uint4 *__restrict__ act, unsigned nact, unsigned G, vec3i *tris,
-                                                  unsigned *next) {
+__global__ void __launch_bounds__(EW * 32, P::CTAS) k_emit(P pol, const unsigned *__restrict__ signs, Out o, const uint4 *__restrict__ act,
+                                                           unsigned nact, unsigned G, vec3i *tris) {
+    const uint4 *__restrict__ words = o.words;
     __shared__ EmitShared shared[EW];
     __shared__ unsigned qt[256];
     for (int i = threadIdx.x; i < 256; i += EW * 32) qt[i] = pol.quick(i);
@@ -475,11 +466,7 @@ __global__ void __launch_bounds__(EW * 32) k_emit(P pol, const unsigned *__restr
     const int lane = threadIdx.x & 31;
     EmitShared &S = shared[threadIdx.x >> 5];
     const unsigned ngroups = (nact + G - 1) / G;
-    for (;;) {
-        unsigned grp = 0;
-        if (lane == 0) grp = atomicAdd(next, 1u);
-        grp = __shfl_sync(FULL, grp, 0);
-        if (grp >= ngroups) break;
+    for (unsigned grp; (grp = next_group(o.ctr + 1, lane)) < ngroups;) {
         const unsigned a = grp * G + (unsigned)lane;
         const bool live = (unsigned)lane < G && a < nact;
         const uint4 e = live ? __ldg(act + a) : make_uint4(0u, 0u, 0u, 0u);
@@ -487,8 +474,9 @@ __global__ void __launch_bounds__(EW * 32) k_emit(P pol, const unsigned *__restr
         uint4 m = make_uint4(0u, 0u, 0u, 0u);
         unsigned mix = 0;
         if (live) {
-            pol.geo(e.x, g);
             m = __ldg(words + e.x);
+            if (P::CVERTS) S.amb[lane] = __ldg(o.amb + e.x);
+            pol.geo(e.x, g);
             const Corners q = load_corners(signs, e.x, g);
             mix = mixed_cubes(q, g);
             S.cor[0][lane] = q.a;
@@ -501,90 +489,137 @@ __global__ void __launch_bounds__(EW * 32) k_emit(P pol, const unsigned *__restr
         unsigned both;
         const unsigned ex = warp_excl((__popc(m.x) + __popc(m.y) + __popc(m.z)) | __popc(mix) << 16, lane, both);
         S.prev[lane] = ex & 0xffffu;
-        S.prec[lane] = ex >> 16;
+        S.pre[lane] = ex >> 16;
         const unsigned nv = both & 0xffffu, nc = both >> 16;
         unsigned tbase = __shfl_sync(FULL, e.y, 0);
-        __syncwarp();
-        // ---- vertices, one per lane
-        for (unsigned k0 = 0; k0 < nv; k0 += 32) {
-            const unsigned k = k0 + (unsigned)lane;
-            const int l = find_lane(S.prev, min(k, nv - 1));
-            const int r = (int)(min(k, nv - 1) - S.prev[l]);
-            const unsigned mx = __shfl_sync(FULL, m.x, l), my = __shfl_sync(FULL, m.y, l), mz = __shfl_sync(FULL, m.z, l),
-                           v0 = __shfl_sync(FULL, m.w, l);
-            const int x0 = __shfl_sync(FULL, g.x0, l), y = __shfl_sync(FULL, g.y, l), z = __shfl_sync(FULL, g.z, l),
-                      tag = __shfl_sync(FULL, g.tag, l);
-            int p = 0, cb = 0;   // the point holding the word's r-th vertex, vertices before it
-#pragma unroll
-            for (int s = 16; s; s >>= 1) {
-                const unsigned lt = (1u << (p + s)) - 1u;
-                const int c = __popc(mx & lt) + __popc(my & lt) + __popc(mz & lt);
-                if (c <= r) {
-                    p += s;
-                    cb = c;
-                }
-            }
-            const bool bx = mx >> p & 1u, by = my >> p & 1u;
-            const int j = r - cb, ax = j == 0 ? (bx ? 0 : (by ? 1 : 2)) : (j == 1 && bx && by ? 1 : 2);
-            if (k < nv) pol.vertex(x0 + p, y, z, ax, tag, (int)(v0 + (unsigned)r));
-        }
-        // ---- cubes, one per lane; their triangles go through the queue
-        unsigned fill = 0, ccount = 0;
-        auto emit = [&](unsigned k, bool ok) {
-            const unsigned t = ok ? S.tri[k] : 0u;
-            const int l = (int)(t >> 27);
-            const unsigned w = __shfl_sync(FULL, e.x, l);
-            const unsigned WX = P::MULTI ? __shfl_sync(FULL, g.WX, l) : g.WX, slice = P::MULTI ? __shfl_sync(FULL, g.slice, l) : g.slice;
-            if (!ok) return;
-            const unsigned b = t >> 22 & 31u;
-            const int off = (int)(t & 0x3fffffu);
-            int tv[3];
-#pragma unroll
-            for (int c = 0; c < 3; c++) {
-                const int code = pol.code(off + c);
-                if (code == 12) {
-                    tv[c] = S.cvert[k];
-                } else {
-                    const unsigned ec = edge_code(code), bb = b + (ec & 1u);
-                    tv[c] = vertex_id(words, w + (bb >> 5) + (ec & 2u ? WX : 0u) + (ec & 4u ? slice : 0u), bb & 31u, (int)(ec >> 3));
-                }
-            }
-            tris[tbase + k] = P::REVERSE ? vec3i{tv[2], tv[1], tv[0]} : vec3i{tv[0], tv[1], tv[2]};
-        };
         if (!P::MULTI) {   // lanes without a word take part in the queue too
             g.WX = __shfl_sync(FULL, g.WX, 0);
             g.slice = __shfl_sync(FULL, g.slice, 0);
         }
+        __syncwarp();
+        // ---- vertices, EV per lane with their values in flight together
+        constexpr int EV = P::EV;
+        for (unsigned k0 = 0; k0 < nv; k0 += 32 * EV) {
+            int x[EV], y[EV], z[EV], ax[EV], id[EV];
+            typename P::Edge v[EV];
+#pragma unroll
+            for (int u = 0; u < EV; u++) {
+                const unsigned k = min(k0 + 32 * u + (unsigned)lane, nv - 1);
+                const int l = find_lane(S.prev, k);
+                const int r = (int)(k - S.prev[l]);
+                const unsigned mx = __shfl_sync(FULL, m.x, l), my = __shfl_sync(FULL, m.y, l), mz = __shfl_sync(FULL, m.z, l),
+                               v0 = __shfl_sync(FULL, m.w, l);
+                x[u] = __shfl_sync(FULL, g.x0, l);
+                y[u] = __shfl_sync(FULL, g.y, l);
+                z[u] = __shfl_sync(FULL, g.z, l);
+                const int tag = P::MULTI ? __shfl_sync(FULL, g.tag, l) : 0;
+                int p = 0, cb = 0;   // the point holding the word's r-th vertex, vertices before it
+#pragma unroll
+                for (int s = 16; s; s >>= 1) {
+                    const unsigned lt = (1u << (p + s)) - 1u;
+                    const int c = __popc(mx & lt) + __popc(my & lt) + __popc(mz & lt);
+                    if (c <= r) {
+                        p += s;
+                        cb = c;
+                    }
+                }
+                const bool bx = mx >> p & 1u, by = my >> p & 1u;
+                const int j = r - cb;
+                ax[u] = j == 0 ? (bx ? 0 : (by ? 1 : 2)) : (j == 1 && bx && by ? 1 : 2);
+                x[u] += p;
+                id[u] = (int)(v0 + (unsigned)r);
+                v[u] = pol.edge(x[u], y[u], z[u], ax[u], tag);
+            }
+#pragma unroll
+            for (int u = 0; u < EV; u++) {
+                const unsigned n = min(32u, nv - min(nv, k0 + 32 * u));
+                vec3d q = {0., 0., 0.};
+                if ((unsigned)lane < n) q = pol.vertex(v[u], x[u], y[u], z[u], ax[u], id[u]);
+                const int id0 = __shfl_sync(FULL, id[u], 0);
+                if (__all_sync(FULL, (unsigned)lane >= n || id[u] == id0 + lane)) {   // consecutive: whole sectors
+                    double *st = (double *)S.tri, *out = (double *)(pol.pts + id0);
+                    __syncwarp();
+                    st[3 * lane] = q.x;
+                    st[3 * lane + 1] = q.y;
+                    st[3 * lane + 2] = q.z;
+                    __syncwarp();
+#pragma unroll
+                    for (int c = 0; c < 3; c++)
+                        if ((unsigned)(32 * c + lane) < 3 * n) out[32 * c + lane] = st[32 * c + lane];
+                } else if ((unsigned)lane < n) {
+                    pol.pts[id[u]] = q;
+                }
+            }
+        }
+        __syncwarp();   // the queue takes over the stage
+        // ---- cubes, one per lane; their triangles go through the queue
+        unsigned fill = 0, ccount = 0;
+        auto emit = [&](unsigned k, unsigned n) {   // queue entries k .. k + n - 1, n <= 32
+            const bool ok = (unsigned)lane < n;
+            const unsigned t = ok ? S.tri[k + lane] : 0u;
+            const int l = (int)(t >> 27);
+            const unsigned w = __shfl_sync(FULL, e.x, l);
+            const unsigned WX = P::MULTI ? __shfl_sync(FULL, g.WX, l) : g.WX, slice = P::MULTI ? __shfl_sync(FULL, g.slice, l) : g.slice;
+            if (ok) {
+                const unsigned b = t >> 22 & 31u;
+                const int off = (int)(t & 0x3fffffu);
+#pragma unroll
+                for (int c = 0; c < 3; c++) {
+                    const int code = pol.code(off + c);
+                    int v;
+                    if (P::CVERTS && code == 12) {
+                        v = S.cvert[k + lane];
+                    } else {
+                        const unsigned ec = edge_code(code), bb = b + (ec & 1u);
+                        v = vertex_id(words, w + (bb >> 5) + (ec & 2u ? WX : 0u) + (ec & 4u ? slice : 0u), bb & 31u, (int)(ec >> 3));
+                    }
+                    S.out[3 * lane + (P::REVERSE ? 2 - c : c)] = v;
+                }
+            }
+            __syncwarp();
+            int *out = (int *)(tris + tbase + k);   // whole sectors
+#pragma unroll
+            for (int c = 0; c < 3; c++)
+                if ((unsigned)(32 * c + lane) < 3 * n) out[32 * c + lane] = S.out[32 * c + lane];
+            __syncwarp();
+        };
         for (unsigned k0 = 0; k0 < nc; k0 += 32) {
-            const unsigned k = k0 + (unsigned)lane;
-            const bool ok = k < nc;
-            const int l = find_lane(S.prec, min(k, nc - 1));
-            const int r = (int)(min(k, nc - 1) - S.prec[l]);
+            const bool ok = k0 + (unsigned)lane < nc;
+            const unsigned k = min(k0 + (unsigned)lane, nc - 1);
+            const int l = find_lane(S.pre, k);
+            const int r = (int)(k - S.pre[l]);
             const int i = nth_bit(S.cor[5][l], r);
             const int lut = cube_index(S.cor[0][l], S.cor[1][l], S.cor[2][l], S.cor[3][l], S.cor[4][l], i);
             const unsigned q = qt[lut];
             CubeTiling T{(int)(q >> 8), ok ? (int)(q & 0xffu) : 0, false};
-            if (__any_sync(FULL, ok && T.n == (int)TESTS)) {
-                const int x0 = __shfl_sync(FULL, g.x0, l), y = __shfl_sync(FULL, g.y, l), z = __shfl_sync(FULL, g.z, l),
-                          tag = __shfl_sync(FULL, g.tag, l);
-                Geo gl{x0, y, z, 0u, 0u, 0u, 0u, false, false, false, tag};
-                if (ok && T.n == (int)TESTS) T = pol.tests(gl, x0 + i, y, z, lut);
-            }
             int v12 = -1;
-            const unsigned cvb = __ballot_sync(FULL, ok && T.cv);
-            if (P::CVERTS) {   // number the c-vertices within their words
-                const unsigned cex = ccount + __popc(cvb & ((1u << lane) - 1u));
-                if (ok && r == 0) S.first_c[l] = cex;
-                __syncwarp();
-                const unsigned c0 = __shfl_sync(FULL, e.z, l);
-                const int x0 = __shfl_sync(FULL, g.x0, l), y = __shfl_sync(FULL, g.y, l), z = __shfl_sync(FULL, g.z, l),
-                          tag = __shfl_sync(FULL, g.tag, l);
-                if (ok && T.cv) {
-                    v12 = (int)(c0 + cex - S.first_c[l]);
-                    Geo gl{x0, y, z, 0u, 0u, 0u, 0u, false, false, false, tag};
-                    pol.cvertex(gl, x0 + i, y, z, v12);
+            if (P::CVERTS) {
+                if (__any_sync(FULL, ok && T.n == (int)TESTS)) {
+                    const int x0 = __shfl_sync(FULL, g.x0, l), y = __shfl_sync(FULL, g.y, l), z = __shfl_sync(FULL, g.z, l),
+                              tag = __shfl_sync(FULL, g.tag, l);
+                    const unsigned c0 = __shfl_sync(FULL, e.z, l), w = __shfl_sync(FULL, e.x, l);
+                    const Geo gl{x0, y, z, 0u, 0u, 0u, 0u, false, false, false, tag};
+                    if (ok && T.n == (int)TESTS) {   // decided by k_amb
+                        const unsigned at = __ldg(o.ambat + w);
+                        if (at != NO_TILING) {
+                            const unsigned t = __ldg(o.tilings + at + __popc(S.amb[l] & ((1u << i) - 1u)));
+                            T = CubeTiling{(int)(t & 0x3fffffu), (int)(t >> 22 & 15u), (t >> 26 & 1u) != 0u};
+                        } else {
+                            T = pol.tests(gl, x0 + i, y, z, lut);
+                        }
+                    }
+                    // number the c-vertices within their words
+                    const unsigned cvb = __ballot_sync(FULL, ok && T.cv), cex = ccount + __popc(cvb & ((1u << lane) - 1u));
+                    if (ok && r == 0) S.first_c[l] = cex;
+                    __syncwarp();
+                    if (ok && T.cv) {
+                        v12 = (int)(c0 + cex - S.first_c[l]);
+                        pol.cvertex(gl, x0 + i, y, z, v12);
+                    }
+                    ccount += __popc(cvb);
+                } else if (ok && r == 0) {
+                    S.first_c[l] = ccount;
                 }
-                ccount += __popc(cvb);
             }
             unsigned made;
             const unsigned at = fill + warp_excl((unsigned)T.n, lane, made);
@@ -595,7 +630,7 @@ __global__ void __launch_bounds__(EW * 32) k_emit(P pol, const unsigned *__restr
             fill += made;
             __syncwarp();
             unsigned head = 0;
-            for (; fill - head >= 32; head += 32) emit(head + (unsigned)lane, true);
+            for (; fill - head >= 32; head += 32) emit(head, 32u);
             if (head) {   // the rest to the front
                 __syncwarp();
                 const unsigned rest = fill - head;
@@ -609,37 +644,30 @@ __global__ void __launch_bounds__(EW * 32) k_emit(P pol, const unsigned *__restr
                 __syncwarp();
             }
         }
-        if (fill) emit((unsigned)lane, (unsigned)lane < fill);
+        if (fill) emit(0u, fill);
         __syncwarp();   // the lists are reused by the next group
     }
 }
 
 // ---- host side ----------------------------------------------------------------------
-// Sub-tiles per tile: about 16 tiles per SM, so that the last block's scan stays short.
-inline unsigned subs_per_tile(size_t nsub) { return (unsigned)std::max<size_t>(1, (nsub + 152 * 16 - 1) / (152 * 16)); }
-
 // buffers of a grid of nwords sign words
 inline n2m_status prepare(McWork &w, size_t nwords, uint4 *d_total, Out &o) {
-    const size_t nsub = (nwords + SUB - 1) / SUB;
+    const size_t nsub = (nwords + SUB - 1) / SUB, tiles = (nsub + TILE - 1) / TILE;
     o.nwords = (unsigned)nwords;
     o.nsub = (unsigned)nsub;
-    o.per = subs_per_tile(nsub);
-    const size_t tiles = (nsub + o.per - 1) / o.per;
     CKS(w.words.ensure(nwords * sizeof(uint4)));
     CKS(w.act.ensure(nwords * sizeof(uint4)));
-    CKS(w.cnt.ensure(3 * nwords * sizeof(unsigned)));
-    CKS(w.staged.ensure(nsub * SUB));
-    CKS(w.sub.ensure(2 * (nsub + tiles) * sizeof(uint2) + 4 * sizeof(unsigned)));
+    CKS(w.cnt.ensure(4 * nwords * sizeof(unsigned)));
+    CKS(w.sub.ensure((2 * nsub + tiles) * sizeof(uint4) + 4 * sizeof(unsigned)));
     o.words = w.words.as<uint4>();
     o.cnt = w.cnt.as<unsigned>();
     o.amb = o.cnt + nwords;
-    o.amblist = o.amb + nwords;
-    o.staged = w.staged.as<unsigned char>();
-    o.sub = w.sub.as<uint2>();
-    o.subt = o.sub + nsub;
-    o.part = o.subt + nsub;
-    o.partt = o.part + tiles;
-    o.ctr = (unsigned *)(o.partt + tiles);
+    o.ambat = o.amb + nwords;
+    o.tilings = o.ambat + nwords;
+    o.sub = w.sub.as<uint4>();
+    o.pre = o.sub + nsub;
+    o.part = o.pre + nsub;
+    o.ctr = (unsigned *)(o.part + tiles);
     o.total = d_total;
     return N2M_OK;
 }
@@ -648,45 +676,46 @@ inline n2m_status prepare(McWork &w, size_t nwords, uint4 *d_total, Out &o) {
 template <class P>
 n2m_status count_signs(const P &pol, const unsigned *signs, const Out &o, const Marks &marks, cudaStream_t s) {
     CK(cudaMemsetAsync(o.ctr, 0, 4 * sizeof(unsigned), s));
-    { k_words<P><<<(o.nsub + o.per - 1) / o.per, SUB, 0, s>>>(pol, signs, o, marks); N2M_COUNT(); }
+    { k_words<P><<<std::max(1u, std::min((o.nsub + 7) / 8, 152u * 32u)), 256, 0, s>>>(pol, signs, o, marks); N2M_COUNT(); }
     CKL();
     return N2M_OK;
 }
 // the rest: values are final
 template <class P>
 n2m_status count_values(const P &pol, const unsigned *signs, McWork &w, const Out &o, bool tests, cudaStream_t s) {
-    if (tests) {
-        const unsigned b = std::max(1u, std::min((o.nwords / 32 + 127) / 128, 152u * 8u));   // 1 word in 32 fills it
-        k_amb<P><<<b, 128, 0, s>>>(pol, signs, o);
-        N2M_COUNT();
-    }
-    { k_sum<P><<<(o.nsub + o.per - 1) / o.per, SUB, 0, s>>>(o); N2M_COUNT(); }
-    { k_finish<P><<<std::max(1u, std::min((o.nsub + 7) / 8, 152u * 8u)), 256, 0, s>>>(pol, o, w.act.as<uint4>()); N2M_COUNT(); }
+    if (tests) { k_amb<P><<<(o.nsub + AMB_S - 1) / AMB_S, AMB_T, 0, s>>>(pol, signs, o); N2M_COUNT(); }
+    { k_sum<P><<<(o.nsub + TILE - 1) / TILE, TILE, 0, s>>>(o); N2M_COUNT(); }
+    { k_finish<P><<<std::max(1u, std::min((o.nsub + 8 * FIN - 1) / (8 * FIN), 152u * 16u)), 256, 0, s>>>(pol, o, w.act.as<uint4>()); N2M_COUNT(); }
     CKL();
+    return N2M_OK;
+}
+
+// CTAs of a kernel that fit the GPU at once, kept per device ordinal
+inline n2m_status resident_ctas(const void *fn, std::atomic<int> (&of)[64], int &n) {
+    int dev = 0;
+    CK(cudaGetDevice(&dev));
+    n = dev < 64 ? of[dev].load(std::memory_order_relaxed) : 0;
+    if (!n) {
+        int sms = 0, per_sm = 0;
+        CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, EW * 32, 0));
+        n = sms * std::max(per_sm, 1);
+        if (dev < 64) of[dev].store(n, std::memory_order_relaxed);
+    }
     return N2M_OK;
 }
 
 template <class P>
 n2m_status emit(const P &pol, const unsigned *signs, McWork &w, const Out &o, unsigned nact, vec3i *d_tris, cudaStream_t s) {
-    // CTAs that fit the GPU at once, per device ordinal (work comes from an atomic counter, so any grid is correct)
-    static std::atomic<int> resident_of[64];
-    int dev = 0;
-    CK(cudaGetDevice(&dev));
-    int resident = dev < 64 ? resident_of[dev].load(std::memory_order_relaxed) : 0;
-    if (!resident) {
-        int sms = 0, per_sm = 0;
-        CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_emit<P>, EW * 32, 0));
-        resident = sms * std::max(per_sm, 1);
-        if (dev < 64) resident_of[dev].store(resident, std::memory_order_relaxed);
-    }
+    static std::atomic<int> resident[64];   // work comes from an atomic counter, so any grid is correct
+    int n = 0;
+    CKS(resident_ctas((const void *)k_emit<P>, resident, n));
     // 32 words per group keep the per-group work small; below two groups per resident warp smaller groups
     // spread the mesh over the GPU instead (8 words still fill the lanes: a word has about 7 vertices)
-    const unsigned warps = (unsigned)resident * EW;
+    const unsigned warps = (unsigned)n * EW;
     const unsigned G = nact >= 64u * warps ? 32u : (nact >= 16u * warps ? 16u : 8u);
-    const unsigned groups = (nact + G - 1) / G;
-    const unsigned blocks = std::min<unsigned>((groups + EW - 1) / EW, (unsigned)resident);
-    { k_emit<P><<<blocks, EW * 32, 0, s>>>(pol, signs, o.words, w.act.as<uint4>(), nact, G, d_tris, o.ctr + 3); N2M_COUNT(); }
+    const unsigned blocks = std::min(((nact + G - 1) / G + EW - 1) / EW, (unsigned)n);
+    { k_emit<P><<<blocks, EW * 32, 0, s>>>(pol, signs, o, w.act.as<uint4>(), nact, G, d_tris); N2M_COUNT(); }
     CKL();
     return N2M_OK;
 }

@@ -235,7 +235,7 @@ struct McWork {
     DevBuf signs;            // sign words of the grid
     DevBuf words;            // per active word {x, y, z crossing masks, vertex offset}
     DevBuf act;              // active words in order {word, triangle offset, c-vertex offset, -}
-    DevBuf cnt, staged, sub; // counting scratch (mcwords.cuh: Out)
+    DevBuf cnt, sub;         // counting scratch (mcwords.cuh: Out)
 };
 struct McCounts {
     unsigned nv_edge, nt, nc, nactive;

@@ -118,56 +118,58 @@ __device__ __forceinline__ void ogeo(const OV &g, unsigned w, mcw::Geo &q) {
 }
 
 // ---- emit pass -------------------------------------------------------------------
-// VertexInterp (src/oldcubes.c:22-40) along one axis: p = p1 + mu*(p2-p1)
-// with mu = (iso - v1)/(v2 - v1); only the coordinate along the edge moves.
-__device__ __forceinline__ double interp(double iso, double p1, double p2, double v1, double v2) {
-    const double mu = __ddiv_rn(__dsub_rn(iso, v1), __dsub_rn(v2, v1));
-    return __dadd_rn(p1, __dmul_rn(mu, __dsub_rn(p2, p1)));
+// exact float -> double and int -> double by assembling the bits: conversions issue on the pipe that this part
+// shares with FP64, which bounds the interpolation below
+__device__ __forceinline__ double f2d(float f) {
+    const unsigned u = __float_as_uint(f), e = (u >> 23) & 0xffu;
+    if (e - 1u < 0xfeu)   // normal
+        return __hiloint2double((int)((u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + 0x38000000u)), (int)(u << 29));
+    return (double)f;
+}
+__device__ __forceinline__ double i2d(int v) {   // v >= 0
+    if (v == 0) return 0.0;
+    const int p = 31 - __clz(v);
+    const unsigned long long m = (unsigned long long)(unsigned)v << (52 - p);
+    return __longlong_as_double((long long)(((unsigned long long)(p + 1023) << 52) + (m & 0xfffffffffffffull)));
 }
 
 // The edge vertex of grid point (x, y, z) along axis ax, interpolated as the
-// last cube (raster order) that lists the edge orients it; a position within
-// 1.5e-5 of a grid coordinate makes the vertex a weld candidate.
-__device__ __forceinline__ void oc_vertex(const OV &g, int x, int y, int z, int ax, int id, vec3d *pts, int *cand,
-                                          unsigned *ncand, int cap) {
+// last cube (raster order) that lists the edge orients it.  VertexInterp
+// (src/oldcubes.c:22-40) moves only the coordinate along the edge:
+// p = p1 + mu*(p2-p1) with mu = (iso - v1)/(v2 - v1), and p2 - p1 is 1 or -1, so the
+// product is mu or -mu.  A vertex near a grid point becomes a weld candidate (a wider
+// float test spares the others the double one).
+__device__ __forceinline__ vec3d oc_vertex(const OV &g, float v0, float v1, int x, int y, int z, int ax, int id, int *cand,
+                                           unsigned *ncand, int cap) {
     const int X = g.lo0 + x, Y = g.lo1 + y, Z = g.lo2 + z;
-    const double iso = (double)g.iso, dX = X, dY = Y, dZ = Z;
-    const double v0 = oval(g, X, Y, Z);
     const int c0 = g.lo0, c1 = g.lo1, c2 = g.lo2, e0 = g.hi0 - 2, e1 = g.hi1 - 2, e2 = g.hi2 - 2;
-    double r;
-    vec3d P;
-    if (ax == 0) {   // last user: (X,Y,Z) fwd > (X,Y-1,Z) rev > (X,Y,Z-1) fwd > (X,Y-1,Z-1) rev
-        const double v1 = oval(g, X + 1, Y, Z);
-        bool fwd;
+    bool fwd = true;   // z: every user lists the edge bottom to top
+    if (ax == 0) {     // last user: (X,Y,Z) fwd > (X,Y-1,Z) rev > (X,Y,Z-1) fwd > (X,Y-1,Z-1) rev
         if (Y <= e1 && Z <= e2) fwd = true;
         else if (Y - 1 >= c1 && Z <= e2) fwd = false;
-        else if (Y <= e1 && Z - 1 >= c2) fwd = true;
-        else fwd = false;
-        r = fwd ? interp(iso, dX, dX + 1.0, v0, v1) : interp(iso, dX + 1.0, dX, v1, v0);
-        P = {r, dY, dZ};
+        else fwd = Y <= e1 && Z - 1 >= c2;
     } else if (ax == 1) {   // (X,Y,Z) rev > (X-1,Y,Z) fwd > (X,Y,Z-1) rev > (X-1,Y,Z-1) fwd
-        const double v3 = oval(g, X, Y + 1, Z);
-        bool fwd;
         if (X <= e0 && Z <= e2) fwd = false;
         else if (X - 1 >= c0 && Z <= e2) fwd = true;
-        else if (X <= e0 && Z - 1 >= c2) fwd = false;
-        else fwd = true;
-        r = fwd ? interp(iso, dY, dY + 1.0, v0, v3) : interp(iso, dY + 1.0, dY, v3, v0);
-        P = {dX, r, dZ};
-    } else {   // every user lists the z edge bottom to top
-        r = interp(iso, dZ, dZ + 1.0, v0, (double)oval(g, X, Y, Z + 1));
-        P = {dX, dY, r};
+        else fwd = !(X <= e0 && Z - 1 >= c2);
     }
-    pts[id] = P;
-    if (fabs(r - rint(r)) < 1.5e-5) {
+    const int i0 = ax == 0 ? X : (ax == 1 ? Y : Z);
+    const float va = fwd ? v0 : v1, vb = fwd ? v1 : v0;
+    const double iso = f2d(g.iso), da = f2d(va), db = f2d(vb);
+    const double mu = __ddiv_rn(__dsub_rn(iso, da), __dsub_rn(db, da));
+    const double r = __dadd_rn(i2d(fwd ? i0 : i0 + 1), fwd ? mu : -mu);
+    const float mf = __fdividef(__fsub_rn(g.iso, va), __fsub_rn(vb, va));   // within 1e-6 of mu, or 0, Inf or NaN
+    if (!(mf > 2e-5f && mf < 1.f - 2e-5f) && fabs(r - rint(r)) < 1.5e-5) {
         const unsigned k = atomicAdd(ncand, 1u);
         if (k < (unsigned)cap) cand[k] = id;
     }
+    return {ax == 0 ? r : i2d(X), ax == 1 ? r : i2d(Y), ax == 2 ? r : i2d(Z)};
 }
 
 // mcwords.cuh's policy for the unpadded classic grid
 struct Policy {
     static constexpr bool MULTI = false, REVERSE = false, CVERTS = false;
+    static constexpr int CTAS = 8, EV = 2;   // of k_emit: CTAs per SM, vertices per lane in flight
     OV g;
     vec3d *pts;
     int *cand;
@@ -187,8 +189,15 @@ struct Policy {
     __device__ __forceinline__ void shifts(const mcw::Out &, unsigned, const uint4 &, unsigned &e, unsigned &c) const { e = c = 0; }
     __device__ __forceinline__ mcw::CubeTiling tests(const mcw::Geo &, int, int, int, int) const { return {0, 0, false}; }
     __device__ __forceinline__ void cvertex(const mcw::Geo &, int, int, int, int) const {}
-    __device__ __forceinline__ void vertex(int x, int y, int z, int ax, int, int id) const {
-        oc_vertex(g, x, y, z, ax, id, pts, cand, ncand, cap);
+    struct Edge {
+        float v0, v1;
+    };
+    __device__ __forceinline__ Edge edge(int x, int y, int z, int ax, int) const {
+        const int X = g.lo0 + x, Y = g.lo1 + y, Z = g.lo2 + z;
+        return Edge{oval(g, X, Y, Z), oval(g, X + (ax == 0), Y + (ax == 1), Z + (ax == 2))};
+    }
+    __device__ __forceinline__ vec3d vertex(const Edge &v, int x, int y, int z, int ax, int id) const {
+        return oc_vertex(g, v.v0, v.v1, x, y, z, ax, id, cand, ncand, cap);
     }
 };
 

@@ -953,14 +953,16 @@ __global__ void __launch_bounds__(256) k_od_resolve(const float *__restrict__ in
 }
 
 // ---- marks -> the exact passes on marked voxels ----------------------------------
-// The marked voxels (whose z outputs are wanted), the voxels whose y values those need
-// (+-2 slices) and the voxels whose x values those need (+-2 rows), each as a list of
-// voxel indices.  A block takes OL_T words of a slice of the row-aligned mark bitmap:
-// the y marks of its words and of two rows either way go to shared memory (five slices
-// OR-ed), the x marks are five of those; one atomic per list and block reserves the
-// room (the lists' order is free), and a warp writes a word's indices with one store.
-// 512^3: 96 us; two dilations, a scan over every word and a scatter took 180 us.
-constexpr int OL_T = 256, OL_MAXW = 128;   // rows of more than OL_MAXW words read their halo from global memory
+// The words of marked voxels (whose z outputs are wanted), of the voxels whose y values
+// those need (+-2 slices) and of the voxels whose x values those need (+-2 rows), each
+// as a list of {voxel of bit 0, bits}.  A block takes OL_T words of OL_Z slices of the
+// row-aligned mark bitmap: the y marks of its words and of two rows either way go to
+// shared memory (a window of five slices slides along z: one load per word and slice
+// and four more per run), the x marks are five of those; one atomic per list and block
+// reserves the room (the lists' order is free).
+// 512^3: 24 us; listing voxels instead of words took 81 us and 250 MB of list traffic,
+// two dilations, a scan over every word and a scatter 180 us.
+constexpr int OL_T = 256, OL_Z = 8, OL_MAXW = 64;   // rows of more than OL_MAXW words read their halo from global memory
 
 __device__ __forceinline__ unsigned y_marks(const unsigned *__restrict__ need, unsigned i, unsigned slice, int z, int nz) {
     unsigned m = 0;
@@ -971,127 +973,176 @@ __device__ __forceinline__ unsigned y_marks(const unsigned *__restrict__ need, u
 }
 
 __global__ void __launch_bounds__(OL_T) k_od_lists(const unsigned *__restrict__ need, int nx, int nz, unsigned W, unsigned slice,
-                                                   unsigned *cnt, unsigned *lz, unsigned *ly, unsigned *lx) {
-    __shared__ unsigned ym[OL_T + 4 * OL_MAXW];
-    __shared__ uint4 wsum[OL_T / 32];
-    __shared__ unsigned base[3];
+                                                   unsigned *cnt, uint2 *lz, uint2 *ly, uint2 *lx) {
+    __shared__ unsigned ym[OL_Z][OL_T + 4 * OL_MAXW];
+    __shared__ unsigned wsum[3][OL_T / 32], base[3];
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const unsigned bps = (slice + OL_T - 1) / OL_T;   // blocks per slice
-    const int z = (int)(blockIdx.x / bps);
-    const unsigned i0 = (blockIdx.x - (unsigned)z * bps) * OL_T, i = i0 + (unsigned)tid;
+    const int z0 = (int)(blockIdx.x / bps) * OL_Z;
+    const unsigned i0 = blockIdx.x % bps * OL_T, i = i0 + (unsigned)tid;
     const bool in = i < slice;
-    unsigned my, mx = 0u;
+    unsigned mx[OL_Z], my[OL_Z], mz[OL_Z], any = 0u;
     if (W <= (unsigned)OL_MAXW) {
         const int h = 2 * (int)W;   // halo words either side
         for (int k = tid; k < OL_T + 2 * h; k += OL_T) {
             const long long q = (long long)i0 + k - h;
-            ym[k] = q >= 0 && q < (long long)slice ? y_marks(need, (unsigned)q, slice, z, nz) : 0u;
-        }
-        __syncthreads();
-        my = ym[tid + h];
+            unsigned v[OL_Z + 4];
 #pragma unroll
-        for (int d = 0; d <= 4; d++) mx |= ym[tid + d * (int)W];
+            for (int d = 0; d < OL_Z + 4; d++) {
+                const int z = z0 - 2 + d;
+                v[d] = q >= 0 && q < (long long)slice && z >= 0 && z < nz ? __ldg(need + (size_t)z * slice + (size_t)q) : 0u;
+            }
+#pragma unroll
+            for (int d = 0; d < OL_Z; d++) {
+                ym[d][k] = z0 + d < nz ? v[d] | v[d + 1] | v[d + 2] | v[d + 3] | v[d + 4] : 0u;
+                any |= ym[d][k];
+            }
+        }
+        if (!__syncthreads_or(any != 0u)) return;
+#pragma unroll
+        for (int d = 0; d < OL_Z; d++) {
+            my[d] = in ? ym[d][tid + h] : 0u;
+            mx[d] = 0u;
+#pragma unroll
+            for (int e = 0; e <= 4; e++) mx[d] |= ym[d][tid + e * (int)W];
+            if (!in) mx[d] = 0u;
+        }
     } else {
-        my = in ? y_marks(need, i, slice, z, nz) : 0u;
 #pragma unroll
-        for (int d = -2; d <= 2; d++) {
-            const long long q = (long long)i + (long long)d * W;
-            if (in && q >= 0 && q < (long long)slice) mx |= d ? y_marks(need, (unsigned)q, slice, z, nz) : my;
+        for (int d = 0; d < OL_Z; d++) {
+            my[d] = in && z0 + d < nz ? y_marks(need, i, slice, z0 + d, nz) : 0u;
+            mx[d] = my[d];
+            for (int e = -2; e <= 2; e++) {
+                const long long q = (long long)i + (long long)e * W;
+                if (e && in && z0 + d < nz && q >= 0 && q < (long long)slice) mx[d] |= y_marks(need, (unsigned)q, slice, z0 + d, nz);
+            }
+            any |= mx[d];
         }
+        if (!__syncthreads_or(any != 0u)) return;
     }
-    if (!in) my = mx = 0u;
-    const unsigned mz = my && in ? __ldg(need + (size_t)z * slice + i) : 0u;
-    if (!__syncthreads_or(mx != 0u)) return;   // every y or z mark is an x mark too
-    const unsigned cz = __popc(mz), cy = __popc(my), cx = __popc(mx);
-    unsigned a = cz | cy << 16, c = cx;   // a block's sums are at most 8192
+    unsigned c[3] = {0u, 0u, 0u};   // this warp's words in each list
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const unsigned ta = __shfl_up_sync(FULL, a, o), tc = __shfl_up_sync(FULL, c, o);
-        if (lane >= o) {
-            a += ta;
-            c += tc;
-        }
+    for (int d = 0; d < OL_Z; d++) {
+        mz[d] = my[d] ? __ldg(need + (size_t)(z0 + d) * slice + i) : 0u;
+        c[0] += __popc(__ballot_sync(FULL, mz[d] != 0u));
+        c[1] += __popc(__ballot_sync(FULL, my[d] != 0u));
+        c[2] += __popc(__ballot_sync(FULL, mx[d] != 0u));
     }
-    if (lane == 31) wsum[wid] = make_uint4(a & 0xffffu, a >> 16, c, 0u);
+    if (lane == 0)
+        for (int l = 0; l < 3; l++) wsum[l][wid] = c[l];
     __syncthreads();
     if (tid < 3) {
         unsigned t = 0;
-        for (int k = 0; k < OL_T / 32; k++) t += tid == 0 ? wsum[k].x : (tid == 1 ? wsum[k].y : wsum[k].z);
+        for (int k = 0; k < OL_T / 32; k++) t += wsum[tid][k];
         base[tid] = t ? atomicAdd(cnt + tid, t) : 0u;
     }
     __syncthreads();
-    unsigned oz = base[0] + (a & 0xffffu) - cz, oy = base[1] + (a >> 16) - cy, ox = base[2] + c - cx;
-    for (int k = 0; k < wid; k++) {
-        oz += wsum[k].x;
-        oy += wsum[k].y;
-        ox += wsum[k].z;
+    unsigned at[3];
+#pragma unroll
+    for (int l = 0; l < 3; l++) {
+        at[l] = base[l];
+        for (int k = 0; k < wid; k++) at[l] += wsum[l][k];
     }
-    const unsigned row = i / W, v0 = ((unsigned)z * (slice / W) + row) * (unsigned)nx + (i - row * W) * 32u;
-    auto write = [&](unsigned m, unsigned o, unsigned v, unsigned *list) {
-        if (m >> lane & 1u) list[o + __popc(m & ((1u << lane) - 1u))] = v + (unsigned)lane;
+    const unsigned ny = slice / W, row = i / W, lt = (1u << lane) - 1u;
+    unsigned v0 = ((unsigned)z0 * ny + row) * (unsigned)nx + (i - row * W) * 32u;
+    auto write = [&](unsigned m, unsigned &o, uint2 *list) {
+        const unsigned b = __ballot_sync(FULL, m != 0u);
+        if (m) list[o + __popc(b & lt)] = make_uint2(v0, m);
+        o += __popc(b);
     };
-    for (unsigned busy = __ballot_sync(FULL, mx != 0u); busy; busy &= busy - 1u) {
-        const int k = __ffs(busy) - 1;
-        const unsigned v = __shfl_sync(FULL, v0, k);
-        write(__shfl_sync(FULL, mz, k), __shfl_sync(FULL, oz, k), v, lz);
-        write(__shfl_sync(FULL, my, k), __shfl_sync(FULL, oy, k), v, ly);
-        write(__shfl_sync(FULL, mx, k), __shfl_sync(FULL, ox, k), v, lx);
+#pragma unroll
+    for (int d = 0; d < OL_Z; d++) {
+        write(mz[d], at[0], lz);
+        write(my[d], at[1], ly);
+        write(mx[d], at[2], lx);
+        v0 += ny * (unsigned)nx;
     }
 }
 
 // one exact pass on the listed voxels: dst[v] = tap sum of src along the axis
-// (stride 1, nx or nx*ny; coordinate along the axis = (v / div) % len), or
-// src[v] on the two face layers; one thread per voxel, OE_U list entries per
-// thread in flight at once (a warp takes OE_U runs of 32 consecutive entries),
-// undecided taps queued per warp for the FP64 fix-up
-constexpr int OE_U = 4;
-__global__ void __launch_bounds__(256) k_od_exact(const unsigned *__restrict__ list, const unsigned *__restrict__ cnt,
-                                                  const float *__restrict__ src, float *dst, unsigned stride,
-                                                  unsigned div, unsigned len, unsigned long long mdiv,
-                                                  unsigned long long mlen) {
-    __shared__ unsigned stage_buf[8][32 * (OE_U + 1)];   // < 32 between drains, + 32 per entry
+// (AXIS 0, 1, 2: x, y, z), or src[v] on the two face layers.  A warp takes 32 listed
+// words, writes their voxels as a dense list in shared memory and works through it,
+// OE_U voxels per lane in flight at once; undecided taps queued per warp for the
+// FP64 fix-up.  Bound by the gathers' latency and instruction issue: the x, y and z passes
+// of the 512^3 CT volume take 92, 91 and 70 us.
+constexpr int OE_U = 4, OE_T = 128;
+template <int AXIS>
+__global__ void __launch_bounds__(OE_T, 10) k_od_exact(const uint2 *__restrict__ list, const unsigned *__restrict__ cnt,
+                                                   const float *__restrict__ src, float *dst, unsigned nx, unsigned ny, unsigned nz,
+                                                   unsigned long long mnx, unsigned long long mny) {
+    __shared__ unsigned stage_buf[OE_T / 32][32 * (OE_U + 1)];   // < 32 between drains, + 32 per entry
+    __shared__ unsigned short item[OE_T / 32][32 * 32];          // word << 5 | bit
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     FixStage<false> F{stage_buf[wid], 0};
     Acc acc;   // unused
+    const unsigned stride = AXIS == 0 ? 1u : (AXIS == 1 ? nx : nx * ny);
     const Pass P{src, dst, stride, 0, 0, 0u, 0.f, nullptr};
-    const unsigned n = *cnt;
-    const unsigned nwarps = gridDim.x * (blockDim.x >> 5), gw = blockIdx.x * (blockDim.x >> 5) + (unsigned)wid;
-    for (unsigned i0 = gw * 32u * OE_U; i0 < n; i0 += nwarps * 32u * OE_U) {   // warp-uniform
-        unsigned v[OE_U];
-        bool act[OE_U], inner[OE_U];
-        float a[OE_U][5];
+    const unsigned n = *cnt, warps = gridDim.x * OE_T / 32u;
+    // words of a warp at a time: fewer when the list is too short to give every warp 32
+    const unsigned per = n >= 64u * warps ? 32u : (n >= 16u * warps ? 16u : (n >= 4u * warps ? 8u : 4u));
+    for (unsigned i0 = ((blockIdx.x * OE_T + threadIdx.x) >> 5) * per; i0 < n; i0 += warps * per) {   // warp-uniform
+        const uint2 e = (unsigned)lane < per && i0 + (unsigned)lane < n ? __ldg(list + i0 + lane) : make_uint2(0u, 0u);
+        // x of bit 0, or whether the word's row (slice) is two rows (slices) away from the faces
+        const unsigned row = nx == 1u ? e.x : (unsigned)__umul64hi(e.x, mnx);   // e.x / nx
+        const unsigned sl = ny == 1u ? row : (unsigned)__umul64hi(row, mny);    // row / ny
+        const unsigned c0 = AXIS == 0 ? e.x - row * nx : (AXIS == 1 ? row - sl * ny : sl);
+        const unsigned len = AXIS == 0 ? nx : (AXIS == 1 ? ny : nz);
+        const bool winner = c0 >= 2u && c0 + 2u < len;
+        unsigned total;
+        {
+            unsigned incl = __popc(e.y);
 #pragma unroll
-        for (int u = 0; u < OE_U; u++) {
-            const unsigned i = i0 + (unsigned)u * 32u + (unsigned)lane;
-            act[u] = i < n;
-            v[u] = act[u] ? __ldg(list + i) : 0u;
-        }
-#pragma unroll
-        for (int u = 0; u < OE_U; u++) {
-            const unsigned q = div == 1u ? v[u] : (unsigned)__umul64hi(v[u], mdiv);   // v / div
-            const unsigned c = q - (unsigned)__umul64hi(q, mlen) * len;               // q % len
-            inner[u] = act[u] && c >= 2u && c + 2u < len;
-            const float *p = src + v[u];
-            if (inner[u]) {
-                a[u][0] = __ldg(p - 2 * (size_t)stride);
-                a[u][1] = __ldg(p - (size_t)stride);
-                a[u][3] = __ldg(p + stride);
-                a[u][4] = __ldg(p + 2 * (size_t)stride);
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned t = __shfl_up_sync(FULL, incl, o);
+                if (lane >= o) incl += t;
             }
-            a[u][2] = act[u] ? __ldg(p) : 0.f;
+            total = __shfl_sync(FULL, incl, 31);
+            unsigned at = incl - __popc(e.y);
+            for (unsigned m = e.y; m; m &= m - 1u) item[wid][at++] = (unsigned short)(lane << 5 | (__ffs(m) - 1));
         }
+        __syncwarp();
+        for (unsigned k0 = 0; k0 < total; k0 += 32u * OE_U) {
+            unsigned v[OE_U];
+            bool act[OE_U], inner[OE_U];
+            float a[OE_U][5];
 #pragma unroll
-        for (int u = 0; u < OE_U; u++) {
-            bool fail = false;
-            if (act[u]) {
-                float r = a[u][2];
-                if (inner[u] && !tap5_split_window(a[u][0], a[u][1], a[u][2], a[u][3], a[u][4], &r))
-                    fail = !tap5_fast(a[u][0], a[u][1], a[u][2], a[u][3], a[u][4], &r);
-                if (!fail) dst[v[u]] = r;
+            for (int u = 0; u < OE_U; u++) {
+                const unsigned k = k0 + (unsigned)u * 32u + (unsigned)lane;
+                act[u] = k < total;
+                const unsigned it = act[u] ? item[wid][k] : 0u, b = it & 31u;
+                v[u] = __shfl_sync(FULL, e.x, (int)(it >> 5)) + b;
+                if (AXIS == 0) {
+                    const unsigned x = __shfl_sync(FULL, c0, (int)(it >> 5)) + b;
+                    inner[u] = act[u] && x >= 2u && x + 2u < len;
+                } else {
+                    inner[u] = __shfl_sync(FULL, winner, (int)(it >> 5)) && act[u];
+                }
+                const float *p = src + v[u];
+                if (inner[u]) {
+                    a[u][0] = __ldg(p - 2 * (size_t)stride);
+                    a[u][1] = __ldg(p - (size_t)stride);
+                    a[u][3] = __ldg(p + stride);
+                    a[u][4] = __ldg(p + 2 * (size_t)stride);
+                }
+                a[u][2] = act[u] ? __ldg(p) : 0.f;
             }
-            F.push(fail, v[u], lane);
+#pragma unroll
+            for (int u = 0; u < OE_U; u++) {
+                bool fail = false;
+                if (act[u]) {
+                    float r = a[u][2];
+                    // undecided by the split: nearly always an exact tie, which tap5_fast cannot decide either
+                    if (inner[u]) {
+                        const int q = tap5_split_state(a[u][0], a[u][1], a[u][2], a[u][3], a[u][4], &r);
+                        fail = q < 0 ? !tap5_fast(a[u][0], a[u][1], a[u][2], a[u][3], a[u][4], &r) : q == 0;
+                    }
+                    if (!fail) dst[v[u]] = r;
+                }
+                F.push(fail, v[u], lane);
+            }
+            F.drain(P, acc, lane);
         }
-        F.drain(P, acc, lane);
+        __syncwarp();   // the item list is reused
     }
     F.finish(P, acc, lane);
 }
@@ -1101,14 +1152,17 @@ __global__ void __launch_bounds__(256) k_od_exact(const unsigned *__restrict__ l
 // with largest, voxels neither kept nor in the kept set's dilation (the
 // 26-neighbourhood without (-1,-1,-1), interior voxels; src/meshify.c:218-264)
 // are the minimum.
-__global__ void k_od_post(const unsigned *__restrict__ list, const unsigned *__restrict__ cnt, float *out, LabelPost L,
-                          int nx, int ny, int nz) {
+__global__ void __launch_bounds__(256) k_od_post(const uint2 *__restrict__ list, const unsigned *__restrict__ cnt, float *out,
+                                                 LabelPost L, int nx, int ny, int nz) {
     const unsigned n = *cnt;
+    const int lane = threadIdx.x & 31;
     auto bit = [&](int x, int y, int z) -> unsigned {
         return (__ldg(L.K + ((size_t)z * ny + y) * L.W + ((unsigned)x >> 5)) >> (x & 31)) & 1u;
     };
-    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const unsigned j = list[i], x = j % (unsigned)nx, r = j / (unsigned)nx, y = r % (unsigned)ny, z = r / (unsigned)ny;
+    for (unsigned i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += (gridDim.x * blockDim.x) >> 5) {   // a warp per word
+        const uint2 e = list[i];
+        if (!(e.y >> lane & 1u)) continue;
+        const unsigned j = e.x + (unsigned)lane, x = j % (unsigned)nx, r = j / (unsigned)nx, y = r % (unsigned)ny, z = r / (unsigned)ny;
         if (bit(x, y, z)) {
             if (L.fill) out[j] = fmaxf(out[j], L.iso);
             continue;
@@ -1250,23 +1304,22 @@ n2m_status od_marks(OdWork &w, const int dim[3], unsigned **need, cudaStream_t s
 n2m_status od_repair(const OdRepair &r, cudaStream_t s) {
     OdWork &w = *r.w;
     const int nx = r.dim[0], ny = r.dim[1], nz = r.dim[2];
-    const long long nvox = (long long)nx * ny * nz;
-    CKS(w.list.ensure((size_t)3 * nvox * sizeof(unsigned)));   // every list fits any marking
+    const unsigned W = (unsigned)(nx + 31) / 32u, slice = W * (unsigned)ny, bps = (slice + OL_T - 1) / OL_T;
+    const size_t nw = (size_t)slice * nz;
+    CKS(w.list.ensure(3 * nw * sizeof(uint2)));   // every list fits any marking
     CKS(w.lcnt.ensure(sizeof(uint4)));
     unsigned *cnt = w.lcnt.as<unsigned>();   // z, y, x counts
-    unsigned *lz = w.list.as<unsigned>(), *ly = lz + nvox, *lx = ly + nvox;
-    const unsigned W = (unsigned)(nx + 31) / 32u, slice = W * (unsigned)ny, bps = (slice + OL_T - 1) / OL_T;
+    uint2 *lz = w.list.as<uint2>(), *ly = lz + nw, *lx = ly + nw;
     CK(cudaMemsetAsync(cnt, 0, sizeof(uint4), s));
-    { k_od_lists<<<bps * (unsigned)nz, OL_T, 0, s>>>(w.need.as<unsigned>(), nx, nz, W, slice, cnt, lz, ly, lx); N2M_COUNT(); }
+    { k_od_lists<<<bps * (unsigned)((nz + OL_Z - 1) / OL_Z), OL_T, 0, s>>>(w.need.as<unsigned>(), nx, nz, W, slice, cnt, lz, ly, lx); N2M_COUNT(); }
     CKL();
-    const int xb = od_grid((const void *)k_od_exact, 256);
-    const unsigned uxy = (unsigned)nx * (unsigned)ny;
-    { k_od_exact<<<xb, 256, 0, s>>>(lx, cnt + 2, r.in, r.tmp1, 1u, 1u, (unsigned)nx, 0ull, od_magic((unsigned)nx)); N2M_COUNT(); }
-    { k_od_exact<<<xb, 256, 0, s>>>(ly, cnt + 1, r.tmp1, r.tmp2, (unsigned)nx, (unsigned)nx, (unsigned)ny,
-                                    od_magic((unsigned)nx), od_magic((unsigned)ny)); N2M_COUNT(); }
-    { k_od_exact<<<xb, 256, 0, s>>>(lz, cnt + 0, r.tmp2, r.out, uxy, uxy, (unsigned)nz, od_magic(uxy),
-                                    od_magic((unsigned)nz)); N2M_COUNT(); }
-    if (r.post) { k_od_post<<<xb, 256, 0, s>>>(lz, cnt + 0, r.out, *r.post, nx, ny, nz); N2M_COUNT(); }
+    const int xb = od_grid((const void *)k_od_exact<0>, OE_T);
+    const unsigned ux = (unsigned)nx, uy = (unsigned)ny, uz = (unsigned)nz;
+    const unsigned long long mx = od_magic(ux), my = od_magic(uy);
+    { k_od_exact<0><<<xb, OE_T, 0, s>>>(lx, cnt + 2, r.in, r.tmp1, ux, uy, uz, mx, my); N2M_COUNT(); }
+    { k_od_exact<1><<<xb, OE_T, 0, s>>>(ly, cnt + 1, r.tmp1, r.tmp2, ux, uy, uz, mx, my); N2M_COUNT(); }
+    { k_od_exact<2><<<xb, OE_T, 0, s>>>(lz, cnt + 0, r.tmp2, r.out, ux, uy, uz, mx, my); N2M_COUNT(); }
+    if (r.post) { k_od_post<<<152 * 8, 256, 0, s>>>(lz, cnt + 0, r.out, *r.post, nx, ny, nz); N2M_COUNT(); }
     CKL();
     return N2M_OK;
 }
