@@ -283,7 +283,7 @@ extern "C" void n2m_context_destroy(n2m_context *c) {
                       &c->aw.ranges, &c->alab, &c->lpts, &c->ltris, &c->gA, &c->gB, &c->gs, &c->gtmp, &c->in, &c->raw, &c->vol, &c->stmp, &c->stats, &c->totals, &c->cand, &c->ncand, &c->ocq, &c->pts_raw,
                       &c->tris_raw, &c->pts, &c->tris, &c->ntf, &c->weld, &c->gath, &c->hmesh,
                       &c->mc.signs, &c->mc.words, &c->mc.act, &c->mc.cnt, &c->mc.sub, &c->scan.part,
-                      &c->lab.lab, &c->lab.mask, &c->lab.keep, &c->lab.cnt, &c->lab.edge, &c->lab.rc, &c->lab.misc,
+                      &c->lab.lab, &c->lab.mask, &c->lab.keep, &c->lab.cnt, &c->lab.edge, &c->lab.rc, &c->lab.misc, &c->lab.list, &c->lab.wlist, &c->lab.cs, &c->lab.filled, &c->lab.shell,
                       &c->deg.flags, &c->deg.tmp, &c->hc.zero, &c->hc.adj, &c->hc.meta, &c->hc.P, &c->hc.Q,
                       &c->hc.B, &c->hc.Lo, &c->th.buf, &c->th.table,
                       &c->stmp2, &c->lubits, &c->od.st, &c->od.unc, &c->od.cmin, &c->od.cmax, &c->od.range, &c->od.need, &c->od.list, &c->od.lcnt, &c->od.vsign,
@@ -370,7 +370,7 @@ struct Prep {
     int lo[3], hi[3];
     bool od = false;          // vol is smoothed approximately: marching cubes makes it exact where it reads it
     const float *src = nullptr;
-    const LabelPost *post = nullptr;   // with od: what the clustering did to vol
+    const LabelPost *post = nullptr;   // what the clustering does to vol (not written)
 };
 
 // The reference's greedy grouping (src/meshify.c:62-78) over elements with
@@ -653,20 +653,26 @@ n2m_status prepare(n2m_context *c, const float *d_src, const int dim[3], const n
     if (verbose) printf("intensity range %g..%g, isolevel %g\n", mn, mx, iso);
     VolStats s1 = s0;
     float min_after = mn;
+    bool lazy = false;   // labelled, but the volume is not written
     if (label) {
         // (a stale isolevel's exact smoothing above left its statistics there)
         CK(cudaMemcpyAsync(dst + 1, &h[1], sizeof(VolStats), cudaMemcpyHostToDevice, c->stream));
-        CKS(run_labelling(vol, nx, ny, nz, iso, mn, o.only_largest, o.fill_bubbles, c->lab, dst + 1, c->stream,
+        const bool above = o.cubes == N2M_CUBES_OLDCUBES;
+        CKS(run_labelling(vol, nx, ny, nz, iso, mn, o.only_largest, o.fill_bubbles, above, c->lab, dst + 1, c->stream,
                           od ? c->od.vsign.as<unsigned>() : nullptr, &c->lpost));
-        CKS(readback(c, &s1, dst + 1));
-        if (od && s1.masked == 0) {   // nothing masked out: the minimum is the labelled values': smooth exactly
-            od = false;
-            CK(cudaMemcpyAsync(dst, h, 2 * sizeof(VolStats), cudaMemcpyHostToDevice, c->stream));
-            CKS(launch_smooth(d_src, vol, c->stmp.as<float>(), nx, ny, nz, iso, dst, c->stream, nullptr));
-            CKS(run_labelling(vol, nx, ny, nz, iso, mn, o.only_largest, o.fill_bubbles, c->lab, dst + 1, c->stream));
+        if (c->lpost.S) CKS(readback(c, &s1, dst + 1));
+        lazy = c->lpost.S && s1.masked;   // some voxel holds mn, every value is >= mn: it is the result's minimum
+        if (!lazy) {   // the whole labelled volume, whose minimum has to be found
+            if (od) {
+                od = false;
+                CK(cudaMemcpyAsync(dst, h, sizeof(VolStats), cudaMemcpyHostToDevice, c->stream));
+                CKS(launch_smooth(d_src, vol, c->stmp.as<float>(), nx, ny, nz, iso, dst, c->stream, nullptr));
+            }
+            CK(cudaMemcpyAsync(dst + 1, &h[1], sizeof(VolStats), cudaMemcpyHostToDevice, c->stream));
+            CKS(lab_write(vol, nx, ny, nz, c->lpost, dst + 1, c->stream));
             CKS(readback(c, &s1, dst + 1));
         }
-        min_after = od ? mn : ord2f(s1.vmin);   // masked voxels hold mn, every exact value is >= mn
+        min_after = lazy ? mn : ord2f(s1.vmin);
     } else if (stale) {
         CKS(launch_stats(v, nx, ny, nz, iso, false, dst + 1, c->stream));
         CKS(readback(c, &s1, dst + 1));
@@ -684,7 +690,7 @@ n2m_status prepare(n2m_context *c, const float *d_src, const int dim[3], const n
     P.mn = mn;
     P.od = od;
     P.src = d_src;
-    P.post = od && label ? &c->lpost : nullptr;
+    P.post = lazy ? &c->lpost : nullptr;
     for (int i = 0; i < 3; i++) {
         P.lo[i] = std::max(s1.lo[i] - 1, 0);
         P.hi[i] = std::min(s1.hi[i] + 2, dim[i]);
@@ -726,10 +732,10 @@ n2m_status march(n2m_context *c, const Prep &P, const int dim[3], int cubes, int
         CKS(c->stmp2.ensure(n * sizeof(float)));
         const OdRepair rep{P.src, c->stmp.as<float>(), c->stmp2.as<float>(), (float *)P.vol, {dim[0], dim[1], dim[2]},
                            &c->od, P.post};
-        if (old) CKS(oc_count(P.vol, dim, P.lo, P.hi, P.iso, P.edge_max, c->mc, dtot, c->stream, &rep));
-        else CKS(mc_count(g, cubes, c->mc, dtot, c->stream, &rep));
-    } else if (old) CKS(oc_count(P.vol, dim, P.lo, P.hi, P.iso, P.edge_max, c->mc, dtot, c->stream));
-    else CKS(mc_count(g, cubes, c->mc, dtot, c->stream));
+        if (old) CKS(oc_count(P.vol, dim, P.lo, P.hi, P.iso, P.edge_max, c->mc, dtot, c->stream, c->od, &rep, P.post));
+        else CKS(mc_count(g, cubes, c->mc, dtot, c->stream, c->od, &rep, P.post));
+    } else if (old) CKS(oc_count(P.vol, dim, P.lo, P.hi, P.iso, P.edge_max, c->mc, dtot, c->stream, c->od, nullptr, P.post));
+    else CKS(mc_count(g, cubes, c->mc, dtot, c->stream, c->od, nullptr, P.post));
     CK(cudaEventRecord(c->evs[3], c->stream));
     uint4 tot;
     CKS(readback(c, &tot, dtot));

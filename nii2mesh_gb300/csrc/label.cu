@@ -11,14 +11,21 @@
 // so the root of a component is its first voxel in raster order: that is how
 // the reference numbers labels (first appearance) and breaks size ties (lowest
 // label wins).  Flattening, face contacts, bubble filling, component sizes and
-// the kept component all work per run; only the final pass over the volume
-// (fill to iso, dilation, mask-out and the range/bbox of the result) touches
-// every voxel.
+// the kept component all work per run, and the labelled volume itself is never
+// written: what marching cubes needs of it follows from the kept set (k_lab_shell).
 //
-// Row kernels give each row `seg` lanes (a power of two, one word per lane,
-// rows of more than 32 words in chunks of 32): the start of the run holding a
-// word's first voxel comes from a max-scan of the last run start of the words
-// before it.
+// A word's thread finds the start of the run of any of its bits by itself: the
+// last start within the word, or, for a run that began in an earlier word, the
+// entry k_run_starts left for the word (one max-scan per row and class; walking or
+// scanning the rows again in every kernel made them bound by instructions).
+//
+// All of it waits on scattered loads of links (L2 latency) and on unions, not on
+// bandwidth: the first contact of a run is its parent without a union, pointers are
+// jumped to roots before the other contacts are looked at, and the kernels run over
+// lists of runs or words, so that no lane idles.  512^3 CT volume (18-connected
+// foreground, 6-connected background): contacts 775 -> 252 us, of it 145 us for the
+// foreground; the sizes 88 -> 16 us where noise makes a million runs (int16 scan);
+// the whole call 2184 -> 1538 us with the volume left unwritten.
 #include <algorithm>
 
 #include "n2m_internal.cuh"
@@ -48,14 +55,6 @@ __device__ __forceinline__ unsigned valid_bits(const LD &d, unsigned w) {
 __device__ __forceinline__ unsigned class_word(const unsigned *B, const LD &d, unsigned r, unsigned w, unsigned want) {
     const unsigned b = B[(size_t)r * d.W + w];
     return want ? b : ~b & valid_bits(d, w);
-}
-
-// the class word after this lane's word (0 past the row); all lanes call it
-__device__ __forceinline__ unsigned next_word(const unsigned *B, const LD &d, unsigned c, bool rowok, unsigned r,
-                                              unsigned w, int li, int seg, unsigned want) {
-    const unsigned dn = __shfl_down_sync(FULL, c, 1, seg);
-    if (li < seg - 1) return w + 1 < d.W ? dn : 0u;
-    return rowok && w + 1 < d.W ? class_word(B, d, r, w + 1, want) : 0u;
 }
 
 // Class bits of the volume: value >= iso (meshify's mask), or value != 0
@@ -95,19 +94,190 @@ __global__ void k_lab_bits_vsign(const unsigned *__restrict__ vsign, LD d, unsig
     }
 }
 
-// every run start of the class links to itself; z8 / z32 (may be null) are
-// zeroed at the run starts (the edge flags and sizes the roots will carry)
-__global__ void k_run_init(const unsigned *__restrict__ B, LD d, unsigned want, int *L, unsigned char *z8,
-                           unsigned *z32) {
-    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < d.nwords; i += gridDim.x * blockDim.x) {
-        const unsigned r = i / d.W, w = i - r * d.W;
-        const unsigned c = class_word(B, d, r, w, want), pc = w ? class_word(B, d, r, w - 1, want) : 0u;
-        const long long base = (long long)r * d.nx + (long long)w * 32;
-        for (unsigned st = c & ~((c << 1) | (pc >> 31)); st; st &= st - 1) {
-            const int s = (int)(base + __ffs(st) - 1);
-            L[s] = s;
-            if (z8) z8[s] = 0;
-            if (z32) z32[s] = 0;
+// Contact directions of a run with the rows before it: row k (0: its own, 1: (y-1, z), 2: (y, z-1), 3: (y-1, z-1),
+// 4: (y+1, z-1)) at x offset dx; 6-connectivity takes the first two, 18- the first eight, 26- all
+__host__ __device__ constexpr int dir_k(int i) { return (int)(0x443343221121ull >> (4 * i) & 15ull); }
+__host__ __device__ constexpr int dir_x(int i) { return (int)(0x202011202011ull >> (4 * i) & 15ull) - 1; }
+__host__ __device__ constexpr int ndirs(int nnb) { return nnb == 3 ? 2 : (nnb == 9 ? 8 : 12); }
+static_assert(dir_k(0) == 1 && dir_k(1) == 2 && dir_k(2) == 1 && dir_k(3) == 1 && dir_k(4) == 2 && dir_k(5) == 2 && dir_k(6) == 3 &&
+                  dir_k(7) == 4 && dir_k(8) == 3 && dir_k(9) == 3 && dir_k(10) == 4 && dir_k(11) == 4, "contact rows");
+static_assert(dir_x(0) == 0 && dir_x(1) == 0 && dir_x(2) == -1 && dir_x(3) == 1 && dir_x(4) == -1 && dir_x(5) == 1 && dir_x(6) == 0 &&
+                  dir_x(7) == 0 && dir_x(8) == -1 && dir_x(9) == 1 && dir_x(10) == -1 && dir_x(11) == 1, "contact offsets");
+
+// cs[i]: where (x) the run that reaches into word i from the word before it starts (-1: no run start before the word).
+// `seg` lanes (a power of two, one word per lane) per row, rows of more than 32 words in chunks of 32.
+__global__ void __launch_bounds__(256) k_run_starts(const unsigned *__restrict__ B, LD d, unsigned want, int *cs) {
+    const int lane = threadIdx.x & 31, seg = d.seg, li = lane & (seg - 1);
+    const unsigned rpw = 32u / (unsigned)seg, rsub = (unsigned)lane / (unsigned)seg;
+    const unsigned nw = (gridDim.x * blockDim.x) >> 5;
+    for (unsigned rb = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * rpw; rb < d.nrows; rb += nw * rpw) {
+        const unsigned r = rb + rsub;
+        int cst = -1;
+        unsigned cwd = 0;
+        for (unsigned c0 = 0; c0 < d.W; c0 += (unsigned)seg) {
+            const unsigned w = c0 + (unsigned)li;
+            const bool ok = r < d.nrows && w < d.W;
+            const WordRuns R = word_runs(ok ? class_word(B, d, r, w, want) : 0u, (int)w * 32, li, seg, cst, cwd);
+            if (ok) cs[(size_t)r * d.W + w] = R.cs;
+        }
+    }
+}
+
+// a word of a row with the words around it
+struct Word {
+    unsigned c, pc, nc;   // this word, the one before, the one after (0 outside the row)
+    unsigned r, w;
+    __device__ __forceinline__ unsigned starts() const { return c & ~((c << 1) | (pc >> 31)); }
+    // bits x whose voxel x + dx is in the class
+    __device__ __forceinline__ unsigned shifted(int dx) const {
+        return dx == 0 ? c : dx == 1 ? (c >> 1) | (nc << 31) : dx == -1 ? (c << 1) | (pc >> 31) : (c << 2) | (pc >> 30);
+    }
+    // voxel index of the start of the run that voxel b (-1 .. 32 of this word) belongs to
+    __device__ __forceinline__ int run(const LD &d, const int *__restrict__ cs, int b) const {
+        const int x0 = (int)w * 32;
+        int x;
+        if (b > 31 && !(c >> 31)) x = x0 + 32;
+        else {
+            x = b < 0 ? -1 : last_start(starts(), x0, min(b, 31));
+            if (x < 0) x = __ldg(cs + (size_t)r * d.W + w);
+        }
+        return (int)((long long)r * d.nx + x);
+    }
+};
+__device__ __forceinline__ Word load_word(const unsigned *__restrict__ B, const LD &d, unsigned r, unsigned w, unsigned want) {
+    return Word{class_word(B, d, r, w, want), w ? class_word(B, d, r, w - 1, want) : 0u,
+                w + 1 < d.W ? class_word(B, d, r, w + 1, want) : 0u, r, w};
+}
+// word w of row r and of the NR - 1 rows before it that touch it
+template <int NNB>
+struct Around {
+    static constexpr int NR = NNB == 3 ? 3 : 5;
+    Word q[NR];
+    __device__ __forceinline__ void load(const unsigned *__restrict__ B, const LD &d, unsigned want, const Word &own) {
+        constexpr int RY[5] = {0, -1, 0, -1, 1}, RZ[5] = {0, 0, -1, -1, -1};
+        const int z = (int)(own.r / (unsigned)d.ny), y = (int)(own.r - (unsigned)z * (unsigned)d.ny);
+        q[0] = own;
+#pragma unroll
+        for (int k = 1; k < NR; k++) {
+            const int yy = y + RY[k], zz = z + RZ[k];
+            const bool ok = yy >= 0 && zz >= 0 && yy < d.ny && zz < d.nz;
+            q[k] = ok ? load_word(B, d, (unsigned)zz * (unsigned)d.ny + (unsigned)yy, own.w, want) : Word{0u, 0u, 0u, 0u, own.w};
+        }
+    }
+};
+
+// The run starts of the class, and the words that hold any of it, as lists (their order
+// is free): the kernels that follow wait on memory most of the time, and by rows of
+// words only a few lanes of a warp had a run (512^3: 0.8 M background runs in 4.2 M
+// words, a foreground in a tenth of them).
+constexpr int LIST_K = 8;   // words per thread
+__global__ void __launch_bounds__(256) k_run_list(const unsigned *__restrict__ B, LD d, unsigned want, int *list, unsigned *wlist,
+                                                  unsigned *nlist, unsigned *nwlist) {
+    __shared__ unsigned wsum[8], base, wbase;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    for (unsigned i0 = blockIdx.x * 256 * LIST_K; i0 < d.nwords; i0 += gridDim.x * 256 * LIST_K) {
+        unsigned st[LIST_K], n = 0, any = 0;   // n: run starts (a block has at most 32768) | words << 16
+#pragma unroll
+        for (int k = 0; k < LIST_K; k++) {
+            const unsigned i = i0 + (unsigned)(k * 256 + tid);
+            st[k] = 0u;
+            if (i < d.nwords) {
+                const unsigned r = i / d.W, w = i - r * d.W;
+                const unsigned c = class_word(B, d, r, w, want), pc = w ? class_word(B, d, r, w - 1, want) : 0u;
+                st[k] = c & ~((c << 1) | (pc >> 31));
+                any |= (c ? 1u : 0u) << k;
+            }
+            n += __popc(st[k]);
+        }
+        n += __popc(any) << 16;
+        unsigned incl = n;
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned t = __shfl_up_sync(FULL, incl, o);
+            if (lane >= o) incl += t;
+        }
+        if (lane == 31) wsum[wid] = incl;
+        __syncthreads();
+        if (tid == 0) {
+            unsigned t = 0;
+            for (int k = 0; k < 8; k++) t += wsum[k];
+            if (t) {
+                base = atomicAdd(nlist, t & 0xffffu);
+                wbase = atomicAdd(nwlist, t >> 16);
+            }
+        }
+        __syncthreads();
+        unsigned before = incl - n;
+        for (int k = 0; k < wid; k++) before += wsum[k];
+        unsigned at = base + (before & 0xffffu), wat = wbase + (before >> 16);
+#pragma unroll
+        for (int k = 0; k < LIST_K; k++) {
+            const unsigned i = i0 + (unsigned)(k * 256 + tid), r = i / d.W;
+            const int x0 = (int)((long long)r * d.nx + (long long)(i - r * d.W) * 32);
+            for (unsigned m = st[k]; m; m &= m - 1) list[at++] = x0 + __ffs(m) - 1;
+            if (any >> k & 1u) wlist[wat++] = i;
+        }
+        __syncthreads();   // wsum and the bases are reused
+    }
+}
+
+// the word holding run start s and the run's piece of it
+__device__ __forceinline__ Word start_word(const unsigned *__restrict__ B, const LD &d, unsigned want, int s, unsigned &piece) {
+    const unsigned r = (unsigned)s / (unsigned)d.nx, x = (unsigned)s - r * (unsigned)d.nx;
+    const Word q = load_word(B, d, r, x >> 5, want);
+    piece = piece_at(q.c, (int)(x & 31u));
+    return q;
+}
+
+// Every run start of the class links to one run before it that it touches (itself
+// if its first word touches none): a forest over all runs, without an atomic, whose
+// trees are nearly the components.  z8 / z32 (may be null) are zeroed at the run
+// starts (the edge flags and sizes the roots will carry).
+template <int NNB>
+__global__ void __launch_bounds__(256) k_run_hook(const unsigned *__restrict__ B, LD d, unsigned want, const int *__restrict__ cs,
+                                                  const int *__restrict__ list, const unsigned *__restrict__ nlist, int *L,
+                                                  unsigned char *z8, unsigned *z32) {
+    const unsigned n = *nlist;
+    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const int s = list[i];
+        unsigned piece;
+        Around<NNB> A;
+        A.load(B, d, want, start_word(B, d, want, s, piece));
+        int parent = s;
+        bool found = false;
+#pragma unroll
+        for (int q = 0; q < ndirs(NNB); q++) {   // the first direction with a contact wins
+            const unsigned t = piece & A.q[dir_k(q)].shifted(dir_x(q));
+            if (!found && t) {
+                found = true;
+                parent = A.q[dir_k(q)].run(d, cs, __ffs(t) - 1 + dir_x(q));
+            }
+        }
+        L[s] = parent;
+        if (z8) z8[s] = 0;
+        if (z32) z32[s] = 0;
+    }
+}
+
+// Every run start points at its root (links only ever move to ancestors, which come
+// before them in raster order, so every walk ends).  The way found so far is left for
+// the others every JUMPS links: they run in raster order more or less, and later
+// walks are a few links long.
+constexpr int JUMPS = 4;
+__global__ void __launch_bounds__(256) k_run_jump(const int *__restrict__ list, const unsigned *__restrict__ nlist, int *L) {
+    const unsigned n = *nlist;
+    volatile int *V = L;
+    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const int s = list[i];
+        int p = V[s], at = p;
+        for (bool more = true; more;) {
+#pragma unroll
+            for (int h = 0; h < JUMPS; h++) {
+                const int q = V[p];
+                more = q != p;
+                p = q;
+                if (!more) break;
+            }
+            if (p != at) V[s] = at = p;
         }
     }
 }
@@ -116,72 +286,46 @@ __global__ void k_run_init(const unsigned *__restrict__ B, LD d, unsigned want, 
 // (y-1, z) and (y, z-1) for 6-connectivity, with x offsets -1..1 for 18 and
 // rows (y-1, z-1), (y+1, z-1) for 18 (x offset 0) and 26 (-1..1).  A contact
 // of voxel x with voxel x+dx of row k counts only if voxels x-1 and x+dx-1
-// do not also touch: one union per overlap of two runs.
+// do not also touch: one union per overlap of two runs.  After the hooks and
+// jumps nearly every contact joins runs with the same link already: the links of all
+// directions' contacts are read together, and only different ones are united.
+// A thread per word of the class (a thread per run walked long runs word by word: the
+// background of the 512^3 CT volume took twice as long).
 template <int NNB>
-__global__ void __launch_bounds__(256, 6) k_run_merge(const unsigned *__restrict__ B, LD d, unsigned want, int *L) {
-    static_assert(NNB == 3 || NNB == 9 || NNB == 13, "6-, 18- or 26-connectivity");
-    constexpr int NR = NNB == 3 ? 3 : 5;
-    const int RY[5] = {0, -1, 0, -1, 1}, RZ[5] = {0, 0, -1, -1, -1};
-    const int lane = threadIdx.x & 31, seg = d.seg, li = lane & (seg - 1);
-    const unsigned rpw = 32u / (unsigned)seg, rsub = (unsigned)lane / (unsigned)seg;
-    const unsigned nw = (gridDim.x * blockDim.x) >> 5;
-    for (unsigned rb = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * rpw; rb < d.nrows; rb += nw * rpw) {
-        const unsigned r = rb + rsub;
-        const bool rowok = r < d.nrows;
-        const int z = rowok ? (int)(r / (unsigned)d.ny) : 0, y = rowok ? (int)(r - (unsigned)z * (unsigned)d.ny) : 0;
-        bool kok[NR];
-        unsigned rk[NR];
+__global__ void __launch_bounds__(256) k_run_merge(const unsigned *__restrict__ B, LD d, unsigned want, const int *__restrict__ cs,
+                                                   const unsigned *__restrict__ wlist, const unsigned *__restrict__ nwlist, int *L) {
+    constexpr int ND = ndirs(NNB);
+    const unsigned n = *nwlist;
+    for (unsigned j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
+        const unsigned i = wlist[j], r = i / d.W;
+        const Word own = load_word(B, d, r, i - r * d.W, want);
+        Around<NNB> A;
+        A.load(B, d, want, own);
+        const unsigned left = own.shifted(-1);
+        unsigned m[ND], any = 0u;
 #pragma unroll
-        for (int k = 0; k < NR; k++) {
-            const int yy = y + RY[k], zz = z + RZ[k];
-            kok[k] = rowok && yy >= 0 && zz >= 0 && yy < d.ny && zz < d.nz;
-            rk[k] = kok[k] ? (unsigned)zz * (unsigned)d.ny + (unsigned)yy : 0u;
+        for (int k = 0; k < ND; k++) {
+            const Word &q = A.q[dir_k(k)];
+            m[k] = own.c & q.shifted(dir_x(k)) & ~(left & q.shifted(dir_x(k) - 1));
+            any |= m[k];
         }
-        int cst[NR];
-        unsigned cwd[NR];
+        while (any) {
+            int a[ND], b[ND];
+            any = 0u;
 #pragma unroll
-        for (int k = 0; k < NR; k++) { cst[k] = -1; cwd[k] = 0u; }
-        for (unsigned c0 = 0; c0 < d.W; c0 += (unsigned)seg) {
-            const unsigned w = c0 + (unsigned)li;
-            const bool ok = w < d.W;
-            const int x0 = (int)w * 32;
-            WordRuns R[NR];
-            unsigned nk[NR];
-#pragma unroll
-            for (int k = 0; k < NR; k++) {
-                const unsigned c = ok && kok[k] ? class_word(B, d, rk[k], w, want) : 0u;
-                R[k] = word_runs(c, x0, li, seg, cst[k], cwd[k]);
-                nk[k] = next_word(B, d, c, kok[k], rk[k], w, li, seg, want);
-            }
-            const unsigned F = R[0].c;
-            if (!F) continue;
-            const unsigned left = (F << 1) | (R[0].pc >> 31);
-            auto S = [&](int k, int dx) -> unsigned {
-                const WordRuns &q = R[k];
-                return dx == 0 ? q.c : dx == 1 ? (q.c >> 1) | (nk[k] << 31)
-                                     : dx == -1 ? (q.c << 1) | (q.pc >> 31) : (q.c << 2) | (q.pc >> 30);
-            };
-            const long long base0 = (long long)r * d.nx;
-            auto link = [&](int k, int dx) {
-                unsigned m = F & S(k, dx) & ~(left & S(k, dx - 1));
-                if (!m) return;
-                const WordRuns &q = R[k];
-                const long long basek = (long long)rk[k] * d.nx;
-                for (; m; m &= m - 1) {
-                    const int b = __ffs(m) - 1, xx = b + dx;
-                    const int sk = xx < 0 ? q.cs : xx > 31 ? ((q.c >> 31) & 1u ? q.start_of(31) : x0 + 32) : q.start_of(xx);
-                    const int i = (int)(base0 + R[0].start_of(b)), j = (int)(basek + sk);
-                    if (L[i] != L[j]) unite(L, i, j);
+            for (int k = 0; k < ND; k++) {
+                a[k] = b[k] = 0;
+                if (m[k]) {
+                    const int x = __ffs(m[k]) - 1;
+                    a[k] = L[own.run(d, cs, x)];
+                    b[k] = L[A.q[dir_k(k)].run(d, cs, x + dir_x(k))];
+                    m[k] &= m[k] - 1u;
+                    any |= m[k];
                 }
-            };
-            link(1, 0);
-            link(2, 0);
-            if constexpr (NNB >= 9) {
-                link(1, -1); link(1, 1); link(2, -1); link(2, 1); link(3, 0); link(4, 0);
             }
-            if constexpr (NNB == 13) {
-                link(3, -1); link(3, 1); link(4, -1); link(4, 1);
-            }
+#pragma unroll
+            for (int k = 0; k < ND; k++)
+                if (a[k] != b[k]) unite(L, a[k], b[k]);
         }
     }
 }
@@ -190,20 +334,16 @@ __global__ void __launch_bounds__(256, 6) k_run_merge(const unsigned *__restrict
 // root search only reads: the one store of this kernel is a start's final
 // root (a path-halving store could overwrite a root another thread has just
 // stored with a lower ancestor).
-__global__ void k_run_flatten(const unsigned *__restrict__ B, LD d, unsigned want, int *L, unsigned *nroots) {
+__global__ void __launch_bounds__(256) k_run_flatten(const int *__restrict__ list, const unsigned *__restrict__ nlist, int *L,
+                                                     unsigned *nroots) {
+    const unsigned n = *nlist;
     unsigned cnt = 0;
-    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < d.nwords; i += gridDim.x * blockDim.x) {
-        const unsigned r = i / d.W, w = i - r * d.W;
-        const unsigned c = class_word(B, d, r, w, want), pc = w ? class_word(B, d, r, w - 1, want) : 0u;
-        const long long base = (long long)r * d.nx + (long long)w * 32;
-        for (unsigned st = c & ~((c << 1) | (pc >> 31)); st; st &= st - 1) {
-            const int s = (int)(base + __ffs(st) - 1);
-            const int root = find_root(L, s);
-            if (root == s) cnt++;
-            else L[s] = root;
-        }
+    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const int s = list[i], root = find_root(L, s);
+        if (root == s) cnt++;
+        else L[s] = root;
     }
-    for (int o = 16; o; o >>= 1) cnt += __shfl_xor_sync(FULL, cnt, o);
+    cnt = __reduce_add_sync(FULL, cnt);
     if ((threadIdx.x & 31) == 0 && cnt) atomicAdd(nroots, cnt);
 }
 
@@ -256,76 +396,86 @@ __global__ void k_run_edges(const unsigned *__restrict__ B, LD d, const int *__r
     }
 }
 
-// bubbles (background components away from every face) become foreground,
-// only when the background has at least two components (src/bwlabel.c:488-491)
-__global__ void __launch_bounds__(256) k_run_fill(unsigned *B, LD d, const int *__restrict__ L,
-                                                  const unsigned char *__restrict__ edge, const unsigned *__restrict__ nbg) {
-    if (*nbg <= 1) return;
-    const int lane = threadIdx.x & 31, seg = d.seg, li = lane & (seg - 1);
-    const unsigned rpw = 32u / (unsigned)seg, rsub = (unsigned)lane / (unsigned)seg;
-    const unsigned nw = (gridDim.x * blockDim.x) >> 5;
-    for (unsigned rb = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * rpw; rb < d.nrows; rb += nw * rpw) {
-        const unsigned r = rb + rsub;
-        const bool rowok = r < d.nrows;
-        const long long base = (long long)r * d.nx;
-        int cst = -1;
-        unsigned cwd = 0;
-        for (unsigned c0 = 0; c0 < d.W; c0 += (unsigned)seg) {
-            const unsigned w = c0 + (unsigned)li;
-            const unsigned c = rowok && w < d.W ? class_word(B, d, r, w, 0u) : 0u;
-            const WordRuns R = word_runs(c, (int)w * 32, li, seg, cst, cwd);
-            unsigned fill = 0;
-            for (unsigned rem = c; rem;) {   // the word's pieces of runs
-                const int b = __ffs(rem) - 1;
-                const unsigned pm = piece_at(rem, b);
-                rem &= ~pm;
-                if (!edge[L[base + R.start_of(b)]]) fill |= pm;
-            }
-            // every lane has read its neighbours' words (word_runs) before any write
-            if (fill) B[(size_t)r * d.W + w] |= fill;
-        }
+// sets the bits of the run that starts at s in out
+__device__ __forceinline__ void put_run(const unsigned *__restrict__ B, const LD &d, unsigned want, int s, unsigned *out) {
+    unsigned piece;
+    for (Word q = start_word(B, d, want, s, piece);;) {
+        atomicOr(out + (size_t)q.r * d.W + q.w, piece);
+        if (!(piece >> 31) || !(q.nc & 1u)) break;
+        q = load_word(B, d, q.r, q.w + 1, want);
+        piece = piece_at(q.c, 0);
     }
 }
 
-// component sizes: every run adds its length to its root (at the run's end)
-__global__ void __launch_bounds__(256) k_run_sizes(const unsigned *__restrict__ B, LD d, const int *__restrict__ L,
-                                                   unsigned *cnt) {
-    const int lane = threadIdx.x & 31, seg = d.seg, li = lane & (seg - 1);
-    const unsigned rpw = 32u / (unsigned)seg, rsub = (unsigned)lane / (unsigned)seg;
-    const unsigned nw = (gridDim.x * blockDim.x) >> 5;
-    for (unsigned rb = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * rpw; rb < d.nrows; rb += nw * rpw) {
-        const unsigned r = rb + rsub;
-        const bool rowok = r < d.nrows;
-        const long long base = (long long)r * d.nx;
-        int cst = -1;
-        unsigned cwd = 0;
-        for (unsigned c0 = 0; c0 < d.W; c0 += (unsigned)seg) {
-            const unsigned w = c0 + (unsigned)li;
-            const unsigned c = rowok && w < d.W ? class_word(B, d, r, w, 1u) : 0u;
-            const WordRuns R = word_runs(c, (int)w * 32, li, seg, cst, cwd);
-            const unsigned nxt = next_word(B, d, c, rowok, r, w, li, seg, 1u);
-            for (unsigned ends = c & ~((c >> 1) | (nxt << 31)); ends; ends &= ends - 1) {
-                const int e = __ffs(ends) - 1, s = R.start_of(e);
-                atomicAdd(&cnt[L[base + s]], (unsigned)(R.x0 + e - s + 1));
-            }
+// bubbles (background components away from every face) become foreground,
+// only when the background has at least two components (src/bwlabel.c:488-491);
+// out: the foreground, a copy (the background's words must stay what they were)
+__global__ void __launch_bounds__(256) k_run_fill(const unsigned *__restrict__ B, LD d, const int *__restrict__ list,
+                                                  const unsigned *__restrict__ nlist, const int *__restrict__ L,
+                                                  const unsigned char *__restrict__ edge, const unsigned *__restrict__ nbg,
+                                                  unsigned *out) {
+    if (*nbg <= 1) return;
+    const unsigned n = *nlist;
+    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const int s = list[i];
+        if (!edge[L[s]]) put_run(B, d, 0u, s, out);
+    }
+}
+
+// Component sizes: every run adds its length to its root.  Most runs belong to a few
+// large components, and one atomic per warp and root on the same counter took 88 us
+// (512^3 int16 scan): a lane keeps the heaviest root it meets to itself, and the block
+// adds up what belongs to the heaviest root of its first lane.
+__global__ void __launch_bounds__(256) k_run_sizes(const unsigned *__restrict__ B, LD d, const int *__restrict__ list,
+                                                   const unsigned *__restrict__ nlist, const int *__restrict__ L, unsigned *cnt) {
+    __shared__ int hot;
+    __shared__ unsigned total;
+    const unsigned n = *nlist;
+    int mine = -1;
+    unsigned sum = 0;
+    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const int s = list[i], root = L[s];
+        unsigned piece;
+        Word q = start_word(B, d, 1u, s, piece);
+        unsigned len = __popc(piece);
+        while ((piece >> 31) && (q.nc & 1u)) {
+            q = load_word(B, d, q.r, q.w + 1, 1u);
+            piece = piece_at(q.c, 0);
+            len += __popc(piece);
+        }
+        if (root == mine) {
+            sum += len;
+        } else if (len <= sum) {
+            atomicAdd(&cnt[root], len);
+        } else {
+            if (sum) atomicAdd(&cnt[mine], sum);
+            mine = root;
+            sum = len;
         }
     }
+    if (threadIdx.x == 0) {
+        hot = mine;
+        total = 0;
+    }
+    __syncthreads();
+    const unsigned w = __reduce_add_sync(FULL, mine == hot ? sum : 0u);
+    if ((threadIdx.x & 31) == 0 && w) atomicAdd(&total, w);
+    if (mine != hot && sum) atomicAdd(&cnt[mine], sum);
+    __syncthreads();
+    if (threadIdx.x == 0 && total) atomicAdd(&cnt[hot], total);
 }
 
 // largest component; ties go to the smallest root (first in raster order)
-__global__ void k_run_best(const unsigned *__restrict__ B, LD d, const int *__restrict__ L,
-                           const unsigned *__restrict__ cnt, unsigned long long *best) {
+__global__ void __launch_bounds__(256) k_run_best(const int *__restrict__ list, const unsigned *__restrict__ nlist,
+                                                  const int *__restrict__ L, const unsigned *__restrict__ cnt,
+                                                  unsigned long long *best) {
+    const unsigned n = *nlist;
     unsigned long long b = 0;
-    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < d.nwords; i += gridDim.x * blockDim.x) {
-        const unsigned r = i / d.W, w = i - r * d.W;
-        const unsigned c = class_word(B, d, r, w, 1u), pc = w ? class_word(B, d, r, w - 1, 1u) : 0u;
-        const long long base = (long long)r * d.nx + (long long)w * 32;
-        for (unsigned st = c & ~((c << 1) | (pc >> 31)); st; st &= st - 1) {
-            const int s = (int)(base + __ffs(st) - 1);
-            if (L[s] != s) continue;
-            const unsigned long long k = ((unsigned long long)cnt[s] << 32) | (0xffffffffu - (unsigned)s);
-            b = k > b ? k : b;
-        }
+    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const int s = list[i];
+        if (L[s] != s) continue;
+        const unsigned long long k = ((unsigned long long)cnt[s] << 32) | (0xffffffffu - (unsigned)s);
+        b = k > b ? k : b;
     }
     for (int o = 16; o; o >>= 1) {
         const unsigned long long t = __shfl_xor_sync(FULL, b, o);
@@ -334,33 +484,17 @@ __global__ void k_run_best(const unsigned *__restrict__ B, LD d, const int *__re
     if ((threadIdx.x & 31) == 0 && b) atomicMax(best, b);
 }
 
-// bits of the voxels of the largest component
-__global__ void __launch_bounds__(256) k_run_keep(const unsigned *__restrict__ B, LD d, const int *__restrict__ L,
+// bits of the voxels of the largest component (K cleared before)
+__global__ void __launch_bounds__(256) k_run_keep(const unsigned *__restrict__ B, LD d, const int *__restrict__ list,
+                                                  const unsigned *__restrict__ nlist, const int *__restrict__ L,
                                                   const unsigned long long *__restrict__ best, unsigned *K) {
     const unsigned long long bk = *best;
-    const int root = bk ? (int)(0xffffffffu - (unsigned)(bk & 0xffffffffu)) : -2;
-    const int lane = threadIdx.x & 31, seg = d.seg, li = lane & (seg - 1);
-    const unsigned rpw = 32u / (unsigned)seg, rsub = (unsigned)lane / (unsigned)seg;
-    const unsigned nw = (gridDim.x * blockDim.x) >> 5;
-    for (unsigned rb = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * rpw; rb < d.nrows; rb += nw * rpw) {
-        const unsigned r = rb + rsub;
-        const bool rowok = r < d.nrows;
-        const long long base = (long long)r * d.nx;
-        int cst = -1;
-        unsigned cwd = 0;
-        for (unsigned c0 = 0; c0 < d.W; c0 += (unsigned)seg) {
-            const unsigned w = c0 + (unsigned)li;
-            const unsigned c = rowok && w < d.W ? class_word(B, d, r, w, 1u) : 0u;
-            const WordRuns R = word_runs(c, (int)w * 32, li, seg, cst, cwd);
-            unsigned keep = 0;
-            for (unsigned rem = c; rem;) {
-                const int b = __ffs(rem) - 1;
-                const unsigned pm = piece_at(rem, b);
-                rem &= ~pm;
-                if (L[base + R.start_of(b)] == root) keep |= pm;
-            }
-            if (rowok && w < d.W) K[(size_t)r * d.W + w] = keep;
-        }
+    if (!bk) return;
+    const int root = (int)(0xffffffffu - (unsigned)(bk & 0xffffffffu));
+    const unsigned n = *nlist;
+    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const int s = list[i];
+        if (L[s] == root) put_run(B, d, 1u, s, K);
     }
 }
 
@@ -368,7 +502,121 @@ __global__ void k_nl_from(const unsigned *nroots, bool only_largest, int *nl) {
     *nl = only_largest ? (*nroots > 0 ? 1 : 0) : (int)*nroots;
 }
 
-// The labelled volume, one warp per row, 32 voxels a word, with the range and
+// The labelled volume (src/meshify.c:330-342) without writing it.  Kept voxels (K) are
+// at or above iso (raised to it when filled); a voxel neither kept nor in the dilation of the
+// kept set (the 26-neighbourhood without (-1,-1,-1), interior voxels only;
+// src/meshify.c:218-264) is the minimum mn, below iso; only the voxels of the
+// dilation's shell keep their values, and only those are read here.  Leaves the sign
+// bitmap of the result (S: value - iso > -FLT_EPSILON, or value >= iso for
+// at_or_above; mn must be on the other side), the kept or dilated voxels (KD), and in
+// *st the bbox of the voxels >= iso and the count of masked ones.  Marching cubes reads
+// values next to sign changes only; they are put right there (lab_apply,
+// smooth.cu: k_od_post).  512^3: 203 us when every voxel was written.
+// With R3 = K(x-1) | K(x) | K(x+1) and R2 = K(x) | K(x+1) of a row, the dilation is R3
+// of rows y-1..y+1 in slices z and z+1, R3 of rows y and y+1 in slice z-1, and R2 of
+// row y-1 in slice z-1.  A lane per word, 32 consecutive words per warp.
+__global__ void __launch_bounds__(256) k_lab_shell(const unsigned *__restrict__ K, LD d, const float *__restrict__ vol, float iso,
+                                                   bool at_or_above, unsigned *S, unsigned *KD, VolStats *st) {
+    smooth::Acc acc;
+    acc.init();
+    unsigned masked = 0;
+    const int lane = threadIdx.x & 31;
+    // rows used: 0..2 = y-1..y+1 in slice z, 3..5 in slice z+1, 6 = (y, z-1), 7 = (y+1, z-1), 8 = (y-1, z-1)
+    constexpr int DY[9] = {-1, 0, 1, -1, 0, 1, 0, 1, -1}, DZ[9] = {0, 0, 0, 1, 1, 1, -1, -1, -1};
+    const unsigned n32 = (d.nwords + 31u) & ~31u, slice = d.W * (unsigned)d.ny;
+    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n32; i += gridDim.x * blockDim.x) {   // whole warps
+        const bool live = i < d.nwords;
+        const unsigned r = live ? i / d.W : 0u, w = live ? i - r * d.W : 0u;
+        const int z = (int)(r / (unsigned)d.ny), y = (int)(r - (unsigned)z * (unsigned)d.ny);
+        const unsigned valid = live ? valid_bits(d, w) : 0u;
+        unsigned on = 0u, kept = 0u;
+#pragma unroll
+        for (int k = 0; k < 9; k++) {
+            const int yy = y + DY[k], zz = z + DZ[k];
+            const bool in = live && yy >= 0 && zz >= 0 && yy < d.ny && zz < d.nz;
+            const unsigned q = in ? i + (unsigned)(DZ[k] * (int)slice + DY[k] * (int)d.W) : 0u;
+            const unsigned cur = in ? __ldg(K + q) : 0u;
+            unsigned prv = __shfl_up_sync(FULL, cur, 1), nxt = __shfl_down_sync(FULL, cur, 1);
+            if (lane == 0) prv = in && w ? __ldg(K + q - 1) : 0u;
+            if (lane == 31) nxt = in && w + 1 < d.W ? __ldg(K + q + 1) : 0u;
+            if (w == 0) prv = 0u;
+            if (w + 1 >= d.W) nxt = 0u;
+            on |= cur | (cur >> 1) | (nxt << 31) | (k < 8 ? (cur << 1) | (prv >> 31) : 0u);   // row 8: no K(x-1)
+            if (k == 1) kept = cur;
+        }
+        // interior voxels only
+        if (y > 0 && z > 0 && y < d.ny - 1 && z < d.nz - 1) {
+            if (w == 0) on &= ~1u;
+            if ((int)w * 32 + 31 >= d.nx - 1) on &= (int)w * 32 < d.nx - 1 ? (1u << (d.nx - 1 - (int)w * 32)) - 1u : 0u;
+        } else {
+            on = 0u;
+        }
+        const unsigned shell = on & ~kept & valid, kd = kept | shell;
+        masked += __popc(valid & ~kd);
+        unsigned sg = kept, ge = kept;
+        const long long base = (long long)r * d.nx + (long long)w * 32;
+        for (unsigned busy = __ballot_sync(FULL, shell != 0u); busy;) {   // the shell's values, four words in flight
+            int j[4];
+            float v[4];
+            unsigned sj[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                j[u] = busy ? __ffs(busy) - 1 : -1;
+                busy &= busy - 1u;
+                sj[u] = __shfl_sync(FULL, shell, j[u] & 31);
+                const long long bj = __shfl_sync(FULL, base, j[u] & 31);
+                v[u] = j[u] >= 0 && (sj[u] >> lane & 1u) ? __ldg(vol + bj + lane) : 0.f;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const bool in = j[u] >= 0 && (sj[u] >> lane & 1u);
+                const unsigned a = __ballot_sync(FULL, in && v[u] >= iso), p = __ballot_sync(FULL, in && __fsub_rn(v[u], iso) > -N2M_FLT_EPS);
+                if (lane == j[u]) {
+                    ge |= a;
+                    sg |= at_or_above ? a : p;
+                }
+            }
+        }
+        if (live) {
+            S[i] = sg;
+            KD[i] = kd;
+        }
+        if (ge) {
+            acc.lo0 = min(acc.lo0, (int)w * 32 + __ffs(ge) - 1); acc.hi0 = max(acc.hi0, (int)w * 32 + 31 - __clz(ge));
+            acc.lo1 = min(acc.lo1, y); acc.hi1 = max(acc.hi1, y);
+            acc.lo2 = min(acc.lo2, z); acc.hi2 = max(acc.hi2, z);
+        }
+    }
+    masked = __reduce_add_sync(FULL, masked);
+    if (lane == 0 && masked) atomicAdd(&st->masked, masked);
+    acc.flush(st, false);
+}
+
+// the labelling's effect on the values marching cubes will read: the marked voxels of `need`
+__global__ void __launch_bounds__(256) k_lab_apply(const unsigned *__restrict__ need, LD d, LabelPost P, float *vol) {
+    const int lane = threadIdx.x & 31;
+    const unsigned n32 = (d.nwords + 31u) & ~31u;
+    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n32; i += gridDim.x * blockDim.x) {   // whole warps
+        const unsigned m = i < d.nwords ? need[i] : 0u, r = i / d.W;
+        unsigned kept = 0u, kd = 0u;
+        if (m) {
+            kept = P.K[i];
+            kd = P.KD[i];
+        }
+        const long long base = (long long)r * d.nx + (long long)(i - r * d.W) * 32;
+        for (unsigned busy = __ballot_sync(FULL, m != 0u); busy; busy &= busy - 1u) {
+            const int k = __ffs(busy) - 1;
+            const unsigned mk = __shfl_sync(FULL, m, k), kk = __shfl_sync(FULL, kept, k), dk = __shfl_sync(FULL, kd, k);
+            float *v = vol + __shfl_sync(FULL, base, k) + lane;
+            if (!(mk >> lane & 1u)) continue;
+            if (!(dk >> lane & 1u)) *v = P.mn;
+            else if (P.fill && (kk >> lane & 1u)) *v = fmaxf(*v, P.iso);
+        }
+    }
+}
+
+// The labelled volume written out (without -l 1, or when nothing is masked out and its
+// minimum has to be found), one warp per row, 32 voxels a word, with the range and
 // bbox of the result.  Kept voxels (K) are raised to iso when FILL; with
 // LARGEST, voxels neither kept nor in the dilation of the kept set (the
 // 26-neighbourhood without (-1,-1,-1), interior voxels only;
@@ -574,49 +822,70 @@ LD make_ld(int nx, int ny, int nz) {
     return d;
 }
 
-n2m_status components(LabelWork &w, const LD &d, unsigned want, int conn, unsigned *d_nroots, unsigned char *z8,
-                      unsigned *z32, cudaStream_t s) {
-    int *L = w.lab.as<int>();
-    const unsigned *B = w.mask.as<unsigned>();
-    { k_run_init<<<gsz(d.nwords), 256, 0, s>>>(B, d, want, L, z8, z32); N2M_COUNT(); }
-    if (conn == 6) { k_run_merge<3><<<rgrid(d), 256, 0, s>>>(B, d, want, L); N2M_COUNT(); }
-    else if (conn == 18) { k_run_merge<9><<<rgrid(d), 256, 0, s>>>(B, d, want, L); N2M_COUNT(); }
-    else { k_run_merge<13><<<rgrid(d), 256, 0, s>>>(B, d, want, L); N2M_COUNT(); }
-    { k_run_flatten<<<gsz(d.nwords), 256, 0, s>>>(B, d, want, L, d_nroots); N2M_COUNT(); }
-    CKL();
-    return N2M_OK;
-}
+// a thread per run, all resident at once
+inline unsigned run_grid(const LD &d) { return std::min(gsz(d.nwords), 152u * 8u); }
 
 struct Misc {
     unsigned nbg, nfg;
     unsigned long long best;
-    int nl, pad;
+    int nl;
+    unsigned nlist[2], nwlist[2];   // run starts and words of the background and the foreground
 };
+
+n2m_status components(LabelWork &w, const LD &d, const unsigned *B, unsigned want, int conn, Misc *misc, unsigned char *z8,
+                      unsigned *z32, cudaStream_t s) {
+    int *L = w.lab.as<int>(), *list = w.list.as<int>();
+    unsigned *nlist = &misc->nlist[want];
+    int *cs = w.cs.as<int>();
+    const unsigned lg = std::max(1u, std::min((d.nwords + 256 * LIST_K - 1) / (256 * LIST_K), 152u * 16u));
+    const unsigned g = run_grid(d), wg = gsz(d.nwords);
+    unsigned *wlist = w.wlist.as<unsigned>(), *nwlist = &misc->nwlist[want];
+    { k_run_starts<<<rgrid(d), 256, 0, s>>>(B, d, want, cs); N2M_COUNT(); }
+    { k_run_list<<<lg, 256, 0, s>>>(B, d, want, list, wlist, nlist, nwlist); N2M_COUNT(); }
+    if (conn == 6) { k_run_hook<3><<<g, 256, 0, s>>>(B, d, want, cs, list, nlist, L, z8, z32); N2M_COUNT(); }
+    else if (conn == 18) { k_run_hook<9><<<g, 256, 0, s>>>(B, d, want, cs, list, nlist, L, z8, z32); N2M_COUNT(); }
+    else { k_run_hook<13><<<g, 256, 0, s>>>(B, d, want, cs, list, nlist, L, z8, z32); N2M_COUNT(); }
+    // once every start points at its tree's root, nearly every contact of the merge joins equal links
+    { k_run_jump<<<g, 256, 0, s>>>(list, nlist, L); N2M_COUNT(); }
+    if (conn == 6) { k_run_merge<3><<<wg, 256, 0, s>>>(B, d, want, cs, wlist, nwlist, L); N2M_COUNT(); }
+    else if (conn == 18) { k_run_merge<9><<<wg, 256, 0, s>>>(B, d, want, cs, wlist, nwlist, L); N2M_COUNT(); }
+    else { k_run_merge<13><<<wg, 256, 0, s>>>(B, d, want, cs, wlist, nwlist, L); N2M_COUNT(); }
+    { k_run_flatten<<<g, 256, 0, s>>>(list, nlist, L, want ? &misc->nfg : &misc->nbg); N2M_COUNT(); }
+    CKL();
+    return N2M_OK;
+}
 
 // the class bits in w.mask on entry; *keep: the kept voxels' bits on return
 // (the foreground after filling, or its largest component)
 n2m_status label_core(LabelWork &w, const LD &d, int conn, bool only_largest, bool fill_bubbles, cudaStream_t s,
                       const unsigned **keep) {
     CKS(w.lab.ensure((size_t)d.n * sizeof(int)));
+    CKS(w.list.ensure(((size_t)d.nrows * ((d.nx + 1) / 2)) * sizeof(int)));   // every second voxel of a row at most
+    CKS(w.wlist.ensure((size_t)d.nwords * sizeof(unsigned)));
     CKS(w.misc.ensure(sizeof(Misc)));
     Misc *misc = w.misc.as<Misc>();
     CK(cudaMemsetAsync(misc, 0, sizeof(Misc), s));
-    unsigned *B = w.mask.as<unsigned>();
+    const unsigned *B = w.mask.as<unsigned>();
+    CKS(w.cs.ensure((size_t)d.nwords * sizeof(int)));
     if (fill_bubbles) {
         CKS(w.edge.ensure((size_t)d.n));
-        CKS(components(w, d, 0u, 6, &misc->nbg, w.edge.as<unsigned char>(), nullptr, s));
+        CKS(w.filled.ensure((size_t)d.nwords * sizeof(unsigned)));
+        CKS(components(w, d, B, 0u, 6, misc, w.edge.as<unsigned char>(), nullptr, s));
         { k_run_edges<<<gsz((long long)d.nrows + 4ll * (d.nx + d.ny + d.nz) * d.W), 256, 0, s>>>(B, d, w.lab.as<int>(), w.edge.as<unsigned char>()); N2M_COUNT(); }
-        { k_run_fill<<<rgrid(d), 256, 0, s>>>(B, d, w.lab.as<int>(), w.edge.as<unsigned char>(), &misc->nbg); N2M_COUNT(); }
+        CK(cudaMemcpyAsync(w.filled.p, B, (size_t)d.nwords * sizeof(unsigned), cudaMemcpyDeviceToDevice, s));
+        { k_run_fill<<<run_grid(d), 256, 0, s>>>(B, d, w.list.as<int>(), &misc->nlist[0], w.lab.as<int>(), w.edge.as<unsigned char>(), &misc->nbg, w.filled.as<unsigned>()); N2M_COUNT(); }
         CKL();
+        B = w.filled.as<unsigned>();
     }
     if (only_largest) CKS(w.cnt.ensure((size_t)d.n * sizeof(unsigned)));
-    CKS(components(w, d, 1u, conn, &misc->nfg, nullptr, only_largest ? w.cnt.as<unsigned>() : nullptr, s));
+    CKS(components(w, d, B, 1u, conn, misc, nullptr, only_largest ? w.cnt.as<unsigned>() : nullptr, s));
     *keep = B;
     if (only_largest) {
         CKS(w.keep.ensure((size_t)d.nwords * sizeof(unsigned)));
-        { k_run_sizes<<<rgrid(d), 256, 0, s>>>(B, d, w.lab.as<int>(), w.cnt.as<unsigned>()); N2M_COUNT(); }
-        { k_run_best<<<gsz(d.nwords), 256, 0, s>>>(B, d, w.lab.as<int>(), w.cnt.as<unsigned>(), &misc->best); N2M_COUNT(); }
-        { k_run_keep<<<rgrid(d), 256, 0, s>>>(B, d, w.lab.as<int>(), &misc->best, w.keep.as<unsigned>()); N2M_COUNT(); }
+        CK(cudaMemsetAsync(w.keep.p, 0, (size_t)d.nwords * sizeof(unsigned), s));
+        { k_run_sizes<<<run_grid(d), 256, 0, s>>>(B, d, w.list.as<int>(), &misc->nlist[1], w.lab.as<int>(), w.cnt.as<unsigned>()); N2M_COUNT(); }
+        { k_run_best<<<run_grid(d), 256, 0, s>>>(w.list.as<int>(), &misc->nlist[1], w.lab.as<int>(), w.cnt.as<unsigned>(), &misc->best); N2M_COUNT(); }
+        { k_run_keep<<<run_grid(d), 256, 0, s>>>(B, d, w.list.as<int>(), &misc->nlist[1], w.lab.as<int>(), &misc->best, w.keep.as<unsigned>()); N2M_COUNT(); }
         *keep = w.keep.as<unsigned>();
     }
     { k_nl_from<<<1, 1, 0, s>>>(&misc->nfg, only_largest, &misc->nl); N2M_COUNT(); }
@@ -636,8 +905,8 @@ n2m_status class_bits(LabelWork &w, const LD &d, const float *vol, float iso, bo
 }
 }  // namespace
 
-n2m_status run_labelling(float *vol, int nx, int ny, int nz, float iso, float mn, bool only_largest,
-                         bool fill_bubbles, LabelWork &w, VolStats *st, cudaStream_t s, const unsigned *vsign,
+n2m_status run_labelling(const float *vol, int nx, int ny, int nz, float iso, float mn, bool only_largest,
+                         bool fill_bubbles, bool at_or_above, LabelWork &w, VolStats *st, cudaStream_t s, const unsigned *vsign,
                          LabelPost *post) {
     const LD d = make_ld(nx, ny, nz);
     if (vsign) {
@@ -653,15 +922,38 @@ n2m_status run_labelling(float *vol, int nx, int ny, int nz, float iso, float mn
     }
     const unsigned *K;
     CKS(label_core(w, d, 18, only_largest, fill_bubbles, s, &K));
-    if (post) *post = LabelPost{K, d.W, mn, iso, fill_bubbles, only_largest};
+    *post = LabelPost{K, nullptr, nullptr, d.W, mn, iso, fill_bubbles, only_largest};
+    volatile float below = mn - iso;
+    if (only_largest && !(below > -N2M_FLT_EPS)) {
+        CKS(w.shell.ensure(2 * (size_t)d.nwords * sizeof(unsigned)));
+        unsigned *S = w.shell.as<unsigned>(), *KD = S + d.nwords;
+        { k_lab_shell<<<std::min(gsz(d.nwords), 152u * 16u), 256, 0, s>>>(K, d, vol, iso, at_or_above, S, KD, st); N2M_COUNT(); }
+        CKL();
+        post->S = S;
+        post->KD = KD;
+    }
+    return N2M_OK;
+}
+
+n2m_status lab_write(float *vol, int nx, int ny, int nz, const LabelPost &P, VolStats *st, cudaStream_t s) {
+    const LD d = make_ld(nx, ny, nz);
     const unsigned g = wgrid(d);
     const bool v4 = nx % 4 == 0 && ((uintptr_t)vol & 15) == 0, one = d.W <= 32;
-    if (only_largest && fill_bubbles && one) { k_lab_final<true, true, true><<<g, 256, 0, s>>>(K, d, vol, iso, mn, st, v4); N2M_COUNT(); }
-    else if (only_largest && fill_bubbles) { k_lab_final<true, true, false><<<g, 256, 0, s>>>(K, d, vol, iso, mn, st, v4); N2M_COUNT(); }
-    else if (only_largest && one) { k_lab_final<true, false, true><<<g, 256, 0, s>>>(K, d, vol, iso, mn, st, v4); N2M_COUNT(); }
-    else if (only_largest) { k_lab_final<true, false, false><<<g, 256, 0, s>>>(K, d, vol, iso, mn, st, v4); N2M_COUNT(); }
-    else if (fill_bubbles) { k_lab_final<false, true, false><<<g, 256, 0, s>>>(K, d, vol, iso, mn, st, v4); N2M_COUNT(); }
+    const unsigned *K = P.K;
+    const float iso = P.iso, mn = P.mn;
+    if (P.largest && P.fill && one) { k_lab_final<true, true, true><<<g, 256, 0, s>>>(K, d, vol, iso, mn, st, v4); N2M_COUNT(); }
+    else if (P.largest && P.fill) { k_lab_final<true, true, false><<<g, 256, 0, s>>>(K, d, vol, iso, mn, st, v4); N2M_COUNT(); }
+    else if (P.largest && one) { k_lab_final<true, false, true><<<g, 256, 0, s>>>(K, d, vol, iso, mn, st, v4); N2M_COUNT(); }
+    else if (P.largest) { k_lab_final<true, false, false><<<g, 256, 0, s>>>(K, d, vol, iso, mn, st, v4); N2M_COUNT(); }
+    else if (P.fill) { k_lab_final<false, true, false><<<g, 256, 0, s>>>(K, d, vol, iso, mn, st, v4); N2M_COUNT(); }
     else { k_lab_final<false, false, false><<<g, 256, 0, s>>>(K, d, vol, iso, mn, st, v4); N2M_COUNT(); }
+    CKL();
+    return N2M_OK;
+}
+
+n2m_status lab_apply(float *vol, int nx, int ny, int nz, const unsigned *need, const LabelPost &P, cudaStream_t s) {
+    const LD d = make_ld(nx, ny, nz);
+    { k_lab_apply<<<std::min(gsz(d.nwords), 152u * 16u), 256, 0, s>>>(need, d, P, vol); N2M_COUNT(); }
     CKL();
     return N2M_OK;
 }

@@ -135,20 +135,29 @@ __global__ void __launch_bounds__(256) k_signs(GV g, unsigned nrows, unsigned *s
     }
 }
 
-// Signs from the volume's sign bitmap (OdWork::vsign, wv words per row, nys groups
-// of 8 rows), one thread per word and no values read: darkening is min(edge_max, v),
-// whose sign is the voxel's bit and edge_max's own, and the padding's sign is the
-// same for every padding point.  512^3 (cold caches): 98 us when the border words (two
-// per row of 16) still read their voxels, 25 us now.
-__global__ void __launch_bounds__(256) k_signs_bits(GV g, unsigned nwords, unsigned *signs,
-                                                    const unsigned *__restrict__ vsign, unsigned wv, unsigned nys) {
+// A sign bitmap of the volume: OdWork::vsign (nys groups of 8 rows per slice), or plain row words (nys 0)
+struct SignMap {
+    const unsigned *bits;
+    unsigned wv, nys;   // words per row
+    int ny;
+    __device__ __forceinline__ unsigned word(int x, int y, int z) const {
+        return __ldg(bits + (nys ? od_vsign_word((unsigned)x, (unsigned)y, (unsigned)z, wv, nys)
+                                 : ((size_t)z * ny + y) * wv + ((unsigned)x >> 5)));
+    }
+};
+
+// Signs from the volume's sign bitmap, one thread per word and no values read:
+// darkening is min(edge_max, v), whose sign is the voxel's bit and edge_max's own, and
+// the padding's sign is the same for every padding point.  512^3 (cold caches): 98 us
+// when the border words (two per row of 16) still read their voxels, 25 us now.
+__global__ void __launch_bounds__(256) k_signs_bits(GV g, unsigned nwords, unsigned *signs, SignMap map) {
     const bool dark = __fsub_rn(g.edge_max, g.iso) > -N2M_FLT_EPS, padp = g.pad > -N2M_FLT_EPS;
     auto voxel = [&](int x, int y, int z) {   // sign of a voxel of a y or z row past the volume too; x = 0
         if (y >= g.dy) {
             y -= g.dy;
             z++;
         }
-        return z < g.dz ? dark && (__ldg(vsign + od_vsign_word((unsigned)x, (unsigned)y, (unsigned)z, wv, nys)) & 1u) : padp;
+        return z < g.dz ? dark && (map.word(x, y, z) & 1u) : padp;
     };
     for (unsigned w = blockIdx.x * blockDim.x + threadIdx.x; w < nwords; w += gridDim.x * blockDim.x) {
         const unsigned xw = w % g.WX, row = w / g.WX;
@@ -163,7 +172,7 @@ __global__ void __launch_bounds__(256) k_signs_bits(GV g, unsigned nwords, unsig
             m = padp ? in : 0u;
         } else {
             const int vb = g.lo0 - g.xoff + 32 * (int)xw;
-            if (vb < g.dx) m = __ldg(vsign + od_vsign_word((unsigned)vb, (unsigned)vy, (unsigned)vz, wv, nys));
+            if (vb < g.dx) m = map.word(vb, vy, vz);
             m &= mcw::bit_range(0, g.dx - vb);
             if (!dark) {
                 if (vy == 0 || vz == 0 || vy == g.dy - 1 || vz == g.dz - 1) m = 0u;
@@ -480,7 +489,8 @@ n2m_status grid_words(const GV &v, size_t &nwords) {
 }
 }  // namespace
 
-n2m_status mc_count(const McGrid &g, int variant, McWork &w, uint4 *d_total, cudaStream_t s, const OdRepair *repair) {
+n2m_status mc_count(const McGrid &g, int variant, McWork &w, uint4 *d_total, cudaStream_t s, OdWork &od, const OdRepair *repair,
+                    const LabelPost *post) {
     const GV v = make_gv(g);
     size_t nwords;
     CKS(grid_words(v, nwords));
@@ -488,22 +498,22 @@ n2m_status mc_count(const McGrid &g, int variant, McWork &w, uint4 *d_total, cud
     CKS(mcw::prepare(w, nwords, d_total, o));
     CKS(w.signs.ensure(nwords * sizeof(unsigned)));
     unsigned *signs = w.signs.as<unsigned>();
-    const unsigned blocks = (unsigned)std::min<size_t>((nwords + 255) / 256, 152u * 16u);
-    if (repair && !repair->post) {
-        k_signs_bits<<<blocks, 256, 0, s>>>(v, (unsigned)nwords, signs, repair->w->vsign.as<unsigned>(),
-                                            (unsigned)(g.dim[0] + 31) / 32, (unsigned)(g.dim[1] + 7) / 8);
-        N2M_COUNT();
+    const unsigned blocks = (unsigned)std::min<size_t>((nwords + 255) / 256, 152u * 16u), wv = (unsigned)(v.dx + 31) / 32u;
+    if (post || repair) {
+        const SignMap map{post ? post->S : od.vsign.as<unsigned>(), wv, post ? 0u : (unsigned)(v.dy + 7) / 8u, v.dy};
+        { k_signs_bits<<<blocks, 256, 0, s>>>(v, (unsigned)nwords, signs, map); N2M_COUNT(); }
     } else {
         const unsigned nrows = (unsigned)g.n[1] * (unsigned)g.n[2];
-        k_signs<<<std::min<unsigned>((nrows + 7) / 8, 152u * 16u), 256, 0, s>>>(v, nrows, signs);
-        N2M_COUNT();
+        { k_signs<<<std::min<unsigned>((nrows + 7) / 8, 152u * 16u), 256, 0, s>>>(v, nrows, signs); N2M_COUNT(); }
     }
     const bool classic = variant == N2M_CUBES_CLASSIC_TABLE;
     const Policy pol{v, classic, nullptr, nullptr, nullptr, nullptr, nullptr, 0};
-    mcw::Marks marks{nullptr, v.dx, v.dy, v.dz, (unsigned)(v.dx + 31) / 32u};
-    if (repair) CKS(od_marks(*repair->w, g.dim, &marks.need, s));
+    mcw::Marks marks{nullptr, v.dx, v.dy, v.dz, wv};
+    if (post || repair) CKS(od_marks(od, g.dim, &marks.need, s));
     CKS(mcw::count_signs(pol, signs, o, marks, s));
-    if (repair) CKS(od_repair(*repair, s));   // exact smoothed values where anything below reads them
+    // final values where anything below reads them
+    if (repair) CKS(od_repair(*repair, s));
+    else if (post) CKS(lab_apply((float *)g.vol, v.dx, v.dy, v.dz, marks.need, *post, s));
     return mcw::count_values(pol, signs, w, o, !classic, s);
 }
 

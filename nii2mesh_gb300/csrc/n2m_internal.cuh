@@ -122,12 +122,12 @@ struct OdWork {
     DevBuf vsign;
     unsigned cap = 0;
 };
-// What meshify's labelling did to each voxel (src/meshify.c:330-342), for the
-// exact values the repair writes afterwards: voxels of K (bit x & 31 of word
-// (z*ny + y)*W + x/32) are raised to iso when fill; with largest, voxels
-// neither in K nor in its dilation are the minimum mn.
+// What meshify's labelling does to each voxel (src/meshify.c:330-342), for the values
+// marching cubes reads: voxels of K (bit x & 31 of word (z*ny + y)*W + x/32) are raised
+// to iso when fill; voxels outside KD (K and its dilation) are the minimum mn.  S: the
+// sign bitmap of the result.  KD and S are null when the volume itself was labelled.
 struct LabelPost {
-    const unsigned *K;
+    const unsigned *K, *KD, *S;
     unsigned W;
     float mn, iso;
     bool fill, largest;
@@ -169,16 +169,20 @@ n2m_status scan_u32(unsigned *d, size_t n, unsigned *d_total, ScanWork &w, cudaS
 
 // label.cu
 struct LabelWork {
-    DevBuf lab, mask, keep, cnt, edge, rc, misc;
+    DevBuf lab, mask, keep, cnt, edge, rc, misc, list, wlist, cs, filled, shell;
 };
-// meshify's labelling of vol in place; st: the range and bbox of the result
-// (accumulated into, like launch_stats) and the count of masked voxels.
-// vsign (may be null): a sign bitmap (OdWork::vsign with od_resolve's
-// at_or_above) to take the mask from instead of vol; post (may be null): what
-// the labelling did, for values computed later
-n2m_status run_labelling(float *vol, int nx, int ny, int nz, float iso, float mn, bool only_largest,
-                         bool fill_bubbles, LabelWork &w, VolStats *st, cudaStream_t s, const unsigned *vsign = nullptr,
-                         LabelPost *post = nullptr);
+// meshify's labelling of vol: the kept set in *post, and with only_largest (and mn
+// clearly below iso) also what follows from it without writing the volume: signs, bbox
+// and count of masked voxels (st).  Otherwise (post->S null), and when st says that no
+// voxel was masked, lab_write labels the volume in place and gives its range and bbox.
+// vsign (may be null): a sign bitmap (OdWork::vsign with od_resolve's at_or_above) to
+// take the mask from; at_or_above: which sign S holds (value >= iso, for oldcubes)
+n2m_status run_labelling(const float *vol, int nx, int ny, int nz, float iso, float mn, bool only_largest,
+                         bool fill_bubbles, bool at_or_above, LabelWork &w, VolStats *st, cudaStream_t s, const unsigned *vsign,
+                         LabelPost *post);
+n2m_status lab_write(float *vol, int nx, int ny, int nz, const LabelPost &P, VolStats *st, cudaStream_t s);
+// the labelling's effect on the marked voxels of vol (marks as od_marks lays them out)
+n2m_status lab_apply(float *vol, int nx, int ny, int nz, const unsigned *need, const LabelPost &P, cudaStream_t s);
 // bwlabel() semantics on a float volume (nonzero = foreground); *d_nl gets the label count
 n2m_status run_bwlabel(float *vol, int nx, int ny, int nz, int conn, bool only_largest, bool fill_bubbles,
                        LabelWork &w, ScanWork &sw, int *d_nl, cudaStream_t s);
@@ -240,12 +244,12 @@ struct McWork {
 struct McCounts {
     unsigned nv_edge, nt, nc, nactive;
 };
-// repair: marks the voxels whose values are needed after the sign pass and runs
-// od_repair before any value is read (null: none)
-// (with a repair and no labelling, the sign words of grid points strictly inside
-// the volume come from repair->w->vsign instead of the values)
-n2m_status mc_count(const McGrid &g, int variant, McWork &w, uint4 *d_total, cudaStream_t s,
-                    const OdRepair *repair = nullptr);
+// post: what a labelling did to the volume (its signs are post->S), repair: the volume
+// was smoothed approximately (without post its signs are repair->w->vsign); with
+// either, the voxels whose values are needed are marked after the sign pass and put
+// right before any value is read.  od: the marks' and the repair's buffers.
+n2m_status mc_count(const McGrid &g, int variant, McWork &w, uint4 *d_total, cudaStream_t s, OdWork &od,
+                    const OdRepair *repair = nullptr, const LabelPost *post = nullptr);
 n2m_status mc_emit(const McGrid &g, int variant, McWork &w, const McCounts &c, vec3d *d_pts, vec3i *d_tris,
                    int *d_cand, unsigned *d_ncand, int cand_cap, cudaStream_t s);
 n2m_status mc_backward(const McGrid &g, int variant, McWork &w, const McCounts &c, const float3 *d_gv, float *d_gs,
@@ -254,9 +258,10 @@ n2m_status mc_ccand_scan(const vec3d *d_pts, int np, const int *d_ccand, int ncc
                          unsigned *d_ncand, int cand_cap, cudaStream_t s);
 
 // oldcubes.cu
-// repair: as for mc_count (vsign must then hold od_resolve's at_or_above sign)
+// as mc_count (the sign bitmaps must then hold value >= iso)
 n2m_status oc_count(const float *vol, const int dim[3], const int lo[3], const int hi[3], float iso, float edge_max,
-                    McWork &w, uint4 *d_total, cudaStream_t s, const OdRepair *repair = nullptr);
+                    McWork &w, uint4 *d_total, cudaStream_t s, OdWork &od, const OdRepair *repair = nullptr,
+                    const LabelPost *post = nullptr);
 n2m_status oc_emit(const float *vol, const int dim[3], const int lo[3], const int hi[3], float iso, float edge_max,
                     McWork &w, const McCounts &c, vec3d *d_pts, vec3i *d_tris, int *d_cand, unsigned *d_ncand,
                     int cand_cap, cudaStream_t s);

@@ -83,9 +83,9 @@ __global__ void __launch_bounds__(256) k_oc_signs(OV g, unsigned nrows, unsigned
     }
 }
 
-// Signs from the volume's sign bitmap with bit = value >= iso (OdWork::vsign, wv words
-// per row, nys groups of 8 rows), one thread per word: the complement, and a
-// darkened point is below the isolevel if its voxel or edge_max is.
+// Signs from a sign bitmap of the volume with bit = value >= iso (OdWork::vsign, wv words
+// per row, nys groups of 8 rows; nys 0: plain row words), one thread per word: the
+// complement, and a darkened point is below the isolevel if its voxel or edge_max is.
 __global__ void __launch_bounds__(256) k_oc_signs_bits(OV g, unsigned nwords, unsigned *signs,
                                                        const unsigned *__restrict__ vsign, unsigned wv, unsigned nys) {
     const bool dark = g.edge_max < g.iso;
@@ -93,7 +93,8 @@ __global__ void __launch_bounds__(256) k_oc_signs_bits(OV g, unsigned nwords, un
         const unsigned row = w / g.WX, xw = w - row * g.WX;
         const int vz = g.lo2 + (int)(row / (unsigned)g.NY), vy = g.lo1 + (int)(row % (unsigned)g.NY);
         const int x0 = 32 * (int)xw - g.xoff, vb = g.lo0 + x0;
-        unsigned m = ~__ldg(vsign + od_vsign_word((unsigned)vb, (unsigned)vy, (unsigned)vz, wv, nys));
+        unsigned m = ~__ldg(vsign + (nys ? od_vsign_word((unsigned)vb, (unsigned)vy, (unsigned)vz, wv, nys)
+                                         : ((size_t)vz * g.dy + vy) * wv + ((unsigned)vb >> 5)));
         if (dark) {
             if (vy == 0 || vz == 0 || vy == g.dy - 1 || vz == g.dz - 1) m = 0xffffffffu;
             else m |= ~mcw::bit_range(vb == 0 ? 1 : 0, g.dx - 1 - vb);
@@ -293,7 +294,7 @@ OV make_ov(const float *vol, const int dim[3], const int lo[3], const int hi[3],
 }  // namespace
 
 n2m_status oc_count(const float *vol, const int dim[3], const int lo[3], const int hi[3], float iso, float edge_max,
-                    McWork &w, uint4 *d_total, cudaStream_t s, const OdRepair *repair) {
+                    McWork &w, uint4 *d_total, cudaStream_t s, OdWork &od, const OdRepair *repair, const LabelPost *post) {
     const OV g = make_ov(vol, dim, lo, hi, iso, edge_max);
     if (g.NX < 2 || g.NY < 2 || g.NZ < 2) {
         CK(cudaMemsetAsync(d_total, 0, sizeof(uint4), s));
@@ -309,17 +310,20 @@ n2m_status oc_count(const float *vol, const int dim[3], const int lo[3], const i
     CKS(w.signs.ensure(nwords * sizeof(unsigned)));
     unsigned *signs = w.signs.as<unsigned>();
     const unsigned wblocks = (unsigned)std::min<size_t>((nwords + 255) / 256, 152u * 16u);
-    if (repair && !repair->post) {
-        { k_oc_signs_bits<<<wblocks, 256, 0, s>>>(g, (unsigned)nwords, signs, repair->w->vsign.as<unsigned>(), (unsigned)(dim[0] + 31) / 32, (unsigned)(dim[1] + 7) / 8); N2M_COUNT(); }
+    const unsigned wv = (unsigned)(g.dx + 31) / 32u;
+    if (post || repair) {
+        { k_oc_signs_bits<<<wblocks, 256, 0, s>>>(g, (unsigned)nwords, signs, post ? post->S : od.vsign.as<unsigned>(), wv, post ? 0u : (unsigned)(g.dy + 7) / 8u); N2M_COUNT(); }
     } else {
         const unsigned nrows = (unsigned)g.NY * (unsigned)g.NZ;
         { k_oc_signs<<<std::min<unsigned>((nrows + 7) / 8, 152u * 16u), 256, 0, s>>>(g, nrows, signs); N2M_COUNT(); }
     }
     const Policy pol{g, nullptr, nullptr, nullptr, 0};
-    mcw::Marks marks{nullptr, g.dx, g.dy, g.dz, (unsigned)(g.dx + 31) / 32u};
-    if (repair) CKS(od_marks(*repair->w, dim, &marks.need, s));
+    mcw::Marks marks{nullptr, g.dx, g.dy, g.dz, wv};
+    if (post || repair) CKS(od_marks(od, dim, &marks.need, s));
     CKS(mcw::count_signs(pol, signs, o, marks, s));
-    if (repair) CKS(od_repair(*repair, s));   // exact smoothed values where the emit reads them
+    // final values where the emit reads them
+    if (repair) CKS(od_repair(*repair, s));
+    else if (post) CKS(lab_apply((float *)vol, g.dx, g.dy, g.dz, marks.need, *post, s));
     return mcw::count_values(pol, signs, w, o, false, s);
 }
 

@@ -1147,35 +1147,20 @@ __global__ void __launch_bounds__(OE_T, 10) k_od_exact(const uint2 *__restrict__
     F.finish(P, acc, lane);
 }
 
-// The labelling's effect on the exact values the z pass just wrote at the
-// listed voxels (src/meshify.c:330-342): kept voxels raised to iso (fill);
-// with largest, voxels neither kept nor in the kept set's dilation (the
-// 26-neighbourhood without (-1,-1,-1), interior voxels; src/meshify.c:218-264)
-// are the minimum.
+// the labelling's effect on the exact values the z pass just wrote at the listed words' voxels
 __global__ void __launch_bounds__(256) k_od_post(const uint2 *__restrict__ list, const unsigned *__restrict__ cnt, float *out,
-                                                 LabelPost L, int nx, int ny, int nz) {
+                                                 LabelPost L, int nx, int ny) {
     const unsigned n = *cnt;
     const int lane = threadIdx.x & 31;
-    auto bit = [&](int x, int y, int z) -> unsigned {
-        return (__ldg(L.K + ((size_t)z * ny + y) * L.W + ((unsigned)x >> 5)) >> (x & 31)) & 1u;
-    };
     for (unsigned i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += (gridDim.x * blockDim.x) >> 5) {   // a warp per word
         const uint2 e = list[i];
+        const unsigned row = e.x / (unsigned)nx;
+        const size_t w = (size_t)row * L.W + ((e.x - row * (unsigned)nx) >> 5);
+        const unsigned kept = L.K[w], kd = L.KD[w];
         if (!(e.y >> lane & 1u)) continue;
-        const unsigned j = e.x + (unsigned)lane, x = j % (unsigned)nx, r = j / (unsigned)nx, y = r % (unsigned)ny, z = r / (unsigned)ny;
-        if (bit(x, y, z)) {
-            if (L.fill) out[j] = fmaxf(out[j], L.iso);
-            continue;
-        }
-        if (!L.largest) continue;
-        bool on = false;
-        if (x > 0 && y > 0 && z > 0 && x + 1 < (unsigned)nx && y + 1 < (unsigned)ny && z + 1 < (unsigned)nz) {
-            for (int dz = -1; dz <= 1 && !on; dz++)
-                for (int dy = -1; dy <= 1 && !on; dy++)
-                    for (int dx = -1; dx <= 1 && !on; dx++)
-                        if (!(dx == -1 && dy == -1 && dz == -1)) on = bit((int)x + dx, (int)y + dy, (int)z + dz);
-        }
-        if (!on) out[j] = L.mn;
+        float *v = out + e.x + (unsigned)lane;
+        if (!(kd >> lane & 1u)) *v = L.mn;
+        else if (L.fill && (kept >> lane & 1u)) *v = fmaxf(*v, L.iso);
     }
 }
 
@@ -1319,7 +1304,7 @@ n2m_status od_repair(const OdRepair &r, cudaStream_t s) {
     { k_od_exact<0><<<xb, OE_T, 0, s>>>(lx, cnt + 2, r.in, r.tmp1, ux, uy, uz, mx, my); N2M_COUNT(); }
     { k_od_exact<1><<<xb, OE_T, 0, s>>>(ly, cnt + 1, r.tmp1, r.tmp2, ux, uy, uz, mx, my); N2M_COUNT(); }
     { k_od_exact<2><<<xb, OE_T, 0, s>>>(lz, cnt + 0, r.tmp2, r.out, ux, uy, uz, mx, my); N2M_COUNT(); }
-    if (r.post) { k_od_post<<<152 * 8, 256, 0, s>>>(lz, cnt + 0, r.out, *r.post, nx, ny, nz); N2M_COUNT(); }
+    if (r.post) { k_od_post<<<152 * 8, 256, 0, s>>>(lz, cnt + 0, r.out, *r.post, nx, ny); N2M_COUNT(); }
     CKL();
     return N2M_OK;
 }
