@@ -81,6 +81,7 @@ __device__ __forceinline__ void hist_flush(int l, int maxlab, unsigned c, int x0
 }
 
 __global__ void k_a_hist(AtlasVol v, int maxlab, unsigned *cnt, int *bb, int *vmax) {
+    grid_wait();
     int mx = 0;
     const unsigned spr = (unsigned)(v.nx + 31) / 32;
     const long long nseg = (long long)spr * v.ny * v.nz;
@@ -130,6 +131,7 @@ struct ArenaSink {
 
 __global__ void __launch_bounds__(smooth::NT, 2) k_a_smooth(AtlasVol v, ABox *boxes, int nb, unsigned nitems,
                                                           unsigned *queue, float *arena, bool smooth_on) {
+    grid_wait();
     __shared__ unsigned item;
     __shared__ int bi;
     for (;;) {
@@ -179,6 +181,7 @@ __global__ void __launch_bounds__(smooth::NT, 2) k_a_smooth(AtlasVol v, ABox *bo
 
 // ---- S2: per-label isolevel (src/meshify.c:305-321 with iso 0.5) ------------------
 __global__ void k_a_iso(ABox *boxes, int nb) {
+    grid_wait();
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= nb) return;
     ABox &B = boxes[b];
@@ -252,6 +255,7 @@ __device__ __forceinline__ unsigned ab_class(const unsigned *Bits, const ABox &B
 // class bits: smoothed value >= the box's isolevel
 __global__ void __launch_bounds__(256) k_ab_bits(const ABox *boxes, int nb, unsigned nrows, const float *arena,
                                                  unsigned *Bits) {
+    grid_wait();
     const int lane = threadIdx.x & 31;
     for (unsigned gr = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; gr < nrows; gr += (gridDim.x * blockDim.x) >> 5) {
         const ABox &B = boxes[find_item(boxes, nb, gr, &ABox::row0)];
@@ -268,6 +272,7 @@ __global__ void __launch_bounds__(256) k_ab_bits(const ABox *boxes, int nb, unsi
 // every run start of the class links to itself; z8 / z32 (may be null) zeroed there
 __global__ void k_ab_init(const ABox *boxes, int nb, unsigned nbw, const unsigned *__restrict__ Bits, unsigned want,
                           int *L, unsigned char *z8, unsigned *z32) {
+    grid_wait();
     for (unsigned gw = blockIdx.x * blockDim.x + threadIdx.x; gw < nbw; gw += gridDim.x * blockDim.x) {
         const ABox &B = boxes[find_item(boxes, nb, gw, &ABox::bw0)];
         const unsigned lw = gw - B.bw0, lr = lw / B.W, w = lw - lr * B.W;
@@ -292,6 +297,7 @@ constexpr int AB_SEG = 4;
 template <int NNB>
 __global__ void __launch_bounds__(256) k_ab_merge(const ABox *boxes, int nb, unsigned nrows,
                                                   const unsigned *__restrict__ Bits, unsigned want, int *L) {
+    grid_wait();
     static_assert(NNB == 3 || NNB == 9, "6- or 18-connectivity");
     constexpr int NR = NNB == 3 ? 3 : 5;
     const int RY[5] = {0, -1, 0, -1, 1}, RZ[5] = {0, 0, -1, -1, -1};
@@ -365,6 +371,7 @@ __global__ void __launch_bounds__(256) k_ab_merge(const ABox *boxes, int nb, uns
 // the final root); roots are counted per box
 __global__ void k_ab_flatten(ABox *boxes, int nb, unsigned nbw, const unsigned *__restrict__ Bits, unsigned want, int *L,
                              bool fg) {
+    grid_wait();
     for (unsigned gw = blockIdx.x * blockDim.x + threadIdx.x; gw < nbw; gw += gridDim.x * blockDim.x) {
         const int b = find_item(boxes, nb, gw, &ABox::bw0);
         const ABox &B = boxes[b];
@@ -386,6 +393,7 @@ __global__ void k_ab_flatten(ABox *boxes, int nb, unsigned nbw, const unsigned *
 // of a row on a y or z face, the runs holding x = 0 and x = n0-1 of the others
 __global__ void k_ab_edges(const ABox *boxes, int nb, unsigned nbw, const unsigned *__restrict__ Bits, const int *L,
                            unsigned char *edge) {
+    grid_wait();
     for (unsigned gw = blockIdx.x * blockDim.x + threadIdx.x; gw < nbw; gw += gridDim.x * blockDim.x) {
         const ABox &B = boxes[find_item(boxes, nb, gw, &ABox::bw0)];
         const int n0 = B.n[0], n1 = B.n[1], n2 = B.n[2];
@@ -427,6 +435,7 @@ __global__ void k_ab_edges(const ABox *boxes, int nb, unsigned nbw, const unsign
 // when the box's background has at least two components (src/bwlabel.c:488-491)
 __global__ void __launch_bounds__(256) k_ab_fill(const ABox *boxes, int nb, unsigned nrows, unsigned *Bits, const int *L,
                                                  const unsigned char *__restrict__ edge) {
+    grid_wait();
     const int lane = threadIdx.x & 31, li = lane & (AB_SEG - 1);
     const unsigned rpw = 32u / AB_SEG, rsub = (unsigned)lane / AB_SEG, nwarps = (gridDim.x * blockDim.x) >> 5;
     for (unsigned rb = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * rpw; rb < nrows; rb += nwarps * rpw) {
@@ -458,6 +467,7 @@ __global__ void __launch_bounds__(256) k_ab_fill(const ABox *boxes, int nb, unsi
 // component sizes at the roots (each run adds its length at its end)
 __global__ void __launch_bounds__(256) k_ab_sizes(const ABox *boxes, int nb, unsigned nrows,
                                                   const unsigned *__restrict__ Bits, const int *L, unsigned *cnt) {
+    grid_wait();
     const int lane = threadIdx.x & 31, li = lane & (AB_SEG - 1);
     const unsigned rpw = 32u / AB_SEG, rsub = (unsigned)lane / AB_SEG, nwarps = (gridDim.x * blockDim.x) >> 5;
     for (unsigned rb = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * rpw; rb < nrows; rb += nwarps * rpw) {
@@ -486,6 +496,7 @@ __global__ void __launch_bounds__(256) k_ab_sizes(const ABox *boxes, int nb, uns
 // largest component per box; ties go to the smallest root (first in raster order)
 __global__ void k_ab_best(ABox *boxes, int nb, unsigned nbw, const unsigned *__restrict__ Bits, const int *L,
                           const unsigned *__restrict__ cnt) {
+    grid_wait();
     for (unsigned gw = blockIdx.x * blockDim.x + threadIdx.x; gw < nbw; gw += gridDim.x * blockDim.x) {
         const int b = find_item(boxes, nb, gw, &ABox::bw0);
         const ABox &B = boxes[b];
@@ -504,6 +515,7 @@ __global__ void k_ab_best(ABox *boxes, int nb, unsigned nbw, const unsigned *__r
 // bits of the voxels of each box's largest component
 __global__ void __launch_bounds__(256) k_ab_keep(const ABox *boxes, int nb, unsigned nrows, const unsigned *__restrict__ Bits,
                                                  const int *L, unsigned *K) {
+    grid_wait();
     const int lane = threadIdx.x & 31, li = lane & (AB_SEG - 1);
     const unsigned rpw = 32u / AB_SEG, rsub = (unsigned)lane / AB_SEG, nwarps = (gridDim.x * blockDim.x) >> 5;
     for (unsigned rb = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * rpw; rb < nrows; rb += nwarps * rpw) {
@@ -540,6 +552,7 @@ __global__ void __launch_bounds__(256) k_ab_keep(const ABox *boxes, int nb, unsi
 template <bool LARGEST, bool FILL>
 __global__ void __launch_bounds__(256) k_ab_final(const ABox *boxes, int nb, unsigned nrows, const unsigned *__restrict__ K,
                                                   float *arena, int nx, int ny, int nz) {
+    grid_wait();
     const int lane = threadIdx.x & 31;
     const int DY[9] = {-1, 0, 1, -1, 0, 1, 0, 1, -1}, DZ[9] = {0, 0, 0, 1, 1, 1, -1, -1, -1};
     for (unsigned gr = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; gr < nrows; gr += (gridDim.x * blockDim.x) >> 5) {
@@ -601,6 +614,7 @@ __global__ void __launch_bounds__(256) k_ab_final(const ABox *boxes, int nb, uns
 // reduced per chunk (all its voxels belong to one box): one set of atomics per chunk
 __global__ void __launch_bounds__(256) k_a_stats(ABox *boxes, int nb, unsigned nch, unsigned *queue, unsigned ch,
                                                  const float *arena) {
+    grid_wait();
     __shared__ unsigned item;
     __shared__ int bi;
     __shared__ int red[8][7];
@@ -651,6 +665,7 @@ __global__ void __launch_bounds__(256) k_a_stats(ABox *boxes, int nb, unsigned n
 }
 
 __global__ void k_a_pad(ABox *boxes, int nb) {
+    grid_wait();
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= nb) return;
     ABox &B = boxes[b];
@@ -694,6 +709,7 @@ constexpr int TY = 8, TZ = 8;
 __global__ void __launch_bounds__(256) k_a_count(AtlasVol v, const ABox *boxes, int nb, unsigned nitems, unsigned *queue,
                                                  const float *arena, bool classic, uint4 *words, uint4 *counts,
                                                  unsigned *active, unsigned *nactive) {
+    grid_wait();
     __shared__ float sv[TZ + 1][TY + 1][33];
     __shared__ unsigned item;
     __shared__ int bi;
@@ -783,6 +799,7 @@ __global__ void k_a_emit(AtlasVol v, const ABox *boxes, const BoxOff *boff, int 
                          const uint4 *__restrict__ offs, const unsigned *__restrict__ active, unsigned nactive,
                          const float *arena, bool classic, vec3d *pts, vec3i *tris, int *cand, unsigned *ncand,
                          int *ccand, unsigned *nccand, int cap) {
+    grid_wait();
     const unsigned lane = threadIdx.x & 31u;
     for (unsigned aw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; aw < nactive; aw += (gridDim.x * blockDim.x) >> 5) {
         const unsigned w = active[aw];
@@ -901,6 +918,7 @@ __global__ void k_a_emit(AtlasVol v, const ABox *boxes, const BoxOff *boff, int 
 
 // scan values at the first word of every box (and the totals after the last)
 __global__ void k_a_boxoff(const ABox *boxes, int nb, const uint4 *offs, uint4 total, BoxOff *boff) {
+    grid_wait();
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b > nb) return;
     if (b == nb) {
@@ -913,11 +931,13 @@ __global__ void k_a_boxoff(const ABox *boxes, int nb, const uint4 *offs, uint4 t
 
 // binarise the whole volume for one label (the per-label loop)
 __global__ void k_binarize(const short *lab, long long n, int label, float *out) {
+    grid_wait();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
         out[i] = lab[i] == label ? 1.f : 0.f;
 }
 
 __global__ void k_offset_tris(vec3i *t, int n, int off) {
+    grid_wait();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         t[i].x -= off; t[i].y -= off; t[i].z -= off;
     }
@@ -943,10 +963,12 @@ uint32_t kbits(float f) {
 }
 
 __global__ void k_a_fill_bb(int *bb, int n) {
+    grid_wait();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) bb[i] = (i % 6) < 3 ? INT_MAX : INT_MIN;
 }
 
 __global__ void k_a_gather(const vec3d *p, const int *ids, int n, vec3d *out) {
+    grid_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) out[i] = p[ids[i]];
 }
@@ -954,6 +976,7 @@ __global__ void k_a_gather(const vec3d *p, const int *ids, int n, vec3d *out) {
 // kept triangles before each box's first triangle, from the degenerate filter's flags
 __global__ void k_a_kept(const unsigned *tri_start, int nb, const unsigned *flags, const unsigned *tile_off, int tile,
                          unsigned total_kept, unsigned *kept_before) {
+    grid_wait();
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b > nb) return;
     const unsigned t = tri_start[b];
@@ -969,6 +992,7 @@ __global__ void k_a_kept(const unsigned *tri_start, int nb, const unsigned *flag
 
 // triangle indices relative to their own mesh
 __global__ void k_a_localize(vec3i *t, unsigned nt, const unsigned *tri_start, const unsigned *vert_start, int nb) {
+    grid_wait();
     for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < nt; i += gridDim.x * blockDim.x) {
         int lo = 0, hi = nb - 1;
         while (lo < hi) {
@@ -1020,8 +1044,9 @@ struct Segment {
     n2m_status enqueue(AtlasWork &w, unsigned ch, unsigned per_sm, unsigned chunks, cudaStream_t s) {
         int qi = 0;
         CK(cudaMemsetAsync(q, 0, 32 * sizeof(unsigned), s));
-        { k_a_smooth<<<pgrid(tiles, 2), dim3(smooth::STX, smooth::STY), 0, s>>>(v, db, nb, tiles, q + qi++, ar, smooth_on); N2M_COUNT(); }
-        { k_a_iso<<<(nb + 127) / 128, 128, 0, s>>>(db, nb); N2M_COUNT(); }
+        n2m_launch(k_a_smooth, pgrid(tiles, 2), dim3(smooth::STX, smooth::STY), 0, s, v, db, nb, tiles, q + qi++, ar,
+                   smooth_on);
+        n2m_launch(k_a_iso, (nb + 127) / 128, 128, 0, s, db, nb);
         const unsigned g = pgrid(chunks, per_sm);
         if (only_largest || fill_bubbles) {
             unsigned *Bm = w.mask.as<unsigned>();
@@ -1029,33 +1054,34 @@ struct Segment {
             const unsigned rg = std::max(1u, std::min((nrows + 7) / 8, 152u * 16u));     // a warp per row
             const unsigned sg = std::max(1u, std::min((nrows * AB_SEG / 32 + 8) / 8, 152u * 16u));   // AB_SEG lanes per row
             const unsigned wg = std::max(1u, std::min((nbw + 255) / 256, 152u * 16u));   // a thread per word
-            { k_ab_bits<<<rg, 256, 0, s>>>(db, nb, nrows, ar, Bm); N2M_COUNT(); }
+            n2m_launch(k_ab_bits, rg, 256, 0, s, db, nb, nrows, ar, Bm);
             if (fill_bubbles) {
                 unsigned char *edge = w.edge.as<unsigned char>();
-                { k_ab_init<<<wg, 256, 0, s>>>(db, nb, nbw, Bm, 0u, L, edge, nullptr); N2M_COUNT(); }
-                { k_ab_merge<3><<<sg, 256, 0, s>>>(db, nb, nrows, Bm, 0u, L); N2M_COUNT(); }
-                { k_ab_flatten<<<wg, 256, 0, s>>>(db, nb, nbw, Bm, 0u, L, false); N2M_COUNT(); }
-                { k_ab_edges<<<wg, 256, 0, s>>>(db, nb, nbw, Bm, L, edge); N2M_COUNT(); }
-                { k_ab_fill<<<sg, 256, 0, s>>>(db, nb, nrows, Bm, L, edge); N2M_COUNT(); }
+                n2m_launch(k_ab_init, wg, 256, 0, s, db, nb, nbw, Bm, 0u, L, edge, nullptr);
+                n2m_launch(k_ab_merge<3>, sg, 256, 0, s, db, nb, nrows, Bm, 0u, L);
+                n2m_launch(k_ab_flatten, wg, 256, 0, s, db, nb, nbw, Bm, 0u, L, false);
+                n2m_launch(k_ab_edges, wg, 256, 0, s, db, nb, nbw, Bm, L, edge);
+                n2m_launch(k_ab_fill, sg, 256, 0, s, db, nb, nrows, Bm, L, edge);
             }
             unsigned *cnt = only_largest ? w.ucnt.as<unsigned>() : nullptr;
-            { k_ab_init<<<wg, 256, 0, s>>>(db, nb, nbw, Bm, 1u, L, nullptr, cnt); N2M_COUNT(); }
-            { k_ab_merge<9><<<sg, 256, 0, s>>>(db, nb, nrows, Bm, 1u, L); N2M_COUNT(); }
-            { k_ab_flatten<<<wg, 256, 0, s>>>(db, nb, nbw, Bm, 1u, L, true); N2M_COUNT(); }
+            n2m_launch(k_ab_init, wg, 256, 0, s, db, nb, nbw, Bm, 1u, L, nullptr, cnt);
+            n2m_launch(k_ab_merge<9>, sg, 256, 0, s, db, nb, nrows, Bm, 1u, L);
+            n2m_launch(k_ab_flatten, wg, 256, 0, s, db, nb, nbw, Bm, 1u, L, true);
             const unsigned *K = Bm;
             if (only_largest) {
                 unsigned *Kb = w.keep.as<unsigned>();
-                { k_ab_sizes<<<sg, 256, 0, s>>>(db, nb, nrows, Bm, L, cnt); N2M_COUNT(); }
-                { k_ab_best<<<wg, 256, 0, s>>>(db, nb, nbw, Bm, L, cnt); N2M_COUNT(); }
-                { k_ab_keep<<<sg, 256, 0, s>>>(db, nb, nrows, Bm, L, Kb); N2M_COUNT(); }
+                n2m_launch(k_ab_sizes, sg, 256, 0, s, db, nb, nrows, Bm, L, cnt);
+                n2m_launch(k_ab_best, wg, 256, 0, s, db, nb, nbw, Bm, L, cnt);
+                n2m_launch(k_ab_keep, sg, 256, 0, s, db, nb, nrows, Bm, L, Kb);
                 K = Kb;
             }
-            if (only_largest && fill_bubbles) { k_ab_final<true, true><<<rg, 256, 0, s>>>(db, nb, nrows, K, ar, nx, ny, nz); N2M_COUNT(); }
-            else if (only_largest) { k_ab_final<true, false><<<rg, 256, 0, s>>>(db, nb, nrows, K, ar, nx, ny, nz); N2M_COUNT(); }
-            else { k_ab_final<false, true><<<rg, 256, 0, s>>>(db, nb, nrows, K, ar, nx, ny, nz); N2M_COUNT(); }
+            if (only_largest && fill_bubbles) n2m_launch(k_ab_final<true, true>, rg, 256, 0, s, db, nb, nrows, K, ar, nx,
+                                                         ny, nz);
+            else if (only_largest) n2m_launch(k_ab_final<true, false>, rg, 256, 0, s, db, nb, nrows, K, ar, nx, ny, nz);
+            else n2m_launch(k_ab_final<false, true>, rg, 256, 0, s, db, nb, nrows, K, ar, nx, ny, nz);
         }
-        { k_a_stats<<<g, 256, 0, s>>>(db, nb, chunks, q + qi++, ch, ar); N2M_COUNT(); }
-        { k_a_pad<<<(nb + 127) / 128, 128, 0, s>>>(db, nb); N2M_COUNT(); }
+        n2m_launch(k_a_stats, g, 256, 0, s, db, nb, chunks, q + qi++, ch, ar);
+        n2m_launch(k_a_pad, (nb + 127) / 128, 128, 0, s, db, nb);
         CKL();
         return N2M_OK;
     }
@@ -1070,9 +1096,10 @@ n2m_status atlas_hist(const short *d_lab, const int dim[3], AtlasWork &w, cudaSt
     CK(cudaMemsetAsync(w.cnt.p, 0, (ML + 1) * sizeof(unsigned), s));
     int *dvmax = (int *)(w.bb.as<int>() + (ML + 1) * 6);
     CK(cudaMemsetAsync(dvmax, 0, sizeof(int), s));
-    { k_a_fill_bb<<<256, 256, 0, s>>>(w.bb.as<int>(), (ML + 1) * 6); N2M_COUNT(); }
+    n2m_launch(k_a_fill_bb, 256, 256, 0, s, w.bb.as<int>(), (ML + 1) * 6);
     AtlasVol v{d_lab, dim[0], dim[1], dim[2], (long long)dim[0] * dim[1], (long long)dim[0] * dim[1] * dim[2]};
-    { k_a_hist<<<pgrid((unsigned)std::min<long long>((v.nvox + 255) / 256, 1u << 30), 32), 256, 0, s>>>(v, ML, w.cnt.as<unsigned>(), w.bb.as<int>(), dvmax); N2M_COUNT(); }
+    n2m_launch(k_a_hist, pgrid((unsigned)std::min<long long>((v.nvox + 255) / 256, 1u << 30), 32), 256, 0, s, v, ML,
+               w.cnt.as<unsigned>(), w.bb.as<int>(), dvmax);
     CKL();
     int mx = 0;
     CK(cudaMemcpyAsync(&mx, dvmax, sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -1089,13 +1116,14 @@ n2m_status atlas_hist(const short *d_lab, const int dim[3], AtlasWork &w, cudaSt
 }
 
 n2m_status atlas_binarize(const short *d_lab, long long n, int label, float *out, cudaStream_t s) {
-    { k_binarize<<<pgrid((unsigned)std::min<long long>((n + 255) / 256, 1u << 30), 32), 256, 0, s>>>(d_lab, n, label, out); N2M_COUNT(); }
+    n2m_launch(k_binarize, pgrid((unsigned)std::min<long long>((n + 255) / 256, 1u << 30), 32), 256, 0, s, d_lab, n, label,
+               out);
     CKL();
     return N2M_OK;
 }
 
 n2m_status atlas_offset_tris(vec3i *t, int n, int off, cudaStream_t s) {
-    if (n > 0 && off) { k_offset_tris<<<pgrid((n + 255) / 256, 16), 256, 0, s>>>(t, n, off); N2M_COUNT(); }
+    if (n > 0 && off) n2m_launch(k_offset_tris, pgrid((n + 255) / 256, 16), 256, 0, s, t, n, off);
     CKL();
     return N2M_OK;
 }
@@ -1256,7 +1284,8 @@ n2m_status atlas_batched(const short *d_lab, const int dim[3], const n2m_options
     unsigned *act = w.active.as<unsigned>();
     CK(cudaMemsetAsync(act + words, 0, sizeof(unsigned), s));
     const bool classic = o.cubes == N2M_CUBES_CLASSIC_TABLE;
-    if (ctiles) { k_a_count<<<pgrid(ctiles, 4), 256, 0, s>>>(v, db, nb, ctiles, q + qi++, ar, classic, w.words.as<uint4>(), w.counts.as<uint4>(), act, act + words); N2M_COUNT(); }
+    if (ctiles) n2m_launch(k_a_count, pgrid(ctiles, 4), 256, 0, s, v, db, nb, ctiles, q + qi++, ar, classic,
+                           w.words.as<uint4>(), w.counts.as<uint4>(), act, act + words);
     CKL();
     uint4 *dtot = w.tot.as<uint4>();
     BoxOff *dboff = (BoxOff *)(dtot + 1);
@@ -1264,7 +1293,7 @@ n2m_status atlas_batched(const short *d_lab, const int dim[3], const n2m_options
     uint4 tot;
     CK(cudaMemcpyAsync(&tot, dtot, sizeof(uint4), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
-    { k_a_boxoff<<<(nb + 128) / 128, 128, 0, s>>>(db, nb, w.counts.as<uint4>(), tot, dboff); N2M_COUNT(); }
+    n2m_launch(k_a_boxoff, (nb + 128) / 128, 128, 0, s, db, nb, w.counts.as<uint4>(), tot, dboff);
     std::vector<BoxOff> boff(nb + 1);
     CK(cudaMemcpyAsync(boff.data(), dboff, (nb + 1) * sizeof(BoxOff), cudaMemcpyDeviceToHost, s));
     const unsigned nv = tot.x + tot.z, nt = tot.y, nact = *(&tot.w);
@@ -1275,7 +1304,9 @@ n2m_status atlas_batched(const short *d_lab, const int dim[3], const n2m_options
     int *cand = w.cand.as<int>();
     unsigned *ncand = (unsigned *)(cand + 2 * cap);
     CK(cudaMemsetAsync(ncand, 0, 2 * sizeof(unsigned), s));
-    if (nact) { k_a_emit<<<pgrid((nact + 7) / 8, 16), 256, 0, s>>>(v, db, dboff, nb, w.words.as<uint4>(), w.counts.as<uint4>(), act, nact, ar, classic, w.pts.as<vec3d>(), w.tris.as<vec3i>(), cand, ncand, cand + cap, ncand + 1, cap); N2M_COUNT(); }
+    if (nact) n2m_launch(k_a_emit, pgrid((nact + 7) / 8, 16), 256, 0, s, v, db, dboff, nb, w.words.as<uint4>(),
+                         w.counts.as<uint4>(), act, nact, ar, classic, w.pts.as<vec3d>(), w.tris.as<vec3i>(),
+                         cand, ncand, cand + cap, ncand + 1, cap);
     CKL();
     unsigned nc[2];
     CK(cudaMemcpyAsync(nc, ncand, 2 * sizeof(unsigned), cudaMemcpyDeviceToHost, s));
@@ -1314,7 +1345,7 @@ n2m_status atlas_batched(const short *d_lab, const int dim[3], const n2m_options
         vec3d *dpos = w.gath.as<vec3d>();
         int *dids = (int *)(dpos + all.size());
         CK(cudaMemcpyAsync(dids, all.data(), all.size() * sizeof(int), cudaMemcpyHostToDevice, s));
-        { k_a_gather<<<((int)all.size() + 255) / 256, 256, 0, s>>>(w.pts.as<vec3d>(), dids, (int)all.size(), dpos); N2M_COUNT(); }
+        n2m_launch(k_a_gather, ((int)all.size() + 255) / 256, 256, 0, s, w.pts.as<vec3d>(), dids, (int)all.size(), dpos);
         std::vector<vec3d> pos(all.size());
         CK(cudaMemcpyAsync(pos.data(), dpos, all.size() * sizeof(vec3d), cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
@@ -1393,7 +1424,8 @@ n2m_status atlas_batched(const short *d_lab, const int dim[3], const n2m_options
     CK(cudaMemcpyAsync(&ntf, dntf, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
     CK(cudaMemcpyAsync(dts, ts.data(), (nb + 1) * sizeof(unsigned), cudaMemcpyHostToDevice, s));
-    if (nt) { k_a_kept<<<(nb + 128) / 128, 128, 0, s>>>(dts, nb, dw.flags.as<unsigned>(), dw.tmp.as<unsigned>(), 256, ntf, dkept); N2M_COUNT(); }
+    if (nt) n2m_launch(k_a_kept, (nb + 128) / 128, 128, 0, s, dts, nb, dw.flags.as<unsigned>(), dw.tmp.as<unsigned>(), 256, ntf,
+                       dkept);
     else CK(cudaMemsetAsync(dkept, 0, (nb + 1) * sizeof(unsigned), s));
     std::vector<unsigned> kept(nb + 1);
     CK(cudaMemcpyAsync(kept.data(), dkept, (nb + 1) * sizeof(unsigned), cudaMemcpyDeviceToHost, s));
@@ -1406,7 +1438,7 @@ n2m_status atlas_batched(const short *d_lab, const int dim[3], const n2m_options
     // ---- triangle indices local to their mesh
     CK(cudaMemcpyAsync(dkept, kept.data(), (nb + 1) * sizeof(unsigned), cudaMemcpyHostToDevice, s));
     CK(cudaMemcpyAsync(dvs, vs_new.data(), (nb + 1) * sizeof(unsigned), cudaMemcpyHostToDevice, s));
-    if (ntf) { k_a_localize<<<pgrid((ntf + 255) / 256, 16), 256, 0, s>>>(tris, ntf, dkept, dvs, nb); N2M_COUNT(); }
+    if (ntf) n2m_launch(k_a_localize, pgrid((ntf + 255) / 256, 16), 256, 0, s, tris, ntf, dkept, dvs, nb);
     CKL();
     CK(cudaStreamSynchronize(s));
     out.clear();

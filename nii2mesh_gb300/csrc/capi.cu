@@ -339,12 +339,14 @@ template <class T> n2m_status readback(n2m_context *c, T *dst, const void *dsrc,
 }
 
 __global__ void k_gather(const vec3d *__restrict__ p, const int *__restrict__ ids, int n, vec3d *out) {
+    grid_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) out[i] = p[ids[i]];
 }
 
 // corner q = 3*t + c of the triangle list takes vertex v, for n (q, v) pairs
 __global__ void k_set_corners(vec3i *tris, const int2 *__restrict__ qv, int n) {
+    grid_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) {
         const int t = qv[i].x / 3, c = qv[i].x - 3 * t;
@@ -444,7 +446,7 @@ n2m_status weld_candidates(n2m_context *c, int nv, int ncand, std::vector<int> &
     vec3d *dpos = c->gath.as<vec3d>();
     int *dids = (int *)(dpos + n);
     CK(cudaMemcpyAsync(dids, ids.data(), n * sizeof(int), cudaMemcpyHostToDevice, c->stream));
-    { k_gather<<<(n + 255) / 256, 256, 0, c->stream>>>(c->pts_raw.as<vec3d>(), dids, n, dpos); N2M_COUNT(); }
+    n2m_launch(k_gather, (n + 255) / 256, 256, 0, c->stream, c->pts_raw.as<vec3d>(), dids, n, dpos);
     CKL();
     std::vector<vec3d> pos(n);
     CK(cudaMemcpyAsync(pos.data(), dpos, n * sizeof(vec3d), cudaMemcpyDeviceToHost, c->stream));
@@ -850,7 +852,7 @@ n2m_status pipeline(n2m_context *c, const float *d_src, const int dim[3], const 
             if (no) CK(cudaMemcpyAsync(dovsrc, ov_src.data(), no * sizeof(int), cudaMemcpyHostToDevice, c->stream));
             if (ncr) {   // split vertices: corners take their copy's group vertex before the renumbering
                 CK(cudaMemcpyAsync(dcr, corners.data(), ncr * sizeof(int2), cudaMemcpyHostToDevice, c->stream));
-                { k_set_corners<<<(ncr + 255) / 256, 256, 0, c->stream>>>(c->tris_raw.as<vec3i>(), dcr, ncr); N2M_COUNT(); }
+                n2m_launch(k_set_corners, (ncr + 255) / 256, 256, 0, c->stream, c->tris_raw.as<vec3i>(), dcr, ncr);
                 CKL();
             }
             c->fwd.removed = drem;

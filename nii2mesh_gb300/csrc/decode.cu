@@ -28,6 +28,7 @@ __device__ __forceinline__ float as_float<float>(float v) { return v; }
 template <class T>
 __global__ void __launch_bounds__(256) k_cast(const T *__restrict__ raw, float *__restrict__ out, long long n,
                                               float slope, float inter) {
+    grid_wait();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
         out[i] = __fadd_rn(__fmul_rn(as_float<T>(raw[i]), slope), inter);
 }
@@ -49,15 +50,16 @@ n2m_status launch_cast(const void *d_raw, int datatype, float slope, float inter
     long long b = (n + 255) / 256;
     const unsigned blocks = (unsigned)(b < 152 * 16 ? b : 152 * 16);
     switch (datatype) {
-    case N2M_DT_UINT8: k_cast<unsigned char><<<blocks, 256, 0, s>>>((const unsigned char *)d_raw, d_out, n, slope, inter); break;
-    case N2M_DT_INT16: k_cast<short><<<blocks, 256, 0, s>>>((const short *)d_raw, d_out, n, slope, inter); break;
-    case N2M_DT_UINT16: k_cast<unsigned short><<<blocks, 256, 0, s>>>((const unsigned short *)d_raw, d_out, n, slope, inter); break;
-    case N2M_DT_FLOAT32: k_cast<float><<<blocks, 256, 0, s>>>((const float *)d_raw, d_out, n, slope, inter); break;
+    case N2M_DT_UINT8: n2m_launch(k_cast<unsigned char>, blocks, 256, 0, s, (const unsigned char *)d_raw, d_out, n, slope,
+                                  inter); break;
+    case N2M_DT_INT16: n2m_launch(k_cast<short>, blocks, 256, 0, s, (const short *)d_raw, d_out, n, slope, inter); break;
+    case N2M_DT_UINT16: n2m_launch(k_cast<unsigned short>, blocks, 256, 0, s, (const unsigned short *)d_raw, d_out, n, slope,
+                                   inter); break;
+    case N2M_DT_FLOAT32: n2m_launch(k_cast<float>, blocks, 256, 0, s, (const float *)d_raw, d_out, n, slope, inter); break;
     default:
         n2m_set_error("unsupported NIfTI datatype %d (uint8 2, int16 4, float32 16, uint16 512)", datatype);
         return N2M_ERR_BAD_ARGS;
     }
-    N2M_COUNT();
     CKL();
     return N2M_OK;
 }

@@ -122,6 +122,7 @@ __device__ __forceinline__ unsigned dist_extra_bits(unsigned d) { return d < 4 ?
 __global__ void __launch_bounds__(32 * LZ_WARPS, 3) k_lz(const unsigned *__restrict__ src, long long n, int nchunks,
                                                          int ch, unsigned *__restrict__ tokens,
                                                          DfInfo *__restrict__ info, unsigned *__restrict__ ghist) {
+    grid_wait();
     extern __shared__ unsigned sm_ht[];   // LZ_WARPS tables of DF_HSIZE buckets
     __shared__ unsigned hist_s[LZ_WARPS][DF_NSYM / 2];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -377,6 +378,7 @@ __constant__ unsigned char c_clorder[19] = {16, 17, 18, 0, 8, 7, 9, 6, 10, 5, 11
 __global__ void __launch_bounds__(32 * DF_WARPS) k_huff(const unsigned *__restrict__ ghist, int nchunks, int G,
                                                         DfInfo *__restrict__ info, unsigned *__restrict__ gcodes,
                                                         unsigned *__restrict__ ghdr, unsigned *__restrict__ sizes) {
+    grid_wait();
     __shared__ HuffScratch sc[DF_WARPS];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int group = blockIdx.x * DF_WARPS + warp;
@@ -546,6 +548,7 @@ __global__ void __launch_bounds__(32 * BITS_WARPS) k_bits(const unsigned char *_
                                                         const unsigned *__restrict__ ghdr, const unsigned *__restrict__ offs,
                                                         int nchunks, int ch, int G, unsigned char *__restrict__ out,
                                                         unsigned *__restrict__ err) {
+    grid_wait();
     __shared__ unsigned ring_s[BITS_WARPS][RING];
     __shared__ unsigned code_s[BITS_WARPS][DF_NLIT + DF_NDIST];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -655,6 +658,7 @@ struct XPow {
 };
 __global__ void __launch_bounds__(256) k_cksum(const unsigned *__restrict__ src, long long n, int adler, XPow xp,
                                              unsigned long long *__restrict__ acc) {
+    grid_wait();
     // slicing-by-4 tables: tab[0] the byte table, tab[k][i] = tab[k-1][i] advanced by one zero byte
     __shared__ unsigned tab[4][256];
     __shared__ unsigned long long red[2][8];
@@ -761,6 +765,7 @@ XPow xpow_table() {   // host: x^(8 * 2^k) mod P by repeated squaring
 // container header and trailer around the stream of `body` bytes
 __global__ void k_wrap(unsigned char *out, int container, unsigned long long body, long long n,
                        const unsigned long long *__restrict__ acc) {
+    grid_wait();
     if (threadIdx.x || blockIdx.x) return;
     if (container == N2M_DEFLATE_GZIP) {
         const unsigned char h[10] = {0x1f, 0x8b, 8, 0, 0, 0, 0, 0, 0, 3};   // no name, mtime 0, OS Unix (as gzopen writes)
@@ -837,9 +842,8 @@ n2m_status deflate_device(const void *d_src, size_t n, int container, DeflateWor
         static const XPow xp = xpow_table();
         CK(cudaEventRecord((cudaEvent_t)w.ev_in, s));
         CK(cudaStreamWaitEvent((cudaStream_t)w.side, (cudaEvent_t)w.ev_in, 0));
-        k_cksum<<<(unsigned)((nseg + 255) / 256), 256, 0, (cudaStream_t)w.side>>>((const unsigned *)d_src, (long long)n,
-                                                                                adler, xp, acc);
-        N2M_COUNT();
+        n2m_launch(k_cksum, (unsigned)((nseg + 255) / 256), 256, 0, (cudaStream_t)w.side, (const unsigned *)d_src, (long long)n,
+                   adler, xp, acc);
         CKL();
         CK(cudaEventRecord((cudaEvent_t)w.ev_ck, (cudaStream_t)w.side));
     }
@@ -848,14 +852,11 @@ n2m_status deflate_device(const void *d_src, size_t n, int container, DeflateWor
     const int ngroups = (nchunks + G - 1) / G;
     const unsigned blocks = (unsigned)((ngroups + DF_WARPS - 1) / DF_WARPS);
     CK(cudaFuncSetAttribute(k_lz, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    k_lz<<<(unsigned)((nchunks + LZ_WARPS - 1) / LZ_WARPS), 32 * LZ_WARPS, smem, s>>>(
-        (const unsigned *)d_src, (long long)n, nchunks, (int)ch, w.tok.as<unsigned>(), w.info.as<DfInfo>(),
-        w.hist.as<unsigned>());
-    N2M_COUNT();
+    n2m_launch(k_lz, (unsigned)((nchunks + LZ_WARPS - 1) / LZ_WARPS), 32 * LZ_WARPS, smem, s, (const unsigned *)d_src,
+               (long long)n, nchunks, (int)ch, w.tok.as<unsigned>(), w.info.as<DfInfo>(), w.hist.as<unsigned>());
     CKL();
-    k_huff<<<blocks, 32 * DF_WARPS, 0, s>>>(w.hist.as<unsigned>(), nchunks, G, w.info.as<DfInfo>(),
-                                           w.codes.as<unsigned>(), w.hdr.as<unsigned>(), w.sizes.as<unsigned>());
-    N2M_COUNT();
+    n2m_launch(k_huff, blocks, 32 * DF_WARPS, 0, s, w.hist.as<unsigned>(), nchunks, G, w.info.as<DfInfo>(),
+               w.codes.as<unsigned>(), w.hdr.as<unsigned>(), w.sizes.as<unsigned>());
     CKL();
     CKS(scan_u32(w.sizes.as<unsigned>(), (size_t)nchunks, w.sizes.as<unsigned>() + nchunks, sw, s));
     unsigned body = 0;
@@ -866,15 +867,13 @@ n2m_status deflate_device(const void *d_src, size_t n, int container, DeflateWor
     const size_t total = head + body + tail;
     CKS(w.out.ensure(total + 16));
     unsigned char *out = w.out.as<unsigned char>();
-    k_bits<<<(unsigned)((nchunks + BITS_WARPS - 1) / BITS_WARPS), 32 * BITS_WARPS, 0, s>>>(
-        (const unsigned char *)d_src, w.tok.as<unsigned>(), w.info.as<DfInfo>(), w.codes.as<unsigned>(),
-        w.hdr.as<unsigned>(), w.sizes.as<unsigned>(), nchunks, (int)ch, G, out + head, (unsigned *)(acc + 2));
-    N2M_COUNT();
+    n2m_launch(k_bits, (unsigned)((nchunks + BITS_WARPS - 1) / BITS_WARPS), 32 * BITS_WARPS, 0, s, (const unsigned char *)d_src,
+               w.tok.as<unsigned>(), w.info.as<DfInfo>(), w.codes.as<unsigned>(), w.hdr.as<unsigned>(),
+               w.sizes.as<unsigned>(), nchunks, (int)ch, G, out + head, (unsigned *)(acc + 2));
     CKL();
     if (cksum) CK(cudaStreamWaitEvent(s, (cudaEvent_t)w.ev_ck, 0));
     if (container != N2M_DEFLATE_RAW) {
-        k_wrap<<<1, 1, 0, s>>>(out, container, body, (long long)n, acc);
-        N2M_COUNT();
+        n2m_launch(k_wrap, 1, 1, 0, s, out, container, body, (long long)n, acc);
         CKL();
     }
     *out_len = total;

@@ -28,6 +28,7 @@ __device__ __forceinline__ bool tri_in_range(const vec3i &T, int np) {
 }
 
 __global__ void k_degree(const vec3i *__restrict__ t, int nt, int np, unsigned *deg, unsigned *bad) {
+    grid_wait();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nt; i += gridDim.x * blockDim.x) {
         const vec3i T = t[i];
         if (!tri_in_range(T, np)) {
@@ -44,6 +45,7 @@ __global__ void k_degree(const vec3i *__restrict__ t, int nt, int np, unsigned *
 // the vertex's segment (k_hc_adj sorts it)
 __global__ void k_fill_adj(const vec3i *__restrict__ t, int nt, int np, const unsigned *__restrict__ start,
                            unsigned *fill, int2 *adj) {
+    grid_wait();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nt; i += gridDim.x * blockDim.x) {
         const vec3i T = t[i];
         if (!tri_in_range(T, np)) continue;
@@ -98,6 +100,7 @@ constexpr int ADJ_S = 32, ADJ_T = 128;
 __global__ void __launch_bounds__(ADJ_T) k_hc_adj(const vec3d *__restrict__ o, const unsigned *__restrict__ start, int np,
                                                   int *adj, Meta *meta, unsigned char *border, float4 *Lo, float4 *Pn,
                                                   float4 *B) {
+    grid_wait();
     __shared__ int col[ADJ_S][ADJ_T];
     const int tid = threadIdx.x;
     for (int i = blockIdx.x * ADJ_T + tid; i < np; i += gridDim.x * ADJ_T) {
@@ -207,6 +210,7 @@ __device__ __forceinline__ Meta load_meta(const Meta *__restrict__ meta, int i) 
 __global__ void __launch_bounds__(128) k_hc_a(const float4 *__restrict__ P, const float4 *__restrict__ Lo,
                                               const Meta *__restrict__ meta, const int *__restrict__ adj, int np,
                                               float alpha1, float4 *Pn, float4 *B) {
+    grid_wait();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < np; i += gridDim.x * blockDim.x) {
         const Meta m = load_meta(meta, i);
         const float4 q = P[i], lo = Lo[i];
@@ -228,6 +232,7 @@ __global__ void __launch_bounds__(128) k_hc_b(const float4 *__restrict__ Pn, con
                                               float beta, float beta1, float4 *P, vec3d *o,
                                               const unsigned char *__restrict__ border, bool lock,
                                               const unsigned *__restrict__ bad) {
+    grid_wait();
     if (o && *bad) return;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < np; i += gridDim.x * blockDim.x) {
         const Meta m = load_meta(meta, i);
@@ -256,6 +261,7 @@ __global__ void __launch_bounds__(128) k_hc_b(const float4 *__restrict__ Pn, con
 // The vectors carry 1 / num_i in .w, so a gather brings both.
 __global__ void k_hcT_init(const float3 *__restrict__ g, const unsigned char *__restrict__ border,
                            const Meta *__restrict__ meta, int np, bool lock, float4 *lam, float3 *go) {
+    grid_wait();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < np; i += gridDim.x * blockDim.x) {
         const bool b = lock && border[i];
         const float3 v = g[i];
@@ -268,6 +274,7 @@ __global__ void k_hcT_init(const float3 *__restrict__ g, const unsigned char *__
 // t1 = L^T lam
 __global__ void __launch_bounds__(128) k_hcT_a(const float4 *__restrict__ lam, const Meta *__restrict__ meta,
                                                const int *__restrict__ adj, int np, float4 *t1) {
+    grid_wait();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < np; i += gridDim.x * blockDim.x) {
         const Meta m = load_meta(meta, i);
         float4 r = lam[i];
@@ -283,6 +290,7 @@ __global__ void __launch_bounds__(128) k_hcT_a(const float4 *__restrict__ lam, c
 __global__ void __launch_bounds__(128) k_hcT_b(float4 *lam, const float4 *__restrict__ t1, const Meta *__restrict__ meta,
                                                const int *__restrict__ adj, float3 *go, int np, float ab, float a1b,
                                                float c0, float c1, float c2, bool last) {
+    grid_wait();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < np; i += gridDim.x * blockDim.x) {
         const Meta m = load_meta(meta, i);
         const float4 l = lam[i], u = t1[i];
@@ -321,21 +329,21 @@ inline unsigned sweep_grid(int np) { return (unsigned)std::max(1, std::min((np +
 
 n2m_status hc_count(const vec3i *d_tris, int np, int nt, const HcBufs &h, cudaStream_t s) {
     CK(cudaMemsetAsync(h.start, 0, h.zero_bytes, s));
-    { k_degree<<<gs(nt), 256, 0, s>>>(d_tris, nt, np, h.start, h.bad); N2M_COUNT(); }
+    n2m_launch(k_degree, gs(nt), 256, 0, s, d_tris, nt, np, h.start, h.bad);
     CKL();
     return N2M_OK;
 }
 // everything after the scan of the degrees; iter >= 1
 n2m_status hc_run(vec3d *d_pts, const vec3i *d_tris, int np, int nt, double alpha, double beta, int iter, bool lock_edges,
                   const HcBufs &h, cudaStream_t s) {
-    { k_fill_adj<<<gs(nt), 256, 0, s>>>(d_tris, nt, np, h.start, h.fill, (int2 *)h.adj); N2M_COUNT(); }
+    n2m_launch(k_fill_adj, gs(nt), 256, 0, s, d_tris, nt, np, h.start, h.fill, (int2 *)h.adj);
     const unsigned g = sweep_grid(np);
-    { k_hc_adj<<<g, ADJ_T, 0, s>>>(d_pts, h.start, np, h.adj, h.meta, h.border, h.Lo, h.Q, h.B); N2M_COUNT(); }
+    n2m_launch(k_hc_adj, g, ADJ_T, 0, s, d_pts, h.start, np, h.adj, h.meta, h.border, h.Lo, h.Q, h.B);
     const float a1 = (float)(1.0 - alpha), b = (float)beta, b1 = (float)(1.0 - beta);
     for (int it = 0; it < iter; it++) {
-        if (it) { k_hc_a<<<g, 128, 0, s>>>(h.P, h.Lo, h.meta, h.adj, np, a1, h.Q, h.B); N2M_COUNT(); }
-        { k_hc_b<<<g, 128, 0, s>>>(h.Q, h.B, h.meta, h.adj, np, b, b1, h.P, it + 1 == iter ? d_pts : nullptr, h.border,
-                                   lock_edges, h.bad); N2M_COUNT(); }
+        if (it) n2m_launch(k_hc_a, g, 128, 0, s, h.P, h.Lo, h.meta, h.adj, np, a1, h.Q, h.B);
+        n2m_launch(k_hc_b, g, 128, 0, s, h.Q, h.B, h.meta, h.adj, np, b, b1, h.P, it + 1 == iter ? d_pts : nullptr, h.border,
+                   lock_edges, h.bad);
     }
     CKL();
     return N2M_OK;
@@ -387,13 +395,13 @@ n2m_status mesh_smooth_hc_backward(int np, double alpha, double beta, int iter, 
     // adjacency and border flags are the forward's; its vectors serve as scratch (P lambda, Q t1)
     const HcBufs h = hc_bufs(w, np);
     const unsigned g = sweep_grid(np);
-    { k_hcT_init<<<gs(np), 256, 0, s>>>(d_g, h.border, h.meta, np, lock_edges, h.P, d_go); N2M_COUNT(); }
+    n2m_launch(k_hcT_init, gs(np), 256, 0, s, d_g, h.border, h.meta, np, lock_edges, h.P, d_go);
     const float al = (float)alpha, be = (float)beta;
     const float ab = al * be, a1b = al * (1.f - be);
     const float c0 = be * (1.f - al), c1 = (1.f - be) * (2.f - al), c2 = 1.f - be;
     for (int it = 0; it < iter; it++) {
-        { k_hcT_a<<<g, 128, 0, s>>>(h.P, h.meta, h.adj, np, h.Q); N2M_COUNT(); }
-        { k_hcT_b<<<g, 128, 0, s>>>(h.P, h.Q, h.meta, h.adj, d_go, np, ab, a1b, c0, c1, c2, it + 1 == iter); N2M_COUNT(); }
+        n2m_launch(k_hcT_a, g, 128, 0, s, h.P, h.meta, h.adj, np, h.Q);
+        n2m_launch(k_hcT_b, g, 128, 0, s, h.P, h.Q, h.meta, h.adj, d_go, np, ab, a1b, c0, c1, c2, it + 1 == iter);
     }
     CKL();
     return N2M_OK;
@@ -422,6 +430,7 @@ static __device__ __align__(256) unsigned char g_noalloc_scratch[NA_TOTAL];
 
 // exclusive scan of n <= NA_V + 1 counts in one CTA (n is small by construction)
 __global__ void __launch_bounds__(1024) k_scan_small(unsigned *d, int n) {
+    grid_wait();
     __shared__ unsigned part[1024];
     __shared__ unsigned carry;
     if (threadIdx.x == 0) carry = 0;
@@ -474,7 +483,7 @@ extern "C" n2m_status n2m_smooth_hc_noalloc(vec3d *d_verts, const vec3i *d_tris,
     h.B = (float4 *)(base + NA_B);
     h.Lo = (float4 *)(base + NA_LO);
     CKS(hc_count(d_tris, nvert, ntri, h, s));
-    { k_scan_small<<<1, 1024, 0, s>>>(h.start, nvert + 1); N2M_COUNT(); }
+    n2m_launch(k_scan_small, 1, 1024, 0, s, h.start, nvert + 1);
     CKS(hc_run(d_verts, d_tris, nvert, ntri, alpha, beta, iter, lock_edges, h, s));
     // the validity flag comes back through pageable host memory: a plain copy, no allocation
     unsigned h_bad = 0;

@@ -39,6 +39,7 @@ __device__ __forceinline__ long long bin_of(float x) {
 }
 
 __global__ void __launch_bounds__(256) k_th_range(const float *__restrict__ v, long long n, ThRange *out) {
+    grid_wait();
     float mn = INFINITY, mx = -INFINITY;
     unsigned long long nn = 0;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
@@ -67,6 +68,7 @@ __global__ void __launch_bounds__(256) k_th_range(const float *__restrict__ v, l
 template <int NBINS>
 __global__ void __launch_bounds__(256) k_th_hist(const float *__restrict__ v, long long n, float mn, float scl,
                                                  unsigned *hist) {
+    grid_wait();
     __shared__ unsigned h[NBINS];
     for (int i = threadIdx.x; i < NBINS; i += blockDim.x) h[i] = 0;
     __syncthreads();
@@ -92,6 +94,7 @@ struct Best {
 };
 
 __global__ void __launch_bounds__(256) k_otsu3(const double *__restrict__ P, int nb, Best *out) {
+    grid_wait();
     const int l = blockIdx.x, m = l + 1 + threadIdx.x;
     Best b = {-INFINITY, 0xffffffffu};
     if (l < nb - 3 && m < nb - 2) {
@@ -174,7 +177,7 @@ n2m_status isolevel_otsu(const float *d_img, long long nvox, int mode123, Thresh
     // (1) range of the non-NaN voxels (src/isolevel.c:47-61)
     *h_r = ThRange{f2ord_host(INFINITY), f2ord_host(-INFINITY), 0, 0};
     CK(cudaMemcpyAsync(d_r, h_r, sizeof(ThRange), cudaMemcpyHostToDevice, s));
-    { k_th_range<<<grid_for(nvox), 256, 0, s>>>(d_img, nvox, d_r); N2M_COUNT(); }
+    n2m_launch(k_th_range, grid_for(nvox), 256, 0, s, d_img, nvox, d_r);
     CKL();
     CK(cudaMemcpyAsync(h_r, d_r, sizeof(ThRange), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
@@ -194,7 +197,7 @@ n2m_status isolevel_otsu(const float *d_img, long long nvox, int mode123, Thresh
                 // (2) percentile histogram (src/isolevel.c:83-101), walk (:102-133)
                 const float scl = (NB_RANGE - 1) / (mx - mn);
                 CK(cudaMemsetAsync(d_h1, 0, NB_RANGE * sizeof(unsigned), s));
-                { k_th_hist<NB_RANGE><<<grid_for(nvox), 256, 0, s>>>(d_img, nvox, mn, scl, d_h1); N2M_COUNT(); }
+                n2m_launch(k_th_hist<NB_RANGE>, grid_for(nvox), 256, 0, s, d_img, nvox, mn, scl, d_h1);
                 CKL();
                 CK(cudaMemcpyAsync(h_hist, d_h1, NB_RANGE * sizeof(unsigned), cudaMemcpyDeviceToHost, s));
                 CK(cudaStreamSynchronize(s));
@@ -226,7 +229,7 @@ n2m_status isolevel_otsu(const float *d_img, long long nvox, int mode123, Thresh
     // (3) Otsu histogram on the robust range (src/isolevel.c:250-262)
     const float scl = (NB_OTSU - 1) / (pct98 - pct2);
     CK(cudaMemsetAsync(d_h2, 0, NB_OTSU * sizeof(unsigned), s));
-    { k_th_hist<NB_OTSU><<<grid_for(nvox), 256, 0, s>>>(d_img, nvox, pct2, scl, d_h2); N2M_COUNT(); }
+    n2m_launch(k_th_hist<NB_OTSU>, grid_for(nvox), 256, 0, s, d_img, nvox, pct2, scl, d_h2);
     CKL();
     CK(cudaMemcpyAsync(h_hist, d_h2, NB_OTSU * sizeof(unsigned), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
@@ -244,7 +247,7 @@ n2m_status isolevel_otsu(const float *d_img, long long nvox, int mode123, Thresh
                                  P[(size_t)(hi + 1) * nb + 255];
             CKS(w.table.ensure((size_t)nb * nb * sizeof(double)));
             CK(cudaMemcpyAsync(w.table.p, P.data(), (size_t)nb * nb * sizeof(double), cudaMemcpyHostToDevice, s));
-            { k_otsu3<<<nb - 3, 256, 0, s>>>(w.table.as<double>(), nb, d_best); N2M_COUNT(); }
+            n2m_launch(k_otsu3, nb - 3, 256, 0, s, w.table.as<double>(), nb, d_best);
             CKL();
             CK(cudaMemcpyAsync(h_best, d_best, (nb - 3) * sizeof(Best), cudaMemcpyDeviceToHost, s));
             CK(cudaStreamSynchronize(s));

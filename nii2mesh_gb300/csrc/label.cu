@@ -61,6 +61,7 @@ __device__ __forceinline__ unsigned class_word(const unsigned *B, const LD &d, u
 // (bwlabel's).  A warp takes whole rows, 16 words at a time in flight.
 __global__ void __launch_bounds__(256) k_lab_bits(const float *__restrict__ vol, LD d, float iso, bool nonzero,
                                                   unsigned *B) {
+    grid_wait();
     constexpr int K = 16;
     const int lane = threadIdx.x & 31;
     for (unsigned r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < d.nrows; r += (gridDim.x * blockDim.x) >> 5) {
@@ -88,6 +89,7 @@ __global__ void __launch_bounds__(256) k_lab_bits(const float *__restrict__ vol,
 // Class bits from a sign bitmap (bit = value >= iso; OdWork::vsign layout:
 // wv = W words per row, the 8 row words of a 32 x 8 tile of a slice adjacent)
 __global__ void k_lab_bits_vsign(const unsigned *__restrict__ vsign, LD d, unsigned nys, unsigned *B) {
+    grid_wait();
     for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < d.nwords; i += gridDim.x * blockDim.x) {
         const unsigned r = i / d.W, w = i - r * d.W, z = r / (unsigned)d.ny, y = r - z * (unsigned)d.ny;
         B[i] = __ldg(vsign + od_vsign_word(w * 32u, y, z, d.W, nys)) & valid_bits(d, w);
@@ -107,6 +109,7 @@ static_assert(dir_x(0) == 0 && dir_x(1) == 0 && dir_x(2) == -1 && dir_x(3) == 1 
 // cs[i]: where (x) the run that reaches into word i from the word before it starts (-1: no run start before the word).
 // `seg` lanes (a power of two, one word per lane) per row, rows of more than 32 words in chunks of 32.
 __global__ void __launch_bounds__(256) k_run_starts(const unsigned *__restrict__ B, LD d, unsigned want, int *cs) {
+    grid_wait();
     const int lane = threadIdx.x & 31, seg = d.seg, li = lane & (seg - 1);
     const unsigned rpw = 32u / (unsigned)seg, rsub = (unsigned)lane / (unsigned)seg;
     const unsigned nw = (gridDim.x * blockDim.x) >> 5;
@@ -173,6 +176,7 @@ struct Around {
 constexpr int LIST_K = 8;   // words per thread
 __global__ void __launch_bounds__(256) k_run_list(const unsigned *__restrict__ B, LD d, unsigned want, int *list, unsigned *wlist,
                                                   unsigned *nlist, unsigned *nwlist) {
+    grid_wait();
     __shared__ unsigned wsum[8], base, wbase;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     for (unsigned i0 = blockIdx.x * 256 * LIST_K; i0 < d.nwords; i0 += gridDim.x * 256 * LIST_K) {
@@ -236,6 +240,7 @@ template <int NNB>
 __global__ void __launch_bounds__(256) k_run_hook(const unsigned *__restrict__ B, LD d, unsigned want, const int *__restrict__ cs,
                                                   const int *__restrict__ list, const unsigned *__restrict__ nlist, int *L,
                                                   unsigned char *z8, unsigned *z32) {
+    grid_wait();
     const unsigned n = *nlist;
     for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const int s = list[i];
@@ -264,6 +269,7 @@ __global__ void __launch_bounds__(256) k_run_hook(const unsigned *__restrict__ B
 // walks are a few links long.
 constexpr int JUMPS = 4;
 __global__ void __launch_bounds__(256) k_run_jump(const int *__restrict__ list, const unsigned *__restrict__ nlist, int *L) {
+    grid_wait();
     const unsigned n = *nlist;
     volatile int *V = L;
     for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -294,6 +300,7 @@ __global__ void __launch_bounds__(256) k_run_jump(const int *__restrict__ list, 
 template <int NNB>
 __global__ void __launch_bounds__(256) k_run_merge(const unsigned *__restrict__ B, LD d, unsigned want, const int *__restrict__ cs,
                                                    const unsigned *__restrict__ wlist, const unsigned *__restrict__ nwlist, int *L) {
+    grid_wait();
     constexpr int ND = ndirs(NNB);
     const unsigned n = *nwlist;
     for (unsigned j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
@@ -336,6 +343,7 @@ __global__ void __launch_bounds__(256) k_run_merge(const unsigned *__restrict__ 
 // stored with a lower ancestor).
 __global__ void __launch_bounds__(256) k_run_flatten(const int *__restrict__ list, const unsigned *__restrict__ nlist, int *L,
                                                      unsigned *nroots) {
+    grid_wait();
     const unsigned n = *nlist;
     unsigned cnt = 0;
     for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -352,6 +360,7 @@ __global__ void __launch_bounds__(256) k_run_flatten(const int *__restrict__ lis
 // after them one word each of the rows on a y or z face (every run in it).  A
 // flag is stored only if it is not set yet (most items name the same root).
 __global__ void k_run_edges(const unsigned *__restrict__ B, LD d, const int *__restrict__ L, unsigned char *edge) {
+    grid_wait();
     const unsigned nzf = d.nz > 1 ? 2u : 1u, nyf = d.ny > 1 ? 2u : 1u;
     const unsigned zrows = nzf * (unsigned)d.ny, yrows = d.nz > 2 ? nyf * (unsigned)(d.nz - 2) : 0u;
     const unsigned total = d.nrows + (zrows + yrows) * d.W;
@@ -414,6 +423,7 @@ __global__ void __launch_bounds__(256) k_run_fill(const unsigned *__restrict__ B
                                                   const unsigned *__restrict__ nlist, const int *__restrict__ L,
                                                   const unsigned char *__restrict__ edge, const unsigned *__restrict__ nbg,
                                                   unsigned *out) {
+    grid_wait();
     if (*nbg <= 1) return;
     const unsigned n = *nlist;
     for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -428,6 +438,7 @@ __global__ void __launch_bounds__(256) k_run_fill(const unsigned *__restrict__ B
 // adds up what belongs to the heaviest root of its first lane.
 __global__ void __launch_bounds__(256) k_run_sizes(const unsigned *__restrict__ B, LD d, const int *__restrict__ list,
                                                    const unsigned *__restrict__ nlist, const int *__restrict__ L, unsigned *cnt) {
+    grid_wait();
     __shared__ int hot;
     __shared__ unsigned total;
     const unsigned n = *nlist;
@@ -469,6 +480,7 @@ __global__ void __launch_bounds__(256) k_run_sizes(const unsigned *__restrict__ 
 __global__ void __launch_bounds__(256) k_run_best(const int *__restrict__ list, const unsigned *__restrict__ nlist,
                                                   const int *__restrict__ L, const unsigned *__restrict__ cnt,
                                                   unsigned long long *best) {
+    grid_wait();
     const unsigned n = *nlist;
     unsigned long long b = 0;
     for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -488,6 +500,7 @@ __global__ void __launch_bounds__(256) k_run_best(const int *__restrict__ list, 
 __global__ void __launch_bounds__(256) k_run_keep(const unsigned *__restrict__ B, LD d, const int *__restrict__ list,
                                                   const unsigned *__restrict__ nlist, const int *__restrict__ L,
                                                   const unsigned long long *__restrict__ best, unsigned *K) {
+    grid_wait();
     const unsigned long long bk = *best;
     if (!bk) return;
     const int root = (int)(0xffffffffu - (unsigned)(bk & 0xffffffffu));
@@ -499,6 +512,7 @@ __global__ void __launch_bounds__(256) k_run_keep(const unsigned *__restrict__ B
 }
 
 __global__ void k_nl_from(const unsigned *nroots, bool only_largest, int *nl) {
+    grid_wait();
     *nl = only_largest ? (*nroots > 0 ? 1 : 0) : (int)*nroots;
 }
 
@@ -517,6 +531,7 @@ __global__ void k_nl_from(const unsigned *nroots, bool only_largest, int *nl) {
 // row y-1 in slice z-1.  A lane per word, 32 consecutive words per warp.
 __global__ void __launch_bounds__(256) k_lab_shell(const unsigned *__restrict__ K, LD d, const float *__restrict__ vol, float iso,
                                                    bool at_or_above, unsigned *S, unsigned *KD, VolStats *st) {
+    grid_wait();
     smooth::Acc acc;
     acc.init();
     unsigned masked = 0;
@@ -594,6 +609,7 @@ __global__ void __launch_bounds__(256) k_lab_shell(const unsigned *__restrict__ 
 
 // the labelling's effect on the values marching cubes will read: the marked voxels of `need`
 __global__ void __launch_bounds__(256) k_lab_apply(const unsigned *__restrict__ need, LD d, LabelPost P, float *vol) {
+    grid_wait();
     const int lane = threadIdx.x & 31;
     const unsigned n32 = (d.nwords + 31u) & ~31u;
     for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n32; i += gridDim.x * blockDim.x) {   // whole warps
@@ -629,6 +645,7 @@ __global__ void __launch_bounds__(256) k_lab_apply(const unsigned *__restrict__ 
 template <bool LARGEST, bool FILL, bool ONE>   // ONE: rows of at most 32 words
 __global__ void __launch_bounds__(256) k_lab_final(const unsigned *__restrict__ K, LD d, float *vol, float iso, float mn,
                                                    VolStats *st, bool vec4) {
+    grid_wait();
     smooth::Acc acc;
     acc.init();
     unsigned masked = 0;
@@ -727,6 +744,7 @@ __global__ void __launch_bounds__(256) k_lab_final(const unsigned *__restrict__ 
 
 // bwlabel() output: 0/1 of the kept set
 __global__ void __launch_bounds__(256) k_write_keep(const unsigned *__restrict__ K, LD d, float *vol) {
+    grid_wait();
     const int lane = threadIdx.x & 31;
     for (unsigned r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < d.nrows; r += (gridDim.x * blockDim.x) >> 5) {
         float *row = vol + (long long)r * d.nx;
@@ -741,6 +759,7 @@ __global__ void __launch_bounds__(256) k_write_keep(const unsigned *__restrict__
 // bwlabel() labels: 1 + rank of the component's root among the roots in
 // raster order.  Roots per word, then (after a scan) each root's rank.
 __global__ void k_root_count(const unsigned *__restrict__ B, LD d, const int *__restrict__ L, unsigned *rc) {
+    grid_wait();
     for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < d.nwords; i += gridDim.x * blockDim.x) {
         const unsigned r = i / d.W, w = i - r * d.W;
         const unsigned c = class_word(B, d, r, w, 1u), pc = w ? class_word(B, d, r, w - 1, 1u) : 0u;
@@ -756,6 +775,7 @@ __global__ void k_root_count(const unsigned *__restrict__ B, LD d, const int *__
 
 __global__ void k_root_rank(const unsigned *__restrict__ B, LD d, const int *__restrict__ L,
                             const unsigned *__restrict__ rc, unsigned *rank) {
+    grid_wait();
     for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < d.nwords; i += gridDim.x * blockDim.x) {
         const unsigned r = i / d.W, w = i - r * d.W;
         const unsigned c = class_word(B, d, r, w, 1u), pc = w ? class_word(B, d, r, w - 1, 1u) : 0u;
@@ -770,6 +790,7 @@ __global__ void k_root_rank(const unsigned *__restrict__ B, LD d, const int *__r
 
 __global__ void __launch_bounds__(256) k_write_labels(const unsigned *__restrict__ B, LD d, const int *__restrict__ L,
                                                       const unsigned *__restrict__ rank, float *vol) {
+    grid_wait();
     const int lane = threadIdx.x & 31;
     for (unsigned r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < d.nrows; r += (gridDim.x * blockDim.x) >> 5) {
         float *row = vol + (long long)r * d.nx;
@@ -840,17 +861,17 @@ n2m_status components(LabelWork &w, const LD &d, const unsigned *B, unsigned wan
     const unsigned lg = std::max(1u, std::min((d.nwords + 256 * LIST_K - 1) / (256 * LIST_K), 152u * 16u));
     const unsigned g = run_grid(d), wg = gsz(d.nwords);
     unsigned *wlist = w.wlist.as<unsigned>(), *nwlist = &misc->nwlist[want];
-    { k_run_starts<<<rgrid(d), 256, 0, s>>>(B, d, want, cs); N2M_COUNT(); }
-    { k_run_list<<<lg, 256, 0, s>>>(B, d, want, list, wlist, nlist, nwlist); N2M_COUNT(); }
-    if (conn == 6) { k_run_hook<3><<<g, 256, 0, s>>>(B, d, want, cs, list, nlist, L, z8, z32); N2M_COUNT(); }
-    else if (conn == 18) { k_run_hook<9><<<g, 256, 0, s>>>(B, d, want, cs, list, nlist, L, z8, z32); N2M_COUNT(); }
-    else { k_run_hook<13><<<g, 256, 0, s>>>(B, d, want, cs, list, nlist, L, z8, z32); N2M_COUNT(); }
+    n2m_launch(k_run_starts, rgrid(d), 256, 0, s, B, d, want, cs);
+    n2m_launch(k_run_list, lg, 256, 0, s, B, d, want, list, wlist, nlist, nwlist);
+    if (conn == 6) n2m_launch(k_run_hook<3>, g, 256, 0, s, B, d, want, cs, list, nlist, L, z8, z32);
+    else if (conn == 18) n2m_launch(k_run_hook<9>, g, 256, 0, s, B, d, want, cs, list, nlist, L, z8, z32);
+    else n2m_launch(k_run_hook<13>, g, 256, 0, s, B, d, want, cs, list, nlist, L, z8, z32);
     // once every start points at its tree's root, nearly every contact of the merge joins equal links
-    { k_run_jump<<<g, 256, 0, s>>>(list, nlist, L); N2M_COUNT(); }
-    if (conn == 6) { k_run_merge<3><<<wg, 256, 0, s>>>(B, d, want, cs, wlist, nwlist, L); N2M_COUNT(); }
-    else if (conn == 18) { k_run_merge<9><<<wg, 256, 0, s>>>(B, d, want, cs, wlist, nwlist, L); N2M_COUNT(); }
-    else { k_run_merge<13><<<wg, 256, 0, s>>>(B, d, want, cs, wlist, nwlist, L); N2M_COUNT(); }
-    { k_run_flatten<<<g, 256, 0, s>>>(list, nlist, L, want ? &misc->nfg : &misc->nbg); N2M_COUNT(); }
+    n2m_launch(k_run_jump, g, 256, 0, s, list, nlist, L);
+    if (conn == 6) n2m_launch(k_run_merge<3>, wg, 256, 0, s, B, d, want, cs, wlist, nwlist, L);
+    else if (conn == 18) n2m_launch(k_run_merge<9>, wg, 256, 0, s, B, d, want, cs, wlist, nwlist, L);
+    else n2m_launch(k_run_merge<13>, wg, 256, 0, s, B, d, want, cs, wlist, nwlist, L);
+    n2m_launch(k_run_flatten, g, 256, 0, s, list, nlist, L, want ? &misc->nfg : &misc->nbg);
     CKL();
     return N2M_OK;
 }
@@ -871,9 +892,11 @@ n2m_status label_core(LabelWork &w, const LD &d, int conn, bool only_largest, bo
         CKS(w.edge.ensure((size_t)d.n));
         CKS(w.filled.ensure((size_t)d.nwords * sizeof(unsigned)));
         CKS(components(w, d, B, 0u, 6, misc, w.edge.as<unsigned char>(), nullptr, s));
-        { k_run_edges<<<gsz((long long)d.nrows + 4ll * (d.nx + d.ny + d.nz) * d.W), 256, 0, s>>>(B, d, w.lab.as<int>(), w.edge.as<unsigned char>()); N2M_COUNT(); }
+        n2m_launch(k_run_edges, gsz((long long)d.nrows + 4ll * (d.nx + d.ny + d.nz) * d.W), 256, 0, s, B, d, w.lab.as<int>(),
+                   w.edge.as<unsigned char>());
         CK(cudaMemcpyAsync(w.filled.p, B, (size_t)d.nwords * sizeof(unsigned), cudaMemcpyDeviceToDevice, s));
-        { k_run_fill<<<run_grid(d), 256, 0, s>>>(B, d, w.list.as<int>(), &misc->nlist[0], w.lab.as<int>(), w.edge.as<unsigned char>(), &misc->nbg, w.filled.as<unsigned>()); N2M_COUNT(); }
+        n2m_launch(k_run_fill, run_grid(d), 256, 0, s, B, d, w.list.as<int>(), &misc->nlist[0], w.lab.as<int>(),
+                   w.edge.as<unsigned char>(), &misc->nbg, w.filled.as<unsigned>());
         CKL();
         B = w.filled.as<unsigned>();
     }
@@ -883,12 +906,15 @@ n2m_status label_core(LabelWork &w, const LD &d, int conn, bool only_largest, bo
     if (only_largest) {
         CKS(w.keep.ensure((size_t)d.nwords * sizeof(unsigned)));
         CK(cudaMemsetAsync(w.keep.p, 0, (size_t)d.nwords * sizeof(unsigned), s));
-        { k_run_sizes<<<run_grid(d), 256, 0, s>>>(B, d, w.list.as<int>(), &misc->nlist[1], w.lab.as<int>(), w.cnt.as<unsigned>()); N2M_COUNT(); }
-        { k_run_best<<<run_grid(d), 256, 0, s>>>(w.list.as<int>(), &misc->nlist[1], w.lab.as<int>(), w.cnt.as<unsigned>(), &misc->best); N2M_COUNT(); }
-        { k_run_keep<<<run_grid(d), 256, 0, s>>>(B, d, w.list.as<int>(), &misc->nlist[1], w.lab.as<int>(), &misc->best, w.keep.as<unsigned>()); N2M_COUNT(); }
+        n2m_launch(k_run_sizes, run_grid(d), 256, 0, s, B, d, w.list.as<int>(), &misc->nlist[1], w.lab.as<int>(),
+                   w.cnt.as<unsigned>());
+        n2m_launch(k_run_best, run_grid(d), 256, 0, s, w.list.as<int>(), &misc->nlist[1], w.lab.as<int>(), w.cnt.as<unsigned>(),
+                   &misc->best);
+        n2m_launch(k_run_keep, run_grid(d), 256, 0, s, B, d, w.list.as<int>(), &misc->nlist[1], w.lab.as<int>(), &misc->best,
+                   w.keep.as<unsigned>());
         *keep = w.keep.as<unsigned>();
     }
-    { k_nl_from<<<1, 1, 0, s>>>(&misc->nfg, only_largest, &misc->nl); N2M_COUNT(); }
+    n2m_launch(k_nl_from, 1, 1, 0, s, &misc->nfg, only_largest, &misc->nl);
     CKL();
     return N2M_OK;
 }
@@ -899,7 +925,7 @@ n2m_status class_bits(LabelWork &w, const LD &d, const float *vol, float iso, bo
         return N2M_ERR_TOO_LARGE;
     }
     CKS(w.mask.ensure((size_t)d.nwords * sizeof(unsigned)));
-    { k_lab_bits<<<wgrid(d), 256, 0, s>>>(vol, d, iso, nonzero, w.mask.as<unsigned>()); N2M_COUNT(); }
+    n2m_launch(k_lab_bits, wgrid(d), 256, 0, s, vol, d, iso, nonzero, w.mask.as<unsigned>());
     CKL();
     return N2M_OK;
 }
@@ -915,7 +941,7 @@ n2m_status run_labelling(const float *vol, int nx, int ny, int nz, float iso, fl
             return N2M_ERR_TOO_LARGE;
         }
         CKS(w.mask.ensure((size_t)d.nwords * sizeof(unsigned)));
-        { k_lab_bits_vsign<<<gsz(d.nwords), 256, 0, s>>>(vsign, d, (unsigned)(ny + 7) / 8, w.mask.as<unsigned>()); N2M_COUNT(); }
+        n2m_launch(k_lab_bits_vsign, gsz(d.nwords), 256, 0, s, vsign, d, (unsigned)(ny + 7) / 8, w.mask.as<unsigned>());
         CKL();
     } else {
         CKS(class_bits(w, d, vol, iso, false, s));
@@ -927,7 +953,7 @@ n2m_status run_labelling(const float *vol, int nx, int ny, int nz, float iso, fl
     if (only_largest && !(below > -N2M_FLT_EPS)) {
         CKS(w.shell.ensure(2 * (size_t)d.nwords * sizeof(unsigned)));
         unsigned *S = w.shell.as<unsigned>(), *KD = S + d.nwords;
-        { k_lab_shell<<<std::min(gsz(d.nwords), 152u * 16u), 256, 0, s>>>(K, d, vol, iso, at_or_above, S, KD, st); N2M_COUNT(); }
+        n2m_launch(k_lab_shell, std::min(gsz(d.nwords), 152u * 16u), 256, 0, s, K, d, vol, iso, at_or_above, S, KD, st);
         CKL();
         post->S = S;
         post->KD = KD;
@@ -941,19 +967,21 @@ n2m_status lab_write(float *vol, int nx, int ny, int nz, const LabelPost &P, Vol
     const bool v4 = nx % 4 == 0 && ((uintptr_t)vol & 15) == 0, one = d.W <= 32;
     const unsigned *K = P.K;
     const float iso = P.iso, mn = P.mn;
-    if (P.largest && P.fill && one) { k_lab_final<true, true, true><<<g, 256, 0, s>>>(K, d, vol, iso, mn, st, v4); N2M_COUNT(); }
-    else if (P.largest && P.fill) { k_lab_final<true, true, false><<<g, 256, 0, s>>>(K, d, vol, iso, mn, st, v4); N2M_COUNT(); }
-    else if (P.largest && one) { k_lab_final<true, false, true><<<g, 256, 0, s>>>(K, d, vol, iso, mn, st, v4); N2M_COUNT(); }
-    else if (P.largest) { k_lab_final<true, false, false><<<g, 256, 0, s>>>(K, d, vol, iso, mn, st, v4); N2M_COUNT(); }
-    else if (P.fill) { k_lab_final<false, true, false><<<g, 256, 0, s>>>(K, d, vol, iso, mn, st, v4); N2M_COUNT(); }
-    else { k_lab_final<false, false, false><<<g, 256, 0, s>>>(K, d, vol, iso, mn, st, v4); N2M_COUNT(); }
+    if (P.largest && P.fill && one) n2m_launch(k_lab_final<true, true, true>, g, 256, 0, s, K, d, vol, iso, mn, st,
+                                               v4);
+    else if (P.largest && P.fill) n2m_launch(k_lab_final<true, true, false>, g, 256, 0, s, K, d, vol, iso, mn, st,
+                                             v4);
+    else if (P.largest && one) n2m_launch(k_lab_final<true, false, true>, g, 256, 0, s, K, d, vol, iso, mn, st, v4);
+    else if (P.largest) n2m_launch(k_lab_final<true, false, false>, g, 256, 0, s, K, d, vol, iso, mn, st, v4);
+    else if (P.fill) n2m_launch(k_lab_final<false, true, false>, g, 256, 0, s, K, d, vol, iso, mn, st, v4);
+    else n2m_launch(k_lab_final<false, false, false>, g, 256, 0, s, K, d, vol, iso, mn, st, v4);
     CKL();
     return N2M_OK;
 }
 
 n2m_status lab_apply(float *vol, int nx, int ny, int nz, const unsigned *need, const LabelPost &P, cudaStream_t s) {
     const LD d = make_ld(nx, ny, nz);
-    { k_lab_apply<<<std::min(gsz(d.nwords), 152u * 16u), 256, 0, s>>>(need, d, P, vol); N2M_COUNT(); }
+    n2m_launch(k_lab_apply, std::min(gsz(d.nwords), 152u * 16u), 256, 0, s, need, d, P, vol);
     CKL();
     return N2M_OK;
 }
@@ -965,17 +993,17 @@ n2m_status run_bwlabel(float *vol, int nx, int ny, int nz, int conn, bool only_l
     const unsigned *K;
     CKS(label_core(w, d, conn, only_largest, fill_bubbles, s, &K));
     if (only_largest) {
-        { k_write_keep<<<wgrid(d), 256, 0, s>>>(K, d, vol); N2M_COUNT(); }
+        n2m_launch(k_write_keep, wgrid(d), 256, 0, s, K, d, vol);
     } else {
         CKS(w.rc.ensure(((size_t)d.nwords + 1) * sizeof(unsigned)));
         CKS(w.cnt.ensure((size_t)d.n * sizeof(unsigned)));
         unsigned *rc = w.rc.as<unsigned>();
         CK(cudaMemsetAsync(rc + d.nwords, 0, sizeof(unsigned), s));
-        { k_root_count<<<gsz(d.nwords), 256, 0, s>>>(K, d, w.lab.as<int>(), rc); N2M_COUNT(); }
+        n2m_launch(k_root_count, gsz(d.nwords), 256, 0, s, K, d, w.lab.as<int>(), rc);
         CKL();
         CKS(scan_u32(rc, (size_t)d.nwords + 1, rc + d.nwords, sw, s));
-        { k_root_rank<<<gsz(d.nwords), 256, 0, s>>>(K, d, w.lab.as<int>(), rc, w.cnt.as<unsigned>()); N2M_COUNT(); }
-        { k_write_labels<<<wgrid(d), 256, 0, s>>>(K, d, w.lab.as<int>(), w.cnt.as<unsigned>(), vol); N2M_COUNT(); }
+        n2m_launch(k_root_rank, gsz(d.nwords), 256, 0, s, K, d, w.lab.as<int>(), rc, w.cnt.as<unsigned>());
+        n2m_launch(k_write_labels, wgrid(d), 256, 0, s, K, d, w.lab.as<int>(), w.cnt.as<unsigned>(), vol);
     }
     CK(cudaMemcpyAsync(d_nl, &w.misc.as<Misc>()->nl, sizeof(int), cudaMemcpyDeviceToDevice, s));
     CKL();

@@ -98,6 +98,7 @@ __device__ __forceinline__ unsigned border_word(const GV &g, long long rb, bool 
 }
 
 __global__ void __launch_bounds__(256) k_signs(GV g, unsigned nrows, unsigned *signs) {
+    grid_wait();
     const int lane = threadIdx.x & 31, WX = (int)g.WX;
     const int vb0 = g.lo0 - g.xoff;   // voxel column of a row's first bit
     // words whose 32 points lie strictly inside the volume in x and inside the grid
@@ -151,6 +152,7 @@ struct SignMap {
 // the padding's sign is the same for every padding point.  512^3 (cold caches): 98 us
 // when the border words (two per row of 16) still read their voxels, 25 us now.
 __global__ void __launch_bounds__(256) k_signs_bits(GV g, unsigned nwords, unsigned *signs, SignMap map) {
+    grid_wait();
     const bool dark = __fsub_rn(g.edge_max, g.iso) > -N2M_FLT_EPS, padp = g.pad > -N2M_FLT_EPS;
     auto voxel = [&](int x, int y, int z) {   // sign of a voxel of a y or z row past the volume too; x = 0
         if (y >= g.dy) {
@@ -386,6 +388,7 @@ __device__ __forceinline__ float comp(const float3 &v, int a) { return a == 0 ? 
 __global__ void __launch_bounds__(256) k_mc_backward(GV g, bool classic, const uint4 *__restrict__ words,
                                                      const uint4 *__restrict__ act, unsigned nactive,
                                                      const float3 *__restrict__ gv, float *gs) {
+    grid_wait();
     const unsigned lane = threadIdx.x & 31u;
     for (unsigned aw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; aw < nactive; aw += (gridDim.x * blockDim.x) >> 5) {
         const uint4 a = act[aw];
@@ -447,6 +450,7 @@ __global__ void __launch_bounds__(256) k_mc_backward(GV g, bool classic, const u
 // vertices within 1.5e-5 of a c-vertex candidate become weld candidates too
 __global__ void k_ccand(const vec3d *__restrict__ pts, int np, const int *__restrict__ cc, int ncc, int *cand,
                         unsigned *ncand, int cap) {
+    grid_wait();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < np; i += gridDim.x * blockDim.x) {
         const vec3d a = pts[i];
         for (int k = 0; k < ncc; k++) {
@@ -501,10 +505,10 @@ n2m_status mc_count(const McGrid &g, int variant, McWork &w, uint4 *d_total, cud
     const unsigned blocks = (unsigned)std::min<size_t>((nwords + 255) / 256, 152u * 16u), wv = (unsigned)(v.dx + 31) / 32u;
     if (post || repair) {
         const SignMap map{post ? post->S : od.vsign.as<unsigned>(), wv, post ? 0u : (unsigned)(v.dy + 7) / 8u, v.dy};
-        { k_signs_bits<<<blocks, 256, 0, s>>>(v, (unsigned)nwords, signs, map); N2M_COUNT(); }
+        n2m_launch(k_signs_bits, blocks, 256, 0, s, v, (unsigned)nwords, signs, map);
     } else {
         const unsigned nrows = (unsigned)g.n[1] * (unsigned)g.n[2];
-        { k_signs<<<std::min<unsigned>((nrows + 7) / 8, 152u * 16u), 256, 0, s>>>(v, nrows, signs); N2M_COUNT(); }
+        n2m_launch(k_signs, std::min<unsigned>((nrows + 7) / 8, 152u * 16u), 256, 0, s, v, nrows, signs);
     }
     const bool classic = variant == N2M_CUBES_CLASSIC_TABLE;
     const Policy pol{v, classic, nullptr, nullptr, nullptr, nullptr, nullptr, 0};
@@ -534,7 +538,8 @@ n2m_status mc_backward(const McGrid &g, int variant, McWork &w, const McCounts &
     const GV v = make_gv(g);
     if (c.nactive == 0) return N2M_OK;
     const unsigned blocks = std::min<unsigned>((c.nactive + 7) / 8, 152u * 16u);
-    { k_mc_backward<<<blocks, 256, 0, s>>>(v, variant == N2M_CUBES_CLASSIC_TABLE, w.words.as<uint4>(), w.act.as<uint4>(), c.nactive, d_gv, d_gs); N2M_COUNT(); }
+    n2m_launch(k_mc_backward, blocks, 256, 0, s, v, variant == N2M_CUBES_CLASSIC_TABLE, w.words.as<uint4>(), w.act.as<uint4>(),
+               c.nactive, d_gv, d_gs);
     CKL();
     return N2M_OK;
 }
@@ -543,7 +548,7 @@ n2m_status mc_ccand_scan(const vec3d *d_pts, int np, const int *d_ccand, int ncc
                          unsigned *d_ncand, int cand_cap, cudaStream_t s) {
     if (nccand <= 0) return N2M_OK;
     const int blocks = (np + 255) / 256 < 4096 ? (np + 255) / 256 : 4096;
-    { k_ccand<<<blocks > 0 ? blocks : 1, 256, 0, s>>>(d_pts, np, d_ccand, nccand, d_cand, d_ncand, cand_cap); N2M_COUNT(); }
+    n2m_launch(k_ccand, blocks > 0 ? blocks : 1, 256, 0, s, d_pts, np, d_ccand, nccand, d_cand, d_ncand, cand_cap);
     CKL();
     return N2M_OK;
 }

@@ -183,6 +183,7 @@ struct Marks {
 
 template <class P>
 __global__ void __launch_bounds__(256) k_words(P pol, const unsigned *__restrict__ signs, Out o, Marks marks) {
+    grid_wait();
     __shared__ unsigned qt[256], pre[8][32], cor[8][6][32], cnt[8][32], amb[8][32];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     qt[threadIdx.x] = pol.quick(threadIdx.x);
@@ -261,6 +262,7 @@ constexpr unsigned NO_TILING = 0xffffffffu;
 constexpr int AMB_T = 128, AMB_S = 32, AMB_W = 8;   // threads of k_amb, sub-tiles of a block, words of a warp at a time
 template <class P>
 __global__ void __launch_bounds__(AMB_T) k_amb(P pol, const unsigned *__restrict__ signs, Out o) {
+    grid_wait();
     __shared__ unsigned short list[AMB_S * SUB];
     __shared__ unsigned nlist, pre[4][32], cor[4][6][32], words[4][32];
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
@@ -339,6 +341,7 @@ __device__ __forceinline__ uint4 block_excl4(uint4 v, uint4 *wsum, int lane, int
 // (a template only so that each unit has its own)
 template <class P>
 __global__ void __launch_bounds__(TILE) k_sum(Out o) {
+    grid_wait();
     __shared__ uint4 wsum[8];
     __shared__ bool last;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
@@ -386,6 +389,7 @@ __device__ __forceinline__ uint4 sub_offset(const Out &o, unsigned s) { return a
 constexpr int FIN = 4;
 template <class P>
 __global__ void __launch_bounds__(256) k_finish(P pol, Out o, uint4 *act) {
+    grid_wait();
     const int lane = threadIdx.x & 31;
     const uint4 total = *o.total;
     for (unsigned s0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * FIN; s0 < o.nsub; s0 += ((gridDim.x * blockDim.x) >> 5) * FIN) {
@@ -458,6 +462,7 @@ struct EmitShared {
 template <class P>
 __global__ void __launch_bounds__(EW * 32, P::CTAS) k_emit(P pol, const unsigned *__restrict__ signs, Out o, const uint4 *__restrict__ act,
                                                            unsigned nact, unsigned G, vec3i *tris) {
+    grid_wait();
     const uint4 *__restrict__ words = o.words;
     __shared__ EmitShared shared[EW];
     __shared__ unsigned qt[256];
@@ -676,16 +681,17 @@ inline n2m_status prepare(McWork &w, size_t nwords, uint4 *d_total, Out &o) {
 template <class P>
 n2m_status count_signs(const P &pol, const unsigned *signs, const Out &o, const Marks &marks, cudaStream_t s) {
     CK(cudaMemsetAsync(o.ctr, 0, 4 * sizeof(unsigned), s));
-    { k_words<P><<<std::max(1u, std::min((o.nsub + 7) / 8, 152u * 32u)), 256, 0, s>>>(pol, signs, o, marks); N2M_COUNT(); }
+    n2m_launch(k_words<P>, std::max(1u, std::min((o.nsub + 7) / 8, 152u * 32u)), 256, 0, s, pol, signs, o, marks);
     CKL();
     return N2M_OK;
 }
 // the rest: values are final
 template <class P>
 n2m_status count_values(const P &pol, const unsigned *signs, McWork &w, const Out &o, bool tests, cudaStream_t s) {
-    if (tests) { k_amb<P><<<(o.nsub + AMB_S - 1) / AMB_S, AMB_T, 0, s>>>(pol, signs, o); N2M_COUNT(); }
-    { k_sum<P><<<(o.nsub + TILE - 1) / TILE, TILE, 0, s>>>(o); N2M_COUNT(); }
-    { k_finish<P><<<std::max(1u, std::min((o.nsub + 8 * FIN - 1) / (8 * FIN), 152u * 16u)), 256, 0, s>>>(pol, o, w.act.as<uint4>()); N2M_COUNT(); }
+    if (tests) n2m_launch(k_amb<P>, (o.nsub + AMB_S - 1) / AMB_S, AMB_T, 0, s, pol, signs, o);
+    n2m_launch(k_sum<P>, (o.nsub + TILE - 1) / TILE, TILE, 0, s, o);
+    n2m_launch(k_finish<P>, std::max(1u, std::min((o.nsub + 8 * FIN - 1) / (8 * FIN), 152u * 16u)), 256, 0, s, pol, o,
+               w.act.as<uint4>());
     CKL();
     return N2M_OK;
 }
@@ -715,7 +721,7 @@ n2m_status emit(const P &pol, const unsigned *signs, McWork &w, const Out &o, un
     const unsigned warps = (unsigned)n * EW;
     const unsigned G = nact >= 64u * warps ? 32u : (nact >= 16u * warps ? 16u : 8u);
     const unsigned blocks = std::min(((nact + G - 1) / G + EW - 1) / EW, (unsigned)n);
-    { k_emit<P><<<blocks, EW * 32, 0, s>>>(pol, signs, o, w.act.as<uint4>(), nact, G, d_tris); N2M_COUNT(); }
+    n2m_launch(k_emit<P>, blocks, EW * 32, 0, s, pol, signs, o, w.act.as<uint4>(), nact, G, d_tris);
     CKL();
     return N2M_OK;
 }

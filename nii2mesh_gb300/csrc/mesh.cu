@@ -27,6 +27,7 @@ __device__ __forceinline__ int lower_bound(const int *a, int n, int v) {
 __global__ void k_weld_verts(const vec3d *__restrict__ in, int np, const int *__restrict__ removed, int nrem,
                              const int *__restrict__ ov_id, const vec3d *__restrict__ ov_pos, int nov,
                              vec3d *__restrict__ out) {
+    grid_wait();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < np; i += gridDim.x * blockDim.x) {
         const int r = lower_bound(removed, nrem, i);
         if (r < nrem && removed[r] == i) continue;
@@ -37,6 +38,7 @@ __global__ void k_weld_verts(const vec3d *__restrict__ in, int np, const int *__
 
 __global__ void k_weld_tris(vec3i *t, int nt, const int *__restrict__ removed, const int *__restrict__ keep,
                             int nrem) {
+    grid_wait();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nt; i += gridDim.x * blockDim.x) {
         int v[3] = {t[i].x, t[i].y, t[i].z};
         for (int k = 0; k < 3; k++) {
@@ -110,6 +112,7 @@ constexpr int CB = 256;   // compaction tile = one CTA
 
 __global__ void __launch_bounds__(CB) k_deg_count(const vec3d *__restrict__ p, const vec3i *__restrict__ t, int nt,
                                                   unsigned *keep, unsigned *tile_cnt) {
+    grid_wait();
     const int i = blockIdx.x * CB + threadIdx.x;
     unsigned k = 0;
     if (i < nt) {
@@ -123,6 +126,7 @@ __global__ void __launch_bounds__(CB) k_deg_count(const vec3d *__restrict__ p, c
 
 __global__ void __launch_bounds__(CB) k_deg_compact(const vec3i *__restrict__ t, int nt, const unsigned *keep,
                                                     const unsigned *tile_off, vec3i *out) {
+    grid_wait();
     __shared__ unsigned wcnt[CB / 32];
     const int i = blockIdx.x * CB + threadIdx.x;
     const unsigned k = i < nt ? keep[i] : 0u;
@@ -140,6 +144,7 @@ __global__ void __launch_bounds__(CB) k_deg_compact(const vec3i *__restrict__ t,
 // position it kept
 __global__ void k_weld_back(const float3 *__restrict__ go, int nv_raw, const int *__restrict__ removed, int nrem,
                             const int *__restrict__ ov_id, const int *__restrict__ ov_src, int nov, float3 *graw) {
+    grid_wait();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nv_raw; i += gridDim.x * blockDim.x) {
         const int r = lower_bound(removed, nrem, i);
         if (r < nrem && removed[r] == i) continue;
@@ -154,6 +159,7 @@ __global__ void k_weld_back(const float3 *__restrict__ go, int nv_raw, const int
 
 __global__ void k_sform(vec3d *p, int np, double a0, double a1, double a2, double a3, double b0, double b1, double b2,
                         double b3, double c0, double c1, double c2, double c3) {
+    grid_wait();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < np; i += gridDim.x * blockDim.x) {
         const vec3d v = p[i];
         p[i].x = __dadd_rn(__dadd_rn(__dadd_rn(__dmul_rn(v.x, a0), __dmul_rn(v.y, a1)), __dmul_rn(v.z, a2)), a3);
@@ -163,6 +169,7 @@ __global__ void k_sform(vec3d *p, int np, double a0, double a1, double a2, doubl
 }
 
 __global__ void k_flip(vec3i *t, int nt) {
+    grid_wait();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nt; i += gridDim.x * blockDim.x) {
         const int x = t[i].x;
         t[i].x = t[i].y;
@@ -180,8 +187,8 @@ inline unsigned gs(size_t n) {
 n2m_status mesh_apply_weld(vec3d *d_pts, vec3i *d_tris, int np, int nt, const int *d_removed, const int *d_keep,
                            int nrem, const int *d_ov_id, const vec3d *d_ov_pos, int nov, vec3d *d_out,
                            cudaStream_t s) {
-    { k_weld_verts<<<gs(np), 256, 0, s>>>(d_pts, np, d_removed, nrem, d_ov_id, d_ov_pos, nov, d_out); N2M_COUNT(); }
-    { k_weld_tris<<<gs(nt), 256, 0, s>>>(d_tris, nt, d_removed, d_keep, nrem); N2M_COUNT(); }
+    n2m_launch(k_weld_verts, gs(np), 256, 0, s, d_pts, np, d_removed, nrem, d_ov_id, d_ov_pos, nov, d_out);
+    n2m_launch(k_weld_tris, gs(nt), 256, 0, s, d_tris, nt, d_removed, d_keep, nrem);
     CKL();
     return N2M_OK;
 }
@@ -195,10 +202,10 @@ n2m_status mesh_remove_degenerate(const vec3d *d_pts, const vec3i *d_tris_in, in
     }
     CKS(w.flags.ensure((size_t)nt * sizeof(unsigned)));
     CKS(w.tmp.ensure((size_t)tiles * sizeof(unsigned)));
-    { k_deg_count<<<tiles, CB, 0, s>>>(d_pts, d_tris_in, nt, w.flags.as<unsigned>(), w.tmp.as<unsigned>()); N2M_COUNT(); }
+    n2m_launch(k_deg_count, tiles, CB, 0, s, d_pts, d_tris_in, nt, w.flags.as<unsigned>(), w.tmp.as<unsigned>());
     CKL();
     CKS(scan_u32(w.tmp.as<unsigned>(), tiles, d_nt_out, sw, s));
-    { k_deg_compact<<<tiles, CB, 0, s>>>(d_tris_in, nt, w.flags.as<unsigned>(), w.tmp.as<unsigned>(), d_tris_out); N2M_COUNT(); }
+    n2m_launch(k_deg_compact, tiles, CB, 0, s, d_tris_in, nt, w.flags.as<unsigned>(), w.tmp.as<unsigned>(), d_tris_out);
     CKL();
     return N2M_OK;
 }
@@ -206,7 +213,7 @@ n2m_status mesh_remove_degenerate(const vec3d *d_pts, const vec3i *d_tris_in, in
 n2m_status mesh_weld_backward(const float3 *d_go, int np_final, int nv_raw, const int *d_removed, int nrem,
                               const int *d_ov_id, const int *d_ov_src, int nov, float3 *d_graw, cudaStream_t s) {
     CK(cudaMemsetAsync(d_graw, 0, (size_t)nv_raw * sizeof(float3), s));
-    { k_weld_back<<<gs(nv_raw), 256, 0, s>>>(d_go, nv_raw, d_removed, nrem, d_ov_id, d_ov_src, nov, d_graw); N2M_COUNT(); }
+    n2m_launch(k_weld_back, gs(nv_raw), 256, 0, s, d_go, nv_raw, d_removed, nrem, d_ov_id, d_ov_src, nov, d_graw);
     CKL();
     (void)np_final;
     return N2M_OK;
@@ -214,12 +221,12 @@ n2m_status mesh_weld_backward(const float3 *d_go, int np_final, int nv_raw, cons
 
 n2m_status mesh_apply_sform(vec3d *d_pts, vec3i *d_tris, int np, int nt, const float sx[4], const float sy[4],
                             const float sz[4], cudaStream_t s) {
-    { k_sform<<<gs(np), 256, 0, s>>>(d_pts, np, sx[0], sx[1], sx[2], sx[3], sy[0], sy[1], sy[2], sy[3], sz[0], sz[1],
-                                   sz[2], sz[3]); N2M_COUNT(); }
+    n2m_launch(k_sform, gs(np), 256, 0, s, d_pts, np, sx[0], sx[1], sx[2], sx[3], sy[0], sy[1], sy[2], sy[3], sz[0], sz[1],
+               sz[2], sz[3]);
     const double px = (double)(sx[0] + sx[1] + sx[2]), py = (double)(sy[0] + sy[1] + sy[2]),
                  pz = (double)(sz[0] + sz[1] + sz[2]);
     const float det = (float)(px * py * pz);
-    if (det < 0.0) { k_flip<<<gs(nt), 256, 0, s>>>(d_tris, nt); N2M_COUNT(); }
+    if (det < 0.0) n2m_launch(k_flip, gs(nt), 256, 0, s, d_tris, nt);
     CKL();
     return N2M_OK;
 }

@@ -56,6 +56,7 @@ __device__ __forceinline__ int ocube_ntri(int ci) {
 // Signs from a volume: a warp per row, OS_W words at a time with all their loads in flight.
 constexpr int OS_W = 16;
 __global__ void __launch_bounds__(256) k_oc_signs(OV g, unsigned nrows, unsigned *signs) {
+    grid_wait();
     const int lane = threadIdx.x & 31;
     for (unsigned row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; row < nrows; row += (gridDim.x * blockDim.x) >> 5) {
         const int y = (int)(row % (unsigned)g.NY), z = (int)(row / (unsigned)g.NY);
@@ -88,6 +89,7 @@ __global__ void __launch_bounds__(256) k_oc_signs(OV g, unsigned nrows, unsigned
 // complement, and a darkened point is below the isolevel if its voxel or edge_max is.
 __global__ void __launch_bounds__(256) k_oc_signs_bits(OV g, unsigned nwords, unsigned *signs,
                                                        const unsigned *__restrict__ vsign, unsigned wv, unsigned nys) {
+    grid_wait();
     const bool dark = g.edge_max < g.iso;
     for (unsigned w = blockIdx.x * blockDim.x + threadIdx.x; w < nwords; w += gridDim.x * blockDim.x) {
         const unsigned row = w / g.WX, xw = w - row * g.WX;
@@ -204,6 +206,7 @@ struct Policy {
 
 // weld candidates as a bitmap over the vertices
 __global__ void k_oc_candbits(const int *__restrict__ cand, unsigned ncand, unsigned *bits) {
+    grid_wait();
     for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < ncand; i += gridDim.x * blockDim.x) {
         const unsigned v = (unsigned)cand[i];
         atomicOr(bits + (v >> 5), 1u << (v & 31u));
@@ -213,6 +216,7 @@ __global__ void k_oc_candbits(const int *__restrict__ cand, unsigned ncand, unsi
 // every triangle corner (3*t + c) that names a weld candidate (bit set)
 __global__ void k_oc_copies(const vec3i *__restrict__ tris, unsigned nt, const unsigned *__restrict__ bits,
                             unsigned *out, unsigned *count, unsigned cap) {
+    grid_wait();
     for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < nt; t += gridDim.x * blockDim.x) {
         const vec3i T = tris[t];
         const int v[3] = {T.x, T.y, T.z};
@@ -238,6 +242,7 @@ __constant__ unsigned char c_edge_ab[12][2] = {{0, 1}, {1, 2}, {2, 3}, {3, 0}, {
 __global__ void k_oc_copy_pos(OV g, const unsigned *__restrict__ signs, const uint4 *__restrict__ act, unsigned nact,
                               const vec3i *__restrict__ tris, const unsigned *__restrict__ qs, unsigned n, int *vid,
                               vec3d *pos) {
+    grid_wait();
     const double iso = (double)g.iso;
     for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const unsigned q = qs[i], t = q / 3u, c = q - 3u * t;
@@ -312,10 +317,11 @@ n2m_status oc_count(const float *vol, const int dim[3], const int lo[3], const i
     const unsigned wblocks = (unsigned)std::min<size_t>((nwords + 255) / 256, 152u * 16u);
     const unsigned wv = (unsigned)(g.dx + 31) / 32u;
     if (post || repair) {
-        { k_oc_signs_bits<<<wblocks, 256, 0, s>>>(g, (unsigned)nwords, signs, post ? post->S : od.vsign.as<unsigned>(), wv, post ? 0u : (unsigned)(g.dy + 7) / 8u); N2M_COUNT(); }
+        n2m_launch(k_oc_signs_bits, wblocks, 256, 0, s, g, (unsigned)nwords, signs, post ? post->S : od.vsign.as<unsigned>(),
+                   wv, post ? 0u : (unsigned)(g.dy + 7) / 8u);
     } else {
         const unsigned nrows = (unsigned)g.NY * (unsigned)g.NZ;
-        { k_oc_signs<<<std::min<unsigned>((nrows + 7) / 8, 152u * 16u), 256, 0, s>>>(g, nrows, signs); N2M_COUNT(); }
+        n2m_launch(k_oc_signs, std::min<unsigned>((nrows + 7) / 8, 152u * 16u), 256, 0, s, g, nrows, signs);
     }
     const Policy pol{g, nullptr, nullptr, nullptr, 0};
     mcw::Marks marks{nullptr, g.dx, g.dy, g.dz, wv};
@@ -341,8 +347,10 @@ n2m_status oc_copies(const vec3i *d_tris, int nt, int nv, const int *d_cand, int
                      unsigned *d_out, unsigned *d_count, unsigned cap, cudaStream_t s) {
     CK(cudaMemsetAsync(d_bits, 0, (size_t)(nv + 31) / 32 * sizeof(unsigned), s));
     CK(cudaMemsetAsync(d_count, 0, sizeof(unsigned), s));
-    { k_oc_candbits<<<(unsigned)std::max(1, std::min((ncand + 255) / 256, 1024)), 256, 0, s>>>(d_cand, (unsigned)ncand, d_bits); N2M_COUNT(); }
-    { k_oc_copies<<<(unsigned)std::max(1, std::min((nt + 255) / 256, 152 * 16)), 256, 0, s>>>(d_tris, (unsigned)nt, d_bits, d_out, d_count, cap); N2M_COUNT(); }
+    n2m_launch(k_oc_candbits, (unsigned)std::max(1, std::min((ncand + 255) / 256, 1024)), 256, 0, s, d_cand, (unsigned)ncand,
+               d_bits);
+    n2m_launch(k_oc_copies, (unsigned)std::max(1, std::min((nt + 255) / 256, 152 * 16)), 256, 0, s, d_tris, (unsigned)nt,
+               d_bits, d_out, d_count, cap);
     CKL();
     return N2M_OK;
 }
@@ -352,7 +360,8 @@ n2m_status oc_copy_positions(const float *vol, const int dim[3], const int lo[3]
                              int n, int *d_vid, vec3d *d_pos, cudaStream_t s) {
     const OV g = make_ov(vol, dim, lo, hi, iso, edge_max);
     if (n <= 0 || nactive == 0) return N2M_OK;
-    { k_oc_copy_pos<<<(unsigned)std::min((n + 127) / 128, 1024), 128, 0, s>>>(g, w.signs.as<unsigned>(), w.act.as<uint4>(), nactive, d_tris, d_q, (unsigned)n, d_vid, d_pos); N2M_COUNT(); }
+    n2m_launch(k_oc_copy_pos, (unsigned)std::min((n + 127) / 128, 1024), 128, 0, s, g, w.signs.as<unsigned>(),
+               w.act.as<uint4>(), nactive, d_tris, d_q, (unsigned)n, d_vid, d_pos);
     CKL();
     return N2M_OK;
 }

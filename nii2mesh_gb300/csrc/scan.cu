@@ -50,6 +50,7 @@ __device__ uint4 block_exscan(uint4 &v) {
 }
 
 __global__ void __launch_bounds__(SB) k_tile_sums(const uint4 *__restrict__ d, size_t n, uint4 *part) {
+    grid_wait();
     const size_t base = (size_t)blockIdx.x * TILE;
     uint4 s = make_uint4(0, 0, 0, 0);
     for (int i = 0; i < SI; i++) {
@@ -61,6 +62,7 @@ __global__ void __launch_bounds__(SB) k_tile_sums(const uint4 *__restrict__ d, s
 }
 
 __global__ void __launch_bounds__(SB) k_scan_parts(uint4 *part, size_t np, uint4 *total) {
+    grid_wait();
     uint4 carry = make_uint4(0, 0, 0, 0);
     for (size_t base = 0; base < np; base += SB) {
         const size_t k = base + threadIdx.x;
@@ -73,6 +75,7 @@ __global__ void __launch_bounds__(SB) k_scan_parts(uint4 *part, size_t np, uint4
 }
 
 __global__ void __launch_bounds__(SB) k_tile_scan(uint4 *d, size_t n, const uint4 *part) {
+    grid_wait();
     // each thread owns SI consecutive items of the tile
     const size_t base = (size_t)blockIdx.x * TILE + (size_t)threadIdx.x * SI;
     uint4 it[SI];
@@ -97,9 +100,9 @@ n2m_status scan_uint4(uint4 *d, size_t n, uint4 *d_total, ScanWork &w, cudaStrea
     }
     const size_t tiles = (n + TILE - 1) / TILE;
     CKS(w.part.ensure(tiles * sizeof(uint4)));
-    { k_tile_sums<<<(unsigned)tiles, SB, 0, s>>>(d, n, w.part.as<uint4>()); N2M_COUNT(); }
-    { k_scan_parts<<<1, SB, 0, s>>>(w.part.as<uint4>(), tiles, d_total); N2M_COUNT(); }
-    { k_tile_scan<<<(unsigned)tiles, SB, 0, s>>>(d, n, w.part.as<uint4>()); N2M_COUNT(); }
+    n2m_launch(k_tile_sums, (unsigned)tiles, SB, 0, s, d, n, w.part.as<uint4>());
+    n2m_launch(k_scan_parts, 1, SB, 0, s, w.part.as<uint4>(), tiles, d_total);
+    n2m_launch(k_tile_scan, (unsigned)tiles, SB, 0, s, d, n, w.part.as<uint4>());
     CKL();
     return N2M_OK;
 }
@@ -137,6 +140,7 @@ __device__ unsigned block_exscan_u32(unsigned &v) {
 }
 
 __global__ void __launch_bounds__(SB) k_tile_sums_u32(const unsigned *__restrict__ d, size_t n, unsigned *part) {
+    grid_wait();
     const size_t base = (size_t)blockIdx.x * TILE;
     unsigned s = 0;
     for (int i = 0; i < SI; i++) {
@@ -148,6 +152,7 @@ __global__ void __launch_bounds__(SB) k_tile_sums_u32(const unsigned *__restrict
 }
 
 __global__ void __launch_bounds__(SB) k_scan_parts_u32(unsigned *part, size_t np, unsigned *total) {
+    grid_wait();
     unsigned carry = 0;
     for (size_t base = 0; base < np; base += SB) {
         const size_t k = base + threadIdx.x;
@@ -160,6 +165,7 @@ __global__ void __launch_bounds__(SB) k_scan_parts_u32(unsigned *part, size_t np
 }
 
 __global__ void __launch_bounds__(SB) k_tile_scan_u32(unsigned *d, size_t n, const unsigned *part) {
+    grid_wait();
     const size_t base = (size_t)blockIdx.x * TILE + (size_t)threadIdx.x * SI;
     unsigned it[SI], s = 0;
     for (int i = 0; i < SI; i++) {
@@ -182,9 +188,9 @@ n2m_status scan_u32(unsigned *d, size_t n, unsigned *d_total, ScanWork &w, cudaS
     }
     const size_t tiles = (n + TILE - 1) / TILE;
     CKS(w.part.ensure(tiles * sizeof(unsigned)));
-    { k_tile_sums_u32<<<(unsigned)tiles, SB, 0, s>>>(d, n, w.part.as<unsigned>()); N2M_COUNT(); }
-    { k_scan_parts_u32<<<1, SB, 0, s>>>(w.part.as<unsigned>(), tiles, d_total); N2M_COUNT(); }
-    { k_tile_scan_u32<<<(unsigned)tiles, SB, 0, s>>>(d, n, w.part.as<unsigned>()); N2M_COUNT(); }
+    n2m_launch(k_tile_sums_u32, (unsigned)tiles, SB, 0, s, d, n, w.part.as<unsigned>());
+    n2m_launch(k_scan_parts_u32, 1, SB, 0, s, w.part.as<unsigned>(), tiles, d_total);
+    n2m_launch(k_tile_scan_u32, (unsigned)tiles, SB, 0, s, d, n, w.part.as<unsigned>());
     CKL();
     return N2M_OK;
 }

@@ -32,6 +32,7 @@ using namespace smooth;
 // stay few; every reduction is a min, max or count, so the order is free
 __global__ void __launch_bounds__(256) k_stats(const float *__restrict__ vol, int nx, int ny, int nz, float iso,
                                                VolStats *st, bool minmax) {
+    grid_wait();
     Acc acc;
     acc.init();
     const long long nrows = (long long)ny * nz;
@@ -175,6 +176,7 @@ __device__ __forceinline__ unsigned taps_run(const float (&w)[K + 4], float (&r)
 
 // x pass: each warp takes whole rows (rows row0 .. row1-1 of the volume).
 __global__ void __launch_bounds__(256) k_pass_x(Pass P, unsigned row0, unsigned row1) {
+    grid_wait();
     __shared__ unsigned stage_buf[8][64];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     FixStage<false> F{stage_buf[w], 0};   // < 32 entries between steps, + 32
@@ -209,6 +211,7 @@ __global__ void __launch_bounds__(256) k_pass_x(Pass P, unsigned row0, unsigned 
 // the neighbours' halves, mostly L1 hits) and one float4 store; voxels whose
 // fast path fails are stored as placeholders and fixed by the same warp.
 __global__ void __launch_bounds__(256) k_pass_x4(Pass P, unsigned row0, unsigned row1) {
+    grid_wait();
     __shared__ unsigned stage_buf[8][32 * 5];   // < 32 between drains, + 4 per lane per step
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     FixStage<false> F{stage_buf[w], 0};
@@ -258,6 +261,7 @@ __global__ void __launch_bounds__(256) k_pass_x4(Pass P, unsigned row0, unsigned
 template <int K, int SEGS, bool STATS>
 __global__ void __launch_bounds__(256, 4) k_pass_axis(Pass P, int len, unsigned outer0, unsigned nouter, int p_lo,
                                                       int p_hi) {
+    grid_wait();
     __shared__ unsigned stage_buf[8][32 * (K + 1)];   // < 32 entries between segments, + up to 32 K per segment
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     FixStage<STATS> F{stage_buf[wid], 0};
@@ -392,8 +396,8 @@ n2m_status launch_smooth(const float *in, float *out, float *tmp, int nx, int ny
     // 16-byte rows: the float4 x pass
     const bool x4 = nx % 4 == 0 && ((uintptr_t)in & 15) == 0 && ((uintptr_t)out & 15) == 0;
     auto pass_x = [&](unsigned r0, unsigned r1, unsigned g) -> n2m_status {
-        if (x4) { k_pass_x4<<<std::min<unsigned>(g, (unsigned)gx4), 256, 0, s>>>(px, r0, r1); N2M_COUNT(); }
-        else { k_pass_x<<<std::min<unsigned>(g, (unsigned)gx), 256, 0, s>>>(px, r0, r1); N2M_COUNT(); }
+        if (x4) n2m_launch(k_pass_x4, std::min<unsigned>(g, (unsigned)gx4), 256, 0, s, px, r0, r1);
+        else n2m_launch(k_pass_x, std::min<unsigned>(g, (unsigned)gx), 256, 0, s, px, r0, r1);
         CKL();
         return N2M_OK;
     };
@@ -413,17 +417,18 @@ n2m_status launch_smooth(const float *in, float *out, float *tmp, int nx, int ny
             CK(cudaStreamWaitEvent(s, stage->ev[k], 0));
             const unsigned r0 = (unsigned)z0 * ny, r1 = (unsigned)z1 * ny;
             CKS(pass_x(r0, r1, std::max<unsigned>(1u, (r1 - r0 + 7) / 8)));
-            { k_pass_axis<KRUN, KSEG, false><<<ga, 256, 0, s>>>(py, ny, (unsigned)z0, (unsigned)(z1 - z0), 0, ny); N2M_COUNT(); }
+            n2m_launch(k_pass_axis<KRUN, KSEG, false>, ga, 256, 0, s, py, ny, (unsigned)z0, (unsigned)(z1 - z0), 0,
+                       ny);
             const int zready = z1 == nz ? nz : z1 - 2;
             if (zready > zdone) {
-                { k_pass_axis<KRUN, KSEG, true><<<gz, 256, 0, s>>>(pz, nz, 0u, 1u, zdone, zready); N2M_COUNT(); }
+                n2m_launch(k_pass_axis<KRUN, KSEG, true>, gz, 256, 0, s, pz, nz, 0u, 1u, zdone, zready);
                 zdone = zready;
             }
         }
     } else {
         CKS(pass_x(0u, (unsigned)ny * nz, 0xffffffffu));
-        { k_pass_axis<KRUN, KSEG, false><<<ga, 256, 0, s>>>(py, ny, 0u, (unsigned)nz, 0, ny); N2M_COUNT(); }
-        { k_pass_axis<KRUN, KSEG, true><<<gz, 256, 0, s>>>(pz, nz, 0u, 1u, 0, nz); N2M_COUNT(); }
+        n2m_launch(k_pass_axis<KRUN, KSEG, false>, ga, 256, 0, s, py, ny, 0u, (unsigned)nz, 0, ny);
+        n2m_launch(k_pass_axis<KRUN, KSEG, true>, gz, 256, 0, s, pz, nz, 0u, 1u, 0, nz);
     }
     CKL();
     return N2M_OK;
@@ -433,6 +438,7 @@ namespace {
 // transposed 5-tap pass along one axis: out_j = sum over interior rows i with
 // |i-j| <= 2 of w_|i-j| g_i, plus g_j where j itself is a row left unfiltered
 __global__ void k_smooth_T(const float *__restrict__ g, float *__restrict__ out, int nx, int ny, int nz, int axis) {
+    grid_wait();
     const long long n = (long long)nx * ny * nz;
     const long long stride = axis == 0 ? 1 : (axis == 1 ? nx : (long long)nx * ny);
     const int len = axis == 0 ? nx : (axis == 1 ? ny : nz);
@@ -453,9 +459,9 @@ __global__ void k_smooth_T(const float *__restrict__ g, float *__restrict__ out,
 n2m_status launch_smooth_adjoint(const float *g, float *tmp, float *out, int nx, int ny, int nz, cudaStream_t s) {
     const long long n = (long long)nx * ny * nz;
     const unsigned blocks = (unsigned)std::min<long long>((n + 255) / 256, 152 * 64);
-    { k_smooth_T<<<blocks, 256, 0, s>>>(g, out, nx, ny, nz, 2); N2M_COUNT(); }
-    { k_smooth_T<<<blocks, 256, 0, s>>>(out, tmp, nx, ny, nz, 1); N2M_COUNT(); }
-    { k_smooth_T<<<blocks, 256, 0, s>>>(tmp, out, nx, ny, nz, 0); N2M_COUNT(); }
+    n2m_launch(k_smooth_T, blocks, 256, 0, s, g, out, nx, ny, nz, 2);
+    n2m_launch(k_smooth_T, blocks, 256, 0, s, out, tmp, nx, ny, nz, 1);
+    n2m_launch(k_smooth_T, blocks, 256, 0, s, tmp, out, nx, ny, nz, 0);
     CKL();
     return N2M_OK;
 }
@@ -464,7 +470,7 @@ n2m_status launch_stats(const float *vol, int nx, int ny, int nz, float iso, boo
                         cudaStream_t s) {
     const long long rows = (long long)ny * nz;
     const unsigned grid = (unsigned)std::max<long long>(1, std::min<long long>((rows + 7) / 8, 152 * 8));   // 8 rows per block
-    { k_stats<<<grid, 256, 0, s>>>(vol, nx, ny, nz, iso, st, minmax); N2M_COUNT(); }
+    n2m_launch(k_stats, grid, 256, 0, s, vol, nx, ny, nz, iso, st, minmax);
     CKL();
     return N2M_OK;
 }
@@ -633,6 +639,7 @@ __device__ __noinline__ unsigned list_undecided(const float *p, int nx, int rows
 __global__ void __launch_bounds__(OA_WARPS * 32, 3) k_od_approx(const __grid_constant__ CUtensorMap tmap, float *out,
                                                              int nx, int ny, int nz, int zrun, float iso, OdStats *st,
                                                              OdLists L) {
+    grid_wait();
     const unsigned FULL = 0xffffffffu;
     __shared__ OaStage stage[OA_WARPS][OA_S];
     __shared__ unsigned long long bars[OA_WARPS][OA_S];
@@ -858,6 +865,7 @@ __global__ void __launch_bounds__(OA_WARPS * 32, 3) k_od_approx(const __grid_con
 constexpr int OS_T = 64;
 __global__ void __launch_bounds__(256) k_od_scan(const float *__restrict__ out, int nx, int ny, int nz, int zrun,
                                                  OdStats *st, OdLists L) {
+    grid_wait();
     __shared__ unsigned todo[OS_T], ntodo;
     if (st->flags) return;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -909,6 +917,7 @@ __global__ void __launch_bounds__(256) k_od_scan(const float *__restrict__ out, 
 // another: 29 us for the 512^3 CT volume's few thousand voxels).
 __global__ void __launch_bounds__(256) k_od_resolve(const float *__restrict__ in, float *out, int nx, int ny, int nz,
                                                     float iso, OdStats *st, OdLists L, bool at_or_above) {
+    grid_wait();
     const unsigned FULL = 0xffffffffu;
     const unsigned nu = st->cnt[0], nmin = st->cnt[1], nmax = st->cnt[2], n = nu + nmin + nmax;
     if (st->flags || nu > L.cap || nmin > L.cap || nmax > L.cap) return;   // the caller falls back
@@ -974,6 +983,7 @@ __device__ __forceinline__ unsigned y_marks(const unsigned *__restrict__ need, u
 
 __global__ void __launch_bounds__(OL_T) k_od_lists(const unsigned *__restrict__ need, int nx, int nz, unsigned W, unsigned slice,
                                                    unsigned *cnt, uint2 *lz, uint2 *ly, uint2 *lx) {
+    grid_wait();
     __shared__ unsigned ym[OL_Z][OL_T + 4 * OL_MAXW];
     __shared__ unsigned wsum[3][OL_T / 32], base[3];
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
@@ -1070,6 +1080,7 @@ template <int AXIS>
 __global__ void __launch_bounds__(OE_T, 10) k_od_exact(const uint2 *__restrict__ list, const unsigned *__restrict__ cnt,
                                                    const float *__restrict__ src, float *dst, unsigned nx, unsigned ny, unsigned nz,
                                                    unsigned long long mnx, unsigned long long mny) {
+    grid_wait();
     __shared__ unsigned stage_buf[OE_T / 32][32 * (OE_U + 1)];   // < 32 between drains, + 32 per entry
     __shared__ unsigned short item[OE_T / 32][32 * 32];          // word << 5 | bit
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -1150,6 +1161,7 @@ __global__ void __launch_bounds__(OE_T, 10) k_od_exact(const uint2 *__restrict__
 // the labelling's effect on the exact values the z pass just wrote at the listed words' voxels
 __global__ void __launch_bounds__(256) k_od_post(const uint2 *__restrict__ list, const unsigned *__restrict__ cnt, float *out,
                                                  LabelPost L, int nx, int ny) {
+    grid_wait();
     const unsigned n = *cnt;
     const int lane = threadIdx.x & 31;
     for (unsigned i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += (gridDim.x * blockDim.x) >> 5) {   // a warp per word
@@ -1252,7 +1264,8 @@ n2m_status od_approx(const float *in, float *out, int nx, int ny, int nz, float 
     h.lmax = INT_MIN;
     CK(cudaMemcpyAsync(w.st.p, &h, sizeof(OdStats), cudaMemcpyHostToDevice, s));
     const unsigned grid = (unsigned)std::min<size_t>((ntask + OA_WARPS - 1) / OA_WARPS, (size_t)od_grid((const void *)k_od_approx, OA_WARPS * 32));
-    { k_od_approx<<<grid, OA_WARPS * 32, 0, s>>>(tmap, out, nx, ny, nz, zrun, iso, w.st.as<OdStats>(), od_lists(w, nx, ny)); N2M_COUNT(); }
+    n2m_launch(k_od_approx, grid, OA_WARPS * 32, 0, s, tmap, out, nx, ny, nz, zrun, iso, w.st.as<OdStats>(),
+               od_lists(w, nx, ny));
     CKL();
     return N2M_OK;
 }
@@ -1262,8 +1275,8 @@ n2m_status od_resolve(const float *in, float *out, int nx, int ny, int nz, float
     const OdLists L = od_lists(w, nx, ny);
     const int zrun = od_zrun(nx, ny, nz);
     const size_t ntask = od_tasks(nx, ny, nz, zrun);
-    { k_od_scan<<<(unsigned)((ntask + OS_T - 1) / OS_T), 256, 0, s>>>(out, nx, ny, nz, zrun, w.st.as<OdStats>(), L); N2M_COUNT(); }
-    { k_od_resolve<<<152 * 8, 256, 0, s>>>(in, out, nx, ny, nz, iso, w.st.as<OdStats>(), L, at_or_above); N2M_COUNT(); }
+    n2m_launch(k_od_scan, (unsigned)((ntask + OS_T - 1) / OS_T), 256, 0, s, out, nx, ny, nz, zrun, w.st.as<OdStats>(), L);
+    n2m_launch(k_od_resolve, 152 * 8, 256, 0, s, in, out, nx, ny, nz, iso, w.st.as<OdStats>(), L, at_or_above);
     CKL();
     return N2M_OK;
 }
@@ -1296,15 +1309,16 @@ n2m_status od_repair(const OdRepair &r, cudaStream_t s) {
     unsigned *cnt = w.lcnt.as<unsigned>();   // z, y, x counts
     uint2 *lz = w.list.as<uint2>(), *ly = lz + nw, *lx = ly + nw;
     CK(cudaMemsetAsync(cnt, 0, sizeof(uint4), s));
-    { k_od_lists<<<bps * (unsigned)((nz + OL_Z - 1) / OL_Z), OL_T, 0, s>>>(w.need.as<unsigned>(), nx, nz, W, slice, cnt, lz, ly, lx); N2M_COUNT(); }
+    n2m_launch(k_od_lists, bps * (unsigned)((nz + OL_Z - 1) / OL_Z), OL_T, 0, s, w.need.as<unsigned>(), nx, nz, W, slice, cnt,
+               lz, ly, lx);
     CKL();
     const int xb = od_grid((const void *)k_od_exact<0>, OE_T);
     const unsigned ux = (unsigned)nx, uy = (unsigned)ny, uz = (unsigned)nz;
     const unsigned long long mx = od_magic(ux), my = od_magic(uy);
-    { k_od_exact<0><<<xb, OE_T, 0, s>>>(lx, cnt + 2, r.in, r.tmp1, ux, uy, uz, mx, my); N2M_COUNT(); }
-    { k_od_exact<1><<<xb, OE_T, 0, s>>>(ly, cnt + 1, r.tmp1, r.tmp2, ux, uy, uz, mx, my); N2M_COUNT(); }
-    { k_od_exact<2><<<xb, OE_T, 0, s>>>(lz, cnt + 0, r.tmp2, r.out, ux, uy, uz, mx, my); N2M_COUNT(); }
-    if (r.post) { k_od_post<<<152 * 8, 256, 0, s>>>(lz, cnt + 0, r.out, *r.post, nx, ny); N2M_COUNT(); }
+    n2m_launch(k_od_exact<0>, xb, OE_T, 0, s, lx, cnt + 2, r.in, r.tmp1, ux, uy, uz, mx, my);
+    n2m_launch(k_od_exact<1>, xb, OE_T, 0, s, ly, cnt + 1, r.tmp1, r.tmp2, ux, uy, uz, mx, my);
+    n2m_launch(k_od_exact<2>, xb, OE_T, 0, s, lz, cnt + 0, r.tmp2, r.out, ux, uy, uz, mx, my);
+    if (r.post) n2m_launch(k_od_post, 152 * 8, 256, 0, s, lz, cnt + 0, r.out, *r.post, nx, ny);
     CKL();
     return N2M_OK;
 }

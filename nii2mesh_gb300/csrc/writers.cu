@@ -33,6 +33,7 @@ __device__ __forceinline__ unsigned f32_bits(double v) { return (unsigned)__floa
 
 // float32 vertices, 12 bytes each (be: byte-swapped as the reference's swap_4bytes)
 __global__ void k_pack_pts(const vec3d *__restrict__ p, int np, unsigned char *__restrict__ dst, int be) {
+    grid_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= np) return;
     const vec3d v = p[i];
@@ -44,6 +45,7 @@ __global__ void k_pack_pts(const vec3d *__restrict__ p, int np, unsigned char *_
 
 enum { TRI_LE12 = 0, TRI_BE12 = 1, TRI_PLY13 = 2, TRI_VTK16 = 3 };
 __global__ void k_pack_tris(const vec3i *__restrict__ t, int nt, unsigned char *__restrict__ dst, int mode) {
+    grid_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nt) return;
     const vec3i f = t[i];
@@ -72,6 +74,7 @@ __global__ void k_pack_tris(const vec3i *__restrict__ t, int nt, unsigned char *
 // outside [0, np) sets *bad and is written as the origin
 __global__ void k_pack_stl(const vec3i *__restrict__ t, const vec3d *__restrict__ p, int nt, int np,
                            unsigned char *__restrict__ dst, unsigned *__restrict__ bad) {
+    grid_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nt) return;
     const vec3i f = t[i];
@@ -92,6 +95,7 @@ __global__ void k_pack_stl(const vec3i *__restrict__ t, const vec3d *__restrict_
 // base64 (RFC 4648 alphabet, '=' padding, no line breaks: base64_encode of src/base64.c without USE_EOLN)
 __constant__ char c_b64[65] = "ABCDEFGHIJKLMNOPQRSTUVWXYZabcdefghijklmnopqrstuvwxyz0123456789+/";
 __global__ void k_base64(const unsigned char *__restrict__ in, long long n, unsigned char *__restrict__ out) {
+    grid_wait();
     const long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     const long long i = 3 * g;
     if (i >= n) return;
@@ -117,6 +121,7 @@ __device__ __forceinline__ void put_word(S &out, unsigned w, int n) {
 template <bool TRI>
 __global__ void k_txt_fmt(const void *__restrict__ src, int n, LineFmt f, unsigned *__restrict__ slots,
                           unsigned *__restrict__ lens) {
+    grid_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     n2mfmt::WordSink out{slots + (size_t)(SLOT / 4) * i};
@@ -138,6 +143,7 @@ constexpr int COPY_WARPS = 8;
 __global__ void __launch_bounds__(32 * COPY_WARPS) k_txt_copy(const unsigned *__restrict__ slots,
                                                               const unsigned *__restrict__ offs, int n,
                                                               unsigned char *__restrict__ dst) {
+    grid_wait();
     __shared__ unsigned sw[COPY_WARPS][32 * SLOT / 4];
     __shared__ unsigned so[COPY_WARPS][33];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -224,13 +230,11 @@ n2m_status encode_text(int format, const vec3i *d_t, const vec3d *d_p, int nt, i
     unsigned *slots = w.pack.as<unsigned>();
     unsigned *lens = w.lens.as<unsigned>();
     if (np) {
-        k_txt_fmt<false><<<grid(np, 128), 128, 0, s>>>(d_p, np, fv, slots, lens);
-        N2M_COUNT();
+        n2m_launch(k_txt_fmt<false>, grid(np, 128), 128, 0, s, d_p, np, fv, slots, lens);
         CKL();
     }
     if (nt) {
-        k_txt_fmt<true><<<grid(nt, 128), 128, 0, s>>>(d_t, nt, ft, slots + (size_t)(SLOT / 4) * np, lens + np);
-        N2M_COUNT();
+        n2m_launch(k_txt_fmt<true>, grid(nt, 128), 128, 0, s, d_t, nt, ft, slots + (size_t)(SLOT / 4) * np, lens + np);
         CKL();
     }
     CKS(scan_u32(lens, (size_t)nl, lens + nl, sw, s));
@@ -245,17 +249,15 @@ n2m_status encode_text(int format, const vec3i *d_t, const vec3d *d_p, int nt, i
     CKS(a.text(head));
     unsigned char *o = w.out.as<unsigned char>();
     if (np) {
-        k_txt_copy<<<grid(np, 32 * COPY_WARPS), 32 * COPY_WARPS, 0, s>>>(slots, lens, np, o + a.pos);
-        N2M_COUNT();
+        n2m_launch(k_txt_copy, grid(np, 32 * COPY_WARPS), 32 * COPY_WARPS, 0, s, slots, lens, np, o + a.pos);
         CKL();
     }
     a.pos += vbytes;
     CKS(a.text(mid));
     if (nt) {
         // offsets of the triangle lines are relative to the start of the body
-        k_txt_copy<<<grid(nt, 32 * COPY_WARPS), 32 * COPY_WARPS, 0, s>>>(slots + (size_t)(SLOT / 4) * np, lens + np, nt,
-                                                                         o + a.pos - vbytes);
-        N2M_COUNT();
+        n2m_launch(k_txt_copy, grid(nt, 32 * COPY_WARPS), 32 * COPY_WARPS, 0, s, slots + (size_t)(SLOT / 4) * np, lens + np, nt,
+                   o + a.pos - vbytes);
         CKL();
     }
     a.pos += body - vbytes;
@@ -307,8 +309,7 @@ n2m_status encode_gii(const vec3i *d_t, const vec3d *d_p, int nt, int np, bool g
     size_t tlen = tb, plen = pb;
     CKS(w.pack2.ensure(pb + 16));
     if (np) {
-        k_pack_pts<<<grid(np, 256), 256, 0, s>>>(d_p, np, w.pack2.as<unsigned char>(), 0);
-        N2M_COUNT();
+        n2m_launch(k_pack_pts, grid(np, 256), 256, 0, s, d_p, np, w.pack2.as<unsigned char>(), 0);
         CKL();
     }
     if (gz) {
@@ -343,15 +344,15 @@ n2m_status encode_gii(const vec3i *d_t, const vec3d *d_p, int nt, int np, bool g
     unsigned char *o = w.out.as<unsigned char>();
     CKS(a.text(head));
     if (tlen) {
-        k_base64<<<grid((long long)(tlen + 2) / 3, 256), 256, 0, s>>>(w.pack.as<unsigned char>(), (long long)tlen, o + a.pos);
-        N2M_COUNT();
+        n2m_launch(k_base64, grid((long long)(tlen + 2) / 3, 256), 256, 0, s, w.pack.as<unsigned char>(), (long long)tlen,
+                   o + a.pos);
         CKL();
     }
     a.pos += t64;
     CKS(a.text(mid));
     if (plen) {
-        k_base64<<<grid((long long)(plen + 2) / 3, 256), 256, 0, s>>>(w.pack2.as<unsigned char>(), (long long)plen, o + a.pos);
-        N2M_COUNT();
+        n2m_launch(k_base64, grid((long long)(plen + 2) / 3, 256), 256, 0, s, w.pack2.as<unsigned char>(), (long long)plen,
+                   o + a.pos);
         CKL();
     }
     a.pos += p64;
@@ -414,8 +415,7 @@ n2m_status encode_mesh_device(int format, const vec3i *d_t, const vec3d *d_p, in
         CK(cudaMemcpyAsync(d, h, 16, cudaMemcpyHostToDevice, s));
         if (nt) CK(cudaMemcpyAsync(d + 16, d_t, tb, cudaMemcpyDeviceToDevice, s));
         if (np) {
-            k_pack_pts<<<grid(np, 256), 256, 0, s>>>(d_p, np, d + 16 + tb, 0);
-            N2M_COUNT();
+            n2m_launch(k_pack_pts, grid(np, 256), 256, 0, s, d_p, np, d + 16 + tb, 0);
             CKL();
         }
         if (gz) {
@@ -451,13 +451,11 @@ n2m_status encode_mesh_device(int format, const vec3i *d_t, const vec3d *d_p, in
         CKS(a.text(head));
         unsigned char *o = w.out.as<unsigned char>();
         if (np) {
-            k_pack_pts<<<grid(np, 256), 256, 0, s>>>(d_p, np, o + a.pos, 1);
-            N2M_COUNT();
+            n2m_launch(k_pack_pts, grid(np, 256), 256, 0, s, d_p, np, o + a.pos, 1);
             CKL();
         }
         if (nt) {
-            k_pack_tris<<<grid(nt, 256), 256, 0, s>>>(d_t, nt, o + a.pos + pb, TRI_BE12);
-            N2M_COUNT();
+            n2m_launch(k_pack_tris, grid(nt, 256), 256, 0, s, d_t, nt, o + a.pos + pb, TRI_BE12);
             CKL();
         }
         *len = a.pos + pb + tb;
@@ -474,13 +472,11 @@ n2m_status encode_mesh_device(int format, const vec3i *d_t, const vec3d *d_p, in
         CKS(a.text(head));
         unsigned char *o = w.out.as<unsigned char>();
         if (np) {
-            k_pack_pts<<<grid(np, 256), 256, 0, s>>>(d_p, np, o + a.pos, 0);
-            N2M_COUNT();
+            n2m_launch(k_pack_pts, grid(np, 256), 256, 0, s, d_p, np, o + a.pos, 0);
             CKL();
         }
         if (nt) {
-            k_pack_tris<<<grid(nt, 256), 256, 0, s>>>(d_t, nt, o + a.pos + pb, TRI_PLY13);
-            N2M_COUNT();
+            n2m_launch(k_pack_tris, grid(nt, 256), 256, 0, s, d_t, nt, o + a.pos + pb, TRI_PLY13);
             CKL();
         }
         *len = a.pos + pb + (size_t)nt * 13;
@@ -497,9 +493,8 @@ n2m_status encode_mesh_device(int format, const vec3i *d_t, const vec3d *d_p, in
         Assembler a{w, s};
         CKS(a.text(head));
         if (nt) {
-            k_pack_stl<<<grid(nt, 256), 256, 0, s>>>(d_t, d_p, nt, np, w.out.as<unsigned char>() + a.pos,
-                                                    w.flag.as<unsigned>());
-            N2M_COUNT();
+            n2m_launch(k_pack_stl, grid(nt, 256), 256, 0, s, d_t, d_p, nt, np, w.out.as<unsigned char>() + a.pos,
+                       w.flag.as<unsigned>());
             CKL();
         }
         unsigned bad = 0;
@@ -521,15 +516,13 @@ n2m_status encode_mesh_device(int format, const vec3i *d_t, const vec3d *d_p, in
         CKS(a.text(head));
         unsigned char *o = w.out.as<unsigned char>();
         if (np) {
-            k_pack_pts<<<grid(np, 256), 256, 0, s>>>(d_p, np, o + a.pos, 1);
-            N2M_COUNT();
+            n2m_launch(k_pack_pts, grid(np, 256), 256, 0, s, d_p, np, o + a.pos, 1);
             CKL();
         }
         a.pos += pb;
         CKS(a.text(mid));
         if (nt) {
-            k_pack_tris<<<grid(nt, 256), 256, 0, s>>>(d_t, nt, o + a.pos, TRI_VTK16);
-            N2M_COUNT();
+            n2m_launch(k_pack_tris, grid(nt, 256), 256, 0, s, d_t, nt, o + a.pos, TRI_VTK16);
             CKL();
         }
         *len = a.pos + (size_t)nt * 16;
