@@ -973,19 +973,19 @@ __global__ void k_a_gather(const vec3d *p, const int *ids, int n, vec3d *out) {
     if (i < n) out[i] = p[ids[i]];
 }
 
-// kept triangles before each box's first triangle, from the degenerate filter's flags
-__global__ void k_a_kept(const unsigned *tri_start, int nb, const unsigned *flags, const unsigned *tile_off, int tile,
-                         unsigned total_kept, unsigned *kept_before) {
+// kept triangles before each box's first triangle, from the degenerate filter's bits
+__global__ void k_a_kept(const unsigned *tri_start, int nb, unsigned nt, const unsigned *bits, const unsigned *tile_off,
+                         const unsigned *total_kept, unsigned *kept_before) {
     grid_wait();
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b > nb) return;
     const unsigned t = tri_start[b];
     unsigned k;
-    if (b == nb) k = total_kept;
+    if (t >= nt) k = *total_kept;
     else {
-        const unsigned tb = t / tile;
-        k = tile_off[tb];
-        for (unsigned i = tb * tile; i < t; i++) k += flags[i];
+        k = tile_off[t / DEG_TILE];
+        for (unsigned w = t / DEG_TILE * (DEG_TILE / 32); w < t / 32; w++) k += __popc(bits[w]);
+        k += __popc(bits[t / 32] & ((1u << (t & 31u)) - 1u));
     }
     kept_before[b] = k;
 }
@@ -1388,6 +1388,7 @@ n2m_status atlas_batched(const short *d_lab, const int dim[3], const n2m_options
         }
     }
     vec3d *pts = w.pts.as<vec3d>();
+    WeldMap map;
     unsigned np = nv;
     std::vector<unsigned> vs_new(vs);
     if (!removed.empty()) {
@@ -1408,8 +1409,7 @@ n2m_status atlas_batched(const short *d_lab, const int dim[3], const n2m_options
         if (no) CK(cudaMemcpyAsync(dovid, ov_id.data(), no * sizeof(int), cudaMemcpyHostToDevice, s));
         np = nv - nr;
         CKS(w.pts2.ensure((size_t)np * sizeof(vec3d)));
-        CKS(mesh_apply_weld(pts, w.tris.as<vec3i>(), (int)nv, (int)nt, drem, dkeep, nr, dovid, dov, no,
-                            w.pts2.as<vec3d>(), s));
+        CKS(mesh_apply_weld(pts, (int)nv, drem, nr, dkeep, dovid, dov, no, w.pts2.as<vec3d>(), dw, map, s));
         pts = w.pts2.as<vec3d>();
         for (int b = 0; b <= nb; b++)
             vs_new[b] = vs[b] - (unsigned)(std::lower_bound(r2.begin(), r2.end(), (int)vs[b]) - r2.begin());
@@ -1419,17 +1419,15 @@ n2m_status atlas_batched(const short *d_lab, const int dim[3], const n2m_options
     CKS(w.tris2.ensure((size_t)std::max(nt, 1u) * sizeof(vec3i)));
     CKS(w.ranges.ensure((size_t)(4 * (nb + 1) + 2) * sizeof(unsigned)));
     unsigned *dts = w.ranges.as<unsigned>(), *dkept = dts + (nb + 1), *dvs = dkept + (nb + 1), *dntf = dvs + (nb + 1);
-    CKS(mesh_remove_degenerate(pts, w.tris.as<vec3i>(), (int)nt, w.tris2.as<vec3i>(), dntf, dw, sw, s));
-    unsigned ntf = 0;
-    CK(cudaMemcpyAsync(&ntf, dntf, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
     CK(cudaMemcpyAsync(dts, ts.data(), (nb + 1) * sizeof(unsigned), cudaMemcpyHostToDevice, s));
-    if (nt) n2m_launch(k_a_kept, (nb + 128) / 128, 128, 0, s, dts, nb, dw.flags.as<unsigned>(), dw.tmp.as<unsigned>(), 256, ntf,
+    CKS(mesh_remove_degenerate(pts, w.tris.as<vec3i>(), (int)nt, map, nullptr, w.tris2.as<vec3i>(), dntf, dw, s));
+    if (nt) n2m_launch(k_a_kept, (nb + 128) / 128, 128, 0, s, dts, nb, nt, dw.bits.as<unsigned>(), dw.tiles.as<unsigned>(), dntf,
                        dkept);
     else CK(cudaMemsetAsync(dkept, 0, (nb + 1) * sizeof(unsigned), s));
     std::vector<unsigned> kept(nb + 1);
     CK(cudaMemcpyAsync(kept.data(), dkept, (nb + 1) * sizeof(unsigned), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
+    const unsigned ntf = kept[nb];
     vec3i *tris = w.tris2.as<vec3i>();
     // ---- HC post-smoothing of all meshes at once (they share no vertex)
     CK(cudaEventRecord(ev[5], s));

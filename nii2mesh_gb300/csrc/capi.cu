@@ -222,6 +222,7 @@ struct n2m_context {
     bool want_host = false;
     HostOut hout;
     size_t hint_pb = 0, hint_tb = 0;   // raw mesh bytes of the last host-memory call (early pre-faulting)
+    const unsigned *marks = nullptr;   // vertices close to a grid point, of the mesh being made
     bool pts_early = false;            // the final vertices are already on their way to the host
     // n2m_meshify_into: caller-owned host output buffers (no allocation, no page faulting)
     vec3i *user_t = nullptr;
@@ -284,7 +285,7 @@ extern "C" void n2m_context_destroy(n2m_context *c) {
                       &c->tris_raw, &c->pts, &c->tris, &c->ntf, &c->weld, &c->gath, &c->hmesh,
                       &c->mc.signs, &c->mc.words, &c->mc.act, &c->mc.cnt, &c->mc.sub, &c->scan.part,
                       &c->lab.lab, &c->lab.mask, &c->lab.keep, &c->lab.cnt, &c->lab.edge, &c->lab.rc, &c->lab.misc, &c->lab.list, &c->lab.wlist, &c->lab.cs, &c->lab.filled, &c->lab.shell,
-                      &c->deg.flags, &c->deg.tmp, &c->hc.zero, &c->hc.adj, &c->hc.meta, &c->hc.P, &c->hc.Q,
+                      &c->deg.bits, &c->deg.tiles, &c->deg.rank, &c->deg.near, &c->hc.zero, &c->hc.adj, &c->hc.meta, &c->hc.P, &c->hc.Q,
                       &c->hc.B, &c->hc.Lo, &c->th.buf, &c->th.table,
                       &c->stmp2, &c->lubits, &c->od.st, &c->od.unc, &c->od.cmin, &c->od.cmax, &c->od.range, &c->od.need, &c->od.list, &c->od.lcnt, &c->od.vsign,
                       &c->wr.mt, &c->wr.mp, &c->wr.pack, &c->wr.pack2, &c->wr.lens, &c->wr.flag, &c->wr.out};
@@ -758,12 +759,19 @@ n2m_status march(n2m_context *c, const Prep &P, const int dim[3], int cubes, int
     CKS(c->ncand.ensure(2 * sizeof(unsigned)));
     CK(cudaMemsetAsync(c->ncand.p, 0, 2 * sizeof(unsigned), c->stream));
     McCounts mcn{tot.x, tot.y, tot.z, tot.w};
+    unsigned *near = nullptr;   // marks for the degenerate filter
+    if (std::max({dim[0], dim[1], dim[2]}) < 1 << 22) {
+        CKS(c->deg.near.ensure((nv + 31) / 32 * sizeof(unsigned)));
+        near = c->deg.near.as<unsigned>();
+        CK(cudaMemsetAsync(near, 0, (nv + 31) / 32 * sizeof(unsigned), c->stream));
+    }
+    c->marks = near;
     if (old) {
         CKS(oc_emit(P.vol, dim, P.lo, P.hi, P.iso, P.edge_max, c->mc, mcn, c->pts_raw.as<vec3d>(),
-                    c->tris_raw.as<vec3i>(), c->cand.as<int>(), c->ncand.as<unsigned>(), cap, c->stream));
+                    c->tris_raw.as<vec3i>(), c->cand.as<int>(), c->ncand.as<unsigned>(), cap, near, c->stream));
     } else {
         CKS(mc_emit(g, cubes, c->mc, mcn, c->pts_raw.as<vec3d>(), c->tris_raw.as<vec3i>(), c->cand.as<int>(),
-                    c->ncand.as<unsigned>(), cap, c->stream));
+                    c->ncand.as<unsigned>(), cap, near, c->stream));
     }
     unsigned nc[2];
     CKS(readback(c, nc, c->ncand.p, 2));
@@ -825,6 +833,7 @@ n2m_status pipeline(n2m_context *c, const float *d_src, const int dim[3], const 
     vec3d *pts = c->pts_raw.as<vec3d>();
     int np = nv;
     int welded = 0;
+    WeldMap map;
     c->fwd.nrem = c->fwd.nov = 0;
     if (ncand > 0) {
         std::vector<int> removed, keep, ov_id, ov_src;
@@ -862,8 +871,7 @@ n2m_status pipeline(n2m_context *c, const float *d_src, const int dim[3], const 
             c->fwd.nov = no;
             np = nv - nr;
             CKS(c->pts.ensure((size_t)np * sizeof(vec3d)));
-            CKS(mesh_apply_weld(pts, c->tris_raw.as<vec3i>(), nv, nt, drem, dkeep, nr, dovid, dov, no,
-                                c->pts.as<vec3d>(), c->stream));
+            CKS(mesh_apply_weld(pts, nv, drem, nr, dkeep, dovid, dov, no, c->pts.as<vec3d>(), c->deg, map, c->stream));
             pts = c->pts.as<vec3d>();
             welded = nr;
             CK(cudaStreamSynchronize(c->stream));   // host vectors go out of scope
@@ -879,8 +887,8 @@ n2m_status pipeline(n2m_context *c, const float *d_src, const int dim[3], const 
     c->pts_early = false;
     const bool early = c->want_host && o.post_smooth <= 0;   // vertices are final after the weld
     if (early) CK(cudaEventRecord(c->stage.ev[0], c->stream));
-    CKS(mesh_remove_degenerate(pts, c->tris_raw.as<vec3i>(), nt, c->tris.as<vec3i>(), c->ntf.as<unsigned>(), c->deg,
-                               c->scan, c->stream));
+    CKS(mesh_remove_degenerate(pts, c->tris_raw.as<vec3i>(), nt, map, c->marks, c->tris.as<vec3i>(),
+                               c->ntf.as<unsigned>(), c->deg, c->stream));
     if (early) {   // copy them out on the second stream while the degenerate filter runs
         void *dst = nullptr;
         if (c->user_p) {

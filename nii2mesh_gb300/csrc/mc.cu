@@ -278,6 +278,7 @@ struct Policy {
     int *cand, *ccand;
     unsigned *ncand, *nccand;
     int cap;
+    unsigned *near;   // marks of vertices close to a grid point, or null
     __device__ __forceinline__ unsigned quick(int lut) const {
         Tiling T = {0, 0, false};
         return quick_tiling(lut, classic, T) ? (unsigned)T.off << 8 | (unsigned)T.n : mcw::TESTS;
@@ -314,6 +315,7 @@ struct Policy {
         float c[8];
         cube_values(g, x, y, z, c);
         emit_cvertex(c, x, y, z, (float)g.lo0, (float)g.lo1, (float)g.lo2, id, pts, ccand, nccand, cap);
+        mark_near(near, id);
     }
     struct Edge {
         float c0, c1;
@@ -333,7 +335,11 @@ struct Policy {
         if (ax == 0) axv = X = __fadd_rn(__fadd_rn(fx, u), flo0);
         else if (ax == 1) axv = Y = __fadd_rn(__fadd_rn(fy, u), flo1);
         else axv = Z = __fadd_rn(__fadd_rn(fz, u), flo2);
-        if (frac_dist(axv) < 1.5e-5f) add_cand(cand, ncand, cap, id);
+        const float d = frac_dist(axv);
+        if (!(d >= NEAR_CORNER)) {
+            mark_near(near, id);
+            if (d < 1.5e-5f) add_cand(cand, ncand, cap, id);
+        }
         return {f2d(X), f2d(Y), f2d(Z)};
     }
 };
@@ -522,14 +528,14 @@ n2m_status mc_count(const McGrid &g, int variant, McWork &w, uint4 *d_total, cud
 }
 
 n2m_status mc_emit(const McGrid &g, int variant, McWork &w, const McCounts &c, vec3d *d_pts, vec3i *d_tris,
-                   int *d_cand, unsigned *d_ncand, int cand_cap, cudaStream_t s) {
+                   int *d_cand, unsigned *d_ncand, int cand_cap, unsigned *d_near, cudaStream_t s) {
     const GV v = make_gv(g);
     if (c.nactive == 0) return N2M_OK;
     size_t nwords;
     CKS(grid_words(v, nwords));
     mcw::Out o;
     CKS(mcw::prepare(w, nwords, nullptr, o));
-    const Policy pol{v, variant == N2M_CUBES_CLASSIC_TABLE, d_pts, d_cand, d_cand + cand_cap, d_ncand, d_ncand + 1, cand_cap};
+    const Policy pol{v, variant == N2M_CUBES_CLASSIC_TABLE, d_pts, d_cand, d_cand + cand_cap, d_ncand, d_ncand + 1, cand_cap, d_near};
     return mcw::emit(pol, w.signs.as<unsigned>(), w, o, c.nactive, d_tris, s);
 }
 

@@ -1,6 +1,7 @@
 // mesh.cu — per-mesh stages after marching cubes:
 //   * weld fix-up (src/meshify.c:45-106): applies the merges the host decided
-//     for the few near-grid-point candidates (vertex compaction + remap);
+//     for the few near-grid-point candidates (vertex compaction; the triangles
+//     are renumbered by the degenerate filter);
 //   * remove_degenerate_triangles (src/meshify.c:113-168): FP32 area filter
 //     with a rigorous error margin, the reference's FP64 predicate for the
 //     rest, stable compaction;
@@ -23,34 +24,34 @@ __device__ __forceinline__ int lower_bound(const int *a, int n, int v) {
     return lo;
 }
 
-// removed[k] (sorted) merges into keep[k]; override ids (sorted) take pos.
-__global__ void k_weld_verts(const vec3d *__restrict__ in, int np, const int *__restrict__ removed, int nrem,
-                             const int *__restrict__ ov_id, const vec3d *__restrict__ ov_pos, int nov,
-                             vec3d *__restrict__ out) {
+// removed[k] (sorted) merges into keep[k]; override ids (sorted) take pos.  rank, per 32
+// vertices: which of them are removed, and how many before them.
+__global__ void __launch_bounds__(256) k_weld_verts(const vec3d *__restrict__ in, int np, const int *__restrict__ removed,
+                                                    int nrem, const int *__restrict__ ov_id,
+                                                    const vec3d *__restrict__ ov_pos, int nov, vec3d *__restrict__ out,
+                                                    uint2 *rank) {
     grid_wait();
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < np; i += gridDim.x * blockDim.x) {
-        const int r = lower_bound(removed, nrem, i);
-        if (r < nrem && removed[r] == i) continue;
-        const int o = lower_bound(ov_id, nov, i);
-        out[i - r] = (o < nov && ov_id[o] == i) ? ov_pos[o] : in[i];
+    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < (((unsigned)np + 31u) & ~31u); i += gridDim.x * blockDim.x) {
+        const int r = lower_bound(removed, nrem, (int)i);
+        const bool gone = r < nrem && removed[r] == (int)i;
+        const unsigned b = __ballot_sync(0xffffffffu, gone);
+        if ((i & 31u) == 0) rank[i / 32] = make_uint2(b, (unsigned)r);
+        if (gone || i >= (unsigned)np) continue;
+        const int o = lower_bound(ov_id, nov, (int)i);
+        out[i - r] = (o < nov && ov_id[o] == (int)i) ? ov_pos[o] : in[i];
     }
 }
 
-__global__ void k_weld_tris(vec3i *t, int nt, const int *__restrict__ removed, const int *__restrict__ keep,
-                            int nrem) {
-    grid_wait();
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nt; i += gridDim.x * blockDim.x) {
-        int v[3] = {t[i].x, t[i].y, t[i].z};
-        for (int k = 0; k < 3; k++) {
-            int r = lower_bound(removed, nrem, v[k]);
-            if (r < nrem && removed[r] == v[k]) {
-                v[k] = keep[r];
-                r = lower_bound(removed, nrem, v[k]);
-            }
-            v[k] -= r;
-        }
-        t[i] = {v[0], v[1], v[2]};
+// vertex v after the weld; the ranks of consecutive vertices share cache lines (a search
+// in the removed ids per corner is a chain of ten loads)
+__device__ __forceinline__ int welded(int v, uint2 k, const WeldMap &m) {
+    int r = (int)k.y + __popc(k.x & ((1u << (v & 31)) - 1u));
+    if (k.x >> (v & 31) & 1u) {
+        v = m.keep[r];
+        k = __ldg(m.rank + v / 32);
+        r = (int)k.y + __popc(k.x & ((1u << (v & 31)) - 1u));
     }
+    return v - r;
 }
 
 // ---- degenerate triangles --------------------------------------------------------
@@ -71,10 +72,9 @@ __device__ bool degenerate_ref(vec3d A, vec3d B, vec3d C) {
     return __dmul_rn(0.25, __dsqrt_rn(q)) < (double)FLT_EPSILON;
 }
 
-// True iff the triangle is degenerate under the reference predicate.  Fast
-// path: the area from an FP32 cross product of (double) edge vectors, minus a
+// Fast path: the area from an FP32 cross product of (double) edge vectors, minus a
 // bound on its rounding error, exceeding 4e-7 (> 3x FLT_EPSILON) proves the
-// triangle is kept.
+// triangle is kept under the reference predicate.
 // float value of d if d is exactly a float (zero or normal), by bit assembly:
 // the F2F conversion issues on the FP64 pipe, a small fraction of the integer
 // rate on this part
@@ -89,7 +89,7 @@ __device__ __forceinline__ bool d2f_exact(double d, float &f) {
     return true;
 }
 
-__device__ __forceinline__ bool degenerate(vec3d A, vec3d B, vec3d C) {
+__device__ __forceinline__ bool surely_kept(vec3d A, vec3d B, vec3d C) {
     float ax, ay, az, bx, by, bz, qx, qy, qz;
     float ux, uy, uz, vx, vy, vz;
     if (d2f_exact(A.x, ax) & d2f_exact(A.y, ay) & d2f_exact(A.z, az) & d2f_exact(B.x, bx) & d2f_exact(B.y, by) &
@@ -104,39 +104,149 @@ __device__ __forceinline__ bool degenerate(vec3d A, vec3d B, vec3d C) {
     const float cx = uy * vz - uz * vy, cy = uz * vx - ux * vz, cz = ux * vy - uy * vx;
     const float cr = sqrtf(cx * cx + cy * cy + cz * cz);
     const float nu = sqrtf(ux * ux + uy * uy + uz * uz), nv = sqrtf(vx * vx + vy * vy + vz * vz);
-    if (0.5f * (cr - 1e-6f * nu * nv) > 4e-7f && isfinite(cr)) return false;
-    return degenerate_ref(A, B, C);
+    return 0.5f * (cr - 1e-6f * nu * nv) > 4e-7f && isfinite(cr);
 }
 
-constexpr int CB = 256;   // compaction tile = one CTA
+constexpr int CB = 256;          // threads of a CTA
+constexpr int DT = DEG_TILE;     // triangles of a CTA
+constexpr int DG = 64;           // tiles of a group
+static_assert(DT == 4 * CB && DT == 32 * 32, "four triangles per thread, a warp of words");
 
-__global__ void __launch_bounds__(CB) k_deg_count(const vec3d *__restrict__ p, const vec3i *__restrict__ t, int nt,
-                                                  unsigned *keep, unsigned *tile_cnt) {
+// Kept triangles as bits, and their number per tile and group of tiles; the weld's
+// renumbering, if there was one, on the way.  Gathering three 24-byte vertices per
+// triangle bounded this (L1 wavefronts), and nearly every triangle is far from
+// degenerate.  NEAR: marching cubes marked the vertices closer than NEAR_CORNER to
+// a grid point (and all cell-centre vertices).  A triangle whose corners are on three edges
+// of a cube, none of them marked, has an area above 3e-6, far above FLT_EPSILON, so only
+// triangles with a marked corner (1 %) are looked at; they are listed, so that they share
+// warps.  The bits of neighbouring vertices share sectors.  Without marks (vertices from
+// elsewhere) every triangle is, four consecutive ones per lane, which share most
+// vertices.  512^3 CT (7.6 M triangles): flags of 4 bytes, a triangle per lane and a pass of
+// its own for the renumbering took 93 + 61 us, the general path here 126 (the whole filter
+// with the copy 164), with the marks the filter takes 111; oldcubes (4.1 M) 132 -> 61.
+template <bool NEAR>
+__global__ void __launch_bounds__(CB, 4) k_deg_count(const vec3d *__restrict__ p, vec3i *t, int nt, WeldMap m,
+                                                     const unsigned *__restrict__ near, unsigned *bits, unsigned *tile_cnt,
+                                                     unsigned *group_cnt) {
     grid_wait();
-    const int i = blockIdx.x * CB + threadIdx.x;
-    unsigned k = 0;
-    if (i < nt) {
-        const vec3i T = t[i];
-        k = !degenerate(p[T.x], p[T.y], p[T.z]);
-        keep[i] = k;
-    }
-    k = __syncthreads_count(k);
-    if (threadIdx.x == 0) tile_cnt[blockIdx.x] = k;
-}
-
-__global__ void __launch_bounds__(CB) k_deg_compact(const vec3i *__restrict__ t, int nt, const unsigned *keep,
-                                                    const unsigned *tile_off, vec3i *out) {
-    grid_wait();
-    __shared__ unsigned wcnt[CB / 32];
-    const int i = blockIdx.x * CB + threadIdx.x;
-    const unsigned k = i < nt ? keep[i] : 0u;
-    const unsigned b = __ballot_sync(0xffffffffu, k);
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    if (lane == 0) wcnt[wid] = __popc(b);
+    __shared__ unsigned kept[DT / 32], nslow;
+    __shared__ unsigned short slow[DT];
+    const int tid = threadIdx.x, lane = tid & 31;
+    const unsigned i0 = blockIdx.x * DT + 4u * tid;
+    const int n = i0 < (unsigned)nt ? (int)min(4u, (unsigned)nt - i0) : 0;
+    if (tid == 0) nslow = 0;
     __syncthreads();
-    unsigned off = tile_off[blockIdx.x];
-    for (int w = 0; w < wid; w++) off += wcnt[w];
-    if (k) out[off + __popc(b & ((1u << lane) - 1u))] = t[i];
+    int v[12];
+    if (n == 4) {
+        const int4 *q = (const int4 *)(t + i0);
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            const int4 x = q[k];
+            v[4 * k] = x.x; v[4 * k + 1] = x.y; v[4 * k + 2] = x.z; v[4 * k + 3] = x.w;
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < 12; k++) v[k] = k < 3 * n ? ((const int *)(t + i0))[k] : 0;
+    }
+    unsigned look = 0;   // corners of triangles to look at
+    if (NEAR && n) {
+#pragma unroll
+        for (int k = 0; k < 12; k++) look |= (__ldg(near + v[k] / 32) >> (v[k] & 31) & 1u) << k;
+    }
+    if (m.rank && n) {
+        uint2 q[12];
+#pragma unroll
+        for (int k = 0; k < 12; k++) q[k] = __ldg(m.rank + v[k] / 32);
+#pragma unroll
+        for (int k = 0; k < 12; k++) v[k] = k < 3 * n ? welded(v[k], q[k], m) : 0;
+        if (n == 4) {
+            int4 *q4 = (int4 *)(t + i0);
+#pragma unroll
+            for (int k = 0; k < 3; k++) q4[k] = make_int4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+        } else {
+#pragma unroll
+            for (int k = 0; k < 12; k++)
+                if (k < 3 * n) ((int *)(t + i0))[k] = v[k];
+        }
+    }
+    unsigned keep = 0;
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+        if (k < n) {
+            if (NEAR ? !(look >> (3 * k) & 7u) : surely_kept(p[v[3 * k]], p[v[3 * k + 1]], p[v[3 * k + 2]])) keep |= 1u << k;
+            else slow[atomicAdd(&nslow, 1u)] = (unsigned short)(4 * tid + k);
+        }
+    unsigned w = keep << (4 * (lane & 7));   // eight lanes make a word
+    for (int o = 1; o < 8; o <<= 1) w |= __shfl_xor_sync(0xffffffffu, w, o);
+    if ((lane & 7) == 0) kept[tid / 8] = w;
+    __syncthreads();
+    for (unsigned k = tid; k < nslow; k += CB) {
+        const int i = slow[k];
+        const vec3i T = t[blockIdx.x * DT + i];
+        if ((NEAR && surely_kept(p[T.x], p[T.y], p[T.z])) || !degenerate_ref(p[T.x], p[T.y], p[T.z])) atomicOr(&kept[i / 32], 1u << (i & 31));
+    }
+    __syncthreads();
+    if (tid < 32) {
+        w = kept[tid];
+        bits[blockIdx.x * (DT / 32) + tid] = w;
+        const unsigned sum = __reduce_add_sync(0xffffffffu, __popc(w));
+        if (tid == 0) {
+            tile_cnt[blockIdx.x] = sum;
+            atomicAdd(&group_cnt[blockIdx.x / DG], sum);
+        }
+    }
+}
+
+// The kept triangles in order.  A tile adds up the groups and tiles before it by itself
+// (a scan in between was three launches); a tile without a degenerate triangle,
+// nearly every one, is a plain copy.  tile_off: kept triangles before each tile.
+// 512^3 CT: 48 us with a lane per 12-byte record.
+__global__ void __launch_bounds__(CB) k_deg_compact(const vec3i *__restrict__ t, int nt, const unsigned *__restrict__ bits,
+                                                    const unsigned *__restrict__ tile_cnt, const unsigned *__restrict__ group_cnt,
+                                                    unsigned *tile_off, vec3i *out, unsigned *nt_out) {
+    grid_wait();
+    __shared__ unsigned wsum[CB / 32], pre[DT / 32];
+    __shared__ int stage[3 * DT];
+    const int tile = blockIdx.x, g = tile / DG, tid = threadIdx.x;
+    unsigned s = 0;
+    for (int k = tid; k < g; k += CB) s += group_cnt[k];
+    if (tid < tile - g * DG) s += tile_cnt[g * DG + tid];
+    s = __reduce_add_sync(0xffffffffu, s);
+    if ((tid & 31) == 0) wsum[tid >> 5] = s;
+    __syncthreads();
+    unsigned off = 0;
+    for (int k = 0; k < CB / 32; k++) off += wsum[k];
+    const int have = min(DT, nt - tile * DT);
+    const unsigned cnt = tile_cnt[tile];
+    if (tid == 0) {
+        tile_off[tile] = off;
+        if (tile == (int)gridDim.x - 1) *nt_out = off + cnt;
+    }
+    const int *src = (const int *)(t + (size_t)tile * DT);
+    int *dst = (int *)(out + off);
+    if (cnt == (unsigned)have) {
+#pragma unroll 4
+        for (int k = tid; k < 3 * have; k += CB) dst[k] = src[k];
+        return;
+    }
+    if (tid < 32) {
+        const unsigned c = __popc(bits[tile * (DT / 32) + tid]);
+        unsigned incl = c;
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned x = __shfl_up_sync(0xffffffffu, incl, o);
+            if (tid >= o) incl += x;
+        }
+        pre[tid] = incl - c;
+    }
+    __syncthreads();
+    for (int i = tid; i < have; i += CB) {
+        const unsigned w = bits[tile * (DT / 32) + i / 32];
+        if (!(w >> (i & 31) & 1u)) continue;
+        const unsigned at = pre[i / 32] + __popc(w & ((1u << (i & 31)) - 1u));
+        for (int c = 0; c < 3; c++) stage[3 * at + c] = src[3 * i + c];
+    }
+    __syncthreads();
+    for (int k = tid; k < 3 * (int)cnt; k += CB) dst[k] = stage[k];
 }
 
 // raw vertex gradient: every kept raw vertex receives its welded vertex's
@@ -184,28 +294,31 @@ inline unsigned gs(size_t n) {
 }
 }  // namespace
 
-n2m_status mesh_apply_weld(vec3d *d_pts, vec3i *d_tris, int np, int nt, const int *d_removed, const int *d_keep,
-                           int nrem, const int *d_ov_id, const vec3d *d_ov_pos, int nov, vec3d *d_out,
+n2m_status mesh_apply_weld(const vec3d *d_pts, int np, const int *d_removed, int nrem, const int *d_keep,
+                           const int *d_ov_id, const vec3d *d_ov_pos, int nov, vec3d *d_out, DegWork &w, WeldMap &map,
                            cudaStream_t s) {
-    n2m_launch(k_weld_verts, gs(np), 256, 0, s, d_pts, np, d_removed, nrem, d_ov_id, d_ov_pos, nov, d_out);
-    n2m_launch(k_weld_tris, gs(nt), 256, 0, s, d_tris, nt, d_removed, d_keep, nrem);
+    CKS(w.rank.ensure(((size_t)np + 31) / 32 * sizeof(uint2)));
+    map.rank = w.rank.as<uint2>();
+    map.keep = d_keep;
+    n2m_launch(k_weld_verts, gs(np), 256, 0, s, d_pts, np, d_removed, nrem, d_ov_id, d_ov_pos, nov, d_out, w.rank.as<uint2>());
     CKL();
     return N2M_OK;
 }
 
-n2m_status mesh_remove_degenerate(const vec3d *d_pts, const vec3i *d_tris_in, int nt, vec3i *d_tris_out,
-                                  unsigned *d_nt_out, DegWork &w, ScanWork &sw, cudaStream_t s) {
-    const int tiles = (nt + CB - 1) / CB;
+n2m_status mesh_remove_degenerate(const vec3d *d_pts, vec3i *d_tris_in, int nt, const WeldMap &weld, const unsigned *d_near,
+                                  vec3i *d_tris_out, unsigned *d_nt_out, DegWork &w, cudaStream_t s) {
     if (nt == 0) {
         CK(cudaMemsetAsync(d_nt_out, 0, sizeof(unsigned), s));
         return N2M_OK;
     }
-    CKS(w.flags.ensure((size_t)nt * sizeof(unsigned)));
-    CKS(w.tmp.ensure((size_t)tiles * sizeof(unsigned)));
-    n2m_launch(k_deg_count, tiles, CB, 0, s, d_pts, d_tris_in, nt, w.flags.as<unsigned>(), w.tmp.as<unsigned>());
-    CKL();
-    CKS(scan_u32(w.tmp.as<unsigned>(), tiles, d_nt_out, sw, s));
-    n2m_launch(k_deg_compact, tiles, CB, 0, s, d_tris_in, nt, w.flags.as<unsigned>(), w.tmp.as<unsigned>(), d_tris_out);
+    const int tiles = (int)(((long long)nt + DT - 1) / DT), groups = (tiles + DG - 1) / DG;
+    CKS(w.bits.ensure((size_t)tiles * (DT / 32) * sizeof(unsigned)));
+    CKS(w.tiles.ensure(((size_t)2 * tiles + groups) * sizeof(unsigned)));
+    unsigned *bits = w.bits.as<unsigned>(), *off = w.tiles.as<unsigned>(), *cnt = off + tiles, *grp = cnt + tiles;
+    CK(cudaMemsetAsync(grp, 0, (size_t)groups * sizeof(unsigned), s));
+    if (d_near) n2m_launch(k_deg_count<true>, tiles, CB, 0, s, d_pts, d_tris_in, nt, weld, d_near, bits, cnt, grp);
+    else n2m_launch(k_deg_count<false>, tiles, CB, 0, s, d_pts, d_tris_in, nt, weld, nullptr, bits, cnt, grp);
+    n2m_launch(k_deg_compact, tiles, CB, 0, s, d_tris_in, nt, bits, cnt, grp, off, d_tris_out, d_nt_out);
     CKL();
     return N2M_OK;
 }

@@ -276,7 +276,7 @@ struct McCounts {
 n2m_status mc_count(const McGrid &g, int variant, McWork &w, uint4 *d_total, cudaStream_t s, OdWork &od,
                     const OdRepair *repair = nullptr, const LabelPost *post = nullptr);
 n2m_status mc_emit(const McGrid &g, int variant, McWork &w, const McCounts &c, vec3d *d_pts, vec3i *d_tris,
-                   int *d_cand, unsigned *d_ncand, int cand_cap, cudaStream_t s);
+                   int *d_cand, unsigned *d_ncand, int cand_cap, unsigned *d_near, cudaStream_t s);
 n2m_status mc_backward(const McGrid &g, int variant, McWork &w, const McCounts &c, const float3 *d_gv, float *d_gs,
                        cudaStream_t s);
 n2m_status mc_ccand_scan(const vec3d *d_pts, int np, const int *d_ccand, int nccand, int *d_cand,
@@ -289,7 +289,7 @@ n2m_status oc_count(const float *vol, const int dim[3], const int lo[3], const i
                     const LabelPost *post = nullptr);
 n2m_status oc_emit(const float *vol, const int dim[3], const int lo[3], const int hi[3], float iso, float edge_max,
                     McWork &w, const McCounts &c, vec3d *d_pts, vec3i *d_tris, int *d_cand, unsigned *d_ncand,
-                    int cand_cap, cudaStream_t s);
+                    int cand_cap, unsigned *d_near, cudaStream_t s);
 // the copies of the ncand weld candidates in the reference's triangle soup: every
 // corner 3*t + c naming one, into d_out (at most cap; *d_count = how many there
 // are); d_bits: nv bits of scratch
@@ -302,14 +302,32 @@ n2m_status oc_copy_positions(const float *vol, const int dim[3], const int lo[3]
                              int n, int *d_vid, vec3d *d_pos, cudaStream_t s);
 
 // mesh.cu
-n2m_status mesh_apply_weld(vec3d *d_pts, vec3i *d_tris, int np, int nt, const int *d_removed, const int *d_keep,
-                           int nrem, const int *d_ov_id, const vec3d *d_ov_pos, int nov, vec3d *d_out,
-                           cudaStream_t s);
+constexpr int DEG_TILE = 1024;   // triangles of a tile of the degenerate filter
 struct DegWork {
-    DevBuf flags, tmp;
+    DevBuf bits;    // a bit per triangle: kept
+    DevBuf tiles;   // kept triangles before each tile of DEG_TILE; counts per tile and group
+    DevBuf rank;    // of the weld
+    DevBuf near;    // a bit per vertex: close to a grid point
 };
-n2m_status mesh_remove_degenerate(const vec3d *d_pts, const vec3i *d_tris_in, int nt, vec3i *d_tris_out,
-                                  unsigned *d_nt_out, DegWork &w, ScanWork &sw, cudaStream_t s);
+// what the weld does to vertex ids: per 32 vertices {removed ones, removed before them}
+// (null: no weld); the k-th removed one merges into keep[k]
+struct WeldMap {
+    const uint2 *rank = nullptr;
+    const int *keep = nullptr;
+};
+n2m_status mesh_apply_weld(const vec3d *d_pts, int np, const int *d_removed, int nrem, const int *d_keep,
+                           const int *d_ov_id, const vec3d *d_ov_pos, int nov, vec3d *d_out, DegWork &w, WeldMap &map,
+                           cudaStream_t s);
+// Vertices of marching cubes closer than this to a grid point are marked for the
+// degenerate filter (mesh.cu: k_deg_count; coordinates below 2^22, where floats still
+// resolve it).
+constexpr float NEAR_CORNER = 1.f / 512;
+__device__ __forceinline__ void mark_near(unsigned *near, int id) {
+    if (near) atomicOr(near + (id >> 5), 1u << (id & 31));
+}
+// d_tris_in is renumbered in place if the weld removed vertices; d_near: the marks by raw id, or null
+n2m_status mesh_remove_degenerate(const vec3d *d_pts, vec3i *d_tris_in, int nt, const WeldMap &weld, const unsigned *d_near,
+                                  vec3i *d_tris_out, unsigned *d_nt_out, DegWork &w, cudaStream_t s);
 struct HcWork {
     DevBuf zero;              // degrees / offsets, cursors, the bad-index flag, border flags
     DevBuf adj, meta;         // neighbour lists and their per-vertex heads

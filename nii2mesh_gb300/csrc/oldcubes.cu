@@ -143,7 +143,7 @@ __device__ __forceinline__ double i2d(int v) {   // v >= 0
 // product is mu or -mu.  A vertex near a grid point becomes a weld candidate (a wider
 // float test spares the others the double one).
 __device__ __forceinline__ vec3d oc_vertex(const OV &g, float v0, float v1, int x, int y, int z, int ax, int id, int *cand,
-                                           unsigned *ncand, int cap) {
+                                           unsigned *ncand, int cap, unsigned *near) {
     const int X = g.lo0 + x, Y = g.lo1 + y, Z = g.lo2 + z;
     const int c0 = g.lo0, c1 = g.lo1, c2 = g.lo2, e0 = g.hi0 - 2, e1 = g.hi1 - 2, e2 = g.hi2 - 2;
     bool fwd = true;   // z: every user lists the edge bottom to top
@@ -162,9 +162,12 @@ __device__ __forceinline__ vec3d oc_vertex(const OV &g, float v0, float v1, int 
     const double mu = __ddiv_rn(__dsub_rn(iso, da), __dsub_rn(db, da));
     const double r = __dadd_rn(i2d(fwd ? i0 : i0 + 1), fwd ? mu : -mu);
     const float mf = __fdividef(__fsub_rn(g.iso, va), __fsub_rn(vb, va));   // within 1e-6 of mu, or 0, Inf or NaN
-    if (!(mf > 2e-5f && mf < 1.f - 2e-5f) && fabs(r - rint(r)) < 1.5e-5) {
-        const unsigned k = atomicAdd(ncand, 1u);
-        if (k < (unsigned)cap) cand[k] = id;
+    if (!(mf > NEAR_CORNER + 1e-5f && mf < 1.f - NEAR_CORNER - 1e-5f)) {
+        mark_near(near, id);
+        if (!(mf > 2e-5f && mf < 1.f - 2e-5f) && fabs(r - rint(r)) < 1.5e-5) {
+            const unsigned k = atomicAdd(ncand, 1u);
+            if (k < (unsigned)cap) cand[k] = id;
+        }
     }
     return {ax == 0 ? r : i2d(X), ax == 1 ? r : i2d(Y), ax == 2 ? r : i2d(Z)};
 }
@@ -178,6 +181,7 @@ struct Policy {
     int *cand;
     unsigned *ncand;
     int cap;
+    unsigned *near;
     __device__ __forceinline__ unsigned quick(int lut) const { return (unsigned)(lut * 16) << 8 | (unsigned)ocube_ntri(lut); }
     __device__ __forceinline__ int code(int off) const { return d_tri[off]; }
     __device__ __forceinline__ bool geo(unsigned w, mcw::Geo &q) const {
@@ -200,7 +204,7 @@ struct Policy {
         return Edge{oval(g, X, Y, Z), oval(g, X + (ax == 0), Y + (ax == 1), Z + (ax == 2))};
     }
     __device__ __forceinline__ vec3d vertex(const Edge &v, int x, int y, int z, int ax, int id) const {
-        return oc_vertex(g, v.v0, v.v1, x, y, z, ax, id, cand, ncand, cap);
+        return oc_vertex(g, v.v0, v.v1, x, y, z, ax, id, cand, ncand, cap, near);
     }
 };
 
@@ -335,12 +339,12 @@ n2m_status oc_count(const float *vol, const int dim[3], const int lo[3], const i
 
 n2m_status oc_emit(const float *vol, const int dim[3], const int lo[3], const int hi[3], float iso, float edge_max,
                     McWork &w, const McCounts &c, vec3d *d_pts, vec3i *d_tris, int *d_cand, unsigned *d_ncand,
-                    int cand_cap, cudaStream_t s) {
+                    int cand_cap, unsigned *d_near, cudaStream_t s) {
     const OV g = make_ov(vol, dim, lo, hi, iso, edge_max);
     if (c.nactive == 0) return N2M_OK;
     mcw::Out o;
     CKS(mcw::prepare(w, (size_t)g.WX * g.NY * g.NZ, nullptr, o));
-    return mcw::emit(Policy{g, d_pts, d_cand, d_ncand, cand_cap}, w.signs.as<unsigned>(), w, o, c.nactive, d_tris, s);
+    return mcw::emit(Policy{g, d_pts, d_cand, d_ncand, cand_cap, d_near}, w.signs.as<unsigned>(), w, o, c.nactive, d_tris, s);
 }
 
 n2m_status oc_copies(const vec3i *d_tris, int nt, int nv, const int *d_cand, int ncand, unsigned *d_bits,
