@@ -181,6 +181,7 @@ struct HostOut {
     }
 };
 
+constexpr size_t N2M_UPLOAD = 49152;
 struct n2m_context {
     int device = 0;
     cudaStream_t stream = nullptr;
@@ -188,7 +189,7 @@ struct n2m_context {
     cudaEvent_t evs[8] = {};   // stage boundaries of the last pipeline run
     cudaEvent_t eva[2] = {};   // around pass A of the exact-on-demand pre-smooth
     bool pass_a = false;       // whether the last pipeline run used it
-    DevBuf in, raw, vol, stmp, stmp2, stats, totals, cand, ncand, ocq, lubits, pts_raw, tris_raw, pts, tris, ntf, weld,
+    DevBuf in, raw, vol, stmp, stmp2, stats, march, cand, ocq, lubits, pts_raw, tris_raw, pts, tris, ntf, weld,
         gath, hmesh;
     OdWork od;   // pre-smooth with exact rounding on demand
     McWork mc;
@@ -198,7 +199,7 @@ struct n2m_context {
     DegWork deg;
     HcWork hc;
     ThresholdWork th;
-    void *pinned = nullptr;   // small readbacks
+    void *pinned = nullptr;   // small readbacks (N2M_READBACK bytes), then small uploads (N2M_UPLOAD)
     DevBuf gA, gB, gs, gtmp;   // adjoint scratch
     AtlasWork aw;
     DevBuf alab, lpts, ltris;   // atlas input copy, per-label-loop output
@@ -222,6 +223,8 @@ struct n2m_context {
     bool want_host = false;
     HostOut hout;
     size_t hint_pb = 0, hint_tb = 0;   // raw mesh bytes of the last host-memory call (early pre-faulting)
+    MarchOut mo;                       // of the last march; mo_cand: it holds every weld candidate
+    bool mo_cand = false;
     const unsigned *marks = nullptr;   // vertices close to a grid point, of the mesh being made
     bool pts_early = false;            // the final vertices are already on their way to the host
     // n2m_meshify_into: caller-owned host output buffers (no allocation, no page faulting)
@@ -250,7 +253,7 @@ extern "C" n2m_status n2m_context_create(n2m_context **out, int device) {
     c->device = device;
     if (cudaSetDevice(device) != cudaSuccess || cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreate(&c->ev0) != cudaSuccess || cudaEventCreate(&c->ev1) != cudaSuccess ||
-        cudaMallocHost(&c->pinned, 4096) != cudaSuccess) {
+        cudaMallocHost(&c->pinned, N2M_READBACK + N2M_UPLOAD) != cudaSuccess) {
         n2m_set_error("context creation failed: %s", cudaGetErrorString(cudaGetLastError()));
         delete c;
         return N2M_ERR_CUDA;
@@ -281,7 +284,7 @@ extern "C" void n2m_context_destroy(n2m_context *c) {
     DevBuf *bufs[] = {&c->aw.cnt, &c->aw.bb, &c->aw.boxes, &c->aw.queue, &c->aw.arena, &c->aw.mask, &c->aw.keep,
                       &c->aw.lab, &c->aw.edge, &c->aw.ucnt, &c->aw.words, &c->aw.counts, &c->aw.active, &c->aw.tot,
                       &c->aw.pts, &c->aw.pts2, &c->aw.tris, &c->aw.tris2, &c->aw.cand, &c->aw.gath, &c->aw.weld,
-                      &c->aw.ranges, &c->alab, &c->lpts, &c->ltris, &c->gA, &c->gB, &c->gs, &c->gtmp, &c->in, &c->raw, &c->vol, &c->stmp, &c->stats, &c->totals, &c->cand, &c->ncand, &c->ocq, &c->pts_raw,
+                      &c->aw.ranges, &c->alab, &c->lpts, &c->ltris, &c->gA, &c->gB, &c->gs, &c->gtmp, &c->in, &c->raw, &c->vol, &c->stmp, &c->stats, &c->march, &c->cand, &c->ocq, &c->pts_raw,
                       &c->tris_raw, &c->pts, &c->tris, &c->ntf, &c->weld, &c->gath, &c->hmesh,
                       &c->mc.signs, &c->mc.words, &c->mc.act, &c->mc.cnt, &c->mc.sub, &c->scan.part,
                       &c->lab.lab, &c->lab.mask, &c->lab.keep, &c->lab.cnt, &c->lab.edge, &c->lab.rc, &c->lab.misc, &c->lab.list, &c->lab.wlist, &c->lab.cs, &c->lab.filled, &c->lab.shell,
@@ -336,6 +339,17 @@ template <class T> n2m_status readback(n2m_context *c, T *dst, const void *dsrc,
     CK(cudaMemcpyAsync(c->pinned, dsrc, n * sizeof(T), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
     memcpy(dst, c->pinned, n * sizeof(T));
+    return N2M_OK;
+}
+
+// a readback, or two in one wait
+template <class T, class U> n2m_status readback2(n2m_context *c, T *a, const void *da, U *b, const void *db, bool both) {
+    static_assert(sizeof(T) + sizeof(U) <= N2M_READBACK, "pinned buffer");
+    CK(cudaMemcpyAsync(c->pinned, da, sizeof(T), cudaMemcpyDeviceToHost, c->stream));
+    if (both) CK(cudaMemcpyAsync((char *)c->pinned + sizeof(T), db, sizeof(U), cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaStreamSynchronize(c->stream));
+    memcpy(a, c->pinned, sizeof(T));
+    if (both) memcpy(b, (char *)c->pinned + sizeof(T), sizeof(U));
     return N2M_OK;
 }
 
@@ -438,20 +452,28 @@ void sort_weld_lists(std::vector<int> &removed, std::vector<int> &keep, std::vec
 n2m_status weld_candidates(n2m_context *c, int nv, int ncand, std::vector<int> &removed, std::vector<int> &keep,
                            std::vector<int> &ov_id, std::vector<vec3d> &ov_pos, std::vector<int> &ov_src, vec3d v0) {
     std::vector<int> ids(ncand);
-    CK(cudaMemcpyAsync(ids.data(), c->cand.p, ncand * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
+    if (c->mo_cand) memcpy(ids.data(), c->mo.cand_id, ncand * sizeof(int));
+    else {
+        CK(cudaMemcpyAsync(ids.data(), c->cand.p, ncand * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+        CK(cudaStreamSynchronize(c->stream));
+    }
     std::sort(ids.begin(), ids.end());
     ids.erase(std::unique(ids.begin(), ids.end()), ids.end());
     const int n = (int)ids.size();
-    CKS(c->gath.ensure((size_t)n * (sizeof(vec3d) + sizeof(int))));
-    vec3d *dpos = c->gath.as<vec3d>();
-    int *dids = (int *)(dpos + n);
-    CK(cudaMemcpyAsync(dids, ids.data(), n * sizeof(int), cudaMemcpyHostToDevice, c->stream));
-    n2m_launch(k_gather, (n + 255) / 256, 256, 0, c->stream, c->pts_raw.as<vec3d>(), dids, n, dpos);
-    CKL();
     std::vector<vec3d> pos(n);
-    CK(cudaMemcpyAsync(pos.data(), dpos, n * sizeof(vec3d), cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
+    if (c->mo_cand) {   // their positions came with the counts
+        for (int k = 0; k < ncand; k++)
+            pos[std::lower_bound(ids.begin(), ids.end(), c->mo.cand_id[k]) - ids.begin()] = c->mo.cand_pos[k];
+    } else {
+        CKS(c->gath.ensure((size_t)n * (sizeof(vec3d) + sizeof(int))));
+        vec3d *dpos = c->gath.as<vec3d>();
+        int *dids = (int *)(dpos + n);
+        CK(cudaMemcpyAsync(dids, ids.data(), n * sizeof(int), cudaMemcpyHostToDevice, c->stream));
+        n2m_launch(k_gather, (n + 255) / 256, 256, 0, c->stream, c->pts_raw.as<vec3d>(), dids, n, dpos);
+        CKL();
+        CK(cudaMemcpyAsync(pos.data(), dpos, n * sizeof(vec3d), cudaMemcpyDeviceToHost, c->stream));
+        CK(cudaStreamSynchronize(c->stream));
+    }
     const std::vector<long long> order(ids.begin(), ids.end());   // the reference's vertex order
     int ng = 0;
     const std::vector<int> grp = weld_groups(pos, order, v0, &ng);
@@ -605,6 +627,19 @@ n2m_status prepare(n2m_context *c, const float *d_src, const int dim[3], const n
     // the last slab)
     bool od = smooth && (!label || o.only_largest) && !c->stage.host && od_eligible(d_src, nx, ny, nz);
     OdStats hod;
+    VolStats s0, s1;
+    // The labelling needs the isolevel only, so it is queued before the statistics that
+    // decide about the isolevel and the exact smoothing are read: one wait less.  In the rare
+    // cases that change either it is done again.
+    bool labelled = false, clean = true;   // clean: dst[1] holds initial values
+    auto labelling = [&]() -> n2m_status {
+        if (!clean) CK(cudaMemcpyAsync(dst + 1, &h[1], sizeof(VolStats), cudaMemcpyHostToDevice, c->stream));
+        clean = false;
+        CKS(run_labelling(vol, nx, ny, nz, iso, o.only_largest, o.fill_bubbles, o.cubes == N2M_CUBES_OLDCUBES, c->lab, dst + 1,
+                          c->stream, od ? c->od.vsign.as<unsigned>() : nullptr, &c->lpost));
+        labelled = true;
+        return N2M_OK;
+    };
     if (smooth) {
         CKS(c->stmp.ensure(n * sizeof(float)));
         const StagedInput *stage = c->stage.host ? &c->stage : nullptr;
@@ -615,11 +650,12 @@ n2m_status prepare(n2m_context *c, const float *d_src, const int dim[3], const n
             c->pass_a = true;
             CKS(od_resolve(d_src, vol, nx, ny, nz, iso, c->od, c->stream, label || o.cubes == N2M_CUBES_OLDCUBES));
             CK(cudaEventRecord(c->evs[1], c->stream));
-            CKS(readback(c, &hod, c->od.st.p));
+            if (label) CKS(labelling());
+            CKS(readback2(c, &hod, c->od.st.p, &s1, dst + 1, label));
             bool fallback = false;
             CKS(od_check(c->od, hod, &fallback));
             if (fallback) {
-                od = false;
+                od = labelled = false;
                 CKS(launch_smooth(d_src, vol, c->stmp.as<float>(), nx, ny, nz, iso, dst, c->stream, nullptr));
             }
         } else {
@@ -629,9 +665,12 @@ n2m_status prepare(n2m_context *c, const float *d_src, const int dim[3], const n
     else CKS(launch_stats(label ? vol : d_src, nx, ny, nz, iso, true, dst, c->stream));
     if (!od) CK(cudaEventRecord(c->evs[1], c->stream));
     const float *v = vol ? vol : d_src;
-    VolStats s0;
-    if (od) s0 = hod.vs;
-    else CKS(readback(c, &s0, dst));
+    if (od) {
+        s0 = hod.vs;
+    } else {
+        if (label) CKS(labelling());
+        CKS(readback2(c, &s0, dst, &s1, dst + 1, label));
+    }
     if (s0.nonfinite) {
         n2m_set_error("%u non-finite voxels in the volume", s0.nonfinite);
         return N2M_ERR_NONFINITE;
@@ -648,23 +687,25 @@ n2m_status prepare(n2m_context *c, const float *d_src, const int dim[3], const n
         if (!g_quiet)
             printf("Suggested isolevel out of range. Intensity range %g..%g, setting isolevel to %g\n", mn, mx, iso);
         stale = true;
+        labelled = false;
         if (od) {   // the approximate pass decided signs against the old isolevel: smooth exactly
-            od = false;
+            od = clean = false;
             CKS(launch_smooth(d_src, vol, c->stmp.as<float>(), nx, ny, nz, iso, dst + 1, c->stream, nullptr));
         }
     }
     if (verbose) printf("intensity range %g..%g, isolevel %g\n", mn, mx, iso);
-    VolStats s1 = s0;
+    if (!label) s1 = s0;
     float min_after = mn;
     bool lazy = false;   // labelled, but the volume is not written
     if (label) {
-        // (a stale isolevel's exact smoothing above left its statistics there)
-        CK(cudaMemcpyAsync(dst + 1, &h[1], sizeof(VolStats), cudaMemcpyHostToDevice, c->stream));
-        const bool above = o.cubes == N2M_CUBES_OLDCUBES;
-        CKS(run_labelling(vol, nx, ny, nz, iso, mn, o.only_largest, o.fill_bubbles, above, c->lab, dst + 1, c->stream,
-                          od ? c->od.vsign.as<unsigned>() : nullptr, &c->lpost));
-        if (c->lpost.S) CKS(readback(c, &s1, dst + 1));
-        lazy = c->lpost.S && s1.masked;   // some voxel holds mn, every value is >= mn: it is the result's minimum
+        if (!labelled) {
+            CKS(labelling());
+            if (c->lpost.S) CKS(readback(c, &s1, dst + 1));
+        }
+        c->lpost.mn = mn;
+        volatile float below = mn - iso;
+        // some voxel holds mn, every value is >= mn: it is the result's minimum; mn has to be outside
+        lazy = c->lpost.S && s1.masked && !(below > -N2M_FLT_EPS);
         if (!lazy) {   // the whole labelled volume, whose minimum has to be found
             if (od) {
                 od = false;
@@ -708,8 +749,9 @@ n2m_status prepare(n2m_context *c, const float *d_src, const int dim[3], const n
 }
 
 // stage 4: marching cubes into pts_raw / tris_raw
-n2m_status march(n2m_context *c, const Prep &P, const int dim[3], int cubes, int *nv_out, int *nt_out,
-                 int *ncand_out) {
+// (filter: and, unless there is something to weld, the degenerate filter: *kept_out >= 0 then)
+n2m_status march(n2m_context *c, const Prep &P, const int dim[3], int cubes, bool filter, int *nv_out, int *nt_out,
+                 int *ncand_out, int *kept_out) {
     c->fwd.valid = false;
     const bool old = cubes == N2M_CUBES_OLDCUBES;
     McGrid g;
@@ -728,8 +770,9 @@ n2m_status march(n2m_context *c, const Prep &P, const int dim[3], int cubes, int
         n2m_set_error("grid of %.0f points exceeds the 32-bit range", ng);
         return N2M_ERR_TOO_LARGE;
     }
-    CKS(c->totals.ensure(sizeof(uint4)));
-    uint4 *dtot = c->totals.as<uint4>();
+    CKS(c->march.ensure(sizeof(MarchOut)));
+    MarchOut *dm = c->march.as<MarchOut>();
+    uint4 *dtot = &dm->tot;
     if (P.od) {
         const size_t n = (size_t)dim[0] * dim[1] * dim[2];
         CKS(c->stmp2.ensure(n * sizeof(float)));
@@ -740,8 +783,48 @@ n2m_status march(n2m_context *c, const Prep &P, const int dim[3], int cubes, int
     } else if (old) CKS(oc_count(P.vol, dim, P.lo, P.hi, P.iso, P.edge_max, c->mc, dtot, c->stream, c->od, nullptr, P.post));
     else CKS(mc_count(g, cubes, c->mc, dtot, c->stream, c->od, nullptr, P.post));
     CK(cudaEventRecord(c->evs[3], c->stream));
-    uint4 tot;
-    CKS(readback(c, &tot, dtot));
+    // The emit and the filter are queued with the buffers of earlier calls and take the counts on the device, so that
+    // one wait brings counts, candidates and the filter's result; a mesh that does not fit (or the context's first)
+    // is emitted after the buffers have grown.
+    c->marks = nullptr;
+    const bool marks = std::max({dim[0], dim[1], dim[2]}) < 1 << 22;   // NEAR_CORNER
+    int cap = 0;
+    auto emit = [&](MeshRoom room) -> n2m_status {
+        CK(cudaMemsetAsync(&dm->ncand, 0, 4 * sizeof(unsigned), c->stream));
+        unsigned *near = nullptr;   // marks for the degenerate filter
+        if (marks) {
+            const size_t nb = ((size_t)room.nv + 31) / 32 * sizeof(unsigned);
+            CKS(c->deg.near.ensure(nb));
+            near = c->deg.near.as<unsigned>();
+            CK(cudaMemsetAsync(near, 0, nb, c->stream));
+        }
+        c->marks = near;
+        vec3d *pts = c->pts_raw.as<vec3d>();
+        vec3i *tris = c->tris_raw.as<vec3i>();
+        int *cand = c->cand.as<int>();
+        if (old) CKS(oc_emit(P.vol, dim, P.lo, P.hi, P.iso, P.edge_max, c->mc, dm, room, pts, tris, cand, cap, near, c->stream));
+        else CKS(mc_emit(g, cubes, c->mc, dm, room, pts, tris, cand, cap, near, c->stream));
+        CK(cudaEventRecord(c->evs[4], c->stream));
+        CK(cudaEventRecord(c->evs[5], c->stream));
+        if (filter) {
+            CKS(mesh_after_emit(pts, tris, room, cand, cap, near, c->tris.as<vec3i>(), dm, c->deg, c->stream));
+            CK(cudaEventRecord(c->evs[6], c->stream));
+            CK(cudaEventRecord(c->ev1, c->stream));
+        } else CKS(mesh_weld_candidates(pts, room, cand, cap, dm, c->stream));
+        return N2M_OK;
+    };
+    MeshRoom room{0u, 0u};
+    if (c->pts_raw.cap && c->tris_raw.cap && c->cand.cap && (!filter || c->tris.cap)) {
+        room.nv = (unsigned)std::min<size_t>(c->pts_raw.cap / sizeof(vec3d), 0x7fffffff);
+        room.nt = (unsigned)std::min<size_t>((filter ? std::min(c->tris_raw.cap, c->tris.cap) : c->tris_raw.cap) / sizeof(vec3i),
+                                             0x7fffffff);
+        cap = (int)std::min<size_t>(c->cand.cap / (2 * sizeof(int)), 1 << 26);
+        if (cap < 1 << 26) room.nv = (unsigned)std::min<size_t>(room.nv, (size_t)std::max(cap - 65536, 0) * 16);   // whose candidates fit
+        CKS(emit(room));
+    }
+    MarchOut &m = c->mo;
+    CKS(readback(c, &m, dm));
+    const uint4 tot = m.tot;
     const unsigned long long nv = (unsigned long long)tot.x + tot.z, nt = tot.y;
     if (nv >= 0x7fffffffULL || nt >= 0x7fffffffULL) {
         n2m_set_error("mesh too large for 32-bit indices");
@@ -752,47 +835,39 @@ n2m_status march(n2m_context *c, const Prep &P, const int dim[3], int cubes, int
         n2m_set_error("marching cubes produced no surface");
         return N2M_ERR_EMPTY;
     }
-    CKS(c->pts_raw.ensure(nv * sizeof(vec3d)));
-    CKS(c->tris_raw.ensure(nt * sizeof(vec3i)));
-    const int cap = (int)std::min<unsigned long long>(nv / 16 + 65536, 1 << 26);
-    CKS(c->cand.ensure((size_t)2 * cap * sizeof(int)));
-    CKS(c->ncand.ensure(2 * sizeof(unsigned)));
-    CK(cudaMemsetAsync(c->ncand.p, 0, 2 * sizeof(unsigned), c->stream));
+    const int need = (int)std::min<unsigned long long>(nv / 16 + 65536, 1 << 26);
+    if (!room.fits(tot)) {   // nothing was emitted
+        CKS(c->pts_raw.ensure(nv * sizeof(vec3d)));
+        CKS(c->tris_raw.ensure(nt * sizeof(vec3i)));
+        CKS(c->cand.ensure((size_t)2 * need * sizeof(int)));
+        if (filter) CKS(c->tris.ensure(nt * sizeof(vec3i)));
+        cap = need;
+        room = MeshRoom{(unsigned)nv, (unsigned)nt};
+        CKS(emit(room));
+        CKS(readback(c, &m, dm));
+    }
     McCounts mcn{tot.x, tot.y, tot.z, tot.w};
-    unsigned *near = nullptr;   // marks for the degenerate filter
-    if (std::max({dim[0], dim[1], dim[2]}) < 1 << 22) {
-        CKS(c->deg.near.ensure((nv + 31) / 32 * sizeof(unsigned)));
-        near = c->deg.near.as<unsigned>();
-        CK(cudaMemsetAsync(near, 0, (nv + 31) / 32 * sizeof(unsigned), c->stream));
-    }
-    c->marks = near;
-    if (old) {
-        CKS(oc_emit(P.vol, dim, P.lo, P.hi, P.iso, P.edge_max, c->mc, mcn, c->pts_raw.as<vec3d>(),
-                    c->tris_raw.as<vec3i>(), c->cand.as<int>(), c->ncand.as<unsigned>(), cap, near, c->stream));
-    } else {
-        CKS(mc_emit(g, cubes, c->mc, mcn, c->pts_raw.as<vec3d>(), c->tris_raw.as<vec3i>(), c->cand.as<int>(),
-                    c->ncand.as<unsigned>(), cap, near, c->stream));
-    }
-    unsigned nc[2];
-    CKS(readback(c, nc, c->ncand.p, 2));
-    if (nc[0] > (unsigned)cap || nc[1] > (unsigned)cap) {
-        n2m_set_error("weld candidate overflow (%u, %u > %d)", nc[0], nc[1], cap);
+    unsigned nc[2] = {m.ncand, m.nccand};
+    if (nc[0] > (unsigned)need || nc[1] > (unsigned)need) {
+        n2m_set_error("weld candidate overflow (%u, %u > %d)", nc[0], nc[1], need);
         return N2M_ERR_INTERNAL;
     }
+    *kept_out = filter && !(nc[0] | nc[1]) ? (int)m.kept : -1;
+    c->mo_cand = nc[1] == 0 && nc[0] <= (unsigned)MARCH_CAND;
     if (nc[1]) {   // c-vertex candidates: collect every vertex near them
         CK(cudaMemcpyAsync(c->cand.as<int>() + nc[0], c->cand.as<int>() + cap, nc[1] * sizeof(int),
                            cudaMemcpyDeviceToDevice, c->stream));
         unsigned tot2 = nc[0] + nc[1];
-        CK(cudaMemcpyAsync(c->ncand.p, &tot2, sizeof(unsigned), cudaMemcpyHostToDevice, c->stream));
+        CK(cudaMemcpyAsync(&dm->ncand, &tot2, sizeof(unsigned), cudaMemcpyHostToDevice, c->stream));
         CKS(mc_ccand_scan(c->pts_raw.as<vec3d>(), (int)nv, c->cand.as<int>() + cap, (int)nc[1], c->cand.as<int>(),
-                          c->ncand.as<unsigned>(), cap, c->stream));
-        CKS(readback(c, nc, c->ncand.p, 1));
+                          &dm->ncand, cap, c->stream));
+        CKS(readback(c, nc, &dm->ncand, 1));
         if (nc[0] > (unsigned)cap) {
             n2m_set_error("weld candidate overflow");
             return N2M_ERR_INTERNAL;
         }
     }
-    CK(cudaEventRecord(c->evs[4], c->stream));
+    if (*kept_out < 0) CK(cudaEventRecord(c->evs[4], c->stream));
     c->fwd.g = g;
     c->fwd.mcn = mcn;
     c->fwd.cubes = cubes;
@@ -822,8 +897,9 @@ n2m_status pipeline(n2m_context *c, const float *d_src, const int dim[3], const 
     CK(cudaEventRecord(c->ev0, c->stream));
     Prep P;
     CKS(prepare(c, d_src, dim, o, o.verbose, P, rep));
-    int nv, nt, ncand;
-    CKS(march(c, P, dim, o.cubes, &nv, &nt, &ncand));
+    const bool early = c->want_host && o.post_smooth <= 0;   // vertices are final after the weld
+    int nv, nt, ncand, kept;
+    CKS(march(c, P, dim, o.cubes, !early, &nv, &nt, &ncand, &kept));
     if (c->want_host && !c->user_p) {   // keep buffers started early if they are large enough, else start them now
         const size_t pb = (size_t)std::max(nv, 1) * sizeof(vec3d), tb = (size_t)std::max(nt, 1) * sizeof(vec3i);
         if (!c->hout.pts || c->hout.pb < pb || c->hout.tb < tb) c->hout.start(pb, tb);
@@ -842,25 +918,33 @@ n2m_status pipeline(n2m_context *c, const float *d_src, const int dim[3], const 
         if (o.cubes == N2M_CUBES_OLDCUBES) {
             CKS(weld_oc(c, P, dim, nv, nt, ncand, removed, keep, ov_id, ov_pos, ov_src, corners));
         } else {
-            vec3d v0;
-            CKS(readback(c, &v0, pts));
+            vec3d v0 = c->mo.first;
+            if (!c->mo_cand) CKS(readback(c, &v0, pts));
             CKS(weld_candidates(c, nv, ncand, removed, keep, ov_id, ov_pos, ov_src, v0));
         }
         if (!removed.empty() || !ov_id.empty()) {
             const int nr = (int)removed.size(), no = (int)ov_id.size(), ncr = (int)corners.size();
-            CKS(c->weld.ensure((size_t)(2 * nr + 2 * no + 2) * sizeof(int) + (size_t)(no + 1) * sizeof(vec3d) +
-                               (size_t)(ncr + 1) * sizeof(int2)));
+            // positions, corners and ids in one upload
+            const size_t bytes = (size_t)no * sizeof(vec3d) + (size_t)ncr * sizeof(int2) + (size_t)(2 * nr + 2 * no) * sizeof(int);
+            CKS(c->weld.ensure(bytes));
+            std::vector<char> large(bytes > N2M_UPLOAD ? bytes : 0);
+            char *const up = bytes > N2M_UPLOAD ? large.data() : (char *)c->pinned + N2M_READBACK;
+            char *to = up;
+            auto put = [&to](const void *from, size_t len) {
+                if (len) memcpy(to, from, len);
+                to += len;
+            };
+            put(ov_pos.data(), no * sizeof(vec3d));
+            put(corners.data(), ncr * sizeof(int2));
+            put(removed.data(), nr * sizeof(int));
+            put(keep.data(), nr * sizeof(int));
+            put(ov_id.data(), no * sizeof(int));
+            put(ov_src.data(), no * sizeof(int));
             vec3d *dov = c->weld.as<vec3d>();
-            int2 *dcr = (int2 *)(dov + no + 1);
-            int *drem = (int *)(dcr + ncr + 1);
-            int *dkeep = drem + nr, *dovid = dkeep + nr, *dovsrc = dovid + no + 1;
-            if (no) CK(cudaMemcpyAsync(dov, ov_pos.data(), no * sizeof(vec3d), cudaMemcpyHostToDevice, c->stream));
-            if (nr) CK(cudaMemcpyAsync(drem, removed.data(), nr * sizeof(int), cudaMemcpyHostToDevice, c->stream));
-            if (nr) CK(cudaMemcpyAsync(dkeep, keep.data(), nr * sizeof(int), cudaMemcpyHostToDevice, c->stream));
-            if (no) CK(cudaMemcpyAsync(dovid, ov_id.data(), no * sizeof(int), cudaMemcpyHostToDevice, c->stream));
-            if (no) CK(cudaMemcpyAsync(dovsrc, ov_src.data(), no * sizeof(int), cudaMemcpyHostToDevice, c->stream));
+            int2 *dcr = (int2 *)(dov + no);
+            int *drem = (int *)(dcr + ncr), *dkeep = drem + nr, *dovid = dkeep + nr, *dovsrc = dovid + no;
+            CK(cudaMemcpyAsync(dov, up, bytes, cudaMemcpyHostToDevice, c->stream));
             if (ncr) {   // split vertices: corners take their copy's group vertex before the renumbering
-                CK(cudaMemcpyAsync(dcr, corners.data(), ncr * sizeof(int2), cudaMemcpyHostToDevice, c->stream));
                 n2m_launch(k_set_corners, (ncr + 255) / 256, 256, 0, c->stream, c->tris_raw.as<vec3i>(), dcr, ncr);
                 CKL();
             }
@@ -874,39 +958,40 @@ n2m_status pipeline(n2m_context *c, const float *d_src, const int dim[3], const 
             CKS(mesh_apply_weld(pts, nv, drem, nr, dkeep, dovid, dov, no, c->pts.as<vec3d>(), c->deg, map, c->stream));
             pts = c->pts.as<vec3d>();
             welded = nr;
-            CK(cudaStreamSynchronize(c->stream));   // host vectors go out of scope
+            if (!large.empty()) CK(cudaStreamSynchronize(c->stream));   // it goes out of scope
         }
     }
-    CK(cudaEventRecord(c->evs[5], c->stream));
     if (np < 3) {
         n2m_set_error("fewer than 3 vertices after the weld");
         return N2M_ERR_EMPTY;
     }
-    CKS(c->tris.ensure((size_t)nt * sizeof(vec3i)));
-    CKS(c->ntf.ensure(sizeof(unsigned)));
     c->pts_early = false;
-    const bool early = c->want_host && o.post_smooth <= 0;   // vertices are final after the weld
-    if (early) CK(cudaEventRecord(c->stage.ev[0], c->stream));
-    CKS(mesh_remove_degenerate(pts, c->tris_raw.as<vec3i>(), nt, map, c->marks, c->tris.as<vec3i>(),
-                               c->ntf.as<unsigned>(), c->deg, c->stream));
-    if (early) {   // copy them out on the second stream while the degenerate filter runs
-        void *dst = nullptr;
-        if (c->user_p) {
-            if ((size_t)np <= c->user_pcap) dst = c->user_p;
-        } else {
-            c->hout.join();
-            if (c->hout.pts && c->hout.pb >= (size_t)np * sizeof(vec3d)) dst = c->hout.pts;
+    if (kept < 0) {   // there were candidates, or the vertices are copied out meanwhile
+        CK(cudaEventRecord(c->evs[5], c->stream));
+        CKS(c->tris.ensure((size_t)nt * sizeof(vec3i)));
+        if (early) CK(cudaEventRecord(c->stage.ev[0], c->stream));
+        MarchOut *dm = c->march.as<MarchOut>();
+        CKS(mesh_remove_degenerate(pts, c->tris_raw.as<vec3i>(), nt, map, c->marks, c->tris.as<vec3i>(), &dm->kept, c->deg,
+                                   c->stream));
+        if (early) {   // copy them out on the second stream while the degenerate filter runs
+            void *dst = nullptr;
+            if (c->user_p) {
+                if ((size_t)np <= c->user_pcap) dst = c->user_p;
+            } else {
+                c->hout.join();
+                if (c->hout.pts && c->hout.pb >= (size_t)np * sizeof(vec3d)) dst = c->hout.pts;
+            }
+            if (dst) {
+                CK(cudaStreamWaitEvent(c->copy, c->stage.ev[0], 0));
+                CK(cudaMemcpyAsync(dst, pts, (size_t)np * sizeof(vec3d), cudaMemcpyDeviceToHost, c->copy));
+                c->pts_early = true;
+            }
         }
-        if (dst) {
-            CK(cudaStreamWaitEvent(c->copy, c->stage.ev[0], 0));
-            CK(cudaMemcpyAsync(dst, pts, (size_t)np * sizeof(vec3d), cudaMemcpyDeviceToHost, c->copy));
-            c->pts_early = true;
-        }
+        CK(cudaEventRecord(c->evs[6], c->stream));
+        CK(cudaEventRecord(c->ev1, c->stream));
+        CKS(readback(c, &kept, &dm->kept));
     }
-    CK(cudaEventRecord(c->evs[6], c->stream));
-    CK(cudaEventRecord(c->ev1, c->stream));
-    unsigned ntf;
-    CKS(readback(c, &ntf, c->ntf.p));
+    const unsigned ntf = (unsigned)kept;
     c->res_pts = pts;
     c->res_tris = c->tris.as<vec3i>();
     c->res_np = np;
@@ -1408,14 +1493,14 @@ extern "C" void laplacian_smoothHC(vec3d *verts, vec3i *tris, int nvert, int ntr
 extern "C" n2m_status n2m_set_threshold_device(n2m_context *c, const float *d_img, int64_t nvox, int mode, float *iso) {
     if (!c || !iso || (nvox > 0 && !d_img)) return N2M_ERR_BAD_ARGS;
     CK(cudaSetDevice(c->device));
-    return isolevel_otsu(d_img, nvox, mode, c->th, c->stream, iso);
+    return isolevel_otsu(d_img, nvox, mode, c->th, c->stream, iso, c->pinned);
 }
 
 extern "C" n2m_status n2m_set_threshold(n2m_context *c, const float *img, int64_t nvox, int mode, float *iso) {
     if (!c || !iso || (nvox > 0 && !img)) return N2M_ERR_BAD_ARGS;
     CK(cudaSetDevice(c->device));
     if (nvox > 0) CKS(upload(c, img, (size_t)nvox));
-    return isolevel_otsu(c->in.as<float>(), nvox, mode, c->th, c->stream, iso);
+    return isolevel_otsu(c->in.as<float>(), nvox, mode, c->th, c->stream, iso, c->pinned);
 }
 
 extern "C" float setThreshold(float *img, int nvox, int darkMediumBright123) {
@@ -1502,8 +1587,8 @@ extern "C" int marchingCubes(float *img, short dim[3], int lo[3], int hi[3], int
             P.mnp = ord2f(h.vmin);
         }
         const int cubes = g_oldcubes ? N2M_CUBES_OLDCUBES : (originalMC ? N2M_CUBES_CLASSIC_TABLE : N2M_CUBES_MC33);
-        int v = 0, t = 0, ncand = 0;
-        if (s == N2M_OK) s = march(c, P, d, cubes, &v, &t, &ncand);
+        int v = 0, t = 0, ncand = 0, kept = -1;
+        if (s == N2M_OK) s = march(c, P, d, cubes, false, &v, &t, &ncand, &kept);
         if (s == N2M_OK) {
             c->res_pts = c->pts_raw.as<vec3d>();
             c->res_tris = c->tris_raw.as<vec3i>();

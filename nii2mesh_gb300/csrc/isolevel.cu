@@ -146,6 +146,31 @@ void otsu_table(const unsigned *H, int nb, std::vector<double> &P) {
         }
 }
 
+// the table's first row and last column, all that one boundary needs (the whole table is 65536 divisions)
+void otsu_edges(const unsigned *H, double *first, double *last) {
+    constexpr int nb = NB_OTSU;
+    double Sum = 0.0;
+    for (int v = 0; v < nb; v++) Sum = Sum + H[v];
+    double P[nb], S[nb], Q[nb], T[nb];
+    P[0] = H[0];
+    S[0] = H[0];
+    for (int v = 1; v < nb; v++) {
+        const double prob = H[v] / Sum;
+        P[v] = P[v - 1] + prob;
+        S[v] = S[v - 1] + (v + 1) * prob;
+    }
+    Q[0] = P[nb - 1];
+    T[0] = S[nb - 1];
+    for (int u = 1; u < nb; u++) {
+        Q[u] = P[nb - 1] - P[u - 1];
+        T[u] = S[nb - 1] - S[u - 1];
+    }
+    for (int k = 0; k < nb; k++) {
+        first[k] = P[k] != 0 ? (S[k] * S[k]) / P[k] : P[k];
+        last[k] = Q[k] != 0 ? (T[k] * T[k]) / Q[k] : Q[k];
+    }
+}
+
 unsigned grid_for(long long n) {
     long long b = (n + 255) / 256;
     if (b > 152 * 8) b = 152 * 8;
@@ -154,7 +179,7 @@ unsigned grid_for(long long n) {
 }  // namespace
 
 n2m_status isolevel_otsu(const float *d_img, long long nvox, int mode123, ThresholdWork &w, cudaStream_t s,
-                         float *result) {
+                         float *result, void *pinned) {
     *result = 1.0f;   // the reference's value when there are no voxels
     if (nvox < 1) return N2M_OK;
     if (nvox > 2147483647ll) {
@@ -167,12 +192,11 @@ n2m_status isolevel_otsu(const float *d_img, long long nvox, int mode123, Thresh
     ThRange *d_r = w.buf.as<ThRange>();
     unsigned *d_h1 = (unsigned *)(d_r + 1), *d_h2 = d_h1 + NB_RANGE;
     Best *d_best = (Best *)((char *)w.buf.p + best_off);
-    ThRange hr;
-    ThRange *h_r = &hr;
-    std::vector<unsigned> hist_v(NB_RANGE);
-    unsigned *h_hist = hist_v.data();
-    std::vector<Best> best_v(256);
-    Best *h_best = best_v.data();
+    ThRange *h_r = (ThRange *)pinned;   // one of the three at a time
+    unsigned *h_hist = (unsigned *)pinned;
+    Best *h_best = (Best *)pinned;
+    static_assert(sizeof(ThRange) <= N2M_READBACK && NB_RANGE * sizeof(unsigned) <= N2M_READBACK && 256 * sizeof(Best) <= N2M_READBACK,
+                  "readbacks fit the pinned buffer");
 
     // (1) range of the non-NaN voxels (src/isolevel.c:47-61)
     *h_r = ThRange{f2ord_host(INFINITY), f2ord_host(-INFINITY), 0, 0};
@@ -237,10 +261,10 @@ n2m_status isolevel_otsu(const float *d_img, long long nvox, int mode123, Thresh
     for (int v = 0; v < NB_OTSU; v++) Sum = Sum + h_hist[v];
     int dark = 0, mid = 0, bright = 0;
     if (Sum > 0) {
-        otsu_table(h_hist, NB_OTSU, w.P);
-        const std::vector<double> &P = w.P;
         const int nb = NB_OTSU;
         if (mode123 == 1 || mode123 == 3) {
+            otsu_table(h_hist, NB_OTSU, w.P);
+            const std::vector<double> &P = w.P;
             // three boundaries (src/isolevel.c:182-205): start from the quartiles, keep the first strict maximum
             int lo = (int)(0.25 * nb), mi = (int)(0.50 * nb), hi = (int)(0.75 * nb);
             const double start = P[lo] + P[(size_t)(lo + 1) * nb + mi] + P[(size_t)(mi + 1) * nb + hi] +
@@ -264,10 +288,12 @@ n2m_status isolevel_otsu(const float *d_img, long long nvox, int mode123, Thresh
             bright = hi;
         } else {
             // one boundary (src/isolevel.c:222-236)
+            double first[NB_OTSU], last[NB_OTSU];
+            otsu_edges(h_hist, first, last);
             int thresh = (int)(0.25 * nb);
-            double best = P[thresh] + P[(size_t)(thresh + 1) * nb + nb - 1];
+            double best = first[thresh] + last[thresh + 1];
             for (int i = 0; i < nb - 1; i++) {
-                const double v = P[i] + P[(size_t)(i + 1) * nb + nb - 1];
+                const double v = first[i] + last[i + 1];
                 if (v > best) {
                     thresh = i;
                     best = v;

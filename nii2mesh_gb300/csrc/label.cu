@@ -931,9 +931,8 @@ n2m_status class_bits(LabelWork &w, const LD &d, const float *vol, float iso, bo
 }
 }  // namespace
 
-n2m_status run_labelling(const float *vol, int nx, int ny, int nz, float iso, float mn, bool only_largest,
-                         bool fill_bubbles, bool at_or_above, LabelWork &w, VolStats *st, cudaStream_t s, const unsigned *vsign,
-                         LabelPost *post) {
+n2m_status run_labelling(const float *vol, int nx, int ny, int nz, float iso, bool only_largest, bool fill_bubbles,
+                         bool at_or_above, LabelWork &w, VolStats *st, cudaStream_t s, const unsigned *vsign, LabelPost *post) {
     const LD d = make_ld(nx, ny, nz);
     if (vsign) {
         if (d.n > 0x7fffffffLL) {
@@ -948,9 +947,8 @@ n2m_status run_labelling(const float *vol, int nx, int ny, int nz, float iso, fl
     }
     const unsigned *K;
     CKS(label_core(w, d, 18, only_largest, fill_bubbles, s, &K));
-    *post = LabelPost{K, nullptr, nullptr, d.W, mn, iso, fill_bubbles, only_largest};
-    volatile float below = mn - iso;
-    if (only_largest && !(below > -N2M_FLT_EPS)) {
+    *post = LabelPost{K, nullptr, nullptr, d.W, 0.f, iso, fill_bubbles, only_largest};
+    if (only_largest) {
         CKS(w.shell.ensure(2 * (size_t)d.nwords * sizeof(unsigned)));
         unsigned *S = w.shell.as<unsigned>(), *KD = S + d.nwords;
         n2m_launch(k_lab_shell, std::min(gsz(d.nwords), 152u * 16u), 256, 0, s, K, d, vol, iso, at_or_above, S, KD, st);

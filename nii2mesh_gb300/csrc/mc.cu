@@ -527,16 +527,16 @@ n2m_status mc_count(const McGrid &g, int variant, McWork &w, uint4 *d_total, cud
     return mcw::count_values(pol, signs, w, o, !classic, s);
 }
 
-n2m_status mc_emit(const McGrid &g, int variant, McWork &w, const McCounts &c, vec3d *d_pts, vec3i *d_tris,
-                   int *d_cand, unsigned *d_ncand, int cand_cap, unsigned *d_near, cudaStream_t s) {
+n2m_status mc_emit(const McGrid &g, int variant, McWork &w, MarchOut *d_out, const MeshRoom &room, vec3d *d_pts, vec3i *d_tris,
+                   int *d_cand, int cand_cap, unsigned *d_near, cudaStream_t s) {
     const GV v = make_gv(g);
-    if (c.nactive == 0) return N2M_OK;
     size_t nwords;
     CKS(grid_words(v, nwords));
     mcw::Out o;
-    CKS(mcw::prepare(w, nwords, nullptr, o));
-    const Policy pol{v, variant == N2M_CUBES_CLASSIC_TABLE, d_pts, d_cand, d_cand + cand_cap, d_ncand, d_ncand + 1, cand_cap, d_near};
-    return mcw::emit(pol, w.signs.as<unsigned>(), w, o, c.nactive, d_tris, s);
+    CKS(mcw::prepare(w, nwords, &d_out->tot, o));
+    const Policy pol{v, variant == N2M_CUBES_CLASSIC_TABLE, d_pts, d_cand, d_cand + cand_cap, &d_out->ncand, &d_out->nccand,
+                     cand_cap, d_near};
+    return mcw::emit(pol, w.signs.as<unsigned>(), w, o, room, d_tris, s);
 }
 
 n2m_status mc_backward(const McGrid &g, int variant, McWork &w, const McCounts &c, const float3 *d_gv, float *d_gs,

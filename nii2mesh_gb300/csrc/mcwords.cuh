@@ -461,8 +461,13 @@ struct EmitShared {
 
 template <class P>
 __global__ void __launch_bounds__(EW * 32, P::CTAS) k_emit(P pol, const unsigned *__restrict__ signs, Out o, const uint4 *__restrict__ act,
-                                                           unsigned nact, unsigned G, vec3i *tris) {
+                                                           unsigned warps, MeshRoom room, vec3i *tris) {
     grid_wait();
+    const uint4 tot = *o.total;
+    if (!room.fits(tot)) return;   // emitted again into larger buffers
+    // 32 words per group keep the per-group work small; below two groups per resident warp smaller groups
+    // spread the mesh over the GPU instead (8 words still fill the lanes: a word has about 7 vertices)
+    const unsigned nact = tot.w, G = nact >= 64u * warps ? 32u : (nact >= 16u * warps ? 16u : 8u);
     const uint4 *__restrict__ words = o.words;
     __shared__ EmitShared shared[EW];
     __shared__ unsigned qt[256];
@@ -711,17 +716,13 @@ inline n2m_status resident_ctas(const void *fn, std::atomic<int> (&of)[64], int 
     return N2M_OK;
 }
 
+// the counts are taken on the device (the grid is what fits the GPU at once); a mesh beyond `room` is not emitted
 template <class P>
-n2m_status emit(const P &pol, const unsigned *signs, McWork &w, const Out &o, unsigned nact, vec3i *d_tris, cudaStream_t s) {
+n2m_status emit(const P &pol, const unsigned *signs, McWork &w, const Out &o, const MeshRoom &room, vec3i *d_tris, cudaStream_t s) {
     static std::atomic<int> resident[64];   // work comes from an atomic counter, so any grid is correct
     int n = 0;
     CKS(resident_ctas((const void *)k_emit<P>, resident, n));
-    // 32 words per group keep the per-group work small; below two groups per resident warp smaller groups
-    // spread the mesh over the GPU instead (8 words still fill the lanes: a word has about 7 vertices)
-    const unsigned warps = (unsigned)n * EW;
-    const unsigned G = nact >= 64u * warps ? 32u : (nact >= 16u * warps ? 16u : 8u);
-    const unsigned blocks = std::min(((nact + G - 1) / G + EW - 1) / EW, (unsigned)n);
-    n2m_launch(k_emit<P>, blocks, EW * 32, 0, s, pol, signs, o, w.act.as<uint4>(), nact, G, d_tris);
+    n2m_launch(k_emit<P>, (unsigned)n, EW * 32, 0, s, pol, signs, o, w.act.as<uint4>(), (unsigned)n * EW, room, d_tris);
     CKL();
     return N2M_OK;
 }

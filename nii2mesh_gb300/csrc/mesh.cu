@@ -125,14 +125,13 @@ static_assert(DT == 4 * CB && DT == 32 * 32, "four triangles per thread, a warp 
 // its own for the renumbering took 93 + 61 us, the general path here 126 (the whole filter
 // with the copy 164), with the marks the filter takes 111; oldcubes (4.1 M) 132 -> 61.
 template <bool NEAR>
-__global__ void __launch_bounds__(CB, 4) k_deg_count(const vec3d *__restrict__ p, vec3i *t, int nt, WeldMap m,
-                                                     const unsigned *__restrict__ near, unsigned *bits, unsigned *tile_cnt,
-                                                     unsigned *group_cnt) {
-    grid_wait();
+__device__ __forceinline__ void deg_count_tile(unsigned tile, const vec3d *__restrict__ p, vec3i *t, int nt, const WeldMap &m,
+                                               const unsigned *__restrict__ near, unsigned *bits, unsigned *tile_cnt,
+                                               unsigned *group_cnt) {
     __shared__ unsigned kept[DT / 32], nslow;
     __shared__ unsigned short slow[DT];
     const int tid = threadIdx.x, lane = tid & 31;
-    const unsigned i0 = blockIdx.x * DT + 4u * tid;
+    const unsigned i0 = tile * DT + 4u * tid;
     const int n = i0 < (unsigned)nt ? (int)min(4u, (unsigned)nt - i0) : 0;
     if (tid == 0) nslow = 0;
     __syncthreads();
@@ -182,18 +181,56 @@ __global__ void __launch_bounds__(CB, 4) k_deg_count(const vec3d *__restrict__ p
     __syncthreads();
     for (unsigned k = tid; k < nslow; k += CB) {
         const int i = slow[k];
-        const vec3i T = t[blockIdx.x * DT + i];
+        const vec3i T = t[tile * DT + i];
         if ((NEAR && surely_kept(p[T.x], p[T.y], p[T.z])) || !degenerate_ref(p[T.x], p[T.y], p[T.z])) atomicOr(&kept[i / 32], 1u << (i & 31));
     }
     __syncthreads();
     if (tid < 32) {
         w = kept[tid];
-        bits[blockIdx.x * (DT / 32) + tid] = w;
+        bits[tile * (DT / 32) + tid] = w;
         const unsigned sum = __reduce_add_sync(0xffffffffu, __popc(w));
         if (tid == 0) {
-            tile_cnt[blockIdx.x] = sum;
-            atomicAdd(&group_cnt[blockIdx.x / DG], sum);
+            tile_cnt[tile] = sum;
+            atomicAdd(&group_cnt[tile / DG], sum);
         }
+    }
+}
+
+// the weld's candidates for the host
+__device__ __forceinline__ void give_candidates(const vec3d *__restrict__ p, const int *__restrict__ cand, MarchOut *mo) {
+    const unsigned n = mo->ncand;
+    for (unsigned k = threadIdx.x; k < min(n, (unsigned)MARCH_CAND); k += blockDim.x) {
+        mo->cand_id[k] = cand[k];
+        mo->cand_pos[k] = p[cand[k]];
+    }
+    if (threadIdx.x == 0) mo->first = p[0];
+}
+
+__global__ void __launch_bounds__(CB) k_weld_candidates(const vec3d *__restrict__ p, MeshRoom room, const int *__restrict__ cand,
+                                                        int cap, MarchOut *mo) {
+    grid_wait();
+    if (mo->ncand && mo->ncand <= (unsigned)cap && room.fits(mo->tot)) give_candidates(p, cand, mo);
+}
+
+// with mo the number of triangles is its count; nothing is done if the mesh did not fit or has to be welded first
+template <bool NEAR>
+__global__ void __launch_bounds__(CB, 4) k_deg_count(const vec3d *__restrict__ p, vec3i *t, int nt, WeldMap m,
+                                                     const unsigned *__restrict__ near, unsigned *bits, unsigned *tile_cnt,
+                                                     unsigned *group_cnt, MarchOut *mo, MeshRoom room, const int *__restrict__ cand,
+                                                     int cap) {
+    grid_wait();
+    if (mo) {
+        if (!room.fits(mo->tot)) return;
+        if (mo->ncand | mo->nccand) {
+            if (blockIdx.x == 0 && mo->ncand && mo->ncand <= (unsigned)cap) give_candidates(p, cand, mo);
+            return;
+        }
+        nt = (int)mo->tot.y;
+    }
+    const unsigned tiles = ((unsigned)nt + DT - 1) / DT;
+    for (unsigned tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        deg_count_tile<NEAR>(tile, p, t, nt, m, near, bits, tile_cnt, group_cnt);
+        __syncthreads();   // the lists are reused by the next tile
     }
 }
 
@@ -201,13 +238,13 @@ __global__ void __launch_bounds__(CB, 4) k_deg_count(const vec3d *__restrict__ p
 // (a scan in between was three launches); a tile without a degenerate triangle,
 // nearly every one, is a plain copy.  tile_off: kept triangles before each tile.
 // 512^3 CT: 48 us with a lane per 12-byte record.
-__global__ void __launch_bounds__(CB) k_deg_compact(const vec3i *__restrict__ t, int nt, const unsigned *__restrict__ bits,
-                                                    const unsigned *__restrict__ tile_cnt, const unsigned *__restrict__ group_cnt,
-                                                    unsigned *tile_off, vec3i *out, unsigned *nt_out) {
-    grid_wait();
+__device__ __forceinline__ void deg_compact_tile(int tile, int tiles, const vec3i *__restrict__ t, int nt,
+                                                 const unsigned *__restrict__ bits, const unsigned *__restrict__ tile_cnt,
+                                                 const unsigned *__restrict__ group_cnt, unsigned *tile_off, vec3i *out,
+                                                 unsigned *nt_out) {
     __shared__ unsigned wsum[CB / 32], pre[DT / 32];
     __shared__ int stage[3 * DT];
-    const int tile = blockIdx.x, g = tile / DG, tid = threadIdx.x;
+    const int g = tile / DG, tid = threadIdx.x;
     unsigned s = 0;
     for (int k = tid; k < g; k += CB) s += group_cnt[k];
     if (tid < tile - g * DG) s += tile_cnt[g * DG + tid];
@@ -220,7 +257,7 @@ __global__ void __launch_bounds__(CB) k_deg_compact(const vec3i *__restrict__ t,
     const unsigned cnt = tile_cnt[tile];
     if (tid == 0) {
         tile_off[tile] = off;
-        if (tile == (int)gridDim.x - 1) *nt_out = off + cnt;
+        if (tile == tiles - 1) *nt_out = off + cnt;
     }
     const int *src = (const int *)(t + (size_t)tile * DT);
     int *dst = (int *)(out + off);
@@ -247,6 +284,22 @@ __global__ void __launch_bounds__(CB) k_deg_compact(const vec3i *__restrict__ t,
     }
     __syncthreads();
     for (int k = tid; k < 3 * (int)cnt; k += CB) dst[k] = stage[k];
+}
+
+__global__ void __launch_bounds__(CB) k_deg_compact(const vec3i *__restrict__ t, int nt, const unsigned *__restrict__ bits,
+                                                    const unsigned *__restrict__ tile_cnt, const unsigned *__restrict__ group_cnt,
+                                                    unsigned *tile_off, vec3i *out, unsigned *nt_out, const MarchOut *mo,
+                                                    MeshRoom room) {
+    grid_wait();
+    if (mo) {
+        if (!room.fits(mo->tot) || (mo->ncand | mo->nccand)) return;
+        nt = (int)mo->tot.y;
+    }
+    const int tiles = (int)(((unsigned)nt + DT - 1) / DT);
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        deg_compact_tile(tile, tiles, t, nt, bits, tile_cnt, group_cnt, tile_off, out, nt_out);
+        __syncthreads();   // the stage is reused by the next tile
+    }
 }
 
 // raw vertex gradient: every kept raw vertex receives its welded vertex's
@@ -305,20 +358,62 @@ n2m_status mesh_apply_weld(const vec3d *d_pts, int np, const int *d_removed, int
     return N2M_OK;
 }
 
+namespace {
+struct DegBufs {
+    unsigned *bits, *off, *cnt, *grp;
+};
+// buffers of the filter for nt triangles; the groups' counters are cleared
+n2m_status deg_buffers(long long nt, DegWork &w, cudaStream_t s, DegBufs &b) {
+    const long long tiles = std::max(1ll, (nt + DT - 1) / DT), groups = (tiles + DG - 1) / DG;
+    CKS(w.bits.ensure((size_t)tiles * (DT / 32) * sizeof(unsigned)));
+    CKS(w.tiles.ensure(((size_t)2 * tiles + groups) * sizeof(unsigned)));
+    b.bits = w.bits.as<unsigned>();
+    b.off = w.tiles.as<unsigned>();
+    b.cnt = b.off + tiles;
+    b.grp = b.cnt + tiles;
+    CK(cudaMemsetAsync(b.grp, 0, (size_t)groups * sizeof(unsigned), s));
+    return N2M_OK;
+}
+}  // namespace
+
 n2m_status mesh_remove_degenerate(const vec3d *d_pts, vec3i *d_tris_in, int nt, const WeldMap &weld, const unsigned *d_near,
                                   vec3i *d_tris_out, unsigned *d_nt_out, DegWork &w, cudaStream_t s) {
     if (nt == 0) {
         CK(cudaMemsetAsync(d_nt_out, 0, sizeof(unsigned), s));
         return N2M_OK;
     }
-    const int tiles = (int)(((long long)nt + DT - 1) / DT), groups = (tiles + DG - 1) / DG;
-    CKS(w.bits.ensure((size_t)tiles * (DT / 32) * sizeof(unsigned)));
-    CKS(w.tiles.ensure(((size_t)2 * tiles + groups) * sizeof(unsigned)));
-    unsigned *bits = w.bits.as<unsigned>(), *off = w.tiles.as<unsigned>(), *cnt = off + tiles, *grp = cnt + tiles;
-    CK(cudaMemsetAsync(grp, 0, (size_t)groups * sizeof(unsigned), s));
-    if (d_near) n2m_launch(k_deg_count<true>, tiles, CB, 0, s, d_pts, d_tris_in, nt, weld, d_near, bits, cnt, grp);
-    else n2m_launch(k_deg_count<false>, tiles, CB, 0, s, d_pts, d_tris_in, nt, weld, nullptr, bits, cnt, grp);
-    n2m_launch(k_deg_compact, tiles, CB, 0, s, d_tris_in, nt, bits, cnt, grp, off, d_tris_out, d_nt_out);
+    const int tiles = (int)(((long long)nt + DT - 1) / DT);
+    DegBufs b;
+    CKS(deg_buffers(nt, w, s, b));
+    const MeshRoom all{0u, 0u};
+    if (d_near) n2m_launch(k_deg_count<true>, tiles, CB, 0, s, d_pts, d_tris_in, nt, weld, d_near, b.bits, b.cnt, b.grp, nullptr,
+                           all, nullptr, 0);
+    else n2m_launch(k_deg_count<false>, tiles, CB, 0, s, d_pts, d_tris_in, nt, weld, nullptr, b.bits, b.cnt, b.grp, nullptr, all,
+                    nullptr, 0);
+    n2m_launch(k_deg_compact, tiles, CB, 0, s, d_tris_in, nt, b.bits, b.cnt, b.grp, b.off, d_tris_out, d_nt_out, nullptr, all);
+    CKL();
+    return N2M_OK;
+}
+
+n2m_status mesh_after_emit(const vec3d *d_pts, vec3i *d_tris_in, const MeshRoom &room, const int *d_cand, int cand_cap,
+                           const unsigned *d_near, vec3i *d_tris_out, MarchOut *d_out, DegWork &w, cudaStream_t s) {
+    DegBufs b;
+    CKS(deg_buffers(room.nt, w, s, b));
+    // the buffers may be much larger than this mesh: no more blocks than stay resident
+    const unsigned g = std::max(1u, std::min((room.nt + DT - 1) / DT, 152u * 6u));
+    const WeldMap none;
+    if (d_near) n2m_launch(k_deg_count<true>, g, CB, 0, s, d_pts, d_tris_in, 0, none, d_near, b.bits, b.cnt, b.grp, d_out, room,
+                           d_cand, cand_cap);
+    else n2m_launch(k_deg_count<false>, g, CB, 0, s, d_pts, d_tris_in, 0, none, nullptr, b.bits, b.cnt, b.grp, d_out, room, d_cand,
+                    cand_cap);
+    n2m_launch(k_deg_compact, g, CB, 0, s, d_tris_in, 0, b.bits, b.cnt, b.grp, b.off, d_tris_out, &d_out->kept, d_out, room);
+    CKL();
+    return N2M_OK;
+}
+
+n2m_status mesh_weld_candidates(const vec3d *d_pts, const MeshRoom &room, const int *d_cand, int cand_cap, MarchOut *d_out,
+                                cudaStream_t s) {
+    n2m_launch(k_weld_candidates, 1, CB, 0, s, d_pts, room, d_cand, cand_cap, d_out);
     CKL();
     return N2M_OK;
 }

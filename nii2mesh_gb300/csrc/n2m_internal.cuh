@@ -58,6 +58,9 @@ inline void n2m_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t share
     g_n2m_launches.fetch_add(1, std::memory_order_relaxed);
 }
 
+// bytes of a context's pinned buffer for small readbacks
+constexpr size_t N2M_READBACK = 16384;
+
 // ---- grow-only device buffers -----------------------------------------------
 struct DevBuf {
     void *p = nullptr;
@@ -202,9 +205,9 @@ struct LabelWork {
 // voxel was masked, lab_write labels the volume in place and gives its range and bbox.
 // vsign (may be null): a sign bitmap (OdWork::vsign with od_resolve's at_or_above) to
 // take the mask from; at_or_above: which sign S holds (value >= iso, for oldcubes)
-n2m_status run_labelling(const float *vol, int nx, int ny, int nz, float iso, float mn, bool only_largest,
-                         bool fill_bubbles, bool at_or_above, LabelWork &w, VolStats *st, cudaStream_t s, const unsigned *vsign,
-                         LabelPost *post);
+// (the minimum, post->mn, is the caller's to fill in)
+n2m_status run_labelling(const float *vol, int nx, int ny, int nz, float iso, bool only_largest, bool fill_bubbles,
+                         bool at_or_above, LabelWork &w, VolStats *st, cudaStream_t s, const unsigned *vsign, LabelPost *post);
 n2m_status lab_write(float *vol, int nx, int ny, int nz, const LabelPost &P, VolStats *st, cudaStream_t s);
 // the labelling's effect on the marked voxels of vol (marks as od_marks lays them out)
 n2m_status lab_apply(float *vol, int nx, int ny, int nz, const unsigned *need, const LabelPost &P, cudaStream_t s);
@@ -250,7 +253,7 @@ struct ThresholdWork {
     std::vector<double> P;
 };
 n2m_status isolevel_otsu(const float *d_img, long long nvox, int mode123, ThresholdWork &w, cudaStream_t s,
-                         float *result);
+                         float *result, void *pinned);
 
 // mc.cu
 struct McGrid {
@@ -269,14 +272,33 @@ struct McWork {
 struct McCounts {
     unsigned nv_edge, nt, nc, nactive;
 };
+// What marching cubes and the stages after it leave for the host, read back at once.
+// The kernels from the emit on take the counts from here, so that they can be queued
+// before the host knows them; each does nothing if the mesh does not fit its buffers.
+constexpr int MARCH_CAND = 256;
+struct MarchOut {
+    uint4 tot;                  // edge vertices, triangles, c-vertices, active words
+    unsigned ncand, nccand;     // weld candidates: edge vertices, c-vertices
+    unsigned kept;              // triangles left by the degenerate filter, if it ran
+    unsigned pad;
+    vec3d first;                // with candidates: the first vertex, and the first MARCH_CAND
+    vec3d cand_pos[MARCH_CAND]; // candidates
+    int cand_id[MARCH_CAND];
+};
+struct MeshRoom {
+    unsigned nv, nt;            // vertices and triangles the buffers hold
+    __host__ __device__ bool fits(uint4 t) const {
+        return (unsigned long long)t.x + t.z <= nv && t.y <= nt;
+    }
+};
 // post: what a labelling did to the volume (its signs are post->S), repair: the volume
 // was smoothed approximately (without post its signs are repair->w->vsign); with
 // either, the voxels whose values are needed are marked after the sign pass and put
 // right before any value is read.  od: the marks' and the repair's buffers.
 n2m_status mc_count(const McGrid &g, int variant, McWork &w, uint4 *d_total, cudaStream_t s, OdWork &od,
                     const OdRepair *repair = nullptr, const LabelPost *post = nullptr);
-n2m_status mc_emit(const McGrid &g, int variant, McWork &w, const McCounts &c, vec3d *d_pts, vec3i *d_tris,
-                   int *d_cand, unsigned *d_ncand, int cand_cap, unsigned *d_near, cudaStream_t s);
+n2m_status mc_emit(const McGrid &g, int variant, McWork &w, MarchOut *d_out, const MeshRoom &room, vec3d *d_pts, vec3i *d_tris,
+                   int *d_cand, int cand_cap, unsigned *d_near, cudaStream_t s);
 n2m_status mc_backward(const McGrid &g, int variant, McWork &w, const McCounts &c, const float3 *d_gv, float *d_gs,
                        cudaStream_t s);
 n2m_status mc_ccand_scan(const vec3d *d_pts, int np, const int *d_ccand, int nccand, int *d_cand,
@@ -288,7 +310,7 @@ n2m_status oc_count(const float *vol, const int dim[3], const int lo[3], const i
                     McWork &w, uint4 *d_total, cudaStream_t s, OdWork &od, const OdRepair *repair = nullptr,
                     const LabelPost *post = nullptr);
 n2m_status oc_emit(const float *vol, const int dim[3], const int lo[3], const int hi[3], float iso, float edge_max,
-                    McWork &w, const McCounts &c, vec3d *d_pts, vec3i *d_tris, int *d_cand, unsigned *d_ncand,
+                    McWork &w, MarchOut *d_out, const MeshRoom &room, vec3d *d_pts, vec3i *d_tris, int *d_cand,
                     int cand_cap, unsigned *d_near, cudaStream_t s);
 // the copies of the ncand weld candidates in the reference's triangle soup: every
 // corner 3*t + c naming one, into d_out (at most cap; *d_count = how many there
@@ -328,6 +350,13 @@ __device__ __forceinline__ void mark_near(unsigned *near, int id) {
 // d_tris_in is renumbered in place if the weld removed vertices; d_near: the marks by raw id, or null
 n2m_status mesh_remove_degenerate(const vec3d *d_pts, vec3i *d_tris_in, int nt, const WeldMap &weld, const unsigned *d_near,
                                   vec3i *d_tris_out, unsigned *d_nt_out, DegWork &w, cudaStream_t s);
+// the same, queued before the host knows the counts: if the mesh fits `room` and nothing can be welded, the filter runs
+// (out->kept), else the weld candidates are left in *out
+n2m_status mesh_after_emit(const vec3d *d_pts, vec3i *d_tris_in, const MeshRoom &room, const int *d_cand, int cand_cap,
+                           const unsigned *d_near, vec3i *d_tris_out, MarchOut *d_out, DegWork &w, cudaStream_t s);
+// only the candidates
+n2m_status mesh_weld_candidates(const vec3d *d_pts, const MeshRoom &room, const int *d_cand, int cand_cap, MarchOut *d_out,
+                                cudaStream_t s);
 struct HcWork {
     DevBuf zero;              // degrees / offsets, cursors, the bad-index flag, border flags
     DevBuf adj, meta;         // neighbour lists and their per-vertex heads

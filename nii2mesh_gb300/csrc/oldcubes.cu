@@ -338,13 +338,12 @@ n2m_status oc_count(const float *vol, const int dim[3], const int lo[3], const i
 }
 
 n2m_status oc_emit(const float *vol, const int dim[3], const int lo[3], const int hi[3], float iso, float edge_max,
-                    McWork &w, const McCounts &c, vec3d *d_pts, vec3i *d_tris, int *d_cand, unsigned *d_ncand,
-                    int cand_cap, unsigned *d_near, cudaStream_t s) {
+                   McWork &w, MarchOut *d_out, const MeshRoom &room, vec3d *d_pts, vec3i *d_tris, int *d_cand,
+                   int cand_cap, unsigned *d_near, cudaStream_t s) {
     const OV g = make_ov(vol, dim, lo, hi, iso, edge_max);
-    if (c.nactive == 0) return N2M_OK;
     mcw::Out o;
-    CKS(mcw::prepare(w, (size_t)g.WX * g.NY * g.NZ, nullptr, o));
-    return mcw::emit(Policy{g, d_pts, d_cand, d_ncand, cand_cap, d_near}, w.signs.as<unsigned>(), w, o, c.nactive, d_tris, s);
+    CKS(mcw::prepare(w, (size_t)g.WX * g.NY * g.NZ, &d_out->tot, o));
+    return mcw::emit(Policy{g, d_pts, d_cand, &d_out->ncand, cand_cap, d_near}, w.signs.as<unsigned>(), w, o, room, d_tris, s);
 }
 
 n2m_status oc_copies(const vec3i *d_tris, int nt, int nv, const int *d_cand, int ncand, unsigned *d_bits,
