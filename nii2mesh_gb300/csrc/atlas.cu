@@ -9,13 +9,16 @@
 // bubble detection and the largest-cluster tie-break are unchanged), and the
 // marching-cubes fetch returns 0 for voxels outside the sub-box.
 //
-// All labels' sub-boxes live in one float arena.  Each stage is ONE launch
-// of persistent CTAs that pull work items (a smoothing column, a chunk of
-// voxels, a marching-cubes tile, an active word) of any label from a global
-// atomic queue, so hundreds of labels of very different sizes share the GPU
-// in each launch.  Vertex/triangle numbering comes from one scan over the
-// words of every label's grid: each label's mesh is a contiguous range in
-// the concatenated output, numbered exactly as the single-volume path.
+// All labels' sub-boxes live in one float arena, and their rows in one array of bit words
+// (a box begins at a multiple of 32 words).  Each stage is one launch over the words,
+// runs or points of every box, so hundreds of labels of very different sizes share the GPU
+// in each launch.  The masks are smoothed from their bits, the components are found on
+// runs listed across the boxes, the clustered values are never written (their signs follow
+// from the kept set, agval applies the rest where marching cubes reads), and the
+// boxes' grids are words of one numbering for the kernels of mcwords.cuh: each label's
+// mesh is a contiguous range in the concatenated output, numbered exactly as the
+// single-volume path.  256^3 atlas of 250 labels: 3834 us when every stage went over the
+// voxels or rows of the arena, 1896 us now.
 #include <string.h>
 
 #include <algorithm>
@@ -23,6 +26,7 @@
 #include <vector>
 
 #include "mc33.cuh"
+#include "mcwords.cuh"
 #include "runs.cuh"
 #include "smooth_core.cuh"
 #include "uf.cuh"
@@ -35,8 +39,7 @@ struct ABox {
     int label;
     int o[3], n[3];            // sub-box origin and size (global voxel coordinates)
     long long arena;           // arena offset of the sub-box
-    unsigned tile0;            // first smoothing column / voxel chunk item of this box
-    unsigned chunk0;
+    unsigned tile0;            // first smoothing unit of this box
     int full;                  // sub-box covers the whole volume
     int fail;                  // N2M status of this label (0 = ok)
     int vmin, vmax;            // ordered-int range of the smoothed sub-box
@@ -47,9 +50,9 @@ struct ABox {
     unsigned long long best;   // largest component (size << 32 | ~root)
     // marching-cubes grid (global origin lo, size gn), filled by the host
     int glo[3], gn[3];
-    unsigned WX, word0, ctile0;
-    // clustering on x-runs: bit words per row, first row and first bit word across the boxes
-    unsigned W, row0, bw0;
+    unsigned WX, word0;
+    // bit words per row, first bit word across the boxes
+    unsigned W, bw0;
 };
 
 struct AtlasVol {
@@ -68,114 +71,316 @@ __device__ __forceinline__ int find_item(const ABox *b, int nb, unsigned item, u
     return lo;
 }
 
-// ---- S0: per-label voxel count, bounding box and the largest label ---------------
-// A thread scans 32 consecutive voxels of a row and issues its atomics once per
-// run of equal labels (labels are spatially coherent, so runs are long).
-__device__ __forceinline__ void hist_flush(int l, int maxlab, unsigned c, int x0, int x1, int y, int z, unsigned *cnt,
-                                           int *bb) {
-    if (l < 1 || l > maxlab || !c) return;
-    atomicAdd(&cnt[l], c);
-    int *b = bb + 6 * l;
-    atomicMin(b + 0, x0); atomicMin(b + 1, y); atomicMin(b + 2, z);
-    atomicMax(b + 3, x1); atomicMax(b + 4, y); atomicMax(b + 5, z);
+// ---- S0: every label's bounding box and the largest label -------------------------
+// A thread takes HV consecutive voxels of a row, loaded at once.  Atomics on a label's box
+// are the bound (a label's rows come in order, so nearly every run moves its box on, and a
+// few hundred boxes are a few dozen cache lines): the lanes of a warp whose runs have the
+// same label agree on one extent, a block keeps the boxes of its consecutive rows in shared
+// memory, and sends them on where they exceed the box as last seen (boxes only grow: an old
+// view is safe).  256^3: 259 us with a thread per 32 voxels and seven global atomics for every
+// run, 234 us without the blocks' tables, 79 us now.
+constexpr int HV = 8, HT = 256;   // voxels of a thread, entries of a block's table
+__device__ __forceinline__ void grow_box(int *b, int x0, int x1, int y0, int y1, int z0, int z1) {
+    volatile int *seen = b;
+    const int b0 = seen[0], b1 = seen[1], b2 = seen[2], b3 = seen[3], b4 = seen[4], b5 = seen[5];
+    if (x0 < b0) atomicMin(b, x0);
+    if (y0 < b1) atomicMin(b + 1, y0);
+    if (z0 < b2) atomicMin(b + 2, z0);
+    if (x1 > b3) atomicMax(b + 3, x1);
+    if (y1 > b4) atomicMax(b + 4, y1);
+    if (z1 > b5) atomicMax(b + 5, z1);
 }
-
-__global__ void k_a_hist(AtlasVol v, int maxlab, unsigned *cnt, int *bb, int *vmax) {
+__global__ void __launch_bounds__(HT) k_a_hist(AtlasVol v, int maxlab, unsigned *present, int *bb, int *vmax) {
     grid_wait();
     int mx = 0;
-    const unsigned spr = (unsigned)(v.nx + 31) / 32;
-    const long long nseg = (long long)spr * v.ny * v.nz;
-    for (long long sg = blockIdx.x * (long long)blockDim.x + threadIdx.x; sg < nseg; sg += (long long)gridDim.x * blockDim.x) {
-        const long long row = sg / spr;
-        const int xs = (int)(sg - row * spr) * 32;
-        const int z = (int)(row / v.ny), y = (int)(row - (long long)z * v.ny);
-        const short *p = v.lab + row * v.nx;
-        int cur = -1, x0 = 0, x1 = 0;
-        unsigned c = 0;
-        const int xe = min(xs + 32, v.nx);
-        for (int x = xs; x < xe; x++) {
-            const int l = p[x];
-            mx = max(mx, l);
-            if (l != cur) {
-                hist_flush(cur, maxlab, c, x0, x1, y, z, cnt, bb);
-                cur = l;
-                c = 0;
-                x0 = x;
-            }
-            c++;
-            x1 = x;
+    const unsigned spr = (unsigned)(v.nx + HV - 1) / HV, lane = threadIdx.x & 31u;
+    const unsigned long long nseg = (unsigned long long)spr * v.ny * v.nz, nseg32 = (nseg + 31) & ~31ull;
+    const bool vec = v.nx % HV == 0 && ((size_t)v.lab & 15) == 0, small = nseg32 < 0x80000000ull;   // cheap divisions
+    __shared__ int key[HT], box[HT][6];
+    key[threadIdx.x] = 0;
+#pragma unroll
+    for (int k = 0; k < 6; k++) box[threadIdx.x][k] = k < 3 ? INT_MAX : INT_MIN;
+    __syncthreads();
+    const unsigned long long per = ((nseg32 + gridDim.x - 1) / gridDim.x + 31) & ~31ull, s0 = per * blockIdx.x;
+    const unsigned long long s1 = min(nseg32, s0 + per);
+    for (unsigned long long sg = s0 + threadIdx.x; sg < s1; sg += HT) {   // whole warps
+        const unsigned row = small ? (unsigned)sg / spr : (unsigned)(sg / spr);
+        const int xs = (int)(sg - (unsigned long long)row * spr) * HV, n = sg < nseg ? min(HV, v.nx - xs) : 0;
+        const int z = (int)(row / (unsigned)v.ny), y = (int)(row - (unsigned)z * (unsigned)v.ny);
+        const short *p = v.lab + (long long)row * v.nx + xs;
+        short l[HV];
+        if (vec && n) {
+            *(int4 *)l = __ldg((const int4 *)p);
+        } else {
+#pragma unroll
+            for (int k = 0; k < HV; k++) l[k] = k < n ? p[k] : (short)0;
         }
-        hist_flush(cur, maxlab, c, x0, x1, y, z, cnt, bb);
+        unsigned ends = 0;   // last voxels of runs of labels
+#pragma unroll
+        for (int k = 0; k < HV; k++) {
+            mx = max(mx, (int)l[k]);
+            if (l[k] > 0 && (int)l[k] <= maxlab && (k == HV - 1 || l[k + (k < HV - 1)] != l[k])) ends |= 1u << k;
+        }
+        unsigned done = 0;   // voxels of runs already sent
+        while (__any_sync(FULL, ends != 0u)) {
+            int lab = 0, first = 0, last = 0;
+            if (ends) {
+                const int e = __ffs(ends) - 1;
+#pragma unroll
+                for (int k = 0; k < HV; k++)
+                    if (k == e) lab = l[k];
+                first = e;
+#pragma unroll
+                for (int k = HV - 2; k >= 0; k--)
+                    if (k < first && k == first - 1 && !(done >> k & 1u) && l[k] == lab) first = k;
+                last = xs + e;
+                done |= (2u << e) - 1u;
+                first += xs;
+                ends &= ends - 1u;
+            }
+            const unsigned peers = __match_any_sync(FULL, lab);
+            const int x0 = __reduce_min_sync(peers, first), x1 = __reduce_max_sync(peers, last);
+            const int y0 = __reduce_min_sync(peers, y), y1 = __reduce_max_sync(peers, y);
+            const int z0 = __reduce_min_sync(peers, z), z1 = __reduce_max_sync(peers, z);
+            if (lab && lane == (unsigned)__ffs(peers) - 1u) {
+                int at = -1;
+                for (int t = 0; t < 4 && at < 0; t++) {
+                    const int i = (lab + 61 * t) & (HT - 1), had = atomicCAS(&key[i], 0, lab);
+                    if (had == 0 || had == lab) at = i;
+                }
+                if (at >= 0) {
+                    grow_box(box[at], x0, x1, y0, y1, z0, z1);
+                } else {
+                    grow_box(bb + 6 * lab, x0, x1, y0, y1, z0, z1);
+                    present[lab] = 1u;
+                }
+            }
+        }
     }
-    for (int o = 16; o; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if ((threadIdx.x & 31) == 0) atomicMax(vmax, mx);
+    __shared__ int bmx;
+    if (threadIdx.x == 0) bmx = 0;
+    __syncthreads();
+    mx = __reduce_max_sync(FULL, mx);
+    if ((threadIdx.x & 31) == 0) atomicMax(&bmx, mx);
+    __syncthreads();
+    if (threadIdx.x == 0) atomicMax(vmax, bmx);
+    if (const int lab = key[threadIdx.x]) {
+        const int *b = box[threadIdx.x];
+        grow_box(bb + 6 * lab, b[0], b[3], b[1], b[4], b[2], b[5]);
+        present[lab] = 1u;
+    }
 }
 
-// ---- S1: binarise + pre-smooth every sub-box (one persistent launch) -------------
-struct MaskSrc {
-    const short *lab;
-    int nx;
-    long long nxy;
-    int label;
-    __device__ __forceinline__ float load(int x, int y, int z) const {
-        return lab[(long long)z * nxy + (long long)y * nx + x] == label ? 1.f : 0.f;
-    }
+// ---- S1: binarise + pre-smooth every sub-box -----------------------------------------
+// The boxes' rows are bit words (bit x & 31 of word B.bw0 + (z*n1 + y)*B.W + x/32, local
+// coordinates; a box begins at a multiple of 32 words, the filling is zero), and a warp
+// takes 32 words of one box at a time.
+struct WordAt {
+    unsigned lr;   // local row
+    int w;         // word of the row
+    bool live;
 };
-struct ArenaSink {
-    float *a;
-    int o0, o1, o2, n0, n1;
-    __device__ __forceinline__ void put(int x, int y, int z, float v) {
-        a[((long long)(z - o2) * n1 + (y - o1)) * n0 + (x - o0)] = v;
+__device__ __forceinline__ WordAt word_at(const ABox &B, unsigned lw) {
+    WordAt a;
+    a.lr = lw / B.W;
+    a.w = (int)(lw - a.lr * B.W);
+    a.live = a.lr < (unsigned)B.n[1] * (unsigned)B.n[2];
+    return a;
+}
+// bits of f(row, x) for the 32 words of a warp, 8 words in flight; load(lr, x) fetches, bit(value) decides
+template <class V, class L, class P> __device__ __forceinline__ unsigned warp_words(const ABox &B, unsigned lw0, int lane, L load, P bit) {
+    const WordAt a = word_at(B, lw0 + (unsigned)lane);
+    const int n = __popc(__ballot_sync(FULL, a.live));
+    unsigned mine = 0;
+    for (int k0 = 0; k0 < n; k0 += 8) {
+        V val[8];
+        bool in[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+            const unsigned lr = __shfl_sync(FULL, a.lr, (k0 + u) & 31);
+            const int x = 32 * __shfl_sync(FULL, a.w, (k0 + u) & 31) + lane;
+            in[u] = k0 + u < n && x < B.n[0];
+            val[u] = in[u] ? load(lr, x) : V(0);
+        }
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+            const unsigned m = __ballot_sync(FULL, in[u] && bit(val[u]));
+            if (lane == k0 + u) mine = m;
+        }
     }
-};
+    return mine;
+}
 
-__global__ void __launch_bounds__(smooth::NT, 2) k_a_smooth(AtlasVol v, ABox *boxes, int nb, unsigned nitems,
-                                                          unsigned *queue, float *arena, bool smooth_on) {
+__global__ void __launch_bounds__(256) k_a_mask(AtlasVol v, const ABox *boxes, int nb, unsigned nbw, unsigned *M,
+                                                unsigned *wbox) {
     grid_wait();
-    __shared__ unsigned item;
-    __shared__ int bi;
-    for (;;) {
-        if (threadIdx.x == 0 && threadIdx.y == 0) {
-            item = atomicAdd(queue, 1u);
-            bi = item < nitems ? find_item(boxes, nb, item, &ABox::tile0) : 0;
-        }
-        __syncthreads();
-        const unsigned it = item;
-        const int b = bi;
-        __syncthreads();
-        if (it >= nitems) return;
-        ABox &B = boxes[b];
-        const unsigned local = it - B.tile0;
-        const int tx = (B.n[0] + smooth::STX - 1) / smooth::STX, ty = (B.n[1] + smooth::STY - 1) / smooth::STY;
-        const int cx = local % tx, cy = (local / tx) % ty, cz = local / (tx * ty);
-        const int x0 = B.o[0] + cx * smooth::STX, y0 = B.o[1] + cy * smooth::STY, z0 = B.o[2] + cz * smooth::SZC;
-        const int zend = min(z0 + smooth::SZC, B.o[2] + B.n[2]);
-        MaskSrc src{v.lab, v.nx, v.nxy, B.label};
-        ArenaSink sink{arena + B.arena, B.o[0], B.o[1], B.o[2], B.n[0], B.n[1]};
-        smooth::Acc acc;
-        acc.init();
-        if (smooth_on) {
-            smooth::column(src, sink, acc, 0.5f, x0, y0, z0, zend, B.o[0] + B.n[0], B.o[1] + B.n[1], v.nx, v.ny, v.nz);
-        } else {
-            const int gx = x0 + threadIdx.x, gy = y0 + threadIdx.y;
-            if (gx < B.o[0] + B.n[0] && gy < B.o[1] + B.n[1])
-                for (int z = z0; z < zend; z++) {
-                    const float o = src.load(gx, gy, z);
-                    sink.put(gx, gy, z, o);
-                    acc.add(o, gx, gy, z, 0.5f);
+    const int lane = threadIdx.x & 31;
+    for (unsigned w0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u; w0 < nbw; w0 += gridDim.x * blockDim.x) {
+        const int b = find_item(boxes, nb, w0, &ABox::bw0);
+        const ABox &B = boxes[b];
+        if (lane == 0) wbox[w0 / 32] = (unsigned)b;   // the box of every 32 words
+        const int n1 = B.n[1], label = B.label;
+        const short *base = v.lab + (long long)B.o[2] * v.nxy + (long long)B.o[1] * v.nx + B.o[0];
+        M[w0 + (unsigned)lane] = warp_words<short>(B, w0 - B.bw0, lane, [&](unsigned lr, int x) {
+            const int z = (int)(lr / (unsigned)n1), y = (int)(lr - (unsigned)z * (unsigned)n1);
+            return __ldg(base + (long long)z * v.nxy + (long long)y * v.nx + x);
+        }, [&](short l) { return l == label; });
+    }
+}
+
+// The three passes on the masks' bits.  A warp takes 32 columns x ARY rows and marches along
+// z.  The x pass of a binary row has 32 possible results (a table); the y and z passes prove
+// the reference's rounding in FP32 (tap5_fast).  What they cannot prove takes the FP64
+// sequence: 0.1 % of the y results at once, 1 % of the z results through a queue that
+// fills warps (FP64 issues at a 32nd of the FP32 rate).  Slices whose rows are empty, or
+// full away from the volume's faces, skip the passes.  Bound by FP32 issue.  23 M arena
+// voxels (250 labels of a 256^3 atlas): 604 us with one CTA per column tile, staging and
+// queueing every pass between barriers; 200 us.
+constexpr int ARY = 4, AZC = 16, AWARPS = 8;
+struct SmoothQueue {
+    float v[5][64];
+    unsigned at[64];
+};
+__global__ void __launch_bounds__(32 * AWARPS) k_a_smooth(ABox *boxes, int nb, unsigned nunits, const unsigned *__restrict__ M,
+                                                          float *arena, int nx, int ny, int nz, bool smooth_on) {
+    grid_wait();
+    __shared__ float lut[32];
+    __shared__ SmoothQueue queues[AWARPS];
+    const int lane = threadIdx.x & 31;
+    auto tap = [](float a, float b, float c, float d, float e) {
+        float r;
+        if (!tap5_fast(a, b, c, d, e, &r)) r = tap5_double(a, b, c, d, e);
+        return r;
+    };
+    if (threadIdx.x < 32)
+        lut[lane] = tap((float)(lane & 1), (float)(lane >> 1 & 1), (float)(lane >> 2 & 1), (float)(lane >> 3 & 1), (float)(lane >> 4 & 1));
+    __syncthreads();
+    const float x1 = lut[31], y1 = tap(x1, x1, x1, x1, x1), z1 = tap(y1, y1, y1, y1, y1);   // of a region all ones
+    SmoothQueue &q = queues[threadIdx.x >> 5];
+    for (unsigned unit = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; unit < nunits; unit += (gridDim.x * blockDim.x) >> 5) {
+        ABox &B = boxes[find_item(boxes, nb, unit, &ABox::tile0)];
+        const int n0 = B.n[0], n1 = B.n[1], n2 = B.n[2], W = (int)B.W;
+        const unsigned local = unit - B.tile0, ny4 = (unsigned)(n1 + ARY - 1) / ARY;
+        const int w = (int)(local % (unsigned)W), y0 = (int)(local / (unsigned)W % ny4) * ARY, z0 = (int)(local / ((unsigned)W * ny4)) * AZC;
+        const int zend = min(z0 + AZC, n2), x = 32 * w + lane, gx = B.o[0] + x;
+        const bool own = x < n0, xin = gx >= 2 && gx <= nx - 3;
+        // no face of the volume within the filter's reach of this unit
+        const bool inner = B.o[0] + 32 * w >= 2 && B.o[0] + 32 * w + 31 <= nx - 3 && B.o[1] + y0 >= 2 && B.o[1] + y0 + ARY - 1 <= ny - 3;
+        const unsigned *Mb = M + B.bw0;
+        float *out = arena + B.arena + x;
+        float mn = INFINITY, mx = -INFINITY;
+        float r[ARY][5];
+#pragma unroll
+        for (int k = 0; k < ARY; k++)
+#pragma unroll
+            for (int t = 0; t < 5; t++) r[k][t] = 0.f;
+        unsigned kinds = 0x3ffu, nq = 0;   // the last five slices: 0 empty, 1 full, 2 neither
+        auto drain = [&](unsigned n) {     // the queue's first n <= 32
+            if ((unsigned)lane < n) {
+                const float v = tap5_double(q.v[0][lane], q.v[1][lane], q.v[2][lane], q.v[3][lane], q.v[4][lane]);
+                arena[B.arena + q.at[lane]] = v;
+                mn = fminf(mn, v);
+                mx = fmaxf(mx, v);
+            }
+            __syncwarp();
+        };
+        const int zlo = smooth_on ? max(z0 - 2, -B.o[2]) : z0, zhi = smooth_on ? min(zend + 2, nz - B.o[2]) : zend;
+        for (int zi = zlo; zi < zhi; zi++) {
+            // rows y0-2 .. y0+ARY+1, three words each: lane 3*row + {0, 1, 2}
+            unsigned word = 0;
+            const int rr = lane / 3, yy = y0 - 2 + rr, ww = w - 1 + lane - 3 * rr;
+            if (rr < ARY + 4 && yy >= 0 && yy < n1 && zi >= 0 && zi < n2 && ww >= 0 && ww < W)
+                word = __ldg(Mb + ((unsigned)zi * (unsigned)n1 + (unsigned)yy) * (unsigned)W + (unsigned)ww);
+            const unsigned prv = __shfl_up_sync(FULL, word, 1), nxt = __shfl_down_sync(FULL, word, 1);
+            // at lane 3*row + 1: bits x-2 .. x+33 of the row
+            const unsigned lo = word << 2 | prv >> 30, hi = nxt << 2 | word >> 30;
+            const bool mid = rr < ARY + 4 && lane - 3 * rr == 1;
+            const bool some = __any_sync(FULL, mid && (lo | (hi & 15u)) != 0u);
+            const bool all = __all_sync(FULL, !mid || (lo == FULL && (hi & 15u) == 15u));
+            const unsigned kind = !smooth_on ? 2u : (!some ? 0u : (all && inner ? 1u : 2u));
+            kinds = (kinds << 2 | kind) & 0x3ffu;
+            const int gz = B.o[2] + zi, zo = zi - 2, gzo = gz - 2;
+            float Y[ARY];
+            if (kind == 2u) {
+                float xs[ARY + 4];
+#pragma unroll
+                for (int k = 0; k < ARY + 4; k++) {
+                    const unsigned a = __shfl_sync(FULL, lo, 3 * k + 1), b = __shfl_sync(FULL, hi, 3 * k + 1);
+                    const unsigned win = __funnelshift_r(a, b, lane) & 31u;
+                    xs[k] = smooth_on && xin ? lut[win] : (float)(win >> 2 & 1u);
                 }
+#pragma unroll
+                for (int k = 0; k < ARY; k++) {
+                    const int gy = B.o[1] + y0 + k;
+                    Y[k] = smooth_on && gy >= 2 && gy <= ny - 3 ? tap(xs[k], xs[k + 1], xs[k + 2], xs[k + 3], xs[k + 4]) : xs[k + 2];
+                }
+            } else {
+#pragma unroll
+                for (int k = 0; k < ARY; k++) Y[k] = kind == 0u ? 0.f : y1;
+            }
+#pragma unroll
+            for (int k = 0; k < ARY; k++) {
+                r[k][0] = r[k][1]; r[k][1] = r[k][2]; r[k][2] = r[k][3]; r[k][3] = r[k][4]; r[k][4] = Y[k];
+            }
+            const bool edge = zi >= z0 && zi < zend && (!smooth_on || gz < 2 || gz > nz - 3);   // rows left unfiltered along z
+            const bool zint = smooth_on && zo >= z0 && zo < zend && gzo >= 2 && gzo <= nz - 3;
+#pragma unroll
+            for (int k = 0; k < ARY; k++) {
+                if (y0 + k >= n1) break;
+                if (edge && own) {
+                    out[((long long)zi * n1 + y0 + k) * n0] = Y[k];
+                    mn = fminf(mn, Y[k]);
+                    mx = fmaxf(mx, Y[k]);
+                }
+                if (!zint) continue;
+                const unsigned at = ((unsigned)zo * (unsigned)n1 + (unsigned)(y0 + k)) * (unsigned)n0;
+                float o = 0.f;
+                bool ok = true;
+                if (kinds == 0x155u) o = z1;
+                else if (kinds) ok = tap5_fast(r[k][0], r[k][1], r[k][2], r[k][3], r[k][4], &o);
+                if (own && ok) {
+                    out[at] = o;
+                    mn = fminf(mn, o);
+                    mx = fmaxf(mx, o);
+                }
+                const unsigned fail = __ballot_sync(FULL, own && !ok);
+                if (fail) {
+                    if (own && !ok) {
+                        const unsigned j = nq + __popc(fail & ((1u << lane) - 1u));
+#pragma unroll
+                        for (int t = 0; t < 5; t++) q.v[t][j] = r[k][t];
+                        q.at[j] = at + (unsigned)x;
+                    }
+                    __syncwarp();
+                    nq += __popc(fail);
+                    if (nq >= 32) {
+                        drain(32);
+                        nq -= 32;
+                        float mv[5];
+                        const unsigned ma = q.at[32 + lane];
+#pragma unroll
+                        for (int t = 0; t < 5; t++) mv[t] = q.v[t][32 + lane];
+                        __syncwarp();
+                        if ((unsigned)lane < nq) {
+#pragma unroll
+                            for (int t = 0; t < 5; t++) q.v[t][lane] = mv[t];
+                            q.at[lane] = ma;
+                        }
+                        __syncwarp();
+                    }
+                }
+            }
         }
-        // range of this column into the box
-        float mn = acc.mn, mx = acc.mx;
+        drain(nq);
         for (int o = 16; o; o >>= 1) {
-            mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
-            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+            mn = fminf(mn, __shfl_xor_sync(FULL, mn, o));
+            mx = fmaxf(mx, __shfl_xor_sync(FULL, mx, o));
         }
-        if (((threadIdx.y * blockDim.x + threadIdx.x) & 31) == 0 && mn <= mx) {
-            atomicMin(&B.vmin, f2ord(mn));
-            atomicMax(&B.vmax, f2ord(mx));
+        if (lane == 0 && mn <= mx) {
+            const int a = f2ord(mn), b = f2ord(mx);
+            if (a < *(volatile int *)&B.vmin) atomicMin(&B.vmin, a);
+            if (b > *(volatile int *)&B.vmax) atomicMax(&B.vmax, b);
         }
-        __syncthreads();
     }
 }
 
@@ -197,51 +402,12 @@ __global__ void k_a_iso(ABox *boxes, int nb) {
 }
 
 // ---- S3: clustering on the arena ----------------------------------------------------
-// voxels are processed in chunks of 1024 of one box
-constexpr int CH = 1024;
-
-struct VoxCtx {
-    int b;
-    long long i;         // arena index
-    int x, y, z;         // local coordinates
-};
-
-template <class F>
-__device__ __forceinline__ void for_chunks(const ABox *boxes, int nb, unsigned nchunks, unsigned *queue, unsigned ch, F f) {
-    __shared__ unsigned item;
-    __shared__ int bi;
-    for (;;) {
-        if (threadIdx.x == 0) {
-            item = atomicAdd(queue, 1u);
-            bi = item < nchunks ? find_item(boxes, nb, item, &ABox::chunk0) : 0;
-        }
-        __syncthreads();
-        const unsigned it = item;
-        const int b = bi;
-        __syncthreads();
-        if (it >= nchunks) return;
-        const ABox &B = boxes[b];
-        const unsigned n0 = (unsigned)B.n[0], n01 = (unsigned)B.n[0] * (unsigned)B.n[1];
-        const unsigned nvb = n01 * (unsigned)B.n[2];
-        for (unsigned k = threadIdx.x; k < ch; k += blockDim.x) {
-            const unsigned loc = (it - B.chunk0) * ch + k;
-            if (loc >= nvb) break;
-            const unsigned z = loc / n01, r = loc - z * n01;
-            const unsigned y = r / n0, x = r - y * n0;
-            f(VoxCtx{b, B.arena + loc, (int)x, (int)y, (int)z}, B);
-        }
-    }
-}
-
-// The clustering of label.cu on every sub-box: class masks as bit words per
-// box (bit x & 31 of word B.bw0 + (z*n1 + y)*B.W + x/32, local coordinates),
-// union-find parents in L (arena-indexed) at the first voxel of each x-run
-// only, boxes independent of one another.  A row kernel takes one row of one
-// box per warp (lanes over its words, 32 at a time); rows and words are
-// numbered across the boxes (B.row0, B.bw0).  The background's face contacts
-// are the box's faces (src/meshify.c:332-336 on the binarised sub-box).
-__device__ __forceinline__ bool skip_box(const ABox &B) { return B.fail != 0; }
-
+// The clustering of label.cu on every sub-box: class masks as bit words, union-find
+// links in L (arena-indexed) at the first voxel of each x-run only, boxes independent of
+// one another.  The background's face contacts are the box's faces (src/meshify.c:332-336
+// on the binarised sub-box).  A warp or a lane per row spent its time on short rows and
+// in chains of links (two merges 410 us of the 256^3 atlas, everything else 160); by lists of
+// runs and words, links at roots before the merge, all of it takes 330.
 __device__ __forceinline__ unsigned ab_valid(const ABox &B, unsigned w) {
     const int x0 = (int)w * 32;
     return x0 + 32 <= B.n[0] ? FULL : (1u << (B.n[0] - x0)) - 1u;
@@ -253,414 +419,413 @@ __device__ __forceinline__ unsigned ab_class(const unsigned *Bits, const ABox &B
 }
 
 // class bits: smoothed value >= the box's isolevel
-__global__ void __launch_bounds__(256) k_ab_bits(const ABox *boxes, int nb, unsigned nrows, const float *arena,
+__global__ void __launch_bounds__(256) k_ab_bits(const ABox *boxes, const unsigned *__restrict__ wbox, unsigned nbw, const float *__restrict__ arena,
                                                  unsigned *Bits) {
     grid_wait();
     const int lane = threadIdx.x & 31;
-    for (unsigned gr = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; gr < nrows; gr += (gridDim.x * blockDim.x) >> 5) {
-        const ABox &B = boxes[find_item(boxes, nb, gr, &ABox::row0)];
-        const unsigned lr = gr - B.row0;
-        const float *rp = arena + B.arena + (long long)lr * B.n[0];
-        for (unsigned w = 0; w < B.W; w++) {
-            const int x = (int)w * 32 + lane;
-            const unsigned m = __ballot_sync(FULL, x < B.n[0] && rp[x] >= B.iso);
-            if (lane == 0) Bits[B.bw0 + lr * B.W + w] = m;
-        }
+    for (unsigned w0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u; w0 < nbw; w0 += gridDim.x * blockDim.x) {
+        const ABox &B = boxes[wbox[w0 / 32]];
+        const float *base = arena + B.arena;
+        const int n0 = B.n[0];
+        const float iso = B.iso;
+        Bits[w0 + (unsigned)lane] = warp_words<float>(B, w0 - B.bw0, lane,
+                                                      [&](unsigned lr, int x) { return __ldg(base + (long long)lr * n0 + x); },
+                                                      [&](float f) { return f >= iso; });
     }
 }
 
-// every run start of the class links to itself; z8 / z32 (may be null) zeroed there
-__global__ void k_ab_init(const ABox *boxes, int nb, unsigned nbw, const unsigned *__restrict__ Bits, unsigned want,
-                          int *L, unsigned char *z8, unsigned *z32) {
-    grid_wait();
-    for (unsigned gw = blockIdx.x * blockDim.x + threadIdx.x; gw < nbw; gw += gridDim.x * blockDim.x) {
-        const ABox &B = boxes[find_item(boxes, nb, gw, &ABox::bw0)];
-        const unsigned lw = gw - B.bw0, lr = lw / B.W, w = lw - lr * B.W;
-        const unsigned c = ab_class(Bits, B, lr, w, want), pc = w ? ab_class(Bits, B, lr, w - 1, want) : 0u;
-        const long long base = B.arena + (long long)lr * B.n[0] + (long long)w * 32;
-        for (unsigned st = c & ~((c << 1) | (pc >> 31)); st; st &= st - 1) {
-            const int s = (int)(base + __ffs(st) - 1);
-            L[s] = s;
-            if (z8) z8[s] = 0;
-            if (z32) z32[s] = 0;
+// A word of a box's row in a class, with the words before and after it (0 outside the row)
+struct AWord {
+    unsigned c, pc, nc, lr;
+    int w;
+    // bits x whose voxel x + dx is in the class
+    __device__ __forceinline__ unsigned shifted(int dx) const {
+        return dx == 0 ? c : dx == 1 ? (c >> 1) | (nc << 31) : dx == -1 ? (c << 1) | (pc >> 31) : (c << 2) | (pc >> 30);
+    }
+};
+__device__ __forceinline__ AWord aword(const unsigned *__restrict__ Bits, const ABox &B, unsigned lr, int w, unsigned want) {
+    return AWord{ab_class(Bits, B, lr, (unsigned)w, want), w ? ab_class(Bits, B, lr, (unsigned)w - 1u, want) : 0u,
+                 w + 1 < (int)B.W ? ab_class(Bits, B, lr, (unsigned)w + 1u, want) : 0u, lr, w};
+}
+// arena index of the start of the run that voxel b (-1 .. 32 of word q) belongs to; rows
+// are a few words long, so runs from before the word are walked back
+__device__ __forceinline__ int arun(const unsigned *__restrict__ Bits, const ABox &B, unsigned want, const AWord &q, int b) {
+    int x = 32 * q.w + 32;
+    if (b <= 31 || q.c >> 31) {
+        const unsigned z = b < 0 ? 0u : ~q.c & ((1u << min(b, 31)) - 1u);
+        x = z ? 32 * q.w + 32 - __clz(z) : 32 * q.w;
+        unsigned p = z ? 0u : q.pc;
+        for (int w = q.w; p >> 31; p = --w ? ab_class(Bits, B, q.lr, (unsigned)w - 1u, want) : 0u) {
+            x = 32 * w - __clz(~p);
+            if (~p) break;
         }
     }
+    return (int)(B.arena + (long long)q.lr * B.n[0] + x);
 }
-
-// union of touching runs with the rows before them in the box (rows (y-1, z),
-// (y, z-1), and for 18-connectivity x offsets -1..1 and rows (y-1, z-1),
-// (y+1, z-1)); a contact counts where the voxels before it do not also touch
-// A row kernel's rows: AB_SEG lanes per row (one word per lane, wider rows in
-// chunks), 32 / AB_SEG rows per warp, each with its own box
-constexpr int AB_SEG = 4;
-
-template <int NNB>
-__global__ void __launch_bounds__(256) k_ab_merge(const ABox *boxes, int nb, unsigned nrows,
-                                                  const unsigned *__restrict__ Bits, unsigned want, int *L) {
-    grid_wait();
-    static_assert(NNB == 3 || NNB == 9, "6- or 18-connectivity");
-    constexpr int NR = NNB == 3 ? 3 : 5;
-    const int RY[5] = {0, -1, 0, -1, 1}, RZ[5] = {0, 0, -1, -1, -1};
-    const int lane = threadIdx.x & 31, li = lane & (AB_SEG - 1);
-    const unsigned rpw = 32u / AB_SEG, rsub = (unsigned)lane / AB_SEG, nwarps = (gridDim.x * blockDim.x) >> 5;
-    for (unsigned rb = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * rpw; rb < nrows; rb += nwarps * rpw) {
-        const unsigned gr = rb + rsub;
-        const ABox &B = boxes[gr < nrows ? find_item(boxes, nb, gr, &ABox::row0) : 0];
-        const bool rowok = gr < nrows && !skip_box(B);
-        const int n0 = B.n[0], n1 = B.n[1], n2 = B.n[2];
-        const unsigned lr = rowok ? gr - B.row0 : 0u, W = rowok ? B.W : 0u;
-        const int z = (int)(lr / (unsigned)n1), y = (int)(lr - (unsigned)z * (unsigned)n1);
-        bool kok[NR];
-        unsigned rk[NR];
+// the rows before (lr) that touch it: (y-1, z), (y, z-1) and, for 18-connectivity, (y-1, z-1), (y+1, z-1)
+template <int NNB> struct ARound {
+    static constexpr int NR = NNB == 3 ? 2 : 4, ND = NNB == 3 ? 2 : 8;
+    AWord q[NR];
+    __device__ __forceinline__ void load(const unsigned *__restrict__ Bits, const ABox &B, unsigned want, unsigned lr, int w) {
+        constexpr int RY[4] = {-1, 0, -1, 1}, RZ[4] = {0, -1, -1, -1};
+        const int n1 = B.n[1], z = (int)(lr / (unsigned)n1), y = (int)(lr - (unsigned)z * (unsigned)n1);
 #pragma unroll
         for (int k = 0; k < NR; k++) {
             const int yy = y + RY[k], zz = z + RZ[k];
-            kok[k] = rowok && yy >= 0 && zz >= 0 && yy < n1 && zz < n2;
-            rk[k] = kok[k] ? (unsigned)zz * (unsigned)n1 + (unsigned)yy : 0u;
+            q[k] = yy >= 0 && zz >= 0 && yy < n1 ? aword(Bits, B, (unsigned)(zz * n1 + yy), w, want) : AWord{0u, 0u, 0u, 0u, w};
         }
-        int cst[NR];
-        unsigned cwd[NR];
+    }
+    // contact directions: the row and the x offset
+    static __device__ __forceinline__ constexpr int row(int d) { return d < 2 ? d : d < 4 ? d - 2 + 2 : (d - 4) / 2; }
+    static __device__ __forceinline__ constexpr int dx(int d) { return d < 4 ? 0 : (d & 1 ? 1 : -1); }
+};
+
+// Run starts of the class as a list {word, arena index}, the words holding any of it as
+// another, and every start's link: to the run of its first contact with the rows before
+// (without a union), else to itself.  z8 / z32 (may be null) are zeroed there.
+constexpr int AL_K = 8;   // words per thread
+template <int NNB>
+__global__ void __launch_bounds__(256) k_al_list(const ABox *boxes, const unsigned *__restrict__ wbox, unsigned nbw,
+                                                 const unsigned *__restrict__ Bits, unsigned want, uint2 *list, unsigned *wlist,
+                                                 unsigned *n, int *L, unsigned char *z8, unsigned *z32) {
+    grid_wait();
+    __shared__ unsigned wsum[8], base, wbase;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    for (unsigned i0 = blockIdx.x * 256 * AL_K; i0 < nbw; i0 += gridDim.x * 256 * AL_K) {
+        unsigned st[AL_K], cnt = 0, any = 0;   // run starts (a block has at most 32768) | words << 16
 #pragma unroll
-        for (int k = 0; k < NR; k++) { cst[k] = -1; cwd[k] = 0u; }
-        const unsigned wmax = __reduce_max_sync(FULL, W);
-        for (unsigned c0 = 0; c0 < wmax; c0 += AB_SEG) {
-            const unsigned w = c0 + (unsigned)li;
-            const bool ok = w < W;
-            const int x0 = (int)w * 32;
-            WordRuns R[NR];
-            unsigned nk[NR];
-#pragma unroll
-            for (int k = 0; k < NR; k++) {
-                const unsigned c = ok && kok[k] ? ab_class(Bits, B, rk[k], w, want) : 0u;
-                R[k] = word_runs(c, x0, li, AB_SEG, cst[k], cwd[k]);
-                const unsigned dn = __shfl_down_sync(FULL, c, 1, AB_SEG);
-                nk[k] = li < AB_SEG - 1 ? (w + 1 < W ? dn : 0u)
-                                        : (kok[k] && w + 1 < W ? ab_class(Bits, B, rk[k], w + 1, want) : 0u);
-            }
-            const unsigned F = R[0].c;
-            if (!F) continue;
-            const unsigned left = (F << 1) | (R[0].pc >> 31);
-            auto S = [&](int k, int dx) -> unsigned {
-                const WordRuns &q = R[k];
-                return dx == 0 ? q.c : dx == 1 ? (q.c >> 1) | (nk[k] << 31)
-                                     : dx == -1 ? (q.c << 1) | (q.pc >> 31) : (q.c << 2) | (q.pc >> 30);
-            };
-            const long long base0 = B.arena + (long long)lr * n0;
-            auto link = [&](int k, int dx) {
-                unsigned m = F & S(k, dx) & ~(left & S(k, dx - 1));
-                if (!m) return;
-                const WordRuns &q = R[k];
-                const long long basek = B.arena + (long long)rk[k] * n0;
-                for (; m; m &= m - 1) {
-                    const int b = __ffs(m) - 1, xx = b + dx;
-                    const int sk = xx < 0 ? q.cs : xx > 31 ? ((q.c >> 31) & 1u ? q.start_of(31) : x0 + 32) : q.start_of(xx);
-                    const int i = (int)(base0 + R[0].start_of(b)), j = (int)(basek + sk);
-                    if (L[i] != L[j]) uf::unite(L, i, j);
+        for (int k = 0; k < AL_K; k++) {
+            const unsigned gw = i0 + (unsigned)(k * 256 + tid);
+            st[k] = 0u;
+            if (gw < nbw) {
+                const ABox &B = boxes[wbox[gw / 32]];
+                const WordAt a = word_at(B, gw - B.bw0);
+                if (a.live && !B.fail) {
+                    const unsigned c = ab_class(Bits, B, a.lr, (unsigned)a.w, want), pc = a.w ? ab_class(Bits, B, a.lr, (unsigned)a.w - 1u, want) : 0u;
+                    st[k] = c & ~((c << 1) | (pc >> 31));
+                    any |= (c ? 1u : 0u) << k;
                 }
-            };
-            link(1, 0);
-            link(2, 0);
-            if constexpr (NNB == 9) {
-                link(1, -1); link(1, 1); link(2, -1); link(2, 1); link(3, 0); link(4, 0);
+            }
+            cnt += __popc(st[k]);
+        }
+        cnt += __popc(any) << 16;
+        unsigned incl = cnt;
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned t = __shfl_up_sync(FULL, incl, o);
+            if (lane >= o) incl += t;
+        }
+        if (lane == 31) wsum[wid] = incl;
+        __syncthreads();
+        if (tid == 0) {
+            unsigned t = 0;
+            for (int k = 0; k < 8; k++) t += wsum[k];
+            if (t) {
+                base = atomicAdd(n, t & 0xffffu);
+                wbase = atomicAdd(n + 1, t >> 16);
+            }
+        }
+        __syncthreads();
+        unsigned before = incl - cnt;
+        for (int k = 0; k < wid; k++) before += wsum[k];
+        unsigned at = base + (before & 0xffffu), wat = wbase + (before >> 16);
+#pragma unroll 1
+        for (int k = 0; k < AL_K; k++) {
+            if (!(any >> k & 1u)) continue;
+            const unsigned gw = i0 + (unsigned)(k * 256 + tid);
+            wlist[wat++] = gw;
+            unsigned m = 0;   // this word's starts, kept in registers by index above
+#pragma unroll
+            for (int j = 0; j < AL_K; j++)
+                if (j == k) m = st[j];
+            if (!m) continue;
+            const ABox &B = boxes[wbox[gw / 32]];
+            const WordAt a = word_at(B, gw - B.bw0);
+            ARound<NNB> A;
+            A.load(Bits, B, want, a.lr, a.w);
+            const unsigned c = ab_class(Bits, B, a.lr, (unsigned)a.w, want);
+            const int row0 = (int)(B.arena + (long long)a.lr * B.n[0] + 32 * a.w);
+            for (; m; m &= m - 1) {
+                const int b = __ffs(m) - 1, s = row0 + b;
+                const unsigned piece = piece_at(c, b);
+                int parent = s;
+                bool found = false;
+#pragma unroll
+                for (int d = 0; d < ARound<NNB>::ND; d++) {
+                    const unsigned t = piece & A.q[A.row(d)].shifted(A.dx(d));
+                    if (!found && t) {
+                        found = true;
+                        parent = arun(Bits, B, want, A.q[A.row(d)], __ffs(t) - 1 + A.dx(d));
+                    }
+                }
+                list[at++] = make_uint2(gw, (unsigned)s);
+                L[s] = parent;
+                if (z8) z8[s] = 0;
+                if (z32) z32[s] = 0;
+            }
+        }
+        __syncthreads();   // wsum and the bases are reused
+    }
+}
+
+// Every run start points at its tree's root (links only move to ancestors, which come before
+// them, so every walk ends); the way found so far is left for the others.
+__global__ void __launch_bounds__(256) k_al_jump(const uint2 *__restrict__ list, const unsigned *__restrict__ n, int *L) {
+    grid_wait();
+    volatile int *V = L;
+    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < *n; i += gridDim.x * blockDim.x) {
+        const int s = (int)list[i].y;
+        int p = V[s], at = p, steps = 0;
+        for (int q = V[p]; q != p; q = V[p]) {
+            p = q;
+            if ((++steps & 3) == 0) V[s] = at = p;
+        }
+        if (p != at) V[s] = p;
+    }
+}
+
+// Unions, a thread per word of the class: one per overlap of two runs (a contact counts where
+// the voxels before it do not also touch), of which nearly all join equal links by now.
+template <int NNB>
+__global__ void __launch_bounds__(256) k_al_merge(const ABox *boxes, const unsigned *__restrict__ wbox,
+                                                  const unsigned *__restrict__ Bits, unsigned want,
+                                                  const unsigned *__restrict__ wlist, const unsigned *__restrict__ n, int *L) {
+    grid_wait();
+    for (unsigned j = blockIdx.x * blockDim.x + threadIdx.x; j < n[1]; j += gridDim.x * blockDim.x) {
+        const unsigned gw = wlist[j];
+        const ABox &B = boxes[wbox[gw / 32]];
+        const WordAt at = word_at(B, gw - B.bw0);
+        const AWord own = aword(Bits, B, at.lr, at.w, want);
+        ARound<NNB> A;
+        A.load(Bits, B, want, at.lr, at.w);
+        const unsigned left = own.shifted(-1);
+#pragma unroll
+        for (int d = 0; d < ARound<NNB>::ND; d++) {
+            const AWord &q = A.q[A.row(d)];
+            for (unsigned m = own.c & q.shifted(A.dx(d)) & ~(left & q.shifted(A.dx(d) - 1)); m; m &= m - 1) {
+                const int x = __ffs(m) - 1;
+                const int a = L[arun(Bits, B, want, own, x)], b = L[arun(Bits, B, want, q, x + A.dx(d))];
+                if (a != b) uf::unite(L, a, b);
             }
         }
     }
 }
 
-// every run start points at its root (read-only root search: the one store is
-// the final root); roots are counted per box
-__global__ void k_ab_flatten(ABox *boxes, int nb, unsigned nbw, const unsigned *__restrict__ Bits, unsigned want, int *L,
-                             bool fg) {
+// links to roots (one store, of the final root); roots are counted per box
+__global__ void __launch_bounds__(256) k_al_flatten(ABox *boxes, const unsigned *__restrict__ wbox, const uint2 *__restrict__ list,
+                                                    const unsigned *__restrict__ n, int *L, bool fg) {
     grid_wait();
-    for (unsigned gw = blockIdx.x * blockDim.x + threadIdx.x; gw < nbw; gw += gridDim.x * blockDim.x) {
-        const int b = find_item(boxes, nb, gw, &ABox::bw0);
-        const ABox &B = boxes[b];
-        const unsigned lw = gw - B.bw0, lr = lw / B.W, w = lw - lr * B.W;
-        const unsigned c = ab_class(Bits, B, lr, w, want), pc = w ? ab_class(Bits, B, lr, w - 1, want) : 0u;
-        const long long base = B.arena + (long long)lr * B.n[0] + (long long)w * 32;
-        unsigned nroots = 0;
-        for (unsigned st = c & ~((c << 1) | (pc >> 31)); st; st &= st - 1) {
-            const int s = (int)(base + __ffs(st) - 1);
-            const int root = uf::find_root(L, s);
-            if (root == s) nroots++;
-            else L[s] = root;
+    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < *n; i += gridDim.x * blockDim.x) {
+        const uint2 e = list[i];
+        const int s = (int)e.y, root = uf::find_root(L, s);
+        if (root != s) {
+            L[s] = root;
+        } else {
+            ABox &B = boxes[wbox[e.x / 32]];
+            atomicAdd(fg ? &B.nfg : &B.nbg, 1u);
         }
-        if (nroots) atomicAdd(fg ? &boxes[b].nfg : &boxes[b].nbg, nroots);
     }
 }
 
-// background components touching a face of the box flag their root: every run
-// of a row on a y or z face, the runs holding x = 0 and x = n0-1 of the others
-__global__ void k_ab_edges(const ABox *boxes, int nb, unsigned nbw, const unsigned *__restrict__ Bits, const int *L,
-                           unsigned char *edge) {
+// f(word index, bits) for the pieces of the run that starts at arena index s in word gw; returns its last local x
+template <class F>
+__device__ __forceinline__ int run_pieces(const unsigned *__restrict__ Bits, const ABox &B, unsigned want, unsigned gw, int s, F f) {
+    const WordAt a = word_at(B, gw - B.bw0);
+    int w = a.w;
+    const int b = s - (int)(B.arena + (long long)a.lr * B.n[0]) - 32 * w;
+    unsigned piece = piece_at(ab_class(Bits, B, a.lr, (unsigned)w, want), b);
+    for (;;) {
+        f(B.bw0 + a.lr * B.W + (unsigned)w, piece);
+        if (!(piece >> 31) || w + 1 >= (int)B.W) break;
+        const unsigned c = ab_class(Bits, B, a.lr, (unsigned)w + 1u, want);
+        if (!(c & 1u)) break;
+        piece = piece_at(c, 0);
+        w++;
+    }
+    return 32 * w + 31 - __clz(piece);
+}
+
+// background components touching a face of the box flag their root
+__global__ void __launch_bounds__(256) k_al_edges(const ABox *boxes, const unsigned *__restrict__ wbox,
+                                                  const unsigned *__restrict__ Bits, const uint2 *__restrict__ list,
+                                                  const unsigned *__restrict__ n, const int *L, unsigned char *edge) {
     grid_wait();
-    for (unsigned gw = blockIdx.x * blockDim.x + threadIdx.x; gw < nbw; gw += gridDim.x * blockDim.x) {
-        const ABox &B = boxes[find_item(boxes, nb, gw, &ABox::bw0)];
-        const int n0 = B.n[0], n1 = B.n[1], n2 = B.n[2];
-        const unsigned lw = gw - B.bw0, lr = lw / B.W, w = lw - lr * B.W;
-        const int z = (int)(lr / (unsigned)n1), y = (int)(lr - (unsigned)z * (unsigned)n1);
-        const unsigned c = ab_class(Bits, B, lr, w, 0u);
-        if (!c) continue;
-        const long long base = B.arena + (long long)lr * n0;
-        auto mark = [&](long long j) {
-            const int r = L[j];
-            if (!edge[r]) edge[r] = 1;
-        };
-        if (y == 0 || z == 0 || y == n1 - 1 || z == n2 - 1) {
-            const unsigned pc = w ? ab_class(Bits, B, lr, w - 1, 0u) : 0u;
-            for (unsigned st = c & ~((c << 1) | (pc >> 31)); st; st &= st - 1) mark(base + w * 32 + __ffs(st) - 1);
-            continue;
-        }
-        if (w == 0 && (c & 1u)) mark(base);
-        if (w == B.W - 1) {
-            int b = (n0 - 1) & 31;
-            if (!((c >> b) & 1u)) continue;
-            unsigned ww = w, cc = c;
-            for (;;) {   // back to the run's start (x = 0 of a background run is one)
-                const unsigned pc = ww ? ab_class(Bits, B, lr, ww - 1, 0u) : 0u;
-                const int ls = last_start(cc & ~((cc << 1) | (pc >> 31)), (int)ww * 32, b);
-                if (ls >= 0) {
-                    mark(base + ls);
-                    break;
-                }
-                ww--;
-                b = 31;
-                cc = pc;
-            }
-        }
+    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < *n; i += gridDim.x * blockDim.x) {
+        const uint2 e = list[i];
+        const ABox &B = boxes[wbox[e.x / 32]];
+        const WordAt a = word_at(B, e.x - B.bw0);
+        const int n1 = B.n[1], z = (int)(a.lr / (unsigned)n1), y = (int)(a.lr - (unsigned)z * (unsigned)n1);
+        const bool face = y == 0 || z == 0 || y == n1 - 1 || z == B.n[2] - 1 || (int)e.y == (int)(B.arena + (long long)a.lr * B.n[0]);
+        if (!face && run_pieces(Bits, B, 0u, e.x, (int)e.y, [](unsigned, unsigned) {}) < B.n[0] - 1) continue;
+        const int r = L[e.y];
+        if (!edge[r]) edge[r] = 1;
     }
 }
 
 // bubbles (background components away from the box faces) become foreground,
 // when the box's background has at least two components (src/bwlabel.c:488-491)
-__global__ void __launch_bounds__(256) k_ab_fill(const ABox *boxes, int nb, unsigned nrows, unsigned *Bits, const int *L,
-                                                 const unsigned char *__restrict__ edge) {
+__global__ void __launch_bounds__(256) k_al_fill(const ABox *boxes, const unsigned *__restrict__ wbox,
+                                                 const unsigned *__restrict__ Bits, const uint2 *__restrict__ list,
+                                                 const unsigned *__restrict__ n, const int *L, const unsigned char *__restrict__ edge,
+                                                 unsigned *out) {
     grid_wait();
-    const int lane = threadIdx.x & 31, li = lane & (AB_SEG - 1);
-    const unsigned rpw = 32u / AB_SEG, rsub = (unsigned)lane / AB_SEG, nwarps = (gridDim.x * blockDim.x) >> 5;
-    for (unsigned rb = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * rpw; rb < nrows; rb += nwarps * rpw) {
-        const unsigned gr = rb + rsub;
-        const ABox &B = boxes[gr < nrows ? find_item(boxes, nb, gr, &ABox::row0) : 0];
-        const bool rowok = gr < nrows && B.nbg > 1;
-        const unsigned lr = rowok ? gr - B.row0 : 0u, W = rowok ? B.W : 0u;
-        const long long base = B.arena + (long long)lr * B.n[0];
-        int cst = -1;
-        unsigned cwd = 0;
-        const unsigned wmax = __reduce_max_sync(FULL, W);
-        for (unsigned c0 = 0; c0 < wmax; c0 += AB_SEG) {
-            const unsigned w = c0 + (unsigned)li;
-            const unsigned c = w < W ? ab_class(Bits, B, lr, w, 0u) : 0u;
-            const WordRuns R = word_runs(c, (int)w * 32, li, AB_SEG, cst, cwd);
-            unsigned fill = 0;
-            for (unsigned rem = c; rem;) {
-                const int b = __ffs(rem) - 1;
-                const unsigned pm = piece_at(rem, b);
-                rem &= ~pm;
-                if (!edge[L[base + R.start_of(b)]]) fill |= pm;
-            }
-            // every lane has read its neighbours' words (word_runs) before any write
-            if (fill) Bits[B.bw0 + lr * B.W + w] |= fill;
-        }
+    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < *n; i += gridDim.x * blockDim.x) {
+        const uint2 e = list[i];
+        const ABox &B = boxes[wbox[e.x / 32]];
+        if (B.nbg < 2 || edge[L[e.y]]) continue;
+        run_pieces(Bits, B, 0u, e.x, (int)e.y, [&](unsigned w, unsigned piece) { atomicOr(out + w, piece); });
     }
 }
 
-// component sizes at the roots (each run adds its length at its end)
-__global__ void __launch_bounds__(256) k_ab_sizes(const ABox *boxes, int nb, unsigned nrows,
-                                                  const unsigned *__restrict__ Bits, const int *L, unsigned *cnt) {
+// component sizes at the roots; lanes whose root is the first one's add up first
+__global__ void __launch_bounds__(256) k_al_sizes(const ABox *boxes, const unsigned *__restrict__ wbox,
+                                                  const unsigned *__restrict__ Bits, const uint2 *__restrict__ list,
+                                                  const unsigned *__restrict__ n, const int *L, unsigned *cnt) {
     grid_wait();
-    const int lane = threadIdx.x & 31, li = lane & (AB_SEG - 1);
-    const unsigned rpw = 32u / AB_SEG, rsub = (unsigned)lane / AB_SEG, nwarps = (gridDim.x * blockDim.x) >> 5;
-    for (unsigned rb = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * rpw; rb < nrows; rb += nwarps * rpw) {
-        const unsigned gr = rb + rsub;
-        const ABox &B = boxes[gr < nrows ? find_item(boxes, nb, gr, &ABox::row0) : 0];
-        const bool rowok = gr < nrows;
-        const unsigned lr = rowok ? gr - B.row0 : 0u, W = rowok ? B.W : 0u;
-        const long long base = B.arena + (long long)lr * B.n[0];
-        int cst = -1;
-        unsigned cwd = 0;
-        const unsigned wmax = __reduce_max_sync(FULL, W);
-        for (unsigned c0 = 0; c0 < wmax; c0 += AB_SEG) {
-            const unsigned w = c0 + (unsigned)li;
-            const unsigned c = w < W ? ab_class(Bits, B, lr, w, 1u) : 0u;
-            const WordRuns R = word_runs(c, (int)w * 32, li, AB_SEG, cst, cwd);
-            const unsigned dn = __shfl_down_sync(FULL, c, 1, AB_SEG);
-            const unsigned nxt = li < AB_SEG - 1 ? (w + 1 < W ? dn : 0u) : (w + 1 < W ? ab_class(Bits, B, lr, w + 1, 1u) : 0u);
-            for (unsigned ends = c & ~((c >> 1) | (nxt << 31)); ends; ends &= ends - 1) {
-                const int e = __ffs(ends) - 1, st = R.start_of(e);
-                atomicAdd(&cnt[L[base + st]], (unsigned)(R.x0 + e - st + 1));
-            }
+    const unsigned n32 = (*n + 31u) & ~31u;
+    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n32; i += gridDim.x * blockDim.x) {   // whole warps
+        int root = -1;
+        unsigned len = 0;
+        if (i < *n) {
+            const uint2 e = list[i];
+            root = L[e.y];
+            run_pieces(Bits, boxes[wbox[e.x / 32]], 1u, e.x, (int)e.y, [&](unsigned, unsigned piece) { len += __popc(piece); });
         }
+        const int r0 = __shfl_sync(FULL, root, 0);   // the first lane always has a run
+        const unsigned sum = __reduce_add_sync(FULL, root == r0 ? len : 0u);
+        if ((threadIdx.x & 31) == 0) atomicAdd(&cnt[r0], sum);
+        else if (root >= 0 && root != r0) atomicAdd(&cnt[root], len);
     }
 }
 
 // largest component per box; ties go to the smallest root (first in raster order)
-__global__ void k_ab_best(ABox *boxes, int nb, unsigned nbw, const unsigned *__restrict__ Bits, const int *L,
-                          const unsigned *__restrict__ cnt) {
+__global__ void __launch_bounds__(256) k_al_best(ABox *boxes, const unsigned *__restrict__ wbox, const uint2 *__restrict__ list,
+                                                 const unsigned *__restrict__ n, const int *L, const unsigned *__restrict__ cnt) {
     grid_wait();
-    for (unsigned gw = blockIdx.x * blockDim.x + threadIdx.x; gw < nbw; gw += gridDim.x * blockDim.x) {
-        const int b = find_item(boxes, nb, gw, &ABox::bw0);
-        const ABox &B = boxes[b];
-        const unsigned lw = gw - B.bw0, lr = lw / B.W, w = lw - lr * B.W;
-        const unsigned c = ab_class(Bits, B, lr, w, 1u), pc = w ? ab_class(Bits, B, lr, w - 1, 1u) : 0u;
-        const long long base = B.arena + (long long)lr * B.n[0] + (long long)w * 32;
-        for (unsigned st = c & ~((c << 1) | (pc >> 31)); st; st &= st - 1) {
-            const int s = (int)(base + __ffs(st) - 1);
-            if (L[s] != s) continue;
-            const unsigned loc = (unsigned)(s - B.arena);
-            atomicMax(&boxes[b].best, ((unsigned long long)cnt[s] << 32) | (0xffffffffu - loc));
-        }
+    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < *n; i += gridDim.x * blockDim.x) {
+        const uint2 e = list[i];
+        const int s = (int)e.y;
+        if (L[s] != s) continue;
+        ABox &B = boxes[wbox[e.x / 32]];
+        atomicMax(&B.best, ((unsigned long long)cnt[s] << 32) | (0xffffffffu - (unsigned)(s - B.arena)));
     }
 }
 
-// bits of the voxels of each box's largest component
-__global__ void __launch_bounds__(256) k_ab_keep(const ABox *boxes, int nb, unsigned nrows, const unsigned *__restrict__ Bits,
-                                                 const int *L, unsigned *K) {
+// bits of the voxels of each box's largest component (K cleared before)
+__global__ void __launch_bounds__(256) k_al_keep(const ABox *boxes, const unsigned *__restrict__ wbox,
+                                                 const unsigned *__restrict__ Bits, const uint2 *__restrict__ list,
+                                                 const unsigned *__restrict__ n, const int *L, unsigned *K) {
     grid_wait();
-    const int lane = threadIdx.x & 31, li = lane & (AB_SEG - 1);
-    const unsigned rpw = 32u / AB_SEG, rsub = (unsigned)lane / AB_SEG, nwarps = (gridDim.x * blockDim.x) >> 5;
-    for (unsigned rb = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * rpw; rb < nrows; rb += nwarps * rpw) {
-        const unsigned gr = rb + rsub;
-        const ABox &B = boxes[gr < nrows ? find_item(boxes, nb, gr, &ABox::row0) : 0];
-        const bool rowok = gr < nrows;
-        const long long root = B.best ? B.arena + (long long)(0xffffffffu - (unsigned)(B.best & 0xffffffffu)) : -2;
-        const unsigned lr = rowok ? gr - B.row0 : 0u, W = rowok ? B.W : 0u;
-        const long long base = B.arena + (long long)lr * B.n[0];
-        int cst = -1;
-        unsigned cwd = 0;
-        const unsigned wmax = __reduce_max_sync(FULL, W);
-        for (unsigned c0 = 0; c0 < wmax; c0 += AB_SEG) {
-            const unsigned w = c0 + (unsigned)li;
-            const unsigned c = w < W ? ab_class(Bits, B, lr, w, 1u) : 0u;
-            const WordRuns R = word_runs(c, (int)w * 32, li, AB_SEG, cst, cwd);
-            unsigned keep = 0;
-            for (unsigned rem = c; rem;) {
-                const int b = __ffs(rem) - 1;
-                const unsigned pm = piece_at(rem, b);
-                rem &= ~pm;
-                if ((long long)L[base + R.start_of(b)] == root) keep |= pm;
-            }
-            if (w < W) K[B.bw0 + lr * B.W + w] = keep;
-        }
+    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < *n; i += gridDim.x * blockDim.x) {
+        const uint2 e = list[i];
+        const ABox &B = boxes[wbox[e.x / 32]];
+        if (!B.best || (long long)L[e.y] != B.arena + (long long)(0xffffffffu - (unsigned)(B.best & 0xffffffffu))) continue;
+        run_pieces(Bits, B, 1u, e.x, (int)e.y, [&](unsigned w, unsigned piece) { atomicOr(K + w, piece); });
     }
 }
 
-// The clustered sub-box (src/meshify.c:332-342): kept voxels (K) raised to the
-// box's isolevel when FILL; with LARGEST, a voxel neither kept nor, away from
-// the volume faces, next to a kept voxel (all 26 neighbours except
-// (-1,-1,-1), src/meshify.c:252) becomes the box minimum.  A warp per row; the
-// dilation bits of 32 words at a time lane-parallel (lane l: word c0 + l).
-template <bool LARGEST, bool FILL>
-__global__ void __launch_bounds__(256) k_ab_final(const ABox *boxes, int nb, unsigned nrows, const unsigned *__restrict__ K,
-                                                  float *arena, int nx, int ny, int nz) {
+// What the clustering does to the values of a sub-box, applied where they are read
+// (agval): kept voxels (K) raised to the box's isolevel when FILL; with LARGEST, a voxel
+// neither kept nor, away from the volume faces, next to a kept voxel (all 26 neighbours
+// except (-1,-1,-1), src/meshify.c:252) becomes the box minimum (src/meshify.c:332-342).
+struct APost {
+    const unsigned *K, *KD;   // kept voxels; with LARGEST, those and their neighbours
+    const unsigned *S;        // sign of value - iso
+    bool fill, largest;
+};
+
+// ---- S4: signs and bbox of the clustered sub-boxes -------------------------------------
+// A lane per word.  Only the voxels whose value the bits do not settle are read (those next to
+// kept ones): 23 M arena voxels took 249 us to write clustered and 67 us to read back,
+// 62 us this way.  A sub-box that is the whole volume has every value read for its
+// minimum; any other one reaches 0, the smallest possible.
+__global__ void __launch_bounds__(256) k_ab_shell(ABox *boxes, const unsigned *__restrict__ wbox, unsigned nbw, APost P, unsigned *S, unsigned *KD,
+                                                  const float *__restrict__ arena, int nx, int ny, int nz) {
     grid_wait();
     const int lane = threadIdx.x & 31;
-    const int DY[9] = {-1, 0, 1, -1, 0, 1, 0, 1, -1}, DZ[9] = {0, 0, 0, 1, 1, 1, -1, -1, -1};
-    for (unsigned gr = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; gr < nrows; gr += (gridDim.x * blockDim.x) >> 5) {
-        const ABox &B = boxes[find_item(boxes, nb, gr, &ABox::row0)];
-        const int n0 = B.n[0], n1 = B.n[1], n2 = B.n[2];
-        const unsigned lr = gr - B.row0, W = B.W;
-        const int z = (int)(lr / (unsigned)n1), y = (int)(lr - (unsigned)z * (unsigned)n1);
-        float *row = arena + B.arena + (long long)lr * n0;
-        const unsigned *K0 = K + B.bw0;
-        if (!LARGEST) {
-            for (unsigned w = 0; w < W; w++) {
-                const unsigned kw = K0[lr * W + w];
-                const int x = (int)w * 32 + lane;
-                if (x < n0 && ((kw >> lane) & 1u)) row[x] = fmaxf(row[x], B.iso);
-            }
-            continue;
-        }
-        const float vmin = ord2f(B.vmin);
-        const int gy = B.o[1] + y, gz = B.o[2] + z;
-        const bool ryz = gy > 0 && gz > 0 && gy < ny - 1 && gz < nz - 1;
-        unsigned carry[9];
-#pragma unroll
-        for (int k = 0; k < 9; k++) carry[k] = 0u;
-        for (unsigned c0 = 0; c0 < W; c0 += 32) {
-            unsigned on = 0u, kept = 0u;
+    // rows used: 0..2 = y-1..y+1 in slice z, 3..5 in slice z+1, 6 = (y, z-1), 7 = (y+1, z-1), 8 = (y-1, z-1)
+    constexpr int DY[9] = {-1, 0, 1, -1, 0, 1, 0, 1, -1}, DZ[9] = {0, 0, 0, 1, 1, 1, -1, -1, -1};
+    for (unsigned w0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u; w0 < nbw; w0 += gridDim.x * blockDim.x) {
+        ABox &B = boxes[wbox[w0 / 32]];
+        const WordAt a = word_at(B, w0 - B.bw0 + (unsigned)lane);
+        const int n1 = B.n[1], n2 = B.n[2], z = (int)(a.lr / (unsigned)n1), y = (int)(a.lr - (unsigned)z * (unsigned)n1);
+        const unsigned valid = a.live ? ab_valid(B, (unsigned)a.w) : 0u, W = B.W;
+        unsigned on = 0u, kept = 0u;
+        if (P.K) {
 #pragma unroll
             for (int k = 0; k < 9; k++) {
+                if (!P.largest && k != 1) continue;
                 const int yy = y + DY[k], zz = z + DZ[k];
-                const bool in = yy >= 0 && zz >= 0 && yy < n1 && zz < n2;
-                const unsigned rb = in ? ((unsigned)zz * (unsigned)n1 + (unsigned)yy) * W : 0u;
-                const unsigned cur = in && c0 + lane < W ? K0[rb + c0 + lane] : 0u;
+                const bool in = a.live && yy >= 0 && zz >= 0 && yy < n1 && zz < n2;
+                const unsigned q = in ? B.bw0 + ((unsigned)zz * (unsigned)n1 + (unsigned)yy) * W + (unsigned)a.w : 0u;
+                const unsigned cur = in ? __ldg(P.K + q) : 0u;
                 unsigned prv = __shfl_up_sync(FULL, cur, 1), nxt = __shfl_down_sync(FULL, cur, 1);
-                if (lane == 0) prv = carry[k];
-                if (lane == 31) nxt = in && c0 + 32 < W ? K0[rb + c0 + 32] : 0u;
-                carry[k] = __shfl_sync(FULL, cur, 31);
+                if (lane == 0) prv = in && a.w ? __ldg(P.K + q - 1) : 0u;
+                if (lane == 31) nxt = in && a.w + 1 < (int)W ? __ldg(P.K + q + 1) : 0u;
+                if (a.w == 0) prv = 0u;
+                if (a.w + 1 >= (int)W) nxt = 0u;
                 on |= cur | (cur >> 1) | (nxt << 31) | (k < 8 ? (cur << 1) | (prv >> 31) : 0u);   // row 8: no K(x-1)
                 if (k == 1) kept = cur;
             }
-            const unsigned wend = min(W, c0 + 32);
-            if (!__any_sync(FULL, on != 0u)) {   // nothing kept within reach
-                for (int x = (int)c0 * 32 + lane; x < min(n0, (int)wend * 32); x += 32) row[x] = vmin;
-                continue;
+        }
+        unsigned shell = valid & ~kept, masked = 0u;
+        if (P.largest) {
+            const int gy = B.o[1] + y, gz = B.o[2] + z, gx0 = B.o[0] + 32 * a.w;
+            if (gy > 0 && gz > 0 && gy < ny - 1 && gz < nz - 1) on &= mcw::bit_range(1 - gx0, nx - 1 - gx0);
+            else on = 0u;
+            shell &= on;
+            masked = valid & ~(kept | shell);
+        }
+        const float iso = B.iso, vmin = ord2f(B.vmin);
+        const unsigned vsig = __fsub_rn(vmin, iso) > -N2M_FLT_EPS ? FULL : 0u, vge = vmin >= iso ? FULL : 0u;
+        unsigned sg = kept | (masked & vsig), ge = kept | (masked & vge);
+        const unsigned read = B.full ? valid & ~masked : shell;
+        float lo = INFINITY;
+        if (B.full && masked) lo = vmin;
+        const float *base = arena + B.arena;
+        for (unsigned busy = __ballot_sync(FULL, read != 0u); busy;) {   // four words in flight
+            int j[4];
+            float val[4];
+            unsigned rj[4], kj[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                j[u] = busy ? __ffs(busy) - 1 : -1;
+                busy &= busy - 1u;
+                rj[u] = __shfl_sync(FULL, read, j[u] & 31);
+                kj[u] = __shfl_sync(FULL, kept, j[u] & 31);
+                const unsigned lr = __shfl_sync(FULL, a.lr, j[u] & 31);
+                const int w = __shfl_sync(FULL, a.w, j[u] & 31);
+                val[u] = j[u] >= 0 && (rj[u] >> lane & 1u) ? __ldg(base + (long long)lr * B.n[0] + 32 * w + lane) : 0.f;
             }
-            for (unsigned w = c0; w < wend; w++) {
-                const unsigned onw = __shfl_sync(FULL, on, (int)(w - c0)), kw = __shfl_sync(FULL, kept, (int)(w - c0));
-                const int x = (int)w * 32 + lane;
-                if (x >= n0) continue;
-                const bool kp = (kw >> lane) & 1u;
-                const int gx = B.o[0] + x;
-                const bool interior = ryz && gx > 0 && gx < nx - 1;
-                if (!(kp || (interior && ((onw >> lane) & 1u)))) row[x] = vmin;
-                else if (FILL && kp) row[x] = fmaxf(row[x], B.iso);
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const bool in = j[u] >= 0 && (rj[u] >> lane & 1u), k = kj[u] >> lane & 1u;
+                if (in) lo = fminf(lo, k && P.fill ? fmaxf(val[u], iso) : val[u]);
+                const unsigned g = __ballot_sync(FULL, in && !k && val[u] >= iso),
+                               p = __ballot_sync(FULL, in && !k && __fsub_rn(val[u], iso) > -N2M_FLT_EPS);
+                if (lane == j[u]) {
+                    ge |= g;
+                    sg |= p;
+                }
             }
         }
-    }
-}
-
-// ---- S4: bbox of voxels >= iso and the range after clustering -------------------------
-// reduced per chunk (all its voxels belong to one box): one set of atomics per chunk
-__global__ void __launch_bounds__(256) k_a_stats(ABox *boxes, int nb, unsigned nch, unsigned *queue, unsigned ch,
-                                                 const float *arena) {
-    grid_wait();
-    __shared__ unsigned item;
-    __shared__ int bi;
-    __shared__ int red[8][7];
-    for (;;) {
-        if (threadIdx.x == 0) {
-            item = atomicAdd(queue, 1u);
-            bi = item < nch ? find_item(boxes, nb, item, &ABox::chunk0) : 0;
+        S[w0 + (unsigned)lane] = sg;   // the filling too
+        if (P.largest) KD[w0 + (unsigned)lane] = kept | shell;
+        if (B.full) {
+            for (int o = 16; o; o >>= 1) lo = fminf(lo, __shfl_xor_sync(FULL, lo, o));
+            if (lane == 0 && lo < INFINITY) atomicMin(&B.amin, f2ord(lo));
         }
-        __syncthreads();
-        const unsigned it = item;
-        const int b = bi;
-        __syncthreads();
-        if (it >= nch) return;
-        const ABox &B = boxes[b];
-        const unsigned n0 = (unsigned)B.n[0], n01 = (unsigned)B.n[0] * (unsigned)B.n[1], nvb = n01 * (unsigned)B.n[2];
-        int v[7] = {INT_MAX, INT_MAX, INT_MAX, INT_MAX, INT_MIN, INT_MIN, INT_MIN};   // amin, lo xyz, hi xyz
-        for (unsigned k = threadIdx.x; k < ch; k += blockDim.x) {
-            const unsigned loc = (it - B.chunk0) * ch + k;
-            if (loc >= nvb) break;
-            const float f = arena[B.arena + loc];
-            v[0] = min(v[0], f2ord(f));
-            if (f >= B.iso) {
-                const unsigned z = loc / n01, r = loc - z * n01, y = r / n0, x = r - y * n0;
-                v[1] = min(v[1], (int)x); v[2] = min(v[2], (int)y); v[3] = min(v[3], (int)z);
-                v[4] = max(v[4], (int)x); v[5] = max(v[5], (int)y); v[6] = max(v[6], (int)z);
+        if (__any_sync(FULL, ge != 0u)) {
+            int x0 = ge ? 32 * a.w + __ffs(ge) - 1 : INT_MAX, x1 = ge ? 32 * a.w + 31 - __clz(ge) : INT_MIN;
+            int e[6] = {__reduce_min_sync(FULL, x0), __reduce_min_sync(FULL, ge ? y : INT_MAX), __reduce_min_sync(FULL, ge ? z : INT_MAX),
+                        __reduce_max_sync(FULL, x1), __reduce_max_sync(FULL, ge ? y : INT_MIN), __reduce_max_sync(FULL, ge ? z : INT_MIN)};
+            if (lane == 0) {
+                for (int k = 0; k < 3; k++) {
+                    const int l = B.o[k] + e[k], h = B.o[k] + e[k + 3];
+                    if (l < *(volatile int *)&B.blo[k]) atomicMin(&B.blo[k], l);
+                    if (h > *(volatile int *)&B.bhi[k]) atomicMax(&B.bhi[k], h);
+                }
             }
         }
-        for (int o = 16; o; o >>= 1)
-            for (int j = 0; j < 7; j++) {
-                const int t = __shfl_xor_sync(0xffffffffu, v[j], o);
-                v[j] = j < 4 ? min(v[j], t) : max(v[j], t);
-            }
-        if ((threadIdx.x & 31) == 0)
-            for (int j = 0; j < 7; j++) red[threadIdx.x >> 5][j] = v[j];
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            for (int w = 1; w < (int)(blockDim.x >> 5); w++)
-                for (int j = 0; j < 7; j++) v[j] = j < 4 ? min(v[j], red[w][j]) : max(v[j], red[w][j]);
-            ABox &W = boxes[b];
-            atomicMin(&W.amin, v[0]);
-            if (v[1] != INT_MAX) {
-                atomicMin(&W.blo[0], B.o[0] + v[1]); atomicMin(&W.blo[1], B.o[1] + v[2]); atomicMin(&W.blo[2], B.o[2] + v[3]);
-                atomicMax(&W.bhi[0], B.o[0] + v[4]); atomicMax(&W.bhi[1], B.o[1] + v[5]); atomicMax(&W.bhi[2], B.o[2] + v[6]);
-            }
-        }
-        __syncthreads();
     }
 }
 
@@ -676,7 +841,7 @@ __global__ void k_a_pad(ABox *boxes, int nb) {
 
 // ---- S5-S7: marching cubes over every label's padded grid ------------------------------
 // grid value (x,y,z) of box B minus isolevel, as the single-volume gval
-__device__ __forceinline__ float agval(const AtlasVol &v, const ABox &B, const float *arena, int x, int y, int z) {
+__device__ __forceinline__ float agval(const AtlasVol &v, const ABox &B, const APost &P, const float *arena, int x, int y, int z) {
     const long long j = (long long)(B.glo[0] + x) + (long long)(y + B.glo[1]) * v.nx + (long long)(z + B.glo[2]) * v.nxy;
     float val;
     if (j < v.nvox) {
@@ -691,9 +856,13 @@ __device__ __forceinline__ float agval(const AtlasVol &v, const ABox &B, const f
             vz++;
         }
         const int lx = vx - B.o[0], ly = vy - B.o[1], lz = vz - B.o[2];
-        val = (lx >= 0 && ly >= 0 && lz >= 0 && lx < B.n[0] && ly < B.n[1] && lz < B.n[2])
-                  ? arena[B.arena + ((long long)lz * B.n[1] + ly) * B.n[0] + lx]
-                  : 0.f;
+        val = 0.f;
+        if (lx >= 0 && ly >= 0 && lz >= 0 && lx < B.n[0] && ly < B.n[1] && lz < B.n[2]) {
+            const unsigned lr = (unsigned)lz * (unsigned)B.n[1] + (unsigned)ly, w = B.bw0 + lr * B.W + ((unsigned)lx >> 5);
+            val = __ldg(arena + B.arena + (long long)lr * B.n[0] + lx);
+            if (P.largest && !(__ldg(P.KD + w) >> (lx & 31) & 1u)) val = ord2f(B.vmin);
+            else if (P.fill && (__ldg(P.K + w) >> (lx & 31) & 1u)) val = fmaxf(val, B.iso);
+        }
         if (vx == 0 || vy == 0 || vz == 0 || vx == v.nx - 1 || vy == v.ny - 1 || vz == v.nz - 1)
             val = fminf(B.edge_max, val);
         val = __fsub_rn(val, B.iso);
@@ -704,229 +873,162 @@ __device__ __forceinline__ float agval(const AtlasVol &v, const ABox &B, const f
     return val;
 }
 
-constexpr int TY = 8, TZ = 8;
+// The grids of all boxes are words of one numbering for mcwords.cuh: each box begins at a
+// multiple of SUB words, so that a sub-tile belongs to one box (subbox).
+__device__ __forceinline__ unsigned agrid_words(const ABox &B) { return B.WX * (unsigned)B.gn[1] * (unsigned)B.gn[2]; }
 
-__global__ void __launch_bounds__(256) k_a_count(AtlasVol v, const ABox *boxes, int nb, unsigned nitems, unsigned *queue,
-                                                 const float *arena, bool classic, uint4 *words, uint4 *counts,
-                                                 unsigned *active, unsigned *nactive) {
+// Sign words from the sub-boxes' sign bits, a thread per word and no values read.  A grid
+// ends at most one voxel past the volume and two past the sub-box, where values are 0; agval's
+// cases by words: darkening is min(edge_max, value), whose sign is both their signs, a
+// coordinate one past the volume wraps into the next row or slice (whose first
+// voxels are on a face), and past the last one there is padding.
+__global__ void __launch_bounds__(256) k_a_signs(AtlasVol v, const ABox *boxes, int nb, unsigned nsub, const unsigned *__restrict__ S,
+                                                 unsigned *signs, unsigned *subbox) {
     grid_wait();
-    __shared__ float sv[TZ + 1][TY + 1][33];
-    __shared__ unsigned item;
-    __shared__ int bi;
-    for (;;) {
-        if (threadIdx.x == 0) {
-            item = atomicAdd(queue, 1u);
-            bi = item < nitems ? find_item(boxes, nb, item, &ABox::ctile0) : 0;
-        }
-        __syncthreads();
-        const unsigned it = item;
-        const int b = bi;
-        if (it >= nitems) return;
+    const unsigned lane = threadIdx.x & 31u;
+    for (unsigned sub = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; sub < nsub; sub += (gridDim.x * blockDim.x) >> 5) {
+        const int b = find_item(boxes, nb, sub * mcw::SUB, &ABox::word0);
         const ABox &B = boxes[b];
-        const unsigned local = it - B.ctile0;
-        const int ty = (B.gn[1] + TY - 1) / TY;
-        const int cx = local % B.WX, cy = (local / B.WX) % ty, cz = local / (B.WX * ty);
-        const int x0 = cx * 32, y0 = cy * TY, z0 = cz * TZ;
-        for (int i = threadIdx.x; i < (TZ + 1) * (TY + 1) * 33; i += 256) {
-            const int xx = i % 33, r = i / 33, yy = r % (TY + 1), zz = r / (TY + 1);
-            sv[zz][yy][xx] = agval(v, B, arena, x0 + xx, y0 + yy, z0 + zz);
-        }
-        __syncthreads();
-        const int wy = threadIdx.x >> 5, lane = threadIdx.x & 31;
-        const int y = y0 + wy, x = x0 + lane;
-        if (y < B.gn[1]) {
-            for (int zz = 0; zz < TZ; zz++) {
-                const int z = z0 + zz;
-                if (z >= B.gn[2]) break;
-                const bool in = x < B.gn[0];
-                const bool hx = in && x < B.gn[0] - 1, hy = in && y < B.gn[1] - 1, hz = in && z < B.gn[2] - 1;
-                const float c0 = sv[zz][wy][lane];
-                const bool s0 = c0 > 0.f;
-                const bool ex = hx && ((sv[zz][wy][lane + 1] > 0.f) != s0);
-                const bool ey = hy && ((sv[zz][wy + 1][lane] > 0.f) != s0);
-                const bool ez = hz && ((sv[zz + 1][wy][lane] > 0.f) != s0);
-                int nt = 0, nc = 0;
-                if (hx && hy && hz) {
-                    float c[8] = {c0, sv[zz][wy][lane + 1], sv[zz][wy + 1][lane + 1], sv[zz][wy + 1][lane],
-                                  sv[zz + 1][wy][lane], sv[zz + 1][wy][lane + 1], sv[zz + 1][wy + 1][lane + 1],
-                                  sv[zz + 1][wy + 1][lane]};
-                    const int lut = cube_lut(c);
-                    if (lut != 0 && lut != 255) {
-                        const Tiling T = select_tiling(c, lut, classic);
-                        nt = T.n;
-                        nc = T.cv;
+        if (lane == 0) subbox[sub] = (unsigned)b;
+        const unsigned lw = sub * mcw::SUB - B.word0 + lane;
+        unsigned m = 0;
+        if (lw < agrid_words(B)) {
+            const unsigned row = lw / B.WX;
+            const int x0 = 32 * (int)(lw - row * B.WX), z = (int)(row / (unsigned)B.gn[1]), y = (int)(row - (unsigned)z * (unsigned)B.gn[1]);
+            const bool dark = __fsub_rn(B.edge_max, B.iso) > -N2M_FLT_EPS, padp = B.pad > -N2M_FLT_EPS;
+            const unsigned zero = __fsub_rn(0.f, B.iso) > -N2M_FLT_EPS ? FULL : 0u;
+            auto bits = [&](int vx, int vy, int vz) -> unsigned {   // signs of voxels vx .. vx+31 of a row, no face rule
+                const int lx = vx - B.o[0], ly = vy - B.o[1], lz = vz - B.o[2];
+                if (ly < 0 || lz < 0 || ly >= B.n[1] || lz >= B.n[2] || lx <= -32 || lx >= B.n[0]) return zero;
+                const unsigned *r = S + B.bw0 + ((unsigned)lz * (unsigned)B.n[1] + (unsigned)ly) * B.W;
+                const unsigned q = (unsigned)(lx < 0 ? 0 : lx) >> 5;
+                const unsigned c = __ldg(r + q);
+                const unsigned n = lx < 0 ? c << -lx : __funnelshift_r(c, q + 1 < B.W ? __ldg(r + q + 1) : 0u, lx & 31);
+                const unsigned in = mcw::bit_range(-lx, B.n[0] - lx);
+                return (n & in) | (zero & ~in);
+            };
+            int vy = B.glo[1] + y, vz = B.glo[2] + z;
+            const int vx = B.glo[0] + x0, pad = v.nx - vx;   // bit of the padding column
+            const unsigned in = mcw::bit_range(0, B.gn[0] - x0);
+            if (vy >= v.ny) {   // the padding row is row 0 of the next slice
+                vy -= v.ny;
+                vz++;
+            }
+            if (vz >= v.nz) {
+                m = padp ? FULL : 0u;
+            } else {
+                m = bits(vx, vy, vz);
+                if (!dark) {
+                    if (vy == 0 || vz == 0 || vy == v.ny - 1 || vz == v.nz - 1) m = 0u;
+                    else m &= mcw::bit_range(1 - vx, v.nx - 1 - vx);
+                }
+                if (pad >= 0 && pad < 32) {
+                    m &= mcw::bit_range(0, pad);
+                    int py = vy + 1, pz = vz;
+                    if (py >= v.ny) {
+                        py -= v.ny;
+                        pz++;
                     }
-                }
-                const unsigned xm = __ballot_sync(0xffffffffu, ex), ym = __ballot_sync(0xffffffffu, ey),
-                               zm = __ballot_sync(0xffffffffu, ez);
-                for (int o = 16; o; o >>= 1) {
-                    nt += __shfl_xor_sync(0xffffffffu, nt, o);
-                    nc += __shfl_xor_sync(0xffffffffu, nc, o);
-                }
-                if (lane == 0) {
-                    const unsigned w = B.word0 + ((unsigned)z * (unsigned)B.gn[1] + (unsigned)y) * B.WX + (unsigned)cx;
-                    const unsigned nv = __popc(xm) + __popc(ym) + __popc(zm);
-                    const bool act = nv | nt | nc;
-                    words[w] = make_uint4(xm, ym, zm, 0u);
-                    counts[w] = make_uint4(nv, (unsigned)nt, (unsigned)nc, act);
-                    if (act) active[atomicAdd(nactive, 1u)] = w;
+                    if (pz < v.nz ? dark && (bits(0, py, pz) & 1u) : padp) m |= 1u << pad;
                 }
             }
+            m &= in;
         }
-        __syncthreads();
+        signs[sub * mcw::SUB + lane] = m;
     }
 }
 
-__device__ __forceinline__ int avid(const uint4 *__restrict__ words, const uint4 *__restrict__ offs, const ABox &B,
-                                    unsigned cshift, int x, int y, int z, int axis) {
-    const unsigned w = B.word0 + ((unsigned)z * (unsigned)B.gn[1] + (unsigned)y) * B.WX + ((unsigned)x >> 5);
-    const unsigned l = (unsigned)x & 31u;
-    const uint4 m = words[w];
-    const unsigned lt = (1u << l) - 1u;
-    unsigned id = offs[w].x + cshift + __popc(m.x & lt) + __popc(m.y & lt) + __popc(m.z & lt);
-    if (axis >= 1) id += (m.x >> l) & 1u;
-    if (axis == 2) id += (m.y >> l) & 1u;
-    return (int)id;
-}
+// mcwords.cuh's policy for the boxes' padded Lewiner grids.  Vertex numbers are contiguous per
+// box: its edge vertices, then its c-vertices.
+struct Policy {
+    static constexpr bool MULTI = true, REVERSE = true, CVERTS = true;
+    static constexpr int CTAS = 8, EV = 1;
+    AtlasVol v;
+    const ABox *boxes;
+    int nb;
+    const unsigned *subbox;
+    APost post;
+    const float *arena;
+    bool classic;
+    vec3d *pts;
+    int *cand, *ccand;
+    unsigned *ncand, *nccand;
+    int cap;
+    unsigned *near;
+    __device__ __forceinline__ unsigned quick(int lut) const {
+        Tiling T = {0, 0, false};
+        return quick_tiling(lut, classic, T) ? (unsigned)T.off << 8 | (unsigned)T.n : mcw::TESTS;
+    }
+    __device__ __forceinline__ int code(int off) const { return d_lut[off]; }
+    __device__ __forceinline__ bool geo(unsigned w, mcw::Geo &q) const {
+        const unsigned b = __ldg(subbox + w / mcw::SUB);
+        const ABox &B = boxes[b];
+        const unsigned lw = w - B.word0, row = lw / B.WX, xw = lw - row * B.WX;
+        q.z = (int)(row / (unsigned)B.gn[1]);
+        if (q.z >= B.gn[2]) return false;   // the filling behind the box's last word
+        q.y = (int)(row - (unsigned)q.z * (unsigned)B.gn[1]);
+        q.x0 = 32 * (int)xw;
+        q.WX = B.WX;
+        q.slice = B.WX * (unsigned)B.gn[1];
+        q.inm = mcw::bit_range(0, B.gn[0] - q.x0);
+        q.hxm = mcw::bit_range(0, B.gn[0] - 1 - q.x0);
+        q.hy = q.y < B.gn[1] - 1;
+        q.hz = q.z < B.gn[2] - 1;
+        q.nx = xw + 1 < B.WX;
+        q.tag = (int)b;
+        return true;
+    }
+    __device__ __forceinline__ void voxel_word(const mcw::Geo &, int &wx, int &vy, int &vz) const { wx = vy = vz = 0; }
+    __device__ __forceinline__ void shifts(const mcw::Out &o, unsigned s, const uint4 &total, unsigned &e, unsigned &c) const {
+        const ABox &B = boxes[__ldg(subbox + s)];
+        const unsigned s0 = B.word0 / mcw::SUB, s1 = s0 + (agrid_words(B) + mcw::SUB - 1) / mcw::SUB;
+        e = mcw::sub_offset(o, s0).z;                             // earlier boxes' c-vertices
+        c = s1 < o.nsub ? mcw::sub_offset(o, s1).x : total.x;     // edge vertices up to the end of this box
+    }
+    __device__ __forceinline__ void corners(const ABox &B, int x, int y, int z, float *c) const {
+        c[0] = agval(v, B, post, arena, x, y, z); c[1] = agval(v, B, post, arena, x + 1, y, z);
+        c[2] = agval(v, B, post, arena, x + 1, y + 1, z); c[3] = agval(v, B, post, arena, x, y + 1, z);
+        c[4] = agval(v, B, post, arena, x, y, z + 1); c[5] = agval(v, B, post, arena, x + 1, y, z + 1);
+        c[6] = agval(v, B, post, arena, x + 1, y + 1, z + 1); c[7] = agval(v, B, post, arena, x, y + 1, z + 1);
+    }
+    __device__ __noinline__ mcw::CubeTiling tests(const mcw::Geo &q, int x, int y, int z, int lut) const {
+        float c[8];
+        corners(boxes[q.tag], x, y, z, c);
+        const Tiling T = select_tiling(c, lut, classic);
+        return mcw::CubeTiling{T.off, T.n, T.cv};
+    }
+    __device__ __forceinline__ void cvertex(const mcw::Geo &q, int x, int y, int z, int id) const {
+        const ABox &B = boxes[q.tag];
+        float c[8];
+        corners(B, x, y, z, c);
+        emit_cvertex(c, x, y, z, (float)B.glo[0], (float)B.glo[1], (float)B.glo[2], id, pts, ccand, nccand, cap);
+        mark_near(near, id);
+    }
+    struct Edge {
+        float c0, c1, flo0, flo1, flo2;
+    };
+    __device__ __forceinline__ Edge edge(int x, int y, int z, int ax, int tag) const {
+        const ABox &B = boxes[tag];
+        return Edge{agval(v, B, post, arena, x, y, z), agval(v, B, post, arena, x + (ax == 0), y + (ax == 1), z + (ax == 2)),
+                    (float)B.glo[0], (float)B.glo[1], (float)B.glo[2]};
+    }
+    __device__ __forceinline__ vec3d vertex(const Edge &c, int x, int y, int z, int ax, int id) const {
+        return edge_vertex(c.c0, c.c1, x, y, z, ax, c.flo0, c.flo1, c.flo2, id, cand, ncand, cap, near);
+    }
+};
 
-// per box: the scan values at its first word (edge vertices, triangles and
-// c-vertices of all earlier boxes), from which its contiguous ranges follow
+// per box: edge vertices, triangles and c-vertices of all earlier boxes, from which its
+// contiguous ranges follow (and the totals after the last)
 struct BoxOff {
     unsigned e, t, c;
 };
-
-__global__ void k_a_emit(AtlasVol v, const ABox *boxes, const BoxOff *boff, int nb, const uint4 *__restrict__ words,
-                         const uint4 *__restrict__ offs, const unsigned *__restrict__ active, unsigned nactive,
-                         const float *arena, bool classic, vec3d *pts, vec3i *tris, int *cand, unsigned *ncand,
-                         int *ccand, unsigned *nccand, int cap) {
-    grid_wait();
-    const unsigned lane = threadIdx.x & 31u;
-    for (unsigned aw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; aw < nactive; aw += (gridDim.x * blockDim.x) >> 5) {
-        const unsigned w = active[aw];
-        const int b = find_item(boxes, nb, w, &ABox::word0);
-        const ABox &B = boxes[b];
-        const unsigned cshift = boff[b].c;                        // c-vertices of earlier boxes
-        const unsigned cbase = boff[b + 1].e + 0u;                // this box's c-vertices follow its edge vertices
-        const unsigned lw = w - B.word0;
-        const unsigned row = lw / B.WX, xw = lw - row * B.WX;
-        const int z = (int)(row / (unsigned)B.gn[1]), y = (int)(row - (unsigned)z * (unsigned)B.gn[1]);
-        const int x = (int)(xw * 32u + lane);
-        const uint4 o = offs[w];
-        const uint4 m = words[w];
-        const bool in = x < B.gn[0];
-        const bool hx = in && x < B.gn[0] - 1, hy = in && y < B.gn[1] - 1, hz = in && z < B.gn[2] - 1;
-        const bool cube = hx && hy && hz;
-        const bool ex = (m.x >> lane) & 1u, ey = (m.y >> lane) & 1u, ez = (m.z >> lane) & 1u;
-        float c[8];
-        if (in) {
-            c[0] = agval(v, B, arena, x, y, z);
-            c[1] = hx ? agval(v, B, arena, x + 1, y, z) : c[0];
-            c[3] = hy ? agval(v, B, arena, x, y + 1, z) : c[0];
-            c[4] = hz ? agval(v, B, arena, x, y, z + 1) : c[0];
-            if (cube) {
-                c[2] = agval(v, B, arena, x + 1, y + 1, z);
-                c[5] = agval(v, B, arena, x + 1, y, z + 1);
-                c[6] = agval(v, B, arena, x + 1, y + 1, z + 1);
-                c[7] = agval(v, B, arena, x, y + 1, z + 1);
-            }
-        }
-        const float flo0 = (float)B.glo[0], flo1 = (float)B.glo[1], flo2 = (float)B.glo[2];
-        if (ex | ey | ez) {
-            const unsigned lt = (1u << lane) - 1u;
-            int id = (int)(o.x + cshift + __popc(m.x & lt) + __popc(m.y & lt) + __popc(m.z & lt));
-            const float fx = (float)x, fy = (float)y, fz = (float)z;
-            if (ex) {
-                const float X = __fadd_rn(__fadd_rn(fx, edge_u(c[0], c[1])), flo0);
-                pts[id] = {(double)X, (double)__fadd_rn(fy, flo1), (double)__fadd_rn(fz, flo2)};
-                if (frac_dist(X) < 1.5e-5f) { unsigned k = atomicAdd(ncand, 1u); if (k < (unsigned)cap) cand[k] = id; }
-                id++;
-            }
-            if (ey) {
-                const float Y = __fadd_rn(__fadd_rn(fy, edge_u(c[0], c[3])), flo1);
-                pts[id] = {(double)__fadd_rn(fx, flo0), (double)Y, (double)__fadd_rn(fz, flo2)};
-                if (frac_dist(Y) < 1.5e-5f) { unsigned k = atomicAdd(ncand, 1u); if (k < (unsigned)cap) cand[k] = id; }
-                id++;
-            }
-            if (ez) {
-                const float Z = __fadd_rn(__fadd_rn(fz, edge_u(c[0], c[4])), flo2);
-                pts[id] = {(double)__fadd_rn(fx, flo0), (double)__fadd_rn(fy, flo1), (double)Z};
-                if (frac_dist(Z) < 1.5e-5f) { unsigned k = atomicAdd(ncand, 1u); if (k < (unsigned)cap) cand[k] = id; }
-            }
-        }
-        Tiling T = {0, 0, false};
-        if (cube) {
-            const int lut = cube_lut(c);
-            if (lut != 0 && lut != 255) T = select_tiling(c, lut, classic);
-        }
-        int tb = T.n, cb = T.cv;
-        for (int d = 1; d < 32; d <<= 1) {
-            const int a = __shfl_up_sync(0xffffffffu, tb, d), bb = __shfl_up_sync(0xffffffffu, cb, d);
-            if ((int)lane >= d) { tb += a; cb += bb; }
-        }
-        tb -= T.n;
-        cb -= T.cv;
-        if (T.n == 0) continue;
-        int v12 = -1;
-        if (T.cv) {
-            v12 = (int)(cbase + o.z + cb);
-            float n = 0.f, sx = 0.f, sy = 0.f, sz = 0.f;
-            for (int e = 0; e < 12; e++) {
-                const int own = k_edge[e][0], ax = k_edge[e][1], ca = k_edge[e][2], cbn = k_edge[e][3];
-                if ((c[ca] > 0.f) == (c[cbn] > 0.f)) continue;
-                const float u = edge_u(c[ca], c[cbn]);
-                float px = (float)(x + ((own ^ (own >> 1)) & 1)), py = (float)(y + ((own >> 1) & 1)),
-                      pz = (float)(z + ((own >> 2) & 1));
-                if (ax == 0) px = __fadd_rn(px, u);
-                else if (ax == 1) py = __fadd_rn(py, u);
-                else pz = __fadd_rn(pz, u);
-                n = __fadd_rn(n, 1.f);
-                sx = __fadd_rn(sx, px); sy = __fadd_rn(sy, py); sz = __fadd_rn(sz, pz);
-            }
-            if (n > 0.f) { sx = __fdiv_rn(sx, n); sy = __fdiv_rn(sy, n); sz = __fdiv_rn(sz, n); }
-            const float X = __fadd_rn(sx, flo0), Y = __fadd_rn(sy, flo1), Z = __fadd_rn(sz, flo2);
-            pts[v12] = {(double)X, (double)Y, (double)Z};
-            if (fminf(frac_dist(X), fminf(frac_dist(Y), frac_dist(Z))) < 1.5e-5f) {
-                unsigned k = atomicAdd(nccand, 1u);
-                if (k < (unsigned)cap) ccand[k] = v12;
-            }
-        }
-        int tv[3];
-        for (int t = 0; t < 3 * T.n; t++) {
-            const int code = d_lut[T.off + t];
-            int vv;
-            switch (code) {
-            case 0: vv = avid(words, offs, B, cshift, x, y, z, 0); break;
-            case 1: vv = avid(words, offs, B, cshift, x + 1, y, z, 1); break;
-            case 2: vv = avid(words, offs, B, cshift, x, y + 1, z, 0); break;
-            case 3: vv = avid(words, offs, B, cshift, x, y, z, 1); break;
-            case 4: vv = avid(words, offs, B, cshift, x, y, z + 1, 0); break;
-            case 5: vv = avid(words, offs, B, cshift, x + 1, y, z + 1, 1); break;
-            case 6: vv = avid(words, offs, B, cshift, x, y + 1, z + 1, 0); break;
-            case 7: vv = avid(words, offs, B, cshift, x, y, z + 1, 1); break;
-            case 8: vv = avid(words, offs, B, cshift, x, y, z, 2); break;
-            case 9: vv = avid(words, offs, B, cshift, x + 1, y, z, 2); break;
-            case 10: vv = avid(words, offs, B, cshift, x + 1, y + 1, z, 2); break;
-            case 11: vv = avid(words, offs, B, cshift, x, y + 1, z, 2); break;
-            case 12: vv = v12; break;
-            default: vv = -1; break;
-            }
-            tv[t % 3] = vv;
-            if (t % 3 == 2) tris[o.y + tb + t / 3] = {tv[2], tv[1], tv[0]};
-        }
-    }
-}
-
-// scan values at the first word of every box (and the totals after the last)
-__global__ void k_a_boxoff(const ABox *boxes, int nb, const uint4 *offs, uint4 total, BoxOff *boff) {
+__global__ void k_a_boxoff(const ABox *boxes, int nb, mcw::Out o, BoxOff *boff) {
     grid_wait();
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b > nb) return;
-    if (b == nb) {
-        boff[b] = {total.x, total.y, total.z};
-        return;
-    }
-    const uint4 o = offs[boxes[b].word0];
-    boff[b] = {o.x, o.y, o.z};
+    const unsigned s = b < nb ? boxes[b].word0 / mcw::SUB : o.nsub;
+    const uint4 q = s < o.nsub ? mcw::sub_offset(o, s) : *o.total;
+    boff[b] = {q.x, q.y, q.z};
 }
 
 // binarise the whole volume for one label (the per-label loop)
@@ -1007,17 +1109,8 @@ __global__ void k_a_localize(vec3i *t, unsigned nt, const unsigned *tri_start, c
 }  // namespace
 
 namespace {
-unsigned set_chunks(std::vector<ABox> &boxes, unsigned ch) {
-    unsigned chunks = 0;
-    for (auto &B : boxes) {
-        B.chunk0 = chunks;
-        chunks += (unsigned)(((long long)B.n[0] * B.n[1] * B.n[2] + ch - 1) / ch);
-    }
-    return chunks;
-}
-
-// smoothing, isolevel, clustering and range/bbox: device-only work (no host
-// synchronisation), enqueued for timing by the autotuner or captured as a graph
+// smoothing, isolevel, clustering and signs/bbox: device-only work (no host
+// synchronisation)
 struct Segment {
     AtlasVol v;
     ABox *db;
@@ -1026,61 +1119,77 @@ struct Segment {
     float *ar;
     bool smooth_on, only_largest, fill_bubbles;
     int nx, ny, nz;
-    unsigned *q;
     long long arena;
     unsigned nrows, nbw;   // rows and bit words of all the boxes
+    APost post;            // what the clustering leaves (enqueue)
 
     n2m_status ensure(AtlasWork &w) {
+        CKS(w.keep.ensure((size_t)nbw * sizeof(unsigned)));
+        CKS(w.shell.ensure((size_t)2 * nbw * sizeof(unsigned)));
+        CKS(w.wbox.ensure((size_t)nbw / 32 * sizeof(unsigned)));
         if (only_largest || fill_bubbles) {
             CKS(w.mask.ensure((size_t)nbw * sizeof(unsigned)));
-            if (only_largest) CKS(w.keep.ensure((size_t)nbw * sizeof(unsigned)));
             CKS(w.lab.ensure((size_t)arena * sizeof(int)));
+            CKS(w.list.ensure(((size_t)arena + nrows) / 2 * sizeof(uint2)));   // every second voxel of a row at most
+            CKS(w.wlist.ensure(((size_t)nbw + 4) * sizeof(unsigned)));
+            if (fill_bubbles) CKS(w.fill.ensure((size_t)nbw * sizeof(unsigned)));
             if (fill_bubbles) CKS(w.edge.ensure((size_t)arena));
             if (only_largest) CKS(w.ucnt.ensure((size_t)arena * sizeof(unsigned)));
         }
         return N2M_OK;
     }
 
-    n2m_status enqueue(AtlasWork &w, unsigned ch, unsigned per_sm, unsigned chunks, cudaStream_t s) {
-        int qi = 0;
-        CK(cudaMemsetAsync(q, 0, 32 * sizeof(unsigned), s));
-        n2m_launch(k_a_smooth, pgrid(tiles, 2), dim3(smooth::STX, smooth::STY), 0, s, v, db, nb, tiles, q + qi++, ar,
-                   smooth_on);
+    n2m_status enqueue(AtlasWork &w, cudaStream_t s) {
+        unsigned *wbox = w.wbox.as<unsigned>();
+        unsigned *M = w.keep.as<unsigned>();   // the labels' masks, until the kept voxels take their place
+        const unsigned wg = std::max(1u, std::min((nbw + 255) / 256, 152u * 16u));   // a thread per word
+        n2m_launch(k_a_mask, wg, 256, 0, s, v, db, nb, nbw, M, wbox);
+        n2m_launch(k_a_smooth, std::max(1u, std::min((tiles + AWARPS - 1) / AWARPS, 152u * 8u)), 32 * AWARPS, 0, s, db, nb, tiles,
+                   M, ar, nx, ny, nz, smooth_on);
         n2m_launch(k_a_iso, (nb + 127) / 128, 128, 0, s, db, nb);
-        const unsigned g = pgrid(chunks, per_sm);
         if (only_largest || fill_bubbles) {
             unsigned *Bm = w.mask.as<unsigned>();
             int *L = w.lab.as<int>();
-            const unsigned rg = std::max(1u, std::min((nrows + 7) / 8, 152u * 16u));     // a warp per row
-            const unsigned sg = std::max(1u, std::min((nrows * AB_SEG / 32 + 8) / 8, 152u * 16u));   // AB_SEG lanes per row
-            const unsigned wg = std::max(1u, std::min((nbw + 255) / 256, 152u * 16u));   // a thread per word
-            n2m_launch(k_ab_bits, rg, 256, 0, s, db, nb, nrows, ar, Bm);
+            // lists by words, then a thread per entry (about one run per word)
+            const unsigned lg = std::max(1u, std::min((nbw + 256 * AL_K - 1) / (256 * AL_K), 152u * 16u)), g = std::min(wg, 152u * 8u);
+            uint2 *list = w.list.as<uint2>();
+            unsigned *wlist = w.wlist.as<unsigned>(), *n = wlist + nbw;   // {runs, words} of the background, of the foreground
+            CK(cudaMemsetAsync(n, 0, 4 * sizeof(unsigned), s));
+            n2m_launch(k_ab_bits, wg, 256, 0, s, db, wbox, nbw, ar, Bm);
+            const unsigned *K = Bm;
             if (fill_bubbles) {
                 unsigned char *edge = w.edge.as<unsigned char>();
-                n2m_launch(k_ab_init, wg, 256, 0, s, db, nb, nbw, Bm, 0u, L, edge, nullptr);
-                n2m_launch(k_ab_merge<3>, sg, 256, 0, s, db, nb, nrows, Bm, 0u, L);
-                n2m_launch(k_ab_flatten, wg, 256, 0, s, db, nb, nbw, Bm, 0u, L, false);
-                n2m_launch(k_ab_edges, wg, 256, 0, s, db, nb, nbw, Bm, L, edge);
-                n2m_launch(k_ab_fill, sg, 256, 0, s, db, nb, nrows, Bm, L, edge);
+                unsigned *Fm = w.fill.as<unsigned>();
+                n2m_launch(k_al_list<3>, lg, 256, 0, s, db, wbox, nbw, Bm, 0u, list, wlist, n, L, edge, nullptr);
+                n2m_launch(k_al_jump, g, 256, 0, s, list, n, L);
+                n2m_launch(k_al_merge<3>, g, 256, 0, s, db, wbox, Bm, 0u, wlist, n, L);
+                n2m_launch(k_al_flatten, g, 256, 0, s, db, wbox, list, n, L, false);
+                n2m_launch(k_al_edges, g, 256, 0, s, db, wbox, Bm, list, n, L, edge);
+                CK(cudaMemcpyAsync(Fm, Bm, (size_t)nbw * sizeof(unsigned), cudaMemcpyDeviceToDevice, s));
+                n2m_launch(k_al_fill, g, 256, 0, s, db, wbox, Bm, list, n, L, edge, Fm);
+                K = Fm;
             }
-            unsigned *cnt = only_largest ? w.ucnt.as<unsigned>() : nullptr;
-            n2m_launch(k_ab_init, wg, 256, 0, s, db, nb, nbw, Bm, 1u, L, nullptr, cnt);
-            n2m_launch(k_ab_merge<9>, sg, 256, 0, s, db, nb, nrows, Bm, 1u, L);
-            n2m_launch(k_ab_flatten, wg, 256, 0, s, db, nb, nbw, Bm, 1u, L, true);
-            const unsigned *K = Bm;
             if (only_largest) {
-                unsigned *Kb = w.keep.as<unsigned>();
-                n2m_launch(k_ab_sizes, sg, 256, 0, s, db, nb, nrows, Bm, L, cnt);
-                n2m_launch(k_ab_best, wg, 256, 0, s, db, nb, nbw, Bm, L, cnt);
-                n2m_launch(k_ab_keep, sg, 256, 0, s, db, nb, nrows, Bm, L, Kb);
+                const unsigned *F = K;   // the (filled) foreground
+                unsigned *cnt = w.ucnt.as<unsigned>(), *Kb = w.keep.as<unsigned>();
+                n2m_launch(k_al_list<9>, lg, 256, 0, s, db, wbox, nbw, F, 1u, list, wlist, n + 2, L, nullptr, cnt);
+                n2m_launch(k_al_jump, g, 256, 0, s, list, n + 2, L);
+                n2m_launch(k_al_merge<9>, g, 256, 0, s, db, wbox, F, 1u, wlist, n + 2, L);
+                n2m_launch(k_al_flatten, g, 256, 0, s, db, wbox, list, n + 2, L, true);
+                n2m_launch(k_al_sizes, g, 256, 0, s, db, wbox, F, list, n + 2, L, cnt);
+                n2m_launch(k_al_best, g, 256, 0, s, db, wbox, list, n + 2, L, cnt);
+                CK(cudaMemsetAsync(Kb, 0, (size_t)nbw * sizeof(unsigned), s));
+                n2m_launch(k_al_keep, g, 256, 0, s, db, wbox, F, list, n + 2, L, Kb);
                 K = Kb;
             }
-            if (only_largest && fill_bubbles) n2m_launch(k_ab_final<true, true>, rg, 256, 0, s, db, nb, nrows, K, ar, nx,
-                                                         ny, nz);
-            else if (only_largest) n2m_launch(k_ab_final<true, false>, rg, 256, 0, s, db, nb, nrows, K, ar, nx, ny, nz);
-            else n2m_launch(k_ab_final<false, true>, rg, 256, 0, s, db, nb, nrows, K, ar, nx, ny, nz);
+            post.K = K;
         }
-        n2m_launch(k_a_stats, g, 256, 0, s, db, nb, chunks, q + qi++, ch, ar);
+        post.fill = fill_bubbles;
+        post.largest = only_largest;
+        unsigned *S = w.shell.as<unsigned>(), *KD = S + nbw;
+        post.S = S;
+        post.KD = KD;
+        n2m_launch(k_ab_shell, wg, 256, 0, s, db, wbox, nbw, post, S, KD, ar, nx, ny, nz);
         n2m_launch(k_a_pad, (nb + 127) / 128, 128, 0, s, db, nb);
         CKL();
         return N2M_OK;
@@ -1098,7 +1207,7 @@ n2m_status atlas_hist(const short *d_lab, const int dim[3], AtlasWork &w, cudaSt
     CK(cudaMemsetAsync(dvmax, 0, sizeof(int), s));
     n2m_launch(k_a_fill_bb, 256, 256, 0, s, w.bb.as<int>(), (ML + 1) * 6);
     AtlasVol v{d_lab, dim[0], dim[1], dim[2], (long long)dim[0] * dim[1], (long long)dim[0] * dim[1] * dim[2]};
-    n2m_launch(k_a_hist, pgrid((unsigned)std::min<long long>((v.nvox + 255) / 256, 1u << 30), 32), 256, 0, s, v, ML,
+    n2m_launch(k_a_hist, pgrid((unsigned)std::min<long long>((v.nvox + 256 * HV - 1) / (256 * HV), 1u << 30), 4), HT, 0, s, v, ML,
                w.cnt.as<unsigned>(), w.bb.as<int>(), dvmax);
     CKL();
     int mx = 0;
@@ -1168,14 +1277,11 @@ n2m_status atlas_batched(const short *d_lab, const int dim[3], const n2m_options
         B.arena = arena;
         arena += (long long)B.n[0] * B.n[1] * B.n[2];
         B.tile0 = tiles;
-        tiles += (unsigned)(((B.n[0] + smooth::STX - 1) / smooth::STX) * ((B.n[1] + smooth::STY - 1) / smooth::STY) *
-                            ((B.n[2] + smooth::SZC - 1) / smooth::SZC));
-        B.chunk0 = 0;   // set per chunk size below
         B.W = (unsigned)(B.n[0] + 31) / 32;
-        B.row0 = rows;
+        tiles += B.W * (unsigned)((B.n[1] + ARY - 1) / ARY) * (unsigned)((B.n[2] + AZC - 1) / AZC);
         B.bw0 = bwords;
         rows += (unsigned long long)B.n[1] * B.n[2];
-        bwords += (unsigned long long)B.W * B.n[1] * B.n[2];
+        bwords += ((unsigned long long)B.W * B.n[1] * B.n[2] + 31) / 32 * 32;
         B.vmin = INT_MAX;
         B.vmax = INT_MIN;
         for (int a = 0; a < 3; a++) { B.blo[a] = INT_MAX; B.bhi[a] = INT_MIN; }
@@ -1187,81 +1293,25 @@ n2m_status atlas_batched(const short *d_lab, const int dim[3], const n2m_options
         return N2M_ERR_TOO_LARGE;
     }
     CKS(w.boxes.ensure((size_t)nb * sizeof(ABox)));
-    CKS(w.queue.ensure(96 * sizeof(unsigned)));
     CKS(w.arena.ensure((size_t)arena * sizeof(float)));
     ABox *db = w.boxes.as<ABox>();
-    unsigned *q = w.queue.as<unsigned>();
     CK(cudaMemcpyAsync(db, boxes.data(), nb * sizeof(ABox), cudaMemcpyHostToDevice, s));
-    CK(cudaMemsetAsync(q, 0, 96 * sizeof(unsigned), s));
     float *ar = w.arena.as<float>();
     const bool smooth_on = o.pre_smooth && dim[0] >= 5 && dim[1] >= 5 && dim[2] >= 5;
-    Segment seg{v, db, nb, tiles, ar, smooth_on, o.only_largest, o.fill_bubbles, dim[0], dim[1], dim[2], q, arena,
-                (unsigned)rows, (unsigned)bwords};
+    Segment seg{v, db, nb, tiles, ar, smooth_on, o.only_largest, o.fill_bubbles, dim[0], dim[1], dim[2], arena,
+                (unsigned)rows, (unsigned)bwords, APost{}};
     CKS(seg.ensure(w));
-    // pick chunk size and persistent-grid width once per context (autotuner)
-    if (!w.tuned) {
-        float best = 1e30f;
-        const unsigned cands[][2] = {{512, 4}, {1024, 8}, {1024, 16}, {2048, 8}, {4096, 8}, {4096, 16}};
-        for (const auto &cd : cands) {
-            std::vector<ABox> bx(boxes);
-            const unsigned nch = set_chunks(bx, cd[0]);
-            CK(cudaMemcpyAsync(db, bx.data(), nb * sizeof(ABox), cudaMemcpyHostToDevice, s));
-            CK(cudaEventRecord(ev[1], s));
-            CKS(seg.enqueue(w, cd[0], cd[1], nch, s));
-            CK(cudaEventRecord(ev[2], s));
-            CK(cudaEventSynchronize(ev[2]));
-            float ms = 0.f;
-            cudaEventElapsedTime(&ms, ev[1], ev[2]);
-            if (ms < best) { best = ms; w.chunk = cd[0]; w.per_sm = cd[1]; }
-        }
-        w.tuned = true;
-        w.tuned_ms = best;
-    }
-    const unsigned chunks = set_chunks(boxes, w.chunk);
-    CK(cudaMemcpyAsync(db, boxes.data(), nb * sizeof(ABox), cudaMemcpyHostToDevice, s));
     CK(cudaEventRecord(ev[1], s));
-    // the smoothing + clustering + range/bbox segment runs as one CUDA graph
-    cudaGraph_t graph = nullptr;
-    CK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-    const n2m_status cst = seg.enqueue(w, w.chunk, w.per_sm, chunks, s);
-    const cudaError_t ce = cudaStreamEndCapture(s, &graph);
-    if (cst != N2M_OK || ce != cudaSuccess) {
-        if (graph) cudaGraphDestroy(graph);
-        CKS(cst);
-        CK(ce);
-    }
-    cudaGraphExec_t exec = (cudaGraphExec_t)w.exec;
-    bool updated = false;
-    if (exec) {
-        cudaGraphExecUpdateResultInfo info;
-        updated = cudaGraphExecUpdate(exec, graph, &info) == cudaSuccess;
-        if (!updated) {
-            cudaGetLastError();
-            cudaGraphExecDestroy(exec);
-            exec = nullptr;
-        }
-    }
-    if (!exec) {
-        const cudaError_t ie = cudaGraphInstantiate(&exec, graph, 0);
-        if (ie != cudaSuccess) {
-            cudaGraphDestroy(graph);
-            CK(ie);
-        }
-    }
-    w.exec = exec;
-    cudaGraphDestroy(graph);
-    CK(cudaGraphLaunch(exec, s));
+    CKS(seg.enqueue(w, s));
     CK(cudaEventRecord(ev[2], s));
-    int qi = 32;
     CK(cudaMemcpyAsync(boxes.data(), db, nb * sizeof(ABox), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
     CK(cudaEventRecord(ev[3], s));
     // ---- marching-cubes grids
-    unsigned words = 0, ctiles = 0;
+    unsigned long long words64 = 0;
     for (auto &B : boxes) {
         if (!B.fail && B.blo[0] > B.bhi[0]) B.fail = N2M_ERR_EMPTY;
-        B.word0 = words;
-        B.ctile0 = ctiles;
+        B.word0 = (unsigned)words64;
         if (B.fail) {
             B.WX = 0;
             for (int a = 0; a < 3; a++) B.gn[a] = 0;
@@ -1273,41 +1323,57 @@ n2m_status atlas_batched(const short *d_lab, const int dim[3], const n2m_options
             B.gn[a] = hi - lo + 1;
         }
         B.WX = (unsigned)((B.gn[0] + 31) / 32);
-        words += B.WX * (unsigned)B.gn[1] * (unsigned)B.gn[2];
-        ctiles += B.WX * (unsigned)((B.gn[1] + TY - 1) / TY) * (unsigned)((B.gn[2] + TZ - 1) / TZ);
+        words64 += ((unsigned long long)B.WX * (unsigned)B.gn[1] * (unsigned)B.gn[2] + mcw::SUB - 1) / mcw::SUB * mcw::SUB;
     }
+    if (words64 >= 0xffffffffULL - mcw::SUB) {
+        n2m_set_error("atlas grids too large");
+        return N2M_ERR_TOO_LARGE;
+    }
+    const unsigned words = (unsigned)words64, nsub = words / mcw::SUB;
     CK(cudaMemcpyAsync(db, boxes.data(), nb * sizeof(ABox), cudaMemcpyHostToDevice, s));
-    CKS(w.words.ensure(((size_t)words + 1) * sizeof(uint4)));
-    CKS(w.counts.ensure(((size_t)words + 1) * sizeof(uint4)));
-    CKS(w.active.ensure(((size_t)words + 2) * sizeof(unsigned)));
-    CKS(w.tot.ensure(sizeof(uint4) + (size_t)(nb + 1) * sizeof(BoxOff)));
-    unsigned *act = w.active.as<unsigned>();
-    CK(cudaMemsetAsync(act + words, 0, sizeof(unsigned), s));
+    CKS(w.tot.ensure(sizeof(MarchOut) + (size_t)(nb + 1) * sizeof(BoxOff)));
+    MarchOut *dm = w.tot.as<MarchOut>();
+    BoxOff *dboff = (BoxOff *)(dm + 1);
     const bool classic = o.cubes == N2M_CUBES_CLASSIC_TABLE;
-    if (ctiles) n2m_launch(k_a_count, pgrid(ctiles, 4), 256, 0, s, v, db, nb, ctiles, q + qi++, ar, classic,
-                           w.words.as<uint4>(), w.counts.as<uint4>(), act, act + words);
-    CKL();
-    uint4 *dtot = w.tot.as<uint4>();
-    BoxOff *dboff = (BoxOff *)(dtot + 1);
-    CKS(scan_uint4(w.counts.as<uint4>(), words, dtot, sw, s));
-    uint4 tot;
-    CK(cudaMemcpyAsync(&tot, dtot, sizeof(uint4), cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
-    n2m_launch(k_a_boxoff, (nb + 128) / 128, 128, 0, s, db, nb, w.counts.as<uint4>(), tot, dboff);
-    std::vector<BoxOff> boff(nb + 1);
-    CK(cudaMemcpyAsync(boff.data(), dboff, (nb + 1) * sizeof(BoxOff), cudaMemcpyDeviceToHost, s));
-    const unsigned nv = tot.x + tot.z, nt = tot.y, nact = *(&tot.w);
+    std::vector<BoxOff> boff(nb + 1, BoxOff{0u, 0u, 0u});
+    mcw::Out mo{};
+    Policy pol{v, db, nb, nullptr, seg.post, ar, classic, nullptr, nullptr, nullptr, &dm->ncand, &dm->nccand, 0, nullptr};
+    CK(cudaMemsetAsync(dm, 0, sizeof(uint4) + 4 * sizeof(unsigned), s));
+    if (words) {
+        CKS(mcw::prepare(w.mc, words, &dm->tot, mo));
+        CKS(w.mc.signs.ensure((size_t)words * sizeof(unsigned)));
+        CKS(w.subbox.ensure((size_t)nsub * sizeof(unsigned)));
+        unsigned *signs = w.mc.signs.as<unsigned>();
+        pol.subbox = w.subbox.as<unsigned>();
+        n2m_launch(k_a_signs, std::max(1u, std::min((nsub + 7) / 8, 152u * 16u)), 256, 0, s, v, db, nb, nsub, seg.post.S, signs,
+                   w.subbox.as<unsigned>());
+        CKS(mcw::count_signs(pol, signs, mo, mcw::Marks{nullptr, 0, 0, 0, 0}, s));
+        CKS(mcw::count_values(pol, signs, w.mc, mo, !classic, s));
+        n2m_launch(k_a_boxoff, (nb + 128) / 128, 128, 0, s, db, nb, mo, dboff);
+        CKL();
+        CK(cudaMemcpyAsync(boff.data(), dboff, (nb + 1) * sizeof(BoxOff), cudaMemcpyDeviceToHost, s));
+        CK(cudaStreamSynchronize(s));
+    }
+    const unsigned nv = boff[nb].e + boff[nb].c, nt = boff[nb].t;
     CKS(w.pts.ensure((size_t)std::max(nv, 1u) * sizeof(vec3d)));
     CKS(w.tris.ensure((size_t)std::max(nt, 1u) * sizeof(vec3i)));
     const int cap = (int)std::min<unsigned>(nv / 16 + 65536, 1u << 26);
-    CKS(w.cand.ensure((size_t)2 * cap * sizeof(int) + 2 * sizeof(unsigned)));
+    CKS(w.cand.ensure((size_t)2 * cap * sizeof(int)));
     int *cand = w.cand.as<int>();
-    unsigned *ncand = (unsigned *)(cand + 2 * cap);
-    CK(cudaMemsetAsync(ncand, 0, 2 * sizeof(unsigned), s));
-    if (nact) n2m_launch(k_a_emit, pgrid((nact + 7) / 8, 16), 256, 0, s, v, db, dboff, nb, w.words.as<uint4>(),
-                         w.counts.as<uint4>(), act, nact, ar, classic, w.pts.as<vec3d>(), w.tris.as<vec3i>(),
-                         cand, ncand, cand + cap, ncand + 1, cap);
-    CKL();
+    unsigned *ncand = &dm->ncand, *near = nullptr;
+    if (std::max({dim[0], dim[1], dim[2]}) < 1 << 22) {   // NEAR_CORNER
+        CKS(dw.near.ensure(((size_t)nv + 31) / 32 * sizeof(unsigned)));
+        near = dw.near.as<unsigned>();
+        CK(cudaMemsetAsync(near, 0, ((size_t)nv + 31) / 32 * sizeof(unsigned), s));
+    }
+    if (nv || nt) {
+        pol.pts = w.pts.as<vec3d>();
+        pol.cand = cand;
+        pol.ccand = cand + cap;
+        pol.cap = cap;
+        pol.near = near;
+        CKS(mcw::emit(pol, w.mc.signs.as<unsigned>(), w.mc, mo, MeshRoom{nv, nt}, w.tris.as<vec3i>(), s));
+    }
     unsigned nc[2];
     CK(cudaMemcpyAsync(nc, ncand, 2 * sizeof(unsigned), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
@@ -1420,7 +1486,7 @@ n2m_status atlas_batched(const short *d_lab, const int dim[3], const n2m_options
     CKS(w.ranges.ensure((size_t)(4 * (nb + 1) + 2) * sizeof(unsigned)));
     unsigned *dts = w.ranges.as<unsigned>(), *dkept = dts + (nb + 1), *dvs = dkept + (nb + 1), *dntf = dvs + (nb + 1);
     CK(cudaMemcpyAsync(dts, ts.data(), (nb + 1) * sizeof(unsigned), cudaMemcpyHostToDevice, s));
-    CKS(mesh_remove_degenerate(pts, w.tris.as<vec3i>(), (int)nt, map, nullptr, w.tris2.as<vec3i>(), dntf, dw, s));
+    CKS(mesh_remove_degenerate(pts, w.tris.as<vec3i>(), (int)nt, map, near, w.tris2.as<vec3i>(), dntf, dw, s));
     if (nt) n2m_launch(k_a_kept, (nb + 128) / 128, 128, 0, s, dts, nb, nt, dw.bits.as<unsigned>(), dw.tiles.as<unsigned>(), dntf,
                        dkept);
     else CK(cudaMemsetAsync(dkept, 0, (nb + 1) * sizeof(unsigned), s));

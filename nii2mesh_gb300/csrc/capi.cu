@@ -281,8 +281,8 @@ extern "C" void n2m_context_destroy(n2m_context *c) {
     if (!c) return;
     cudaSetDevice(c->device);
     cudaStreamSynchronize(c->stream);
-    DevBuf *bufs[] = {&c->aw.cnt, &c->aw.bb, &c->aw.boxes, &c->aw.queue, &c->aw.arena, &c->aw.mask, &c->aw.keep,
-                      &c->aw.lab, &c->aw.edge, &c->aw.ucnt, &c->aw.words, &c->aw.counts, &c->aw.active, &c->aw.tot,
+    DevBuf *bufs[] = {&c->aw.cnt, &c->aw.bb, &c->aw.boxes, &c->aw.arena, &c->aw.mask, &c->aw.keep, &c->aw.fill, &c->aw.shell, &c->aw.wbox, &c->aw.list, &c->aw.wlist,
+                      &c->aw.lab, &c->aw.edge, &c->aw.ucnt, &c->aw.mc.signs, &c->aw.mc.words, &c->aw.mc.act, &c->aw.mc.cnt, &c->aw.mc.sub, &c->aw.subbox, &c->aw.tot,
                       &c->aw.pts, &c->aw.pts2, &c->aw.tris, &c->aw.tris2, &c->aw.cand, &c->aw.gath, &c->aw.weld,
                       &c->aw.ranges, &c->alab, &c->lpts, &c->ltris, &c->gA, &c->gB, &c->gs, &c->gtmp, &c->in, &c->raw, &c->vol, &c->stmp, &c->stats, &c->march, &c->cand, &c->ocq, &c->pts_raw,
                       &c->tris_raw, &c->pts, &c->tris, &c->ntf, &c->weld, &c->gath, &c->hmesh,
@@ -294,7 +294,6 @@ extern "C" void n2m_context_destroy(n2m_context *c) {
                       &c->wr.mt, &c->wr.mp, &c->wr.pack, &c->wr.pack2, &c->wr.lens, &c->wr.flag, &c->wr.out};
     for (DevBuf *b : bufs) b->release();
     deflate_release(c->wr.df);
-    if (c->aw.exec) cudaGraphExecDestroy((cudaGraphExec_t)c->aw.exec);
     if (c->pinned) cudaFreeHost(c->pinned);
     if (c->wr.host) cudaFreeHost(c->wr.host);
     for (int i = 0; i < 8; i++)

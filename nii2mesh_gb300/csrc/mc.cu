@@ -194,59 +194,6 @@ __device__ __forceinline__ float ival(const GV &g, const float *p) {
     return fabsf(v) < N2M_FLT_EPS ? N2M_FLT_EPS : v;
 }
 
-// exact float -> double by assembling the bits in integer registers (a
-// conversion instruction would issue on the pipe this part shares with FP64;
-// a predicated one still issues)
-__device__ __noinline__ double f2d_rare(float f) {   // zero, subnormal, Inf, NaN
-    const unsigned u = __float_as_uint(f), e = (u >> 23) & 0xffu, m = u & 0x7fffffu;
-    const unsigned long long sign = (unsigned long long)(u & 0x80000000u) << 32;
-    unsigned long long de = 0, dm = 0;
-    if (e == 0xffu) {
-        de = 0x7ffull;
-        dm = (unsigned long long)m << 29;
-    } else if (m != 0u) {           // m * 2^-149, leading bit p
-        const int p = 31 - __clz((int)m);
-        de = (unsigned long long)(p - 149 + 1023);
-        dm = ((unsigned long long)m << (52 - p)) & 0xfffffffffffffull;
-    }
-    return __longlong_as_double((long long)(sign | (de << 52) | dm));
-}
-__device__ __forceinline__ double f2d(float f) {
-    const unsigned u = __float_as_uint(f);
-    if (((u >> 23) & 0xffu) - 1u < 0xfeu)
-        return __hiloint2double((int)((u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + 0x38000000u)), (int)(u << 29));
-    return u == 0u ? 0.0 : f2d_rare(f);
-}
-
-// exact float of 0 <= v < 2^23 by bit assembly (no I2F conversion)
-__device__ __forceinline__ float i2f_small(int v) { return __int_as_float(0x4B000000 | v) - 8388608.f; }
-
-__device__ __forceinline__ void add_cand(int *cand, unsigned *n, int cap, int id) {
-    const unsigned k = atomicAdd(n, 1u);
-    if (k < (unsigned)cap) cand[k] = id;
-}
-
-// c-vertex of a cube: mean of its crossing edge vertices (src/MarchingCubes.c:1029-1082)
-__device__ __noinline__ void emit_cvertex(const float *c, int x, int y, int z, float flo0, float flo1, float flo2,
-                                          int v12, vec3d *pts, int *ccand, unsigned *nccand, int cap) {
-    float n = 0.f, sx = 0.f, sy = 0.f, sz = 0.f;
-    for (int e = 0; e < 12; e++) {
-        const int own = k_edge[e][0], ax = k_edge[e][1], ca = k_edge[e][2], cbn = k_edge[e][3];
-        if ((c[ca] > 0.f) == (c[cbn] > 0.f)) continue;
-        const float u = edge_u(c[ca], c[cbn]);
-        float px = (float)(x + ((own ^ (own >> 1)) & 1)), py = (float)(y + ((own >> 1) & 1)), pz = (float)(z + ((own >> 2) & 1));
-        if (ax == 0) px = __fadd_rn(px, u);
-        else if (ax == 1) py = __fadd_rn(py, u);
-        else pz = __fadd_rn(pz, u);
-        n = __fadd_rn(n, 1.f);
-        sx = __fadd_rn(sx, px); sy = __fadd_rn(sy, py); sz = __fadd_rn(sz, pz);
-    }
-    if (n > 0.f) { sx = __fdiv_rn(sx, n); sy = __fdiv_rn(sy, n); sz = __fdiv_rn(sz, n); }
-    const float X = __fadd_rn(sx, flo0), Y = __fadd_rn(sy, flo1), Z = __fadd_rn(sz, flo2);
-    pts[v12] = {f2d(X), f2d(Y), f2d(Z)};
-    if (fminf(frac_dist(X), fminf(frac_dist(Y), frac_dist(Z))) < 1.5e-5f) add_cand(ccand, nccand, cap, v12);
-}
-
 // corner values of cube (x, y, z), by gval's rules
 __device__ __noinline__ void cube_values(const GV &g, int x, int y, int z, float *c) {
     const int vx = g.lo0 + x, vy = g.lo1 + y, vz = g.lo2 + z;
@@ -329,18 +276,7 @@ struct Policy {
         return Edge{gval(g, x, y, z), gval(g, x + (ax == 0), y + (ax == 1), z + (ax == 2))};
     }
     __device__ __forceinline__ vec3d vertex(const Edge &c, int x, int y, int z, int ax, int id) const {
-        const float u = edge_u(c.c0, c.c1), flo0 = (float)g.lo0, flo1 = (float)g.lo1, flo2 = (float)g.lo2;
-        const float fx = i2f_small(x), fy = i2f_small(y), fz = i2f_small(z);
-        float X = __fadd_rn(fx, flo0), Y = __fadd_rn(fy, flo1), Z = __fadd_rn(fz, flo2), axv;
-        if (ax == 0) axv = X = __fadd_rn(__fadd_rn(fx, u), flo0);
-        else if (ax == 1) axv = Y = __fadd_rn(__fadd_rn(fy, u), flo1);
-        else axv = Z = __fadd_rn(__fadd_rn(fz, u), flo2);
-        const float d = frac_dist(axv);
-        if (!(d >= NEAR_CORNER)) {
-            mark_near(near, id);
-            if (d < 1.5e-5f) add_cand(cand, ncand, cap, id);
-        }
-        return {f2d(X), f2d(Y), f2d(Z)};
+        return edge_vertex(c.c0, c.c1, x, y, z, ax, (float)g.lo0, (float)g.lo1, (float)g.lo2, id, cand, ncand, cap, near);
     }
 };
 

@@ -192,7 +192,6 @@ void stats_init_host(VolStats *h);
 struct ScanWork {
     DevBuf part;
 };
-n2m_status scan_uint4(uint4 *d, size_t n, uint4 *d_total, ScanWork &w, cudaStream_t s);
 n2m_status scan_u32(unsigned *d, size_t n, unsigned *d_total, ScanWork &w, cudaStream_t s);
 
 // label.cu
@@ -383,12 +382,9 @@ n2m_status mesh_apply_sform(vec3d *d_pts, vec3i *d_tris, int np, int nt, const f
 // atlas.cu
 #include <vector>
 struct AtlasWork {
-    DevBuf cnt, bb, boxes, queue, arena, mask, keep, lab, edge, ucnt, words, counts, active, tot, pts, pts2, tris, tris2,
+    McWork mc;
+    DevBuf cnt, bb, boxes, arena, mask, keep, fill, shell, wbox, list, wlist, lab, edge, ucnt, subbox, tot, pts, pts2, tris, tris2,
         cand, gath, weld, ranges;
-    void *exec = nullptr;            // cudaGraphExec_t of the smoothing + clustering segment
-    bool tuned = false;              // autotuned work-item size and grid width
-    unsigned chunk = 1024, per_sm = 8;
-    float tuned_ms = 0.f;
 };
 n2m_status atlas_hist(const short *d_lab, const int dim[3], AtlasWork &w, cudaStream_t s, int *maxlab,
                       std::vector<unsigned> &cnt, std::vector<int> &bb);

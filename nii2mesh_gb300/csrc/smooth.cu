@@ -8,8 +8,8 @@
 // decides ~97 % of the taps, the rest are batched per warp and recomputed in
 // FP64 by full warps; the z pass also reduces the range (min/max), the count
 // of non-finite voxels and the bbox of voxels >= iso.  Traffic: 8 B per voxel
-// per pass, three passes.  (The batched atlas smooths its sub-boxes with the
-// fused column routine of smooth_core.cuh instead.)
+// per pass, three passes.  (The batched atlas smooths its binary
+// sub-boxes from their bits instead, atlas.cu.)
 #include <float.h>
 #include <math.h>
 #include <stddef.h>
