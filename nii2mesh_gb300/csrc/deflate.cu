@@ -37,7 +37,11 @@
 namespace {
 constexpr int DF_CHUNK_MIN = 16384, DF_CHUNK_MAX = 32768;   // input bytes per block (chosen per call)
 constexpr int DF_HBITS = 10, DF_HSIZE = 1 << DF_HBITS;   // hash buckets per chunk, two positions each
-constexpr int LZ_WARPS = 16;                     // chunks per CTA of k_lz (4.6 KB of shared memory each: 48 warps / SM)
+// Chunks per CTA of k_lz (4.6 KB of shared memory each).  A CTA stays until its slowest chunk is done, and few large
+// CTAs fill the SMs unevenly: a 92 MB mesh took 1934 us with 16, 1836 with 8, 1802 with 4, and with fewer
+// instructions per tile 1778, 1711 and 1744.
+constexpr int LZ_WARPS = 8;
+constexpr int LZ_SLOTS = 48;                     // chunks per SM that the chunk size aims at
 constexpr int DF_WARPS = 4;                      // chunks per CTA of k_huff
 constexpr int BITS_WARPS = 8;                    // chunks per CTA of k_bits
 constexpr int DF_MAXLEN = 258;
@@ -54,21 +58,19 @@ struct DfInfo {
     unsigned len;        // input bytes of the chunk
 };
 
-__device__ __forceinline__ unsigned load4(const unsigned *__restrict__ w, long long p) {
-    const long long i = p >> 2;
-    const unsigned sh = (unsigned)(p & 3) * 8u;
-    const unsigned lo = __ldg(w + i);
-    if (!sh) return lo;
-    return __funnelshift_r(lo, __ldg(w + i + 1), sh);
-}
-
-// length of the match of p against c (first 4 bytes known equal), at most maxl
-__device__ __forceinline__ int match_len(const unsigned *__restrict__ src, long long p, long long c, int maxl) {
-    int l = 4;
-    while (l < maxl) {
-        const unsigned x = load4(src, p + l) ^ load4(src, c + l);
+// Length (0, or 4 .. maxl) of the match of byte p against byte c < p, w4 the 4 bytes at p and next the word after the one
+// that holds p.  One word of each side per step, the other half of a byte-shifted word kept from the step before.
+__device__ __forceinline__ int match_len(const unsigned *__restrict__ src, int p, int c, unsigned w4, unsigned next, int maxl) {
+    const unsigned *__restrict__ a = src + (p >> 2) + 2, *__restrict__ b = src + (c >> 2) + 2;
+    const unsigned sa = 8u * (p & 3), sb = 8u * (c & 3);
+    unsigned lb = __ldg(b - 1), la = next;
+    if (__funnelshift_r(__ldg(b - 2), lb, sb) != w4) return 0;
+    for (int l = 4; l < maxl; l += 4) {
+        const unsigned ha = __ldg(a++), hb = __ldg(b++);
+        const unsigned x = __funnelshift_r(la, ha, sa) ^ __funnelshift_r(lb, hb, sb);
         if (x) return min(l + ((__ffs(x) - 1) >> 3), maxl);
-        l += 4;
+        la = ha;
+        lb = hb;
     }
     return maxl;
 }
@@ -116,10 +118,15 @@ __device__ __forceinline__ unsigned len_extra_bits(unsigned sym) { return (sym <
 __device__ __forceinline__ unsigned dist_extra_bits(unsigned d) { return d < 4 ? 0u : d / 2 - 1; }
 
 // ---- match finding and parsing --------------------------------------------------------------
+// Bound by the latency of a chunk's tile after tile (memory at 26 %, issue at 42 %): the
+// compares keep the half word that the next step needs, and the parse takes one step per match.
+// 92 MB mesh: 1344 us with two loads per side and compare and a step per deferred match,
+// 1131 now.  Looking a tile ahead (2009 us for the whole stream), first bytes from other
+// lanes and long matches by the warp (2288) cost more instructions than they hid.
 // src must have n + 8 readable bytes (4-byte aligned); chunks of ch bytes; tokens: ch per chunk.
 // Hash bucket: the chunk offsets of the two most recent positions with that hash
 // (newest in the low half, 0xFFFF = none).  Histogram: 16-bit counts in pairs.
-__global__ void __launch_bounds__(32 * LZ_WARPS, 3) k_lz(const unsigned *__restrict__ src, long long n, int nchunks,
+__global__ void __launch_bounds__(32 * LZ_WARPS, LZ_SLOTS / LZ_WARPS) k_lz(const unsigned *__restrict__ src, long long n, int nchunks,
                                                          int ch, unsigned *__restrict__ tokens,
                                                          DfInfo *__restrict__ info, unsigned *__restrict__ ghist) {
     grid_wait();
@@ -135,13 +142,15 @@ __global__ void __launch_bounds__(32 * LZ_WARPS, 3) k_lz(const unsigned *__restr
     __syncwarp();
     const long long c0 = (long long)chunk * ch;
     const int len_c = (int)min((long long)ch, n - c0);
+    const unsigned *__restrict__ csrc = src + (c0 >> 2);   // chunks begin at multiples of 4096 bytes
     unsigned *tok = tokens + (size_t)chunk * ch;
     const unsigned lt = (1u << lane) - 1;
     int next = 0, ntk = 0;
     for (int t0 = 0; t0 < len_c; t0 += 32) {
         const int o = t0 + lane;
         const bool in = o < len_c, valid = o + 4 <= len_c;
-        const unsigned w4 = in ? load4(src, c0 + o) : 0u;
+        const unsigned own = in ? __ldg(csrc + (o >> 2)) : 0u, after = in ? __ldg(csrc + (o >> 2) + 1) : 0u;
+        const unsigned w4 = __funnelshift_r(own, after, 8u * (o & 3));
         const unsigned h = valid ? (w4 * 2654435761u) >> (32 - DF_HBITS) : (0x10000u | (unsigned)lane);   // lanes
         // without 4 bytes get keys no hash can take
         const unsigned same = __match_any_sync(0xffffffffu, h);
@@ -169,41 +178,36 @@ __global__ void __launch_bounds__(32 * LZ_WARPS, 3) k_lz(const unsigned *__restr
         int mlen = 0, mdist = 0;
         if (valid) {
             const int maxl = min(DF_MAXLEN, len_c - o);
-            if (c1 >= 0 && load4(src, c0 + c1) == w4) {
-                mlen = match_len(src, c0 + o, c0 + c1, maxl);
+            if (c1 >= 0) {
+                mlen = match_len(csrc, o, c1, w4, after, maxl);
                 mdist = o - c1;
             }
-            if (c2 >= 0 && mlen < maxl && load4(src, c0 + c2) == w4) {
-                const int l = match_len(src, c0 + o, c0 + c2, maxl);
+            if (c2 >= 0 && mlen < maxl) {
+                const int l = match_len(csrc, o, c2, w4, after, maxl);
                 if (l > mlen) {
                     mlen = l;
                     mdist = o - c2;
                 }
             }
         }
-        // greedy parse with one-step lazy evaluation over the match starts of this tile
-        const unsigned mm = __ballot_sync(0xffffffffu, mlen >= 4);
+        // greedy parse with one-step lazy evaluation over the match starts of this tile: a match
+        // gives way to a longer one that starts at the next byte (which is a match start too), so from any
+        // position the first start that does not give way is taken
+        const int follow = __shfl_down_sync(0xffffffffu, mlen, 1);
+        const unsigned starts = __ballot_sync(0xffffffffu, mlen >= 4 && !(lane < 31 && follow > mlen));
         const unsigned tmask = (len_c - t0 >= 32) ? 0xffffffffu : ((1u << (len_c - t0)) - 1);
-        unsigned lit = 0, mat = 0;
         int pos = next - t0;
+        unsigned mat = 0, lit = pos < 32 ? 0xffffffffu << pos : 0u;
         while (pos < 32) {
-            const unsigned rest = mm & (0xffffffffu << pos);
+            const unsigned rest = starts & (0xffffffffu << pos);
             if (!rest) {
-                lit |= 0xffffffffu << pos;
                 pos = 32;
                 break;
             }
             const int q = __ffs(rest) - 1;
-            lit |= ((1u << q) - 1) & (0xffffffffu << pos);
-            const int lq = __shfl_sync(0xffffffffu, mlen, q);
-            const int lq1 = __shfl_sync(0xffffffffu, mlen, (q + 1) & 31);
-            if (q < 31 && lq1 > lq) {
-                lit |= 1u << q;
-                pos = q + 1;
-                continue;
-            }
             mat |= 1u << q;
-            pos = q + lq;
+            pos = q + __shfl_sync(0xffffffffu, mlen, q);
+            lit &= ~(0xffffffffu << q) | (pos < 32 ? 0xffffffffu << pos : 0u);   // without [q, pos)
         }
         next = t0 + pos;
         lit &= tmask;
@@ -251,18 +255,16 @@ struct HuffScratch {
     unsigned hdr[DF_HDR_WORDS];
 };
 
-// warp-wide bitonic sort of keys[0, n), n a power of two
+// warp-wide bitonic sort of keys[0, n), n a power of two from 32
 __device__ void warp_sort(unsigned *keys, int n, int lane) {
     for (int k = 2; k <= n; k <<= 1)
         for (int j = k >> 1; j > 0; j >>= 1) {
-            for (int i = lane; i < n; i += 32) {
-                const int l = i ^ j;
-                if (l > i) {
-                    const unsigned a = keys[i], b = keys[l];
-                    if ((a > b) == ((i & k) == 0)) {
-                        keys[i] = b;
-                        keys[l] = a;
-                    }
+            for (int t = lane; t < n / 2; t += 32) {   // pairs
+                const int i = (t & ~(j - 1)) << 1 | (t & (j - 1)), l = i | j;
+                const unsigned a = keys[i], b = keys[l];
+                if ((a > b) == ((i & k) == 0)) {
+                    keys[i] = b;
+                    keys[l] = a;
                 }
             }
             __syncwarp();
@@ -271,59 +273,79 @@ __device__ void warp_sort(unsigned *keys, int n, int lane) {
 
 // Huffman code lengths (<= limit) of f[0, nsym) into L[0, nsym); at least two
 // symbols of f must be nonzero.  Frequencies are halved until the tree fits.
+// A chain of dependent shared-memory accesses sets the time: only the used symbols are
+// sorted, the merge keeps the next two of either queue in registers, and depths are
+// found 32 nodes at a time (one lane walking keys, tree and depths: k_huff 199 us for a
+// 92 MB mesh, 147 now).
 __device__ void build_lengths(HuffScratch &S, const unsigned *f, int nsym, int limit, unsigned char *L, int lane) {
-    const int padn = nsym <= 32 ? 32 : 512;
+    constexpr unsigned NONE = 0xFFFFFFFFu;
     for (int shift = 0;; shift++) {
-        for (int i = lane; i < padn; i += 32) {
-            unsigned k = 0xFFFFFFFFu;
-            if (i < nsym && f[i]) k = ((shift ? ((f[i] >> shift) | 1u) : f[i]) << 9) | (unsigned)i;
-            S.keys[i] = k;
+        int m = 0;   // used symbols
+        for (int i0 = 0; i0 < nsym; i0 += 32) {
+            const int i = i0 + lane;
+            const unsigned fi = i < nsym ? f[i] : 0u, used = __ballot_sync(0xffffffffu, fi != 0u);
+            if (fi) S.keys[m + __popc(used & ((1u << lane) - 1u))] = ((shift ? ((fi >> shift) | 1u) : fi) << 9) | (unsigned)i;
+            m += __popc(used);
         }
+        int n = 32;
+        while (n < m) n <<= 1;
+        for (int i = m + lane; i < n; i += 32) S.keys[i] = NONE;
         __syncwarp();
-        warp_sort(S.keys, padn, lane);
-        int ok = 1, m = 0;
+        warp_sort(S.keys, n, lane);
+        const int root = 2 * m - 2;
         if (lane == 0) {
-            while (m < padn && S.keys[m] != 0xFFFFFFFFu) m++;
-            // two queues: sorted leaves 0..m-1 and internal nodes m.. in creation order
-            int li = 0, ii = m, ni = m;
-            for (int k = 0; k < m - 1; k++) {
-                int ab[2];
-                unsigned wab[2];
+            // two queues: sorted leaves 0..m-1 and internal nodes m.. in creation order, the heads and the ones after in registers
+            int li = 0, ii = m;
+            unsigned l0 = S.keys[0] >> 9, l1 = m > 1 ? S.keys[1] >> 9 : NONE, w0 = NONE, w1 = NONE;
+            for (int ni = m; ni <= root; ni++) {
+                unsigned sum = 0;
+#pragma unroll
                 for (int t = 0; t < 2; t++) {
-                    if (li < m && (ii >= ni || (S.keys[li] >> 9) <= S.w[ii])) {
-                        ab[t] = li;
-                        wab[t] = S.keys[li] >> 9;
-                        li++;
+                    if (li < m && l0 <= w0) {
+                        sum += l0;
+                        S.par[li++] = (unsigned short)ni;
+                        l0 = l1;
+                        l1 = li + 1 < m ? S.keys[li + 1] >> 9 : NONE;
                     } else {
-                        ab[t] = ii;
-                        wab[t] = S.w[ii];
-                        ii++;
+                        sum += w0;
+                        S.par[ii++] = (unsigned short)ni;
+                        w0 = w1;
+                        w1 = ii + 1 < ni ? S.w[ii + 1] : NONE;
                     }
                 }
-                S.w[ni] = wab[0] + wab[1];
-                S.par[ab[0]] = (unsigned short)ni;
-                S.par[ab[1]] = (unsigned short)ni;
-                ni++;
+                S.w[ni] = sum;
+                if (ii == ni) w0 = sum;
+                else if (ii + 1 == ni) w1 = sum;
             }
-            const int root = 2 * m - 2;
             S.dep[root] = 0;
-            int maxd = 0;
-            for (int j = root - 1; j >= 0; j--) {
-                S.dep[j] = S.dep[S.par[j]] + 1;
-                if (j < m && S.dep[j] > maxd) maxd = S.dep[j];
-            }
-            ok = maxd <= limit;
         }
-        ok = __shfl_sync(0xffffffffu, ok, 0);
-        m = __shfl_sync(0xffffffffu, m, 0);
         __syncwarp();
-        if (ok) {
+        int maxd = 0;
+        for (int top = root - 1; top >= 0; top -= 32) {   // a node's parent comes after it
+            const int j = top - lane, p = j >= 0 ? S.par[j] : root;
+            int d = -1;
+            for (unsigned known = 0; known != 0xffffffffu; known = __ballot_sync(0xffffffffu, d >= 0)) {
+                const int from = __shfl_sync(0xffffffffu, d, (top - p) & 31);   // a parent among these nodes
+                if (d < 0) {
+                    if (j < 0) d = 0;
+                    else if (p > top) d = S.dep[p] + 1;
+                    else if (from >= 0) d = from + 1;
+                }
+            }
+            if (j >= 0) {
+                S.dep[j] = (unsigned char)d;
+                if (j < m) maxd = max(maxd, d);
+            }
+            __syncwarp();
+        }
+        if (__reduce_max_sync(0xffffffffu, maxd) <= limit) {
             for (int i = lane; i < nsym; i += 32) L[i] = 0;
             __syncwarp();
             for (int i = lane; i < m; i += 32) L[S.keys[i] & 511u] = S.dep[i];
             __syncwarp();
             return;
         }
+        __syncwarp();   // the keys are written again
     }
 }
 
@@ -812,8 +834,7 @@ n2m_status deflate_device(const void *d_src, size_t n, int container, DeflateWor
         CK(cudaGetDevice(&dev));
         CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
         CK(cudaFuncSetAttribute(k_lz, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_lz, 32 * LZ_WARPS, smem));
-        w.lz_slots = std::max(1, sms * per_sm * LZ_WARPS);
+        w.lz_slots = sms * LZ_SLOTS;
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_huff, 32 * DF_WARPS, 0));
         w.huff_slots = std::max(1, sms * per_sm * DF_WARPS);
         CK(cudaStreamCreateWithFlags((cudaStream_t *)&w.side, cudaStreamNonBlocking));
