@@ -290,7 +290,7 @@ extern "C" void n2m_context_destroy(n2m_context *c) {
                       &c->lab.lab, &c->lab.mask, &c->lab.keep, &c->lab.cnt, &c->lab.edge, &c->lab.rc, &c->lab.misc, &c->lab.list, &c->lab.wlist, &c->lab.cs, &c->lab.filled, &c->lab.shell,
                       &c->deg.bits, &c->deg.tiles, &c->deg.rank, &c->deg.near, &c->hc.zero, &c->hc.adj, &c->hc.meta, &c->hc.P, &c->hc.Q,
                       &c->hc.B, &c->hc.Lo, &c->th.buf, &c->th.table,
-                      &c->stmp2, &c->lubits, &c->od.st, &c->od.unc, &c->od.cmin, &c->od.cmax, &c->od.range, &c->od.need, &c->od.list, &c->od.lcnt, &c->od.vsign,
+                      &c->stmp2, &c->lubits, &c->od.st, &c->od.unc, &c->od.cmin, &c->od.cmax, &c->od.range, &c->od.need, &c->od.list, &c->od.lcnt, &c->od.vsign, &c->od.pad,
                       &c->wr.mt, &c->wr.mp, &c->wr.pack, &c->wr.pack2, &c->wr.lens, &c->wr.flag, &c->wr.out};
     for (DevBuf *b : bufs) b->release();
     deflate_release(c->wr.df);
@@ -624,7 +624,7 @@ n2m_status prepare(n2m_context *c, const float *d_src, const int dim[3], const n
     // Otherwise the exact three passes; a volume arriving from host memory in slabs is
     // smoothed while it arrives that way (the on-demand repair could only start after
     // the last slab)
-    bool od = smooth && (!label || o.only_largest) && !c->stage.host && od_eligible(d_src, nx, ny, nz);
+    bool od = smooth && (!label || o.only_largest) && !c->stage.host && od_eligible(nx, ny, nz);
     OdStats hod;
     VolStats s0, s1;
     // The labelling needs the isolevel only, so it is queued before the statistics that

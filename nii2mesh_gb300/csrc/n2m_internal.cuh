@@ -148,6 +148,7 @@ struct OdWork {
     // od_resolve's at_or_above, the value is >= iso (the complement of oldcubes'
     // sign); exact for every voxel once od_resolve has run
     DevBuf vsign;
+    DevBuf pad;   // the input with rows of a multiple of 16 bytes
     unsigned cap = 0;
 };
 // What meshify's labelling does to each voxel (src/meshify.c:330-342), for the values
@@ -173,8 +174,8 @@ struct OdRepair {
 __host__ __device__ __forceinline__ size_t od_vsign_word(unsigned x, unsigned y, unsigned z, unsigned wv, unsigned nys) {
     return (((size_t)z * nys + (y >> 3)) * wv + (x >> 5)) * 8u + (y & 7u);
 }
-// whether the on-demand path applies: rows a multiple of 16 bytes (TMA tiles), fewer than 2^32 voxels
-bool od_eligible(const float *in, int nx, int ny, int nz);
+// whether the on-demand path applies: at least 5 voxels along each axis, fewer than 2^32
+bool od_eligible(int nx, int ny, int nz);
 n2m_status od_approx(const float *in, float *out, int nx, int ny, int nz, float iso, OdWork &w, cudaStream_t s);
 n2m_status od_resolve(const float *in, float *out, int nx, int ny, int nz, float iso, OdWork &w, cudaStream_t s,
                       bool at_or_above = false);
