@@ -28,58 +28,86 @@ struct ThRange {
     unsigned long long pad;
 };
 
-// (int)round(x) for the bin of a finite product; NaN (0 * inf on a constant
-// volume) goes to bin 0, like the reference's clamp does on every platform
-__device__ __forceinline__ long long bin_of(float x) {
-    if (!(x == x)) return 0;
-    const float r = roundf(x);
-    if (r >= 9.0e18f) return 9000000000000000000ll;
-    if (r <= -9.0e18f) return -9000000000000000000ll;
-    return (long long)r;
+// f(value, is there one) for every voxel, by 16-byte loads where the volume's alignment allows,
+// four in flight; a warp's lanes call f together
+template <class F> __device__ __forceinline__ void each_voxel(const float *__restrict__ v, long long n, F f) {
+    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x, step = (long long)gridDim.x * blockDim.x;
+    const long long n4 = ((size_t)v & 15) ? 0 : n / 4;
+    const float4 *v4 = (const float4 *)v;
+    for (long long i = t; (i & ~31ll) < n4; i += 4 * step) {
+        float4 q[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) q[u] = i + u * step < n4 ? __ldg(v4 + i + u * step) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const bool in = i + u * step < n4;
+            f(q[u].x, in); f(q[u].y, in); f(q[u].z, in); f(q[u].w, in);
+        }
+    }
+    for (long long i = 4 * n4 + t; 4 * n4 + ((i - 4 * n4) & ~31ll) < n; i += step) f(i < n ? __ldg(v + i) : 0.f, i < n);
 }
 
+// Bound by the blocks' atomics on the one result (7 M voxels: 20 us with a set per warp and
+// 4-byte loads, 9.5 with one per block where it still changes something).
 __global__ void __launch_bounds__(256) k_th_range(const float *__restrict__ v, long long n, ThRange *out) {
     grid_wait();
     float mn = INFINITY, mx = -INFINITY;
-    unsigned long long nn = 0;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const float x = __ldg(v + i);
-        if (x != x) { nn++; continue; }
-        mn = fminf(mn, x);
+    unsigned nn = 0;   // at most 2^31 voxels
+    each_voxel(v, n, [&](float x, bool in) {
+        if (!in) return;
+        if (x != x) nn++;
+        mn = fminf(mn, x);   // a NaN is the other operand's
         mx = fmaxf(mx, x);
+    });
+    __shared__ int lo, hi;
+    __shared__ unsigned nan;
+    if (threadIdx.x == 0) {
+        lo = INT_MAX;
+        hi = INT_MIN;
+        nan = 0;
     }
-    for (int o = 16; o; o >>= 1) {
-        mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
-        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        nn += __shfl_xor_sync(0xffffffffu, nn, o);
-    }
+    __syncthreads();
+    const bool any = mn <= mx;
+    const int l = __reduce_min_sync(0xffffffffu, any ? f2ord(mn) : INT_MAX), h = __reduce_max_sync(0xffffffffu, any ? f2ord(mx) : INT_MIN);
+    nn = __reduce_add_sync(0xffffffffu, nn);
     if ((threadIdx.x & 31) == 0) {
-        if (mn <= mx) {
-            atomicMin(&out->vmin, f2ord(mn));
-            atomicMax(&out->vmax, f2ord(mx));
+        atomicMin(&lo, l);
+        atomicMax(&hi, h);
+        if (nn) atomicAdd(&nan, nn);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        if (lo <= hi) {
+            if (lo < *(volatile int *)&out->vmin) atomicMin(&out->vmin, lo);
+            if (hi > *(volatile int *)&out->vmax) atomicMax(&out->vmax, hi);
         }
-        if (nn) atomicAdd(&out->nnan, nn);
+        if (nan) atomicAdd(&out->nnan, (unsigned long long)nan);
     }
 }
 
-// histogram of bin_of((v - mn) * scl) over the non-NaN voxels, bins clamped
-// to [0, nb-1] (the 256-bin pass clamps like the reference; the 1001-bin
-// indices are in range for every finite volume)
+// Histogram of (int)round((v - mn) * scl) over the non-NaN voxels, rounded half away from
+// zero, clamped to [0, nb-1] (the 256-bin pass clamps like the reference; the 1001-bin
+// indices are in range for every finite volume; a NaN product, 0 * inf on a constant
+// volume, is bin 0, like the reference's clamp makes it).  Few large blocks: every block
+// adds its bins to the same addresses.  A warp whose lanes all have one bin (background)
+// sends one shared atomic.  7 M voxels: 28 and 23 us with 1216 blocks of 256 and an atomic per
+// voxel, 13.7 and 13.2 now.
+constexpr int TH_T = 1024;
 template <int NBINS>
-__global__ void __launch_bounds__(256) k_th_hist(const float *__restrict__ v, long long n, float mn, float scl,
-                                                 unsigned *hist) {
+__global__ void __launch_bounds__(TH_T) k_th_hist(const float *__restrict__ v, long long n, float mn, float scl,
+                                                  unsigned *hist) {
     grid_wait();
     __shared__ unsigned h[NBINS];
     for (int i = threadIdx.x; i < NBINS; i += blockDim.x) h[i] = 0;
     __syncthreads();
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const float x = __ldg(v + i);
-        if (x != x) continue;
-        long long b = bin_of(__fmul_rn(__fsub_rn(x, mn), scl));
-        b = b < NBINS - 1 ? b : NBINS - 1;
-        b = b > 0 ? b : 0;
-        atomicAdd(&h[b], 1u);
-    }
+    const int lane = threadIdx.x & 31;
+    each_voxel(v, n, [&](float x, bool in) {
+        const float r = roundf(__fmul_rn(__fsub_rn(x, mn), scl));
+        const int b = !in || x != x ? -1 : (r > 0.f ? (r < (float)(NBINS - 1) ? (int)r : NBINS - 1) : 0);
+        int same;
+        __match_all_sync(0xffffffffu, b, &same);
+        if (b >= 0 && (!same || lane == 0)) atomicAdd(&h[b], same ? 32u : 1u);
+    });
     __syncthreads();
     for (int i = threadIdx.x; i < NBINS; i += blockDim.x)
         if (h[i]) atomicAdd(&hist[i], h[i]);
@@ -176,6 +204,7 @@ unsigned grid_for(long long n) {
     if (b > 152 * 8) b = 152 * 8;
     return b > 0 ? (unsigned)b : 1u;
 }
+unsigned hist_grid(long long n) { return (unsigned)std::max<long long>(1, std::min<long long>((n + 4 * TH_T - 1) / (4 * TH_T), 152 * 2)); }
 }  // namespace
 
 n2m_status isolevel_otsu(const float *d_img, long long nvox, int mode123, ThresholdWork &w, cudaStream_t s,
@@ -221,7 +250,7 @@ n2m_status isolevel_otsu(const float *d_img, long long nvox, int mode123, Thresh
                 // (2) percentile histogram (src/isolevel.c:83-101), walk (:102-133)
                 const float scl = (NB_RANGE - 1) / (mx - mn);
                 CK(cudaMemsetAsync(d_h1, 0, NB_RANGE * sizeof(unsigned), s));
-                n2m_launch(k_th_hist<NB_RANGE>, grid_for(nvox), 256, 0, s, d_img, nvox, mn, scl, d_h1);
+                n2m_launch(k_th_hist<NB_RANGE>, hist_grid(nvox), TH_T, 0, s, d_img, nvox, mn, scl, d_h1);
                 CKL();
                 CK(cudaMemcpyAsync(h_hist, d_h1, NB_RANGE * sizeof(unsigned), cudaMemcpyDeviceToHost, s));
                 CK(cudaStreamSynchronize(s));
@@ -253,7 +282,7 @@ n2m_status isolevel_otsu(const float *d_img, long long nvox, int mode123, Thresh
     // (3) Otsu histogram on the robust range (src/isolevel.c:250-262)
     const float scl = (NB_OTSU - 1) / (pct98 - pct2);
     CK(cudaMemsetAsync(d_h2, 0, NB_OTSU * sizeof(unsigned), s));
-    n2m_launch(k_th_hist<NB_OTSU>, grid_for(nvox), 256, 0, s, d_img, nvox, pct2, scl, d_h2);
+    n2m_launch(k_th_hist<NB_OTSU>, hist_grid(nvox), TH_T, 0, s, d_img, nvox, pct2, scl, d_h2);
     CKL();
     CK(cudaMemcpyAsync(h_hist, d_h2, NB_OTSU * sizeof(unsigned), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
