@@ -24,7 +24,7 @@
 // jumped to roots before the other contacts are looked at, and the kernels run over
 // lists of runs or words, so that no lane idles.  512^3 CT volume (18-connected
 // foreground, 6-connected background): contacts 775 -> 252 us, of it 145 us for the
-// foreground; the sizes 88 -> 16 us where noise makes a million runs (int16 scan);
+// foreground; the sizes 91 -> 48 us where noise makes a million runs (int16 scan);
 // the whole call 2184 -> 1538 us with the volume left unwritten.
 #include <algorithm>
 
@@ -234,12 +234,12 @@ __device__ __forceinline__ Word start_word(const unsigned *__restrict__ B, const
 
 // Every run start of the class links to one run before it that it touches (itself
 // if its first word touches none): a forest over all runs, without an atomic, whose
-// trees are nearly the components.  z8 / z32 (may be null) are zeroed at the run
-// starts (the edge flags and sizes the roots will carry).
+// trees are nearly the components.  z8 (may be null) is zeroed at the run starts (the
+// edge flags the roots will carry), len (may be null) takes the run's length.
 template <int NNB>
 __global__ void __launch_bounds__(256) k_run_hook(const unsigned *__restrict__ B, LD d, unsigned want, const int *__restrict__ cs,
                                                   const int *__restrict__ list, const unsigned *__restrict__ nlist, int *L,
-                                                  unsigned char *z8, unsigned *z32) {
+                                                  unsigned char *z8, unsigned *len) {
     grid_wait();
     const unsigned n = *nlist;
     for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -259,7 +259,16 @@ __global__ void __launch_bounds__(256) k_run_hook(const unsigned *__restrict__ B
         }
         L[s] = parent;
         if (z8) z8[s] = 0;
-        if (z32) z32[s] = 0;
+        if (len) {
+            Word q = A.q[0];
+            unsigned l = __popc(piece);
+            while ((piece >> 31) && (q.nc & 1u)) {
+                q = load_word(B, d, q.r, q.w + 1, want);
+                piece = piece_at(q.c, 0);
+                l += __popc(piece);
+            }
+            len[s] = l;
+        }
     }
 }
 
@@ -351,8 +360,13 @@ __global__ void __launch_bounds__(256) k_run_flatten(const int *__restrict__ lis
         if (root == s) cnt++;
         else L[s] = root;
     }
+    __shared__ unsigned all;   // one atomic per block: a few ns each on the one address, 13 us by warps
+    if (threadIdx.x == 0) all = 0;
+    __syncthreads();
     cnt = __reduce_add_sync(FULL, cnt);
-    if ((threadIdx.x & 31) == 0 && cnt) atomicAdd(nroots, cnt);
+    if ((threadIdx.x & 31) == 0 && cnt) atomicAdd(&all, cnt);
+    __syncthreads();
+    if (threadIdx.x == 0 && all) atomicAdd(nroots, all);
 }
 
 // Background components touching a face of the volume flag their root:
@@ -432,12 +446,13 @@ __global__ void __launch_bounds__(256) k_run_fill(const unsigned *__restrict__ B
     }
 }
 
-// Component sizes: every run adds its length to its root.  Most runs belong to a few
-// large components, and one atomic per warp and root on the same counter took 88 us
-// (512^3 int16 scan): a lane keeps the heaviest root it meets to itself, and the block
-// adds up what belongs to the heaviest root of its first lane.
-__global__ void __launch_bounds__(256) k_run_sizes(const unsigned *__restrict__ B, LD d, const int *__restrict__ list,
-                                                   const unsigned *__restrict__ nlist, const int *__restrict__ L, unsigned *cnt) {
+// Component sizes, from the runs' lengths (k_run_hook): every run that is no root adds
+// its own to its root's.  Most runs belong to a few large components, so a lane keeps the
+// heaviest root it meets to itself, and the block adds up what belongs to the
+// heaviest root of its first lane (an atomic per warp and root, roots included, with the run walked
+// again took 91 us for an int16 scan's million runs, 48 now).
+__global__ void __launch_bounds__(256) k_run_sizes(const int *__restrict__ list, const unsigned *__restrict__ nlist,
+                                                   const int *__restrict__ L, unsigned *cnt) {
     grid_wait();
     __shared__ int hot;
     __shared__ unsigned total;
@@ -446,14 +461,8 @@ __global__ void __launch_bounds__(256) k_run_sizes(const unsigned *__restrict__ 
     unsigned sum = 0;
     for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const int s = list[i], root = L[s];
-        unsigned piece;
-        Word q = start_word(B, d, 1u, s, piece);
-        unsigned len = __popc(piece);
-        while ((piece >> 31) && (q.nc & 1u)) {
-            q = load_word(B, d, q.r, q.w + 1, 1u);
-            piece = piece_at(q.c, 0);
-            len += __popc(piece);
-        }
+        if (root == s) continue;
+        const unsigned len = cnt[s];   // only roots' change
         if (root == mine) {
             sum += len;
         } else if (len <= sum) {
@@ -493,7 +502,12 @@ __global__ void __launch_bounds__(256) k_run_best(const int *__restrict__ list, 
         const unsigned long long t = __shfl_xor_sync(FULL, b, o);
         b = t > b ? t : b;
     }
-    if ((threadIdx.x & 31) == 0 && b) atomicMax(best, b);
+    __shared__ unsigned long long all;   // one atomic per block, and only while it changes something
+    if (threadIdx.x == 0) all = 0;
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0 && b) atomicMax(&all, b);
+    __syncthreads();
+    if (threadIdx.x == 0 && all > *(volatile unsigned long long *)best) atomicMax(best, all);
 }
 
 // bits of the voxels of the largest component (K cleared before)
@@ -906,7 +920,7 @@ n2m_status label_core(LabelWork &w, const LD &d, int conn, bool only_largest, bo
     if (only_largest) {
         CKS(w.keep.ensure((size_t)d.nwords * sizeof(unsigned)));
         CK(cudaMemsetAsync(w.keep.p, 0, (size_t)d.nwords * sizeof(unsigned), s));
-        n2m_launch(k_run_sizes, run_grid(d), 256, 0, s, B, d, w.list.as<int>(), &misc->nlist[1], w.lab.as<int>(),
+        n2m_launch(k_run_sizes, run_grid(d), 256, 0, s, w.list.as<int>(), &misc->nlist[1], w.lab.as<int>(),
                    w.cnt.as<unsigned>());
         n2m_launch(k_run_best, run_grid(d), 256, 0, s, w.list.as<int>(), &misc->nlist[1], w.lab.as<int>(), w.cnt.as<unsigned>(),
                    &misc->best);

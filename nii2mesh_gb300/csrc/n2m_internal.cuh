@@ -185,8 +185,9 @@ n2m_status od_marks(OdWork &w, const int dim[3], unsigned **need, cudaStream_t s
 n2m_status od_repair(const OdRepair &r, cudaStream_t s);
 // transposed pre-smooth: g_img = Sx^T Sy^T Sz^T g (tmp: one volume of scratch)
 n2m_status launch_smooth_adjoint(const float *g, float *tmp, float *out, int nx, int ny, int nz, cudaStream_t s);
+// (z0: slice of vol in the whole volume)
 n2m_status launch_stats(const float *vol, int nx, int ny, int nz, float iso, bool minmax, VolStats *st,
-                        cudaStream_t s);
+                        cudaStream_t s, int z0 = 0);
 void stats_init_host(VolStats *h);
 
 // scan.cu: exclusive scan of uint4 (component-wise) in place; total -> *d_total

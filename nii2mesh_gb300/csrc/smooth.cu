@@ -30,7 +30,7 @@ using namespace smooth;
 // range / bbox / non-finite count of an existing volume: a bounded grid whose
 // warps stride over the rows, so the block flushes (one set of atomics each)
 // stay few; every reduction is a min, max or count, so the order is free
-__global__ void __launch_bounds__(256) k_stats(const float *__restrict__ vol, int nx, int ny, int nz, float iso,
+__global__ void __launch_bounds__(256) k_stats(const float *__restrict__ vol, int nx, int ny, int nz, int z0, float iso,
                                                VolStats *st, bool minmax) {
     grid_wait();
     Acc acc;
@@ -41,7 +41,7 @@ __global__ void __launch_bounds__(256) k_stats(const float *__restrict__ vol, in
         const int z = (int)(r / ny), y = (int)(r - (long long)z * ny);
         const float *row = vol + r * nx;
 #pragma unroll 4
-        for (int x = lane; x < nx; x += 32) acc.add(__ldg(row + x), x, y, z, iso);
+        for (int x = lane; x < nx; x += 32) acc.add(__ldg(row + x), x, y, z0 + z, iso);
     }
     acc.flush(st, minmax);
 }
@@ -467,10 +467,10 @@ n2m_status launch_smooth_adjoint(const float *g, float *tmp, float *out, int nx,
 }
 
 n2m_status launch_stats(const float *vol, int nx, int ny, int nz, float iso, bool minmax, VolStats *st,
-                        cudaStream_t s) {
+                        cudaStream_t s, int z0) {
     const long long rows = (long long)ny * nz;
     const unsigned grid = (unsigned)std::max<long long>(1, std::min<long long>((rows + 7) / 8, 152 * 8));   // 8 rows per block
-    n2m_launch(k_stats, grid, 256, 0, s, vol, nx, ny, nz, iso, st, minmax);
+    n2m_launch(k_stats, grid, 256, 0, s, vol, nx, ny, nz, z0, iso, st, minmax);
     CKL();
     return N2M_OK;
 }

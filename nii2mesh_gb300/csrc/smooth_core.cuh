@@ -72,13 +72,16 @@ struct Acc {
                 a.hi0 = max(a.hi0, b.hi0); a.hi1 = max(a.hi1, b.hi1); a.hi2 = max(a.hi2, b.hi2);
                 a.nf += b.nf;
             }
+            // hundreds of blocks at one cache line: only what still changes something
+            auto low = [](int *p, int v) { if (v < *(volatile int *)p) atomicMin(p, v); };
+            auto high = [](int *p, int v) { if (v > *(volatile int *)p) atomicMax(p, v); };
             if (minmax && a.mn <= a.mx) {
-                atomicMin(&st->vmin, f2ord(a.mn));
-                atomicMax(&st->vmax, f2ord(a.mx));
+                low(&st->vmin, f2ord(a.mn));
+                high(&st->vmax, f2ord(a.mx));
             }
             if (a.lo0 != INT_MAX) {
-                atomicMin(&st->lo[0], a.lo0); atomicMin(&st->lo[1], a.lo1); atomicMin(&st->lo[2], a.lo2);
-                atomicMax(&st->hi[0], a.hi0); atomicMax(&st->hi[1], a.hi1); atomicMax(&st->hi[2], a.hi2);
+                low(&st->lo[0], a.lo0); low(&st->lo[1], a.lo1); low(&st->lo[2], a.lo2);
+                high(&st->hi[0], a.hi0); high(&st->hi[1], a.hi1); high(&st->hi[2], a.hi2);
             }
             if (a.nf) atomicAdd(&st->nonfinite, a.nf);
         }
