@@ -187,23 +187,26 @@ __device__ __forceinline__ WordAt word_at(const ABox &B, unsigned lw) {
     a.live = a.lr < (unsigned)B.n[1] * (unsigned)B.n[2];
     return a;
 }
-// bits of f(row, x) for the 32 words of a warp, 8 words in flight; load(lr, x) fetches, bit(value) decides
-template <class V, class L, class P> __device__ __forceinline__ unsigned warp_words(const ABox &B, unsigned lw0, int lane, L load, P bit) {
+// bits of the 32 words of a warp, AW_U words in flight: off(row) is where a row's values begin in p (found once per
+// word, by its own lane), bit(value) decides
+constexpr int AW_U = 16;
+template <class V, class O, class P>
+__device__ __forceinline__ unsigned warp_words(const ABox &B, unsigned lw0, int lane, const V *__restrict__ p, O off, P bit) {
     const WordAt a = word_at(B, lw0 + (unsigned)lane);
-    const int n = __popc(__ballot_sync(FULL, a.live));
+    const int n = __popc(__ballot_sync(FULL, a.live)), left = B.n[0] - 32 * a.w;   // columns from the word's first on
+    const long long at = a.live ? off(a.lr) + 32 * a.w : 0;
     unsigned mine = 0;
-    for (int k0 = 0; k0 < n; k0 += 8) {
-        V val[8];
-        bool in[8];
+    for (int k0 = 0; k0 < n; k0 += AW_U) {
+        V val[AW_U];
+        bool in[AW_U];
 #pragma unroll
-        for (int u = 0; u < 8; u++) {
-            const unsigned lr = __shfl_sync(FULL, a.lr, (k0 + u) & 31);
-            const int x = 32 * __shfl_sync(FULL, a.w, (k0 + u) & 31) + lane;
-            in[u] = k0 + u < n && x < B.n[0];
-            val[u] = in[u] ? load(lr, x) : V(0);
+        for (int u = 0; u < AW_U; u++) {
+            const long long q = __shfl_sync(FULL, at, (k0 + u) & 31);
+            in[u] = k0 + u < n && lane < __shfl_sync(FULL, left, (k0 + u) & 31);
+            val[u] = in[u] ? __ldg(p + q + lane) : V(0);
         }
 #pragma unroll
-        for (int u = 0; u < 8; u++) {
+        for (int u = 0; u < AW_U; u++) {
             const unsigned m = __ballot_sync(FULL, in[u] && bit(val[u]));
             if (lane == k0 + u) mine = m;
         }
@@ -221,9 +224,9 @@ __global__ void __launch_bounds__(256) k_a_mask(AtlasVol v, const ABox *boxes, i
         if (lane == 0) wbox[w0 / 32] = (unsigned)b;   // the box of every 32 words
         const int n1 = B.n[1], label = B.label;
         const short *base = v.lab + (long long)B.o[2] * v.nxy + (long long)B.o[1] * v.nx + B.o[0];
-        M[w0 + (unsigned)lane] = warp_words<short>(B, w0 - B.bw0, lane, [&](unsigned lr, int x) {
+        M[w0 + (unsigned)lane] = warp_words(B, w0 - B.bw0, lane, base, [&](unsigned lr) {
             const int z = (int)(lr / (unsigned)n1), y = (int)(lr - (unsigned)z * (unsigned)n1);
-            return __ldg(base + (long long)z * v.nxy + (long long)y * v.nx + x);
+            return (long long)z * v.nxy + (long long)y * v.nx;
         }, [&](short l) { return l == label; });
     }
 }
@@ -236,7 +239,7 @@ __global__ void __launch_bounds__(256) k_a_mask(AtlasVol v, const ABox *boxes, i
 // full away from the volume's faces, skip the passes.  Bound by FP32 issue.  23 M arena
 // voxels (250 labels of a 256^3 atlas): 604 us with one CTA per column tile, staging and
 // queueing every pass between barriers; 200 us.
-constexpr int ARY = 4, AZC = 16, AWARPS = 8;
+constexpr int ARY = 4, AZC = 24, AWARPS = 8;
 struct SmoothQueue {
     float v[5][64];
     unsigned at[64];
@@ -428,9 +431,8 @@ __global__ void __launch_bounds__(256) k_ab_bits(const ABox *boxes, const unsign
         const float *base = arena + B.arena;
         const int n0 = B.n[0];
         const float iso = B.iso;
-        Bits[w0 + (unsigned)lane] = warp_words<float>(B, w0 - B.bw0, lane,
-                                                      [&](unsigned lr, int x) { return __ldg(base + (long long)lr * n0 + x); },
-                                                      [&](float f) { return f >= iso; });
+        Bits[w0 + (unsigned)lane] = warp_words(B, w0 - B.bw0, lane, base, [&](unsigned lr) { return (long long)lr * n0; },
+                                               [&](float f) { return f >= iso; });
     }
 }
 

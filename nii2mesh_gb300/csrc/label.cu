@@ -173,7 +173,7 @@ struct Around {
 // is free): the kernels that follow wait on memory most of the time, and by rows of
 // words only a few lanes of a warp had a run (512^3: 0.8 M background runs in 4.2 M
 // words, a foreground in a tenth of them).
-constexpr int LIST_K = 8;   // words per thread
+constexpr int LIST_K = 2;   // words per thread (8: a block for 2048 words left most SMs of a small volume idle)
 __global__ void __launch_bounds__(256) k_run_list(const unsigned *__restrict__ B, LD d, unsigned want, int *list, unsigned *wlist,
                                                   unsigned *nlist, unsigned *nwlist) {
     grid_wait();
@@ -877,15 +877,15 @@ n2m_status components(LabelWork &w, const LD &d, const unsigned *B, unsigned wan
     unsigned *wlist = w.wlist.as<unsigned>(), *nwlist = &misc->nwlist[want];
     n2m_launch(k_run_starts, rgrid(d), 256, 0, s, B, d, want, cs);
     n2m_launch(k_run_list, lg, 256, 0, s, B, d, want, list, wlist, nlist, nwlist);
-    if (conn == 6) n2m_launch(k_run_hook<3>, g, 256, 0, s, B, d, want, cs, list, nlist, L, z8, z32);
-    else if (conn == 18) n2m_launch(k_run_hook<9>, g, 256, 0, s, B, d, want, cs, list, nlist, L, z8, z32);
-    else n2m_launch(k_run_hook<13>, g, 256, 0, s, B, d, want, cs, list, nlist, L, z8, z32);
+    if (conn == 6) n2m_launch(k_run_hook<3>, 2 * g, 128, 0, s, B, d, want, cs, list, nlist, L, z8, z32);
+    else if (conn == 18) n2m_launch(k_run_hook<9>, 2 * g, 128, 0, s, B, d, want, cs, list, nlist, L, z8, z32);
+    else n2m_launch(k_run_hook<13>, 2 * g, 128, 0, s, B, d, want, cs, list, nlist, L, z8, z32);
     // once every start points at its tree's root, nearly every contact of the merge joins equal links
-    n2m_launch(k_run_jump, g, 256, 0, s, list, nlist, L);
-    if (conn == 6) n2m_launch(k_run_merge<3>, wg, 256, 0, s, B, d, want, cs, wlist, nwlist, L);
-    else if (conn == 18) n2m_launch(k_run_merge<9>, wg, 256, 0, s, B, d, want, cs, wlist, nwlist, L);
-    else n2m_launch(k_run_merge<13>, wg, 256, 0, s, B, d, want, cs, wlist, nwlist, L);
-    n2m_launch(k_run_flatten, g, 256, 0, s, list, nlist, L, want ? &misc->nfg : &misc->nbg);
+    n2m_launch(k_run_jump, 2 * g, 128, 0, s, list, nlist, L);
+    if (conn == 6) n2m_launch(k_run_merge<3>, 4 * wg, 64, 0, s, B, d, want, cs, wlist, nwlist, L);
+    else if (conn == 18) n2m_launch(k_run_merge<9>, 4 * wg, 64, 0, s, B, d, want, cs, wlist, nwlist, L);
+    else n2m_launch(k_run_merge<13>, 4 * wg, 64, 0, s, B, d, want, cs, wlist, nwlist, L);
+    n2m_launch(k_run_flatten, 2 * g, 128, 0, s, list, nlist, L, want ? &misc->nfg : &misc->nbg);
     CKL();
     return N2M_OK;
 }
