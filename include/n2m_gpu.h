@@ -261,7 +261,7 @@ n2m_status n2m_smooth_hc_device(n2m_context *ctx, vec3d *d_verts, const vec3i *d
  * n2m_smooth_hc_device) for callers that cannot call cudaMalloc: code inside
  * another framework's captured or allocation-controlled region, or programs
  * whose device memory all comes from their own pool.  All scratch lives in one
- * fixed device array inside the library (about 18 MB, held by every GPU that
+ * fixed device array inside the library (about 22 MB, held by every GPU that
  * loads the library until the process exits), so meshes are limited to
  * N2M_NOALLOC_MAX_VERTS vertices and N2M_NOALLOC_MAX_TRIS triangles; larger
  * meshes fail with N2M_ERR_TOO_LARGE before any work is queued.  d_verts and

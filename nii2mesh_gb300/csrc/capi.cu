@@ -289,7 +289,7 @@ extern "C" void n2m_context_destroy(n2m_context *c) {
                       &c->tris_raw, &c->pts, &c->tris, &c->ntf, &c->weld, &c->gath, &c->hmesh,
                       &c->mc.signs, &c->mc.words, &c->mc.act, &c->mc.cnt, &c->mc.sub, &c->scan.part,
                       &c->lab.lab, &c->lab.mask, &c->lab.keep, &c->lab.cnt, &c->lab.edge, &c->lab.rc, &c->lab.misc, &c->lab.list, &c->lab.wlist, &c->lab.cs, &c->lab.filled, &c->lab.shell,
-                      &c->deg.bits, &c->deg.tiles, &c->deg.rank, &c->deg.near, &c->hc.zero, &c->hc.adj, &c->hc.meta, &c->hc.P, &c->hc.Q,
+                      &c->deg.bits, &c->deg.tiles, &c->deg.rank, &c->deg.near, &c->hc.zero, &c->hc.adj, &c->hc.ell, &c->hc.meta, &c->hc.P, &c->hc.Q,
                       &c->hc.B, &c->hc.Lo, &c->th.buf, &c->th.table,
                       &c->stmp2, &c->lubits, &c->od.st, &c->od.unc, &c->od.cmin, &c->od.cmax, &c->od.range, &c->od.need, &c->od.list, &c->od.lcnt, &c->od.vsign, &c->od.pad,
                       &c->wr.mt, &c->wr.mp, &c->wr.pack, &c->wr.pack2, &c->wr.lens, &c->wr.flag, &c->wr.out};

@@ -79,6 +79,10 @@ __device__ __noinline__ void heapsort_ids(int *a, int n) {
 // One vertex's neighbours.  The smoothing sums the two other vertices of every
 // reference, so inside a closed surface each neighbour comes twice: the list
 // holds n2 ids that count twice (summed once, doubled), then n1 that count once.
+// The first ELL_K of the doubled ids also stand in `ell`, entry k of 32 consecutive
+// vertices together, so that a warp reads them in whole lines.
+constexpr unsigned ELL_K = 8;
+__device__ __forceinline__ size_t ell_at(int i, unsigned k) { return (size_t)(i >> 5) * (32 * ELL_K) + 32 * k + (i & 31); }
 struct __align__(16) Meta {
     unsigned at;      // first entry in adj
     unsigned n2, n1;
@@ -98,8 +102,8 @@ struct __align__(16) Meta {
 // for the separate sort, Lo and border kernels that walked triangle references.
 constexpr int ADJ_S = 32, ADJ_T = 128;
 __global__ void __launch_bounds__(ADJ_T) k_hc_adj(const vec3d *__restrict__ o, const unsigned *__restrict__ start, int np,
-                                                  int *adj, Meta *meta, unsigned char *border, float4 *Lo, float4 *Pn,
-                                                  float4 *B) {
+                                                  int *adj, int *ell, Meta *meta, unsigned char *border, float4 *Lo,
+                                                  float4 *Pn, float4 *B) {
     grid_wait();
     __shared__ int col[ADJ_S][ADJ_T];
     const int tid = threadIdx.x;
@@ -147,7 +151,10 @@ __global__ void __launch_bounds__(ADJ_T) k_hc_adj(const vec3d *__restrict__ o, c
                     const int id = col[k][tid];
                     unsigned e = k + 1;
                     while (e < n && col[e][tid] == id) e++;
-                    for (unsigned c = (e - k) >> 1; c; c--) g[w2++] = id;
+                    for (unsigned c = (e - k) >> 1; c; c--) {
+                        if (w2 < ELL_K) ell[ell_at(i, w2)] = id;
+                        g[w2++] = id;
+                    }
                     if ((e - k) & 1u) g[w1++] = id;
                     k = e;
                 }
@@ -167,38 +174,51 @@ __global__ void __launch_bounds__(ADJ_T) k_hc_adj(const vec3d *__restrict__ o, c
     }
 }
 
-// Sum of X over the neighbours (W: each scaled by its own .w).  A sweep is bound
-// by the latency of its three dependent loads (list, ids, vectors), so eight
-// ids and then their eight 16-byte vectors are in flight at once: one round for
-// the usual valence of 6.  At 250k vertices with cold caches a half-iteration
-// takes 10.0 us; through the triangle references (twelve 12-byte vectors behind
-// a fourth dependent load) it took 14.0.
+// Sum of X over the neighbours (W: each scaled by its own .w).  A sweep is bound by the
+// latency of its three dependent loads (list, ids, vectors) and by L1: eight ids and
+// then their eight 16-byte vectors are in flight at once, one round for the usual valence
+// of 6, and the ids come in whole lines from `ell` (per-vertex lists lie 48 bytes apart: a
+// warp's load of one id each touched 12 lines).  At 250k vertices with cold caches a
+// half-iteration takes 9.4 us; with the ids from the lists it took 10.5, through the
+// triangle references (twelve 12-byte vectors behind a fourth dependent load) 14.0.
+template <bool W> __device__ __forceinline__ void add_vectors(const float4 *__restrict__ X, const int (&id)[8], float &sx, float &sy, float &sz) {
+    float4 v[8];
+#pragma unroll
+    for (int u = 0; u < 8; u++) v[u] = id[u] >= 0 ? __ldg(X + id[u]) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int u = 0; u < 8; u++) {
+        if (W) {
+            sx += v[u].x * v[u].w; sy += v[u].y * v[u].w; sz += v[u].z * v[u].w;
+        } else {
+            sx += v[u].x; sy += v[u].y; sz += v[u].z;
+        }
+    }
+}
 template <bool W>
 __device__ __forceinline__ void add_ids(const float4 *__restrict__ X, const int *__restrict__ p, unsigned n, float &sx,
                                         float &sy, float &sz) {
     for (unsigned k = 0; k < n; k += 8) {
         int id[8];
-        float4 v[8];
 #pragma unroll
         for (int u = 0; u < 8; u++) id[u] = k + u < n ? __ldg(p + k + u) : -1;
-#pragma unroll
-        for (int u = 0; u < 8; u++) v[u] = id[u] >= 0 ? __ldg(X + id[u]) : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-        for (int u = 0; u < 8; u++) {
-            if (W) {
-                sx += v[u].x * v[u].w; sy += v[u].y * v[u].w; sz += v[u].z * v[u].w;
-            } else {
-                sx += v[u].x; sy += v[u].y; sz += v[u].z;
-            }
-        }
+        add_vectors<W>(X, id, sx, sy, sz);
     }
 }
+struct Lists {
+    const int *adj, *ell;
+};
 template <bool W>
-__device__ __forceinline__ float3 sum_neighbours(const float4 *__restrict__ X, const int *__restrict__ adj, const Meta &m) {
+__device__ __forceinline__ float3 sum_neighbours(const float4 *__restrict__ X, const Lists &l, int i, const Meta &m) {
     float ax = 0.f, ay = 0.f, az = 0.f;
-    add_ids<W>(X, adj + m.at, m.n2, ax, ay, az);
+    const int *__restrict__ e = l.ell + ell_at(i, 0);
+    int id[8];
+    static_assert(ELL_K == 8, "one round");
+#pragma unroll
+    for (int u = 0; u < 8; u++) id[u] = (unsigned)u < m.n2 ? __ldg(e + 32 * u) : -1;
+    add_vectors<W>(X, id, ax, ay, az);
+    if (m.n2 > ELL_K) add_ids<W>(X, l.adj + m.at + ELL_K, m.n2 - ELL_K, ax, ay, az);
     ax += ax; ay += ay; az += az;
-    if (m.n1) add_ids<W>(X, adj + m.at + m.n2, m.n1, ax, ay, az);
+    if (m.n1) add_ids<W>(X, l.adj + m.at + m.n2, m.n1, ax, ay, az);
     return make_float3(ax, ay, az);
 }
 __device__ __forceinline__ Meta load_meta(const Meta *__restrict__ meta, int i) {
@@ -208,7 +228,7 @@ __device__ __forceinline__ Meta load_meta(const Meta *__restrict__ meta, int i) 
 
 // first half of an HC iteration: Pn = L(p) - o, B = Pn - (1-alpha) Q
 __global__ void __launch_bounds__(128) k_hc_a(const float4 *__restrict__ P, const float4 *__restrict__ Lo,
-                                              const Meta *__restrict__ meta, const int *__restrict__ adj, int np,
+                                              const Meta *__restrict__ meta, Lists lists, int np,
                                               float alpha1, float4 *Pn, float4 *B) {
     grid_wait();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < np; i += gridDim.x * blockDim.x) {
@@ -216,7 +236,7 @@ __global__ void __launch_bounds__(128) k_hc_a(const float4 *__restrict__ P, cons
         const float4 q = P[i], lo = Lo[i];
         float4 pn = q;
         if (m.inv != 0.f) {
-            const float3 l = sum_neighbours<false>(P, adj, m);
+            const float3 l = sum_neighbours<false>(P, lists, i, m);
             pn = make_float4(lo.x + l.x * m.inv, lo.y + l.y * m.inv, lo.z + l.z * m.inv, 0.f);
         }
         Pn[i] = pn;
@@ -228,7 +248,7 @@ __global__ void __launch_bounds__(128) k_hc_a(const float4 *__restrict__ P, cons
 // vertices instead: o += P, except border vertices when locked, and none at all
 // when a triangle index was out of range
 __global__ void __launch_bounds__(128) k_hc_b(const float4 *__restrict__ Pn, const float4 *__restrict__ B,
-                                              const Meta *__restrict__ meta, const int *__restrict__ adj, int np,
+                                              const Meta *__restrict__ meta, Lists lists, int np,
                                               float beta, float beta1, float4 *P, vec3d *o,
                                               const unsigned char *__restrict__ border, bool lock,
                                               const unsigned *__restrict__ bad) {
@@ -239,7 +259,7 @@ __global__ void __launch_bounds__(128) k_hc_b(const float4 *__restrict__ Pn, con
         const float4 b = B[i], pn = Pn[i];
         float3 lb = make_float3(b.x, b.y, b.z);
         if (m.inv != 0.f) {
-            lb = sum_neighbours<false>(B, adj, m);
+            lb = sum_neighbours<false>(B, lists, i, m);
             lb = make_float3(lb.x * m.inv, lb.y * m.inv, lb.z * m.inv);
         }
         const float3 d = make_float3(pn.x - (beta * b.x + beta1 * lb.x), pn.y - (beta * b.y + beta1 * lb.y),
@@ -273,13 +293,13 @@ __global__ void k_hcT_init(const float3 *__restrict__ g, const unsigned char *__
 
 // t1 = L^T lam
 __global__ void __launch_bounds__(128) k_hcT_a(const float4 *__restrict__ lam, const Meta *__restrict__ meta,
-                                               const int *__restrict__ adj, int np, float4 *t1) {
+                                               Lists lists, int np, float4 *t1) {
     grid_wait();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < np; i += gridDim.x * blockDim.x) {
         const Meta m = load_meta(meta, i);
         float4 r = lam[i];
         if (m.inv != 0.f) {
-            const float3 s = sum_neighbours<true>(lam, adj, m);
+            const float3 s = sum_neighbours<true>(lam, lists, i, m);
             r = make_float4(s.x, s.y, s.z, m.inv);
         }
         t1[i] = r;
@@ -288,14 +308,14 @@ __global__ void __launch_bounds__(128) k_hcT_a(const float4 *__restrict__ lam, c
 
 // t2 = L^T t1; go += ab*lam + a1b*t1; lam = c0*lam + c1*t1 - c2*t2 (added to go by the last iteration)
 __global__ void __launch_bounds__(128) k_hcT_b(float4 *lam, const float4 *__restrict__ t1, const Meta *__restrict__ meta,
-                                               const int *__restrict__ adj, float3 *go, int np, float ab, float a1b,
+                                               Lists lists, float3 *go, int np, float ab, float a1b,
                                                float c0, float c1, float c2, bool last) {
     grid_wait();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < np; i += gridDim.x * blockDim.x) {
         const Meta m = load_meta(meta, i);
         const float4 l = lam[i], u = t1[i];
         float3 v = make_float3(u.x, u.y, u.z);
-        if (m.inv != 0.f) v = sum_neighbours<true>(t1, adj, m);
+        if (m.inv != 0.f) v = sum_neighbours<true>(t1, lists, i, m);
         float3 g = go[i];
         g.x += ab * l.x + a1b * u.x; g.y += ab * l.y + a1b * u.y; g.z += ab * l.z + a1b * u.z;
         const float4 n = make_float4(c0 * l.x + c1 * u.x - c2 * v.x, c0 * l.y + c1 * u.y - c2 * v.y,
@@ -314,7 +334,7 @@ struct HcBufs {
     unsigned *start, *fill, *bad;
     unsigned char *border;
     size_t zero_bytes;
-    int *adj;
+    int *adj, *ell;
     Meta *meta;
     float4 *P, *Q, *B, *Lo;
 };
@@ -338,11 +358,11 @@ n2m_status hc_run(vec3d *d_pts, const vec3i *d_tris, int np, int nt, double alph
                   const HcBufs &h, cudaStream_t s) {
     n2m_launch(k_fill_adj, gs(nt), 256, 0, s, d_tris, nt, np, h.start, h.fill, (int2 *)h.adj);
     const unsigned g = sweep_grid(np);
-    n2m_launch(k_hc_adj, g, ADJ_T, 0, s, d_pts, h.start, np, h.adj, h.meta, h.border, h.Lo, h.Q, h.B);
+    n2m_launch(k_hc_adj, g, ADJ_T, 0, s, d_pts, h.start, np, h.adj, h.ell, h.meta, h.border, h.Lo, h.Q, h.B);
     const float a1 = (float)(1.0 - alpha), b = (float)beta, b1 = (float)(1.0 - beta);
     for (int it = 0; it < iter; it++) {
-        if (it) n2m_launch(k_hc_a, g, 128, 0, s, h.P, h.Lo, h.meta, h.adj, np, a1, h.Q, h.B);
-        n2m_launch(k_hc_b, g, 128, 0, s, h.Q, h.B, h.meta, h.adj, np, b, b1, h.P, it + 1 == iter ? d_pts : nullptr, h.border,
+        if (it) n2m_launch(k_hc_a, g, 128, 0, s, h.P, h.Lo, h.meta, Lists{h.adj, h.ell}, np, a1, h.Q, h.B);
+        n2m_launch(k_hc_b, g, 128, 0, s, h.Q, h.B, h.meta, Lists{h.adj, h.ell}, np, b, b1, h.P, it + 1 == iter ? d_pts : nullptr, h.border,
                    lock_edges, h.bad);
     }
     CKL();
@@ -352,6 +372,7 @@ HcBufs hc_bufs(const HcWork &w, int np) {
     HcBufs h;
     hc_zero_layout(np, w.zero.p, h);
     h.adj = w.adj.as<int>();
+    h.ell = w.ell.as<int>();
     h.meta = w.meta.as<Meta>();
     h.P = w.P.as<float4>();
     h.Q = w.Q.as<float4>();
@@ -367,6 +388,7 @@ n2m_status mesh_smooth_hc(vec3d *d_pts, const vec3i *d_tris, int np, int nt, dou
     HcBufs h;
     CKS(w.zero.ensure(hc_zero_layout(np, nullptr, h)));
     CKS(w.adj.ensure((size_t)6 * (nt > 0 ? nt : 1) * sizeof(int)));
+    CKS(w.ell.ensure(((size_t)np + 31) / 32 * 32 * ELL_K * sizeof(int)));
     CKS(w.meta.ensure((size_t)np * sizeof(Meta)));
     CKS(w.P.ensure((size_t)np * sizeof(float4)));
     CKS(w.Q.ensure((size_t)np * sizeof(float4)));
@@ -400,8 +422,8 @@ n2m_status mesh_smooth_hc_backward(int np, double alpha, double beta, int iter, 
     const float ab = al * be, a1b = al * (1.f - be);
     const float c0 = be * (1.f - al), c1 = (1.f - be) * (2.f - al), c2 = 1.f - be;
     for (int it = 0; it < iter; it++) {
-        n2m_launch(k_hcT_a, g, 128, 0, s, h.P, h.meta, h.adj, np, h.Q);
-        n2m_launch(k_hcT_b, g, 128, 0, s, h.P, h.Q, h.meta, h.adj, d_go, np, ab, a1b, c0, c1, c2, it + 1 == iter);
+        n2m_launch(k_hcT_a, g, 128, 0, s, h.P, h.meta, Lists{h.adj, h.ell}, np, h.Q);
+        n2m_launch(k_hcT_b, g, 128, 0, s, h.P, h.Q, h.meta, Lists{h.adj, h.ell}, d_go, np, ab, a1b, c0, c1, c2, it + 1 == iter);
     }
     CKL();
     return N2M_OK;
@@ -414,7 +436,7 @@ n2m_status mesh_smooth_hc_backward(int np, double alpha, double beta, int iter, 
 // smoothing (neighbour lists, displacement buffers, flags) lives in one
 // file-scope device array of fixed size, so the entry point allocates nothing.
 // Limits: N2M_NOALLOC_MAX_VERTS vertices and N2M_NOALLOC_MAX_TRIS triangles
-// (about 18 MB, held by every GPU that loads the library until exit).
+// (about 22 MB, held by every GPU that loads the library until exit).
 namespace {
 constexpr size_t NA_V = N2M_NOALLOC_MAX_VERTS, NA_T = N2M_NOALLOC_MAX_TRIS;
 constexpr size_t na_align(size_t b) { return (b + 255) & ~(size_t)255; }
@@ -424,7 +446,8 @@ constexpr size_t NA_P = NA_META + na_align(NA_V * 16);
 constexpr size_t NA_Q = NA_P + na_align(NA_V * 16);
 constexpr size_t NA_B = NA_Q + na_align(NA_V * 16);
 constexpr size_t NA_LO = NA_B + na_align(NA_V * 16);
-constexpr size_t NA_TOTAL = NA_LO + na_align(NA_V * 16);
+constexpr size_t NA_ELL = NA_LO + na_align(NA_V * 16);
+constexpr size_t NA_TOTAL = NA_ELL + na_align((NA_V + 31) / 32 * 32 * ELL_K * 4);
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[NA_TOTAL];
 
@@ -482,6 +505,7 @@ extern "C" n2m_status n2m_smooth_hc_noalloc(vec3d *d_verts, const vec3i *d_tris,
     h.Q = (float4 *)(base + NA_Q);
     h.B = (float4 *)(base + NA_B);
     h.Lo = (float4 *)(base + NA_LO);
+    h.ell = (int *)(base + NA_ELL);
     CKS(hc_count(d_tris, nvert, ntri, h, s));
     n2m_launch(k_scan_small, 1, 1024, 0, s, h.start, nvert + 1);
     CKS(hc_run(d_verts, d_tris, nvert, ntri, alpha, beta, iter, lock_edges, h, s));

@@ -360,9 +360,8 @@ n2m_status mesh_weld_candidates(const vec3d *d_pts, const MeshRoom &room, const 
                                 cudaStream_t s);
 struct HcWork {
     DevBuf zero;              // degrees / offsets, cursors, the bad-index flag, border flags
-    DevBuf adj, meta;         // neighbour lists and their per-vertex heads
+    DevBuf adj, ell, meta;    // neighbour lists, their first entries by 32 vertices, per-vertex heads
     DevBuf P, Q, B, Lo;       // displacements
-
 };
 // Triangles with an index outside [0, np) are skipped and flagged; the flag
 // makes the last kernel leave d_pts unchanged.  mesh_smooth_hc_check waits for
