@@ -38,18 +38,17 @@ WORKLOAD = "ct512: 512^3 f32 CT-like, iso 300, -p 1 -l 0 -b 0 -o 0 -r 1 -s 0 (Le
 ISO = 300.0
 # DRAM bytes (read + write) per step of each stage on this workload: one ncu capture of
 # `bench.py --profile 384` (dram__bytes_read.sum + dram__bytes_write.sum of the stage's kernels),
-# scaled by the voxel count to 512^3 (profiles/meshify_ct512_kernels.md): smooth = pass A + pass B,
-# count = signs, marks, exact passes on marked voxels, words, scans, emit = k_emit, weld, degenerate
+# scaled by the voxel count to 512^3: smooth = pass A + pass B, count = sign words, marks, exact
+# passes on marked voxels, tests, numbering, emit = k_emit, weld, degenerate
 SCALE_384 = (512 / 384) ** 3
-NCU_TRAFFIC = {"smooth": 437.9e6 * SCALE_384, "count": 654.6e6 * SCALE_384, "emit": 138.0e6 * SCALE_384,
-               "weld": 74.0e6 * SCALE_384, "degenerate": 125.6e6 * SCALE_384}
-PASS_A_TRAFFIC = 437.6e6 * SCALE_384   # k_od_approx alone
-# what bounds each stage (measured in the same profiles)
-STAGE_BOUND = {"smooth": "FP32 instruction issue in pass A (74 % issue active, ~92 instructions per voxel); "
-                         "DRAM 7.7 B/voxel, no re-reads",
-               "count": "the exact passes on the ~10 % marked voxels (issue + sector-granular gathers) and the "
-                        "sign/word passes",
-               "emit": "latency (neighbour-word and value loads) and divergent listing"}
+NCU_TRAFFIC = {"smooth": 431.2e6 * SCALE_384, "count": 333.7e6 * SCALE_384, "emit": 107.3e6 * SCALE_384,
+               "weld": 37.0e6 * SCALE_384, "degenerate": 77.7e6 * SCALE_384}
+PASS_A_TRAFFIC = 430.9e6 * SCALE_384   # k_od_approx alone
+# what bounds each stage (measured)
+STAGE_BOUND = {"smooth": "FP32 instruction issue in pass A (53 % of the slots, 38 instructions per voxel; registers allow "
+                         "12 warps per SM); DRAM 7.6 B/voxel, no re-reads",
+               "count": "the exact passes on the ~10 % marked voxels (gathers' latency and issue) and the word passes",
+               "emit": "issue and value loads"}
 STAGE_NAMES = ("smooth", "cluster", "count", "emit", "weld", "degenerate", "hc")
 
 
@@ -755,7 +754,7 @@ def main():
             "kernel_ms": round(pa_ms, 4), "algorithmic_bytes": pa_bytes, "traffic": PASS_A_TRAFFIC,
             "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one k_od_approx launch at 384^3, "
                               "scaled by the voxel count",
-            "limited_by": "FP32 instruction issue (74 % issue active); memory 1.9-2.4 TB/s",
+            "limited_by": "FP32 instruction issue (53 % of the slots, 12 warps per SM); memory 4.1 TB/s",
             "whole_path": {"bytes": whole, "achieved": round(whole_gbs, 1), "frac": round(whole_gbs / peak, 4),
                            "formula": "(4 N_vox + 24 N_vert + 12 N_tri) / ms_per_step / peak",
                            "dram_bytes": round(sum(NCU_TRAFFIC.values())),
