@@ -291,7 +291,7 @@ extern "C" void n2m_context_destroy(n2m_context *c) {
                       &c->lab.lab, &c->lab.mask, &c->lab.keep, &c->lab.cnt, &c->lab.edge, &c->lab.rc, &c->lab.misc, &c->lab.list, &c->lab.wlist, &c->lab.cs, &c->lab.filled, &c->lab.shell,
                       &c->deg.bits, &c->deg.tiles, &c->deg.rank, &c->deg.near, &c->hc.zero, &c->hc.adj, &c->hc.ell, &c->hc.meta, &c->hc.P, &c->hc.Q,
                       &c->hc.B, &c->hc.Lo, &c->th.buf, &c->th.table,
-                      &c->stmp2, &c->lubits, &c->od.st, &c->od.unc, &c->od.cmin, &c->od.cmax, &c->od.range, &c->od.need, &c->od.list, &c->od.lcnt, &c->od.vsign, &c->od.pad,
+                      &c->stmp2, &c->lubits, &c->od.st, &c->od.need, &c->od.list, &c->od.lcnt, &c->od.vsign,
                       &c->wr.mt, &c->wr.mp, &c->wr.pack, &c->wr.pack2, &c->wr.lens, &c->wr.flag, &c->wr.out};
     for (DevBuf *b : bufs) b->release();
     deflate_release(c->wr.df);
@@ -646,11 +646,11 @@ n2m_status prepare(n2m_context *c, const float *d_src, const int dim[3], const n
         return N2M_OK;
     };
     if (smooth) {
-        CKS(c->stmp.ensure(n * sizeof(float)));
+        CKS(c->stmp.ensure(od ? od_scratch(d_src, nx, ny, nz) : n * sizeof(float)));
         const StagedInput *stage = c->stage.host ? &c->stage : nullptr;
         if (od) {
             CK(cudaEventRecord(c->eva[0], c->stream));
-            CKS(od_approx(d_src, vol, nx, ny, nz, iso, c->od, c->stream));
+            CKS(od_approx(d_src, vol, nx, ny, nz, iso, c->stmp.as<float>(), c->od, c->stream));
             CK(cudaEventRecord(c->eva[1], c->stream));
             c->pass_a = true;
             CKS(od_resolve(d_src, vol, nx, ny, nz, iso, c->od, c->stream, label || o.cubes == N2M_CUBES_OLDCUBES));

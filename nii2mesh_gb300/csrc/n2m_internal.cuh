@@ -142,13 +142,12 @@ struct OdLists {
     unsigned wv, nys;        // the bitmap's words per row, groups of 8 rows per slice
 };
 struct OdWork {
-    DevBuf st, unc, cmin, cmax, range, need, list, lcnt;
+    DevBuf st, need, list, lcnt;   // st: OdStats, the lists of undecided voxels and range candidates, the tasks' ranges
     // bit x & 31 of word od_vsign_word(x, y, z): the smoothed value of voxel (x, y, z)
     // minus iso is above -FLT_EPSILON (Lewiner's sign before edge darkening), or with
     // od_resolve's at_or_above, the value is >= iso (the complement of oldcubes'
     // sign); exact for every voxel once od_resolve has run
     DevBuf vsign;
-    DevBuf pad;   // the input with rows of a multiple of 16 bytes
     unsigned cap = 0;
 };
 // What meshify's labelling does to each voxel (src/meshify.c:330-342), for the values
@@ -176,7 +175,9 @@ __host__ __device__ __forceinline__ size_t od_vsign_word(unsigned x, unsigned y,
 }
 // whether the on-demand path applies: at least 5 voxels along each axis, fewer than 2^32
 bool od_eligible(int nx, int ny, int nz);
-n2m_status od_approx(const float *in, float *out, int nx, int ny, int nz, float iso, OdWork &w, cudaStream_t s);
+// bytes of od_approx's scratch (the input with rows of a multiple of 16 bytes, if its own are not); at least the volume's
+size_t od_scratch(const float *in, int nx, int ny, int nz);
+n2m_status od_approx(const float *in, float *out, int nx, int ny, int nz, float iso, float *scratch, OdWork &w, cudaStream_t s);
 n2m_status od_resolve(const float *in, float *out, int nx, int ny, int nz, float iso, OdWork &w, cudaStream_t s,
                       bool at_or_above = false);
 n2m_status od_check(const OdWork &w, const OdStats &h, bool *fallback);

@@ -1235,6 +1235,13 @@ bool od_eligible(int nx, int ny, int nz) {
 }
 
 namespace {
+bool od_odd(const float *in, int nx) { return nx % 4 != 0 || ((uintptr_t)in & 15u) != 0; }
+}  // namespace
+size_t od_scratch(const float *in, int nx, int ny, int nz) {
+    return (size_t)(od_odd(in, nx) ? (nx + 3) / 4 * 4 : nx) * ny * nz * sizeof(float);
+}
+
+namespace {
 // rows of nx values with a pitch of px (a multiple of 4), a thread per four
 __global__ void __launch_bounds__(256) k_od_pad(const float *__restrict__ in, float *out, int nx, int px, size_t n4) {
     grid_wait();
@@ -1264,28 +1271,29 @@ int od_zrun(int nx, int ny, int nz) {
 size_t od_tasks(int nx, int ny, int nz, int zrun) {
     return (size_t)((nx + OA_X - 1) / OA_X) * ((ny + OA_Y - 1) / OA_Y) * ((nz + zrun - 1) / zrun);
 }
+constexpr size_t OD_LISTS = (sizeof(OdStats) + 255) / 256 * 256;   // where the lists begin behind the statistics
 OdLists od_lists(const OdWork &w, int nx, int ny) {
-    return OdLists{w.unc.as<unsigned>(), w.cmin.as<unsigned>(), w.cmax.as<unsigned>(),
-                   (unsigned *)((char *)w.st.p + offsetof(OdStats, cnt)), w.cap, w.vsign.as<unsigned>(), w.range.as<float4>(),
+    unsigned *const unc = (unsigned *)((char *)w.st.p + OD_LISTS);   // three lists, then the ranges
+    return OdLists{unc, unc + w.cap, unc + 2 * (size_t)w.cap,
+                   (unsigned *)((char *)w.st.p + offsetof(OdStats, cnt)), w.cap, w.vsign.as<unsigned>(), (float4 *)(unc + 3 * (size_t)w.cap),
                    (unsigned)(nx + 31) / 32, (unsigned)(ny + 7) / 8};
 }
 }  // namespace
 
-n2m_status od_approx(const float *in, float *out, int nx, int ny, int nz, float iso, OdWork &w, cudaStream_t s) {
+n2m_status od_approx(const float *in, float *out, int nx, int ny, int nz, float iso, float *scratch, OdWork &w, cudaStream_t s) {
     const size_t n = (size_t)nx * ny * nz;
     auto encode = tensor_map_encoder();
     if (!encode) {
         n2m_set_error("cuTensorMapEncodeTiled is not available from the driver");
         return N2M_ERR_CUDA;
     }
-    const bool odd = nx % 4 != 0 || ((uintptr_t)in & 15u) != 0 || ((uintptr_t)out & 15u) != 0;
+    const bool odd = od_odd(in, nx) || ((uintptr_t)out & 15u) != 0;
     const int px = (nx + 3) / 4 * 4;
     const float *rows = in;
     if (odd) {
         const size_t n4 = (size_t)px / 4 * ny * nz;
-        CKS(w.pad.ensure(n4 * sizeof(float4)));
-        n2m_launch(k_od_pad, (unsigned)std::min<size_t>((n4 + 255) / 256, 152u * 32u), 256, 0, s, in, w.pad.as<float>(), nx, px, n4);
-        rows = w.pad.as<float>();
+        n2m_launch(k_od_pad, (unsigned)std::min<size_t>((n4 + 255) / 256, 152u * 32u), 256, 0, s, in, scratch, nx, px, n4);
+        rows = scratch;
     }
     CUtensorMap tmap;
     {
@@ -1300,14 +1308,10 @@ n2m_status od_approx(const float *in, float *out, int nx, int ny, int nz, float 
             return N2M_ERR_CUDA;
         }
     }
-    w.cap = (unsigned)std::min<size_t>(n / 64 + 4096, 1u << 22);
+    w.cap = (unsigned)std::min<size_t>(n / 64 + 4096, 1u << 22) & ~3u;   // the ranges behind the lists stay aligned
     const int zrun = od_zrun(nx, ny, nz);
     const size_t nys = (size_t)(ny + 7) / 8, wv = (size_t)(nx + 31) / 32, ntask = od_tasks(nx, ny, nz, zrun);
-    CKS(w.st.ensure(sizeof(OdStats)));
-    CKS(w.unc.ensure((size_t)w.cap * sizeof(unsigned)));
-    CKS(w.cmin.ensure((size_t)w.cap * sizeof(unsigned)));
-    CKS(w.cmax.ensure((size_t)w.cap * sizeof(unsigned)));
-    CKS(w.range.ensure(ntask * sizeof(float4)));
+    CKS(w.st.ensure(OD_LISTS + 3 * (size_t)w.cap * sizeof(unsigned) + ntask * sizeof(float4)));
     CKS(w.vsign.ensure((size_t)nz * nys * wv * 8 * sizeof(unsigned)));
     OdStats h{};
     stats_init_host(&h.vs);   // vmin / vmax are filled by pass B from the candidates
