@@ -119,9 +119,10 @@ bool smooth_can_stage(int nx, int ny, int nz);
 // whole volume approximately (one fused FP32 pass, rigorous error bound), lists
 // the voxels whose sign against iso it cannot decide and leaves the range of each
 // task; od_resolve gives those voxels, and every voxel that can be the volume's
-// minimum or maximum, their exact values, which completes w.st (exact range and
-// bbox in its vs).  Once the host has read w.st, od_check says whether the caller
-// has to run launch_smooth instead (a non-finite or huge input, a list overflow).
+// minimum or maximum (or of a plateau of those, some), their exact values, which
+// completes w.st (exact range and bbox in its vs).  Once the host has read w.st, od_check
+// says whether the caller has to run launch_smooth instead (a non-finite or huge input, more
+// undecided voxels than the list holds, a plateau whose value does not follow from the raw volume).
 // Marching cubes marks the voxels whose values it reads in `need` (mcwords.cuh:
 // k_words, with an OdRepair): the ends of the edges the surface crosses and the
 // corners of ambiguous cubes; od_repair writes the reference's exact value at every
@@ -132,6 +133,8 @@ struct OdStats {
     unsigned flags;
     unsigned cnt[3];         // undecided, min candidates, max candidates
     int umin, lmax;          // ordered: smallest task min + B, largest task max - B
+    unsigned done;           // blocks of od_resolve that are through, when a list of candidates is too short
+    int rlo[4], rhi[4];      // then, ordered: raw range of the voxels in the face layers of at least 0 .. 3 axes
 };
 struct OdLists {
     unsigned *unc, *cmin, *cmax;   // voxels
