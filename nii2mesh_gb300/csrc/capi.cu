@@ -658,9 +658,9 @@ n2m_status prepare(n2m_context *c, const float *d_src, const int dim[3], const n
             if (label) CKS(labelling());
             CKS(readback2(c, &hod, c->od.st.p, &s1, dst + 1, label));
             bool fallback = false;
-            CKS(od_check(c->od, hod, &fallback));
+            CKS(od_check(hod, &fallback));
             if (fallback) {
-                od = labelled = false;
+                od = labelled = c->pass_a = false;
                 CKS(launch_smooth(d_src, vol, c->stmp.as<float>(), nx, ny, nz, iso, dst, c->stream, nullptr));
             }
         } else {

@@ -130,7 +130,7 @@ bool smooth_can_stage(int nx, int ny, int nz);
 enum : unsigned { OD_FALLBACK = 1u, OD_TIMEOUT = 2u };
 struct OdStats {
     VolStats vs;             // bbox of decided voxels >= iso; exact range after od_resolve
-    unsigned flags;
+    unsigned flags;          // final after od_resolve
     unsigned cnt[3];         // undecided, min candidates, max candidates
     int umin, lmax;          // ordered: smallest task min + B, largest task max - B
     unsigned done;           // blocks of od_resolve that are through, when a list of candidates is too short
@@ -183,7 +183,7 @@ size_t od_scratch(const float *in, int nx, int ny, int nz);
 n2m_status od_approx(const float *in, float *out, int nx, int ny, int nz, float iso, float *scratch, OdWork &w, cudaStream_t s);
 n2m_status od_resolve(const float *in, float *out, int nx, int ny, int nz, float iso, OdWork &w, cudaStream_t s,
                       bool at_or_above = false);
-n2m_status od_check(const OdWork &w, const OdStats &h, bool *fallback);
+n2m_status od_check(const OdStats &h, bool *fallback);
 // the cleared mark bitmap: bit x & 31 of word (z*ny + y)*ceil(nx/32) + x/32
 n2m_status od_marks(OdWork &w, const int dim[3], unsigned **need, cudaStream_t s);
 n2m_status od_repair(const OdRepair &r, cudaStream_t s);

@@ -622,21 +622,35 @@ __device__ __forceinline__ unsigned or_rows(const unsigned (&p)[OA_R], int lane)
 }
 
 // lists the lane's undecided voxels (any: it has some), in `rows` rows of `cols` from p; returns its row word's bits of them.
-// Out of line: rare, and the kernel's slice loop is unrolled five times.
+// Out of line: rare, and the kernel's slice loop is unrolled five times.  With the isolevel on a plateau (a mask meshed at
+// its own value) half the volume comes here: one atomic per warp, and none once the list is full and the caller falls
+// back anyway (1.4 M voxels of a 181 x 217 x 181 mask, an atomic each: 0.83 ms for the exact smoothing with the attempt).
 __device__ __noinline__ unsigned list_undecided(const float *p, int nx, int rows, int cols, unsigned j, bool any, float band, float iso,
                                                 unsigned *cnt, unsigned *list, unsigned cap, int lane) {
-    unsigned uw[OA_R];
+    const unsigned FULL = 0xffffffffu;
+    const unsigned listed = lane == 0 ? *(volatile unsigned *)cnt : 0u;
+    if (__shfl_sync(FULL, listed, 0) > cap) return 0u;
+    unsigned uw[OA_R], mine = 0u;
 #pragma unroll
     for (int r = 0; r < OA_R; r++) {
         unsigned m = 0u;
         for (int c = 0; any && r < rows && c < cols; c++)
-            if (fabsf(__fsub_rn(p[(size_t)r * nx + c], iso)) <= band) {
-                m |= 1u << (4 * (lane & 7) + c);
-                const unsigned q = atomicAdd(cnt, 1u);
-                if (q < cap) list[q] = j + (unsigned)(r * nx + c);
-            }
+            if (fabsf(__fsub_rn(p[(size_t)r * nx + c], iso)) <= band) m |= 1u << (4 * (lane & 7) + c);
         uw[r] = m;
+        mine += __popc(m);
     }
+    unsigned incl = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned t = __shfl_up_sync(FULL, incl, o);
+        if (lane >= o) incl += t;
+    }
+    unsigned at = lane == 31 ? atomicAdd(cnt, incl) : 0u;
+    at = __shfl_sync(FULL, at, 31) + incl - mine;
+#pragma unroll
+    for (int r = 0; r < OA_R; r++)
+        for (unsigned m = uw[r]; m; m &= m - 1u, at++)
+            if (at < cap) list[at] = j + (unsigned)(r * nx + (__ffs(m) - 1 - 4 * (lane & 7)));
     return or_rows(uw, lane);
 }
 
@@ -840,6 +854,7 @@ __global__ void __launch_bounds__(OA_WARPS * 32, 3) k_od_approx(const __grid_con
             }
         }
         if (timed_out) break;
+        const bool full = *(volatile unsigned *)L.cnt > L.cap;   // of undecided voxels: the caller falls back
         // huge, infinite or NaN input (an unbounded B), or a non-finite output
         float na, nb;
         unpack2(nanacc, na, nb);
@@ -871,6 +886,7 @@ __global__ void __launch_bounds__(OA_WARPS * 32, 3) k_od_approx(const __grid_con
             if (um < *(volatile int *)&st->umin) atomicMin(&st->umin, um);
             if (lm > *(volatile int *)&st->lmax) atomicMax(&st->lmax, lm);
         }
+        if (__any_sync(FULL, full)) break;
     }
     if (timed_out) {
         // no further copies are issued; wait (bounded) for the ones in flight before leaving
@@ -896,7 +912,7 @@ __global__ void __launch_bounds__(256) k_od_scan(const float *__restrict__ out, 
                                                  OdStats *st, OdLists L) {
     grid_wait();
     __shared__ unsigned todo[OS_T], ntodo;
-    if (st->flags) return;
+    if (st->flags || st->cnt[0] > L.cap) return;   // not every task has a range
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const unsigned nxs = (unsigned)(nx + OA_X - 1) / OA_X, nys = (unsigned)(ny + OA_Y - 1) / OA_Y;
     const unsigned ntask = nxs * nys * ((unsigned)(nz + zrun - 1) / (unsigned)zrun);
@@ -1041,7 +1057,10 @@ __global__ void __launch_bounds__(256) k_od_resolve(const float *__restrict__ in
     const unsigned FULL = 0xffffffffu;
     const bool low = st->cnt[1] > L.cap, high = st->cnt[2] > L.cap;   // lists that do not hold every candidate
     const unsigned nu = st->cnt[0], nmin = low ? OD_SAMPLE : st->cnt[1], nmax = high ? OD_SAMPLE : st->cnt[2], n = nu + nmin + nmax;
-    if (st->flags || nu > L.cap) return;   // the caller falls back
+    if (st->flags || nu > L.cap || !nmin || !nmax) {   // the caller falls back
+        if (blockIdx.x == 0 && threadIdx.x == 0) od_flag(st, OD_FALLBACK);
+        return;
+    }
     const int lane = threadIdx.x & 31;
     const unsigned every = L.cap / OD_SAMPLE;
     for (unsigned i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += (gridDim.x * blockDim.x) >> 5) {
@@ -1444,12 +1463,12 @@ n2m_status od_resolve(const float *in, float *out, int nx, int ny, int nz, float
     return N2M_OK;
 }
 
-n2m_status od_check(const OdWork &w, const OdStats &h, bool *fallback) {
+n2m_status od_check(const OdStats &h, bool *fallback) {
     if (h.flags & OD_TIMEOUT) {
         n2m_set_error("pre-smooth: a tile copy did not complete");
         return N2M_ERR_TIMEOUT;
     }
-    *fallback = (h.flags & OD_FALLBACK) != 0 || h.cnt[0] > w.cap || h.cnt[1] == 0 || h.cnt[2] == 0;
+    *fallback = (h.flags & OD_FALLBACK) != 0;
     return N2M_OK;
 }
 

@@ -77,3 +77,17 @@ def test_plateau_takes_the_path_of_noise(dims, kind):
     o = dict(only_largest=True, fill_bubbles=True)
     flat, noisy = _run(_volume(dims, kind), **o)[1], _run(_volume(dims, kind, 1.0), **o)[1]
     assert abs(flat["kernel_launches"] - noisy["kernel_launches"]) <= 6
+
+
+@pytest.mark.parametrize("label", [False, True])
+@pytest.mark.parametrize("cubes", [n2m.MC33, n2m.OLDCUBES])
+@pytest.mark.parametrize("dims", DIMS)
+def test_isolevel_on_a_plateau(oracle, dims, cubes, label):
+    """a mask meshed at its own value: more undecided voxels than their list holds, so the exact passes run, and the
+    report says so"""
+    v = (_volume(dims, "mask") > 0).astype(np.float32) * 54.0
+    got, rep = _run(v, cubes, only_largest=label, fill_bubbles=label)
+    want = oracle.meshify(v, 54.0, OLDCUBES if cubes == n2m.OLDCUBES else MC33, True, label, label)
+    ok, d, msg = mesh_equal(got, want, 0.0)
+    assert ok, msg
+    assert rep["ms_smooth_pass_a"] == 0.0
