@@ -175,9 +175,10 @@ struct Around {
 // words, a foreground in a tenth of them).
 constexpr int LIST_K = 2;   // words per thread (8: a block for 2048 words left most SMs of a small volume idle)
 __global__ void __launch_bounds__(256) k_run_list(const unsigned *__restrict__ B, LD d, unsigned want, int *list, unsigned *wlist,
-                                                  unsigned *nlist, unsigned *nwlist) {
+                                                  unsigned *nlist, unsigned *nwlist, const unsigned *__restrict__ skip) {
     grid_wait();
     __shared__ unsigned wsum[8], base, wbase;
+    const unsigned off = skip ? __ldg(skip) : 0u;   // looked at late: no wait for it at the start
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     for (unsigned i0 = blockIdx.x * 256 * LIST_K; i0 < d.nwords; i0 += gridDim.x * 256 * LIST_K) {
         unsigned st[LIST_K], n = 0, any = 0;   // n: run starts (a block has at most 32768) | words << 16
@@ -200,6 +201,7 @@ __global__ void __launch_bounds__(256) k_run_list(const unsigned *__restrict__ B
             if (lane >= o) incl += t;
         }
         if (lane == 31) wsum[wid] = incl;
+        if (off) return;   // empty lists: nothing to do for the kernels that follow
         __syncthreads();
         if (tid == 0) {
             unsigned t = 0;
@@ -373,14 +375,16 @@ __global__ void __launch_bounds__(256) k_run_flatten(const int *__restrict__ lis
 // items [0, nrows) take the runs holding x = 0 and x = nx-1 of a row, the items
 // after them one word each of the rows on a y or z face (every run in it).  A
 // flag is stored only if it is not set yet (most items name the same root).
-__global__ void k_run_edges(const unsigned *__restrict__ B, LD d, const int *__restrict__ L, unsigned char *edge) {
+__global__ void k_run_edges(const unsigned *__restrict__ B, LD d, const int *__restrict__ L, unsigned char *edge,
+                            const unsigned *__restrict__ skip) {
     grid_wait();
+    const unsigned off = skip ? __ldg(skip) : 0u;   // then no run has a link
     const unsigned nzf = d.nz > 1 ? 2u : 1u, nyf = d.ny > 1 ? 2u : 1u;
     const unsigned zrows = nzf * (unsigned)d.ny, yrows = d.nz > 2 ? nyf * (unsigned)(d.nz - 2) : 0u;
     const unsigned total = d.nrows + (zrows + yrows) * d.W;
     auto mark = [&](long long j) {
         const int root = L[j];
-        if (!edge[root]) edge[root] = 1;
+        if (!off && !edge[root]) edge[root] = 1;
     };
     for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
         if (t < d.nrows) {
@@ -868,7 +872,7 @@ struct Misc {
 };
 
 n2m_status components(LabelWork &w, const LD &d, const unsigned *B, unsigned want, int conn, Misc *misc, unsigned char *z8,
-                      unsigned *z32, cudaStream_t s) {
+                      unsigned *z32, const unsigned *skip, cudaStream_t s) {
     int *L = w.lab.as<int>(), *list = w.list.as<int>();
     unsigned *nlist = &misc->nlist[want];
     int *cs = w.cs.as<int>();
@@ -876,7 +880,7 @@ n2m_status components(LabelWork &w, const LD &d, const unsigned *B, unsigned wan
     const unsigned g = run_grid(d), wg = gsz(d.nwords);
     unsigned *wlist = w.wlist.as<unsigned>(), *nwlist = &misc->nwlist[want];
     n2m_launch(k_run_starts, rgrid(d), 256, 0, s, B, d, want, cs);
-    n2m_launch(k_run_list, lg, 256, 0, s, B, d, want, list, wlist, nlist, nwlist);
+    n2m_launch(k_run_list, lg, 256, 0, s, B, d, want, list, wlist, nlist, nwlist, skip);
     if (conn == 6) n2m_launch(k_run_hook<3>, 2 * g, 128, 0, s, B, d, want, cs, list, nlist, L, z8, z32);
     else if (conn == 18) n2m_launch(k_run_hook<9>, 2 * g, 128, 0, s, B, d, want, cs, list, nlist, L, z8, z32);
     else n2m_launch(k_run_hook<13>, 2 * g, 128, 0, s, B, d, want, cs, list, nlist, L, z8, z32);
@@ -891,9 +895,9 @@ n2m_status components(LabelWork &w, const LD &d, const unsigned *B, unsigned wan
 }
 
 // the class bits in w.mask on entry; *keep: the kept voxels' bits on return
-// (the foreground after filling, or its largest component)
-n2m_status label_core(LabelWork &w, const LD &d, int conn, bool only_largest, bool fill_bubbles, cudaStream_t s,
-                      const unsigned **keep) {
+// (the foreground after filling, or its largest component); skip: see run_labelling
+n2m_status label_core(LabelWork &w, const LD &d, int conn, bool only_largest, bool fill_bubbles, const unsigned *skip,
+                      cudaStream_t s, const unsigned **keep) {
     CKS(w.lab.ensure((size_t)d.n * sizeof(int)));
     CKS(w.list.ensure(((size_t)d.nrows * ((d.nx + 1) / 2)) * sizeof(int)));   // every second voxel of a row at most
     CKS(w.wlist.ensure((size_t)d.nwords * sizeof(unsigned)));
@@ -905,9 +909,9 @@ n2m_status label_core(LabelWork &w, const LD &d, int conn, bool only_largest, bo
     if (fill_bubbles) {
         CKS(w.edge.ensure((size_t)d.n));
         CKS(w.filled.ensure((size_t)d.nwords * sizeof(unsigned)));
-        CKS(components(w, d, B, 0u, 6, misc, w.edge.as<unsigned char>(), nullptr, s));
+        CKS(components(w, d, B, 0u, 6, misc, w.edge.as<unsigned char>(), nullptr, skip, s));
         n2m_launch(k_run_edges, gsz((long long)d.nrows + 4ll * (d.nx + d.ny + d.nz) * d.W), 256, 0, s, B, d, w.lab.as<int>(),
-                   w.edge.as<unsigned char>());
+                   w.edge.as<unsigned char>(), skip);
         CK(cudaMemcpyAsync(w.filled.p, B, (size_t)d.nwords * sizeof(unsigned), cudaMemcpyDeviceToDevice, s));
         n2m_launch(k_run_fill, run_grid(d), 256, 0, s, B, d, w.list.as<int>(), &misc->nlist[0], w.lab.as<int>(),
                    w.edge.as<unsigned char>(), &misc->nbg, w.filled.as<unsigned>());
@@ -915,7 +919,7 @@ n2m_status label_core(LabelWork &w, const LD &d, int conn, bool only_largest, bo
         B = w.filled.as<unsigned>();
     }
     if (only_largest) CKS(w.cnt.ensure((size_t)d.n * sizeof(unsigned)));
-    CKS(components(w, d, B, 1u, conn, misc, nullptr, only_largest ? w.cnt.as<unsigned>() : nullptr, s));
+    CKS(components(w, d, B, 1u, conn, misc, nullptr, only_largest ? w.cnt.as<unsigned>() : nullptr, skip, s));
     *keep = B;
     if (only_largest) {
         CKS(w.keep.ensure((size_t)d.nwords * sizeof(unsigned)));
@@ -946,7 +950,8 @@ n2m_status class_bits(LabelWork &w, const LD &d, const float *vol, float iso, bo
 }  // namespace
 
 n2m_status run_labelling(const float *vol, int nx, int ny, int nz, float iso, bool only_largest, bool fill_bubbles,
-                         bool at_or_above, LabelWork &w, VolStats *st, cudaStream_t s, const unsigned *vsign, LabelPost *post) {
+                         bool at_or_above, LabelWork &w, VolStats *st, cudaStream_t s, const unsigned *vsign, const unsigned *skip,
+                         LabelPost *post) {
     const LD d = make_ld(nx, ny, nz);
     if (vsign) {
         if (d.n > 0x7fffffffLL) {
@@ -960,7 +965,7 @@ n2m_status run_labelling(const float *vol, int nx, int ny, int nz, float iso, bo
         CKS(class_bits(w, d, vol, iso, false, s));
     }
     const unsigned *K;
-    CKS(label_core(w, d, 18, only_largest, fill_bubbles, s, &K));
+    CKS(label_core(w, d, 18, only_largest, fill_bubbles, skip, s, &K));
     *post = LabelPost{K, nullptr, nullptr, d.W, 0.f, iso, fill_bubbles, only_largest};
     if (only_largest) {
         CKS(w.shell.ensure(2 * (size_t)d.nwords * sizeof(unsigned)));
@@ -1003,7 +1008,7 @@ n2m_status run_bwlabel(float *vol, int nx, int ny, int nz, int conn, bool only_l
     const LD d = make_ld(nx, ny, nz);
     CKS(class_bits(w, d, vol, 0.0f, true, s));
     const unsigned *K;
-    CKS(label_core(w, d, conn, only_largest, fill_bubbles, s, &K));
+    CKS(label_core(w, d, conn, only_largest, fill_bubbles, nullptr, s, &K));
     if (only_largest) {
         n2m_launch(k_write_keep, wgrid(d), 256, 0, s, K, d, vol);
     } else {

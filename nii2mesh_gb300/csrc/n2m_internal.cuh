@@ -209,10 +209,13 @@ struct LabelWork {
 // and count of masked voxels (st).  Otherwise (post->S null), and when st says that no
 // voxel was masked, lab_write labels the volume in place and gives its range and bbox.
 // vsign (may be null): a sign bitmap (OdWork::vsign with od_resolve's at_or_above) to
-// take the mask from; at_or_above: which sign S holds (value >= iso, for oldcubes)
+// take the mask from; at_or_above: which sign S holds (value >= iso, for oldcubes);
+// skip (may be null): a device word that, if not zero, leaves the labelling undone (it was
+// queued before the smoothing was known to hold; its results are not read then)
 // (the minimum, post->mn, is the caller's to fill in)
 n2m_status run_labelling(const float *vol, int nx, int ny, int nz, float iso, bool only_largest, bool fill_bubbles,
-                         bool at_or_above, LabelWork &w, VolStats *st, cudaStream_t s, const unsigned *vsign, LabelPost *post);
+                         bool at_or_above, LabelWork &w, VolStats *st, cudaStream_t s, const unsigned *vsign, const unsigned *skip,
+                         LabelPost *post);
 n2m_status lab_write(float *vol, int nx, int ny, int nz, const LabelPost &P, VolStats *st, cudaStream_t s);
 // the labelling's effect on the marked voxels of vol (marks as od_marks lays them out)
 n2m_status lab_apply(float *vol, int nx, int ny, int nz, const unsigned *need, const LabelPost &P, cudaStream_t s);

@@ -91,3 +91,21 @@ def test_isolevel_on_a_plateau(oracle, dims, cubes, label):
     ok, d, msg = mesh_equal(got, want, 0.0)
     assert ok, msg
     assert rep["ms_smooth_pass_a"] == 0.0
+
+
+def test_labelling_waits_for_the_smoothing():
+    """half of the volume is a plateau at the isolevel (the approximate smoothing does not hold), half is noise (clusters
+    take long): what the labelled call spends before the exact smoothing is done is not another labelling"""
+    rng = np.random.default_rng(5)
+    v = rng.uniform(0, 108, (160, 192, 196)).astype(np.float32)
+    v[:, :, :100] = 54.0
+    d = torch.from_numpy(v).cuda()
+    torch.cuda.synchronize()
+    ctx = n2m.Context()
+    ms = {}
+    for label in (False, True):
+        reps = [ctx.meshify_device(d.data_ptr(), v.shape[::-1], 54.0, only_largest=label, fill_bubbles=label)[4] for _ in range(8)]
+        assert all(r["ms_smooth_pass_a"] == 0.0 for r in reps)
+        ms[label] = min(r["ms_stage"][0] for r in reps), min(r["ms_stage"][1] for r in reps)
+    ctx.close()
+    assert ms[True][0] - ms[False][0] < 0.5 * ms[True][1], ms
