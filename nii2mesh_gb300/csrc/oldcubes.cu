@@ -341,6 +341,7 @@ n2m_status oc_emit(const float *vol, const int dim[3], const int lo[3], const in
                    McWork &w, MarchOut *d_out, const MeshRoom &room, vec3d *d_pts, vec3i *d_tris, int *d_cand,
                    int cand_cap, unsigned *d_near, cudaStream_t s) {
     const OV g = make_ov(vol, dim, lo, hi, iso, edge_max);
+    if (g.NX < 2 || g.NY < 2 || g.NZ < 2) return N2M_OK;   // no cube: oc_count left zero counts and no words
     mcw::Out o;
     CKS(mcw::prepare(w, (size_t)g.WX * g.NY * g.NZ, &d_out->tot, o));
     return mcw::emit(Policy{g, d_pts, d_cand, &d_out->ncand, cand_cap, d_near}, w.signs.as<unsigned>(), w, o, room, d_tris, s);
