@@ -68,6 +68,7 @@ n2m_status DevBuf::ensure(size_t bytes) {
     size_t want = bytes + bytes / 8 + 256;
     cudaError_t e = cudaMalloc(&p, want);
     if (e != cudaSuccess) {
+        cudaGetLastError();   // else the next call's first launch check finds it
         p = nullptr;
         cap = 0;
         n2m_set_error("cudaMalloc(%zu): %s", want, cudaGetErrorString(e));

@@ -19,6 +19,7 @@ void n2m_set_error(const char *fmt, ...);
         cudaError_t e_ = (call);                                                          \
         if (e_ != cudaSuccess) {                                                          \
             n2m_set_error("%s:%d %s: %s", __FILE__, __LINE__, #call, cudaGetErrorString(e_)); \
+            (void)cudaGetLastError();   /* not left for the next call */                  \
             return e_ == cudaErrorMemoryAllocation ? N2M_ERR_OOM : N2M_ERR_CUDA;          \
         }                                                                                 \
     } while (0)
