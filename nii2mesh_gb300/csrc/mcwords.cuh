@@ -466,9 +466,11 @@ __global__ void __launch_bounds__(EW * 32, P::CTAS) k_emit(P pol, const unsigned
     const uint4 tot = *o.total;
     if (!room.fits(tot)) return;   // emitted again into larger buffers
     // Words per group: more fill the lanes better and share the group's start, fewer leave no SM
-    // waiting for a last group.  32 only from eight rounds of groups per resident warp on, 8 (a
-    // word has about 7 vertices) below one round of 16: 512^3 CT (0.6 M active words, four rounds of 32)
-    // 247 us with 32, 239 with 16; brain (14 k words) 157 with 32, 23 with 8.
+    // waiting for a last group.  32 only from eight rounds of groups per resident warp on (1.25 M
+    // active words), 8 (a word has about 7 vertices) below one round of 16.  The emit stage with
+    // the other choice: 512^3 CT without pre-smoothing (19 M triangles) 513 us with 32, 581 with 16;
+    // pre-smoothed (0.6 M active words, four rounds of 32) 249 with 32, 240 with 16; brain (14 k
+    // words) 157 with 32, 23 with 8.
     const unsigned nact = tot.w, G = nact >= 256u * warps ? 32u : (nact >= 16u * warps ? 16u : 8u);
     const uint4 *__restrict__ words = o.words;
     __shared__ EmitShared shared[EW];
