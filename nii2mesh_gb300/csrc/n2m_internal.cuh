@@ -350,8 +350,11 @@ n2m_status mesh_apply_weld(const vec3d *d_pts, int np, const int *d_removed, int
                            const int *d_ov_id, const vec3d *d_ov_pos, int nov, vec3d *d_out, DegWork &w, WeldMap &map,
                            cudaStream_t s);
 // Vertices of marching cubes closer than this to a grid point are marked for the
-// degenerate filter (mesh.cu: k_deg_count; coordinates below 2^22, where floats still
-// resolve it).
+// degenerate filter (mesh.cu: k_deg_count).  Lewiner's distance is that of the stored
+// coordinate, already rounded (at 2^15 a float is a 256th of a voxel): an unmarked vertex is
+// where it is stored, at least this far from the ends of its edge, and so the bound on the area
+// holds for the stored triangle.  (Oldcubes takes the fraction along the edge: its positions are
+// doubles.)  Coordinates below 2^22: mc33::frac_dist rounds to integers there.
 constexpr float NEAR_CORNER = 1.f / 512;
 __device__ __forceinline__ void mark_near(unsigned *near, int id) {
     if (near) atomicOr(near + (id >> 5), 1u << (id & 31));
