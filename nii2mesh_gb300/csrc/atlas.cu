@@ -486,6 +486,7 @@ template <int NNB> struct ARound {
 // another, and every start's link: to the run of its first contact with the rows before
 // (without a union), else to itself.  z8 / z32 (may be null) are zeroed there.
 constexpr int AL_K = 8;   // words per thread
+static_assert(256 * AL_K * 16 < 65536, "a block's run starts and words share one 32-bit sum");
 template <int NNB>
 __global__ void __launch_bounds__(256) k_al_list(const ABox *boxes, const unsigned *__restrict__ wbox, unsigned nbw,
                                                  const unsigned *__restrict__ Bits, unsigned want, uint2 *list, unsigned *wlist,
@@ -494,7 +495,7 @@ __global__ void __launch_bounds__(256) k_al_list(const ABox *boxes, const unsign
     __shared__ unsigned wsum[8], base, wbase;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     for (unsigned i0 = blockIdx.x * 256 * AL_K; i0 < nbw; i0 += gridDim.x * 256 * AL_K) {
-        unsigned st[AL_K], cnt = 0, any = 0;   // run starts (a block has at most 32768) | words << 16
+        unsigned st[AL_K], cnt = 0, any = 0;   // run starts | words << 16
 #pragma unroll
         for (int k = 0; k < AL_K; k++) {
             const unsigned gw = i0 + (unsigned)(k * 256 + tid);

@@ -450,7 +450,7 @@ void sort_weld_lists(std::vector<int> &removed, std::vector<int> &keep, std::vec
 // each is one element in the reference's vertex order.  Outputs the removed
 // ids (sorted), the id each merges into, and position overrides (the group's
 // last writer in the reference's vertex order).
-n2m_status weld_candidates(n2m_context *c, int nv, int ncand, std::vector<int> &removed, std::vector<int> &keep,
+n2m_status weld_candidates(n2m_context *c, int ncand, std::vector<int> &removed, std::vector<int> &keep,
                            std::vector<int> &ov_id, std::vector<vec3d> &ov_pos, std::vector<int> &ov_src, vec3d v0) {
     std::vector<int> ids(ncand);
     if (c->mo_cand) memcpy(ids.data(), c->mo.cand_id, ncand * sizeof(int));
@@ -499,7 +499,6 @@ n2m_status weld_candidates(n2m_context *c, int nv, int ncand, std::vector<int> &
         }
     }
     sort_weld_lists(removed, keep, ov_id, ov_pos, ov_src);
-    (void)nv;
     return N2M_OK;
 }
 
@@ -928,7 +927,7 @@ n2m_status pipeline(n2m_context *c, const float *d_src, const int dim[3], const 
         } else {
             vec3d v0 = c->mo.first;
             if (!c->mo_cand) CKS(readback(c, &v0, pts));
-            CKS(weld_candidates(c, nv, ncand, removed, keep, ov_id, ov_pos, ov_src, v0));
+            CKS(weld_candidates(c, ncand, removed, keep, ov_id, ov_pos, ov_src, v0));
         }
         if (!removed.empty() || !ov_id.empty()) {
             const int nr = (int)removed.size(), no = (int)ov_id.size(), ncr = (int)corners.size();
@@ -1289,7 +1288,7 @@ extern "C" n2m_status n2m_meshify_backward(n2m_context *c, const float *d_grad_p
     }
     const float3 *graw = go;
     if (c->fwd.nrem > 0) {
-        CKS(mesh_weld_backward(go, np, nvr, c->fwd.removed, c->fwd.nrem, c->fwd.ov_id, c->fwd.ov_src, c->fwd.nov,
+        CKS(mesh_weld_backward(go, nvr, c->fwd.removed, c->fwd.nrem, c->fwd.ov_id, c->fwd.ov_src, c->fwd.nov,
                                c->gB.as<float3>(), c->stream));
         graw = c->gB.as<float3>();
     }

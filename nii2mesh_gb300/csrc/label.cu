@@ -120,8 +120,8 @@ __global__ void __launch_bounds__(256) k_run_starts(const unsigned *__restrict__
         for (unsigned c0 = 0; c0 < d.W; c0 += (unsigned)seg) {
             const unsigned w = c0 + (unsigned)li;
             const bool ok = r < d.nrows && w < d.W;
-            const WordRuns R = word_runs(ok ? class_word(B, d, r, w, want) : 0u, (int)w * 32, li, seg, cst, cwd);
-            if (ok) cs[(size_t)r * d.W + w] = R.cs;
+            const int start = run_before(ok ? class_word(B, d, r, w, want) : 0u, (int)w * 32, li, seg, cst, cwd);
+            if (ok) cs[(size_t)r * d.W + w] = start;
         }
     }
 }
@@ -174,6 +174,7 @@ struct Around {
 // words only a few lanes of a warp had a run (512^3: 0.8 M background runs in 4.2 M
 // words, a foreground in a tenth of them).
 constexpr int LIST_K = 2;   // words per thread (8: a block for 2048 words left most SMs of a small volume idle)
+static_assert(256 * LIST_K * 16 < 65536, "a block's run starts and words share one 32-bit sum");
 __global__ void __launch_bounds__(256) k_run_list(const unsigned *__restrict__ B, LD d, unsigned want, int *list, unsigned *wlist,
                                                   unsigned *nlist, unsigned *nwlist, const unsigned *__restrict__ skip) {
     grid_wait();
@@ -181,7 +182,7 @@ __global__ void __launch_bounds__(256) k_run_list(const unsigned *__restrict__ B
     const unsigned off = skip ? __ldg(skip) : 0u;   // looked at late: no wait for it at the start
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     for (unsigned i0 = blockIdx.x * 256 * LIST_K; i0 < d.nwords; i0 += gridDim.x * 256 * LIST_K) {
-        unsigned st[LIST_K], n = 0, any = 0;   // n: run starts (a block has at most 32768) | words << 16
+        unsigned st[LIST_K], n = 0, any = 0;   // n: run starts | words << 16
 #pragma unroll
         for (int k = 0; k < LIST_K; k++) {
             const unsigned i = i0 + (unsigned)(k * 256 + tid);

@@ -418,12 +418,11 @@ n2m_status mesh_weld_candidates(const vec3d *d_pts, const MeshRoom &room, const 
     return N2M_OK;
 }
 
-n2m_status mesh_weld_backward(const float3 *d_go, int np_final, int nv_raw, const int *d_removed, int nrem,
+n2m_status mesh_weld_backward(const float3 *d_go, int nv_raw, const int *d_removed, int nrem,
                               const int *d_ov_id, const int *d_ov_src, int nov, float3 *d_graw, cudaStream_t s) {
     CK(cudaMemsetAsync(d_graw, 0, (size_t)nv_raw * sizeof(float3), s));
     n2m_launch(k_weld_back, gs(nv_raw), 256, 0, s, d_go, nv_raw, d_removed, nrem, d_ov_id, d_ov_src, nov, d_graw);
     CKL();
-    (void)np_final;
     return N2M_OK;
 }
 

@@ -386,7 +386,7 @@ n2m_status mesh_smooth_hc_check(HcWork &w, int np, int iter, cudaStream_t s);
 n2m_status mesh_smooth_hc_backward(int np, double alpha, double beta, int iter, bool lock_edges, HcWork &w,
                                    const float3 *d_g, float3 *d_go, cudaStream_t s);
 // grad of raw (pre-weld) vertices from grad of welded vertices
-n2m_status mesh_weld_backward(const float3 *d_go, int np_final, int nv_raw, const int *d_removed, int nrem,
+n2m_status mesh_weld_backward(const float3 *d_go, int nv_raw, const int *d_removed, int nrem,
                               const int *d_ov_id, const int *d_ov_src, int nov, float3 *d_graw, cudaStream_t s);
 n2m_status mesh_apply_sform(vec3d *d_pts, vec3i *d_tris, int np, int nt, const float sx[4], const float sy[4],
                             const float sz[4], cudaStream_t s);
