@@ -477,16 +477,17 @@ n2m_status launch_stats(const float *vol, int nx, int ny, int nz, float iso, boo
 
 // ==== pre-smooth with exact rounding on demand ===================================
 // Marching cubes reads the smoothed volume in two ways only: the sign of every
-// grid point (value >= iso, and value - iso against the FLT_EPSILON clamp) and
-// the values at the corners of the cubes the surface crosses.  So the volume
+// grid point (value >= iso, and value - iso against the FLT_EPSILON clamp), and
+// the values at the ends of the edges the surface crosses and at the corners of
+// ambiguous cubes.  So the volume
 // is first smoothed approximately in one fused FP32 pass (pass A: one read and
 // one write per voxel), with a rigorous error bound; the few voxels whose sign
 // the bound leaves open, and the candidates for the volume's minimum and
 // maximum, are recomputed with the reference's double sequence (pass B).
-// After the sign words, the corners of every cube with mixed signs are marked
-// (mc.cu: k_need) and the exact three-pass smoothing runs on those voxels
+// With the sign words the voxels whose values will be read are marked
+// (mcwords.cuh: k_words) and the exact three-pass smoothing runs on those voxels
 // only, the x and y passes on the voxels those depend on (marks dilated by +-2
-// slices, then +-2 rows), each pass one thread per marked voxel.  Every value
+// slices, then +-2 rows), by lists of bit words.  Every value
 // marching cubes reads is then the reference's float, bit for bit.
 //
 // Error bound of pass A: each pass evaluates the tap sum as an FP32 FMA chain
@@ -905,14 +906,16 @@ __global__ void __launch_bounds__(OA_WARPS * 32, 3) k_od_approx(const __grid_con
 // reads the few that qualify again with all its warps, a slice's 16 loads of a warp in
 // flight at once (a warp per task and one row after another took 246 us for the
 // 512^3 CT volume's handful).  A list that is full (a plateau at that extreme) takes no
-// more; k_od_resolve then finds that extreme without it.
+// more; k_od_resolve then finds that extreme without it.  8.4 us for the 512^3 CT volume; 73
+// padded with one value (107 with an atomic per voxel there too).
 constexpr int OS_T = 64;
 constexpr unsigned OD_SAMPLE = 4096;   // at most a list's capacity
 __global__ void __launch_bounds__(256) k_od_scan(const float *__restrict__ out, int nx, int ny, int nz, int zrun,
                                                  OdStats *st, OdLists L) {
     grid_wait();
     __shared__ unsigned todo[OS_T], ntodo;
-    if (st->flags || st->cnt[0] > L.cap) return;   // not every task has a range
+    const unsigned flags = st->flags, undecided = st->cnt[0];   // read together
+    if (flags || undecided > L.cap) return;   // not every task has a range
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const unsigned nxs = (unsigned)(nx + OA_X - 1) / OA_X, nys = (unsigned)(ny + OA_Y - 1) / OA_Y;
     const unsigned ntask = nxs * nys * ((unsigned)(nz + zrun - 1) / (unsigned)zrun);
@@ -926,13 +929,21 @@ __global__ void __launch_bounds__(256) k_od_scan(const float *__restrict__ out, 
         if (task < ntask && (__fsub_rd(t.x, t.z) <= umin || __fadd_ru(t.y, t.z) >= lmax)) todo[atomicAdd(&ntodo, 1u)] = task;
     }
     __syncthreads();
-    // one atomic per warp and list
-    auto put = [&](bool want, unsigned j, unsigned *n, unsigned *list) {
-        const unsigned m = __ballot_sync(FULL, want);
-        if (!m) return;
-        unsigned at = lane == 0 ? atomicAdd(n, (unsigned)__popc(m)) : 0u;
-        at = __shfl_sync(FULL, at, 0) + __popc(m & ((1u << lane) - 1u));
-        if (want && at < L.cap) list[at] = j;
+    // bit k of m: the lane's voxel of row k / 2, columns 32 (k & 1) on, j being that of k = 0; one atomic per warp
+    auto put = [&](unsigned m, unsigned j, unsigned *n, unsigned *list) {
+        if (!__any_sync(FULL, m != 0u)) return;
+        unsigned incl = __popc(m);
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned t = __shfl_up_sync(FULL, incl, o);
+            if (lane >= o) incl += t;
+        }
+        unsigned at = lane == 31 ? atomicAdd(n, incl) : 0u;
+        at = __shfl_sync(FULL, at, 31) + incl - __popc(m);
+        for (; m; m &= m - 1u, at++) {
+            const unsigned k = (unsigned)__ffs(m) - 1u;
+            if (at < L.cap) list[at] = j + (k >> 1) * (unsigned)nx + 32u * (k & 1u);
+        }
     };
     unsigned open = 3u;   // lists (1: minimum, 2: maximum) that this warp has not seen full
     for (unsigned i = 0; i < ntodo; i++) {
@@ -940,8 +951,10 @@ __global__ void __launch_bounds__(256) k_od_scan(const float *__restrict__ out, 
         const float4 t = L.range[task];
         const unsigned want = (__fsub_rd(t.x, t.z) <= umin ? 1u : 0u) | (__fadd_ru(t.y, t.z) >= lmax ? 2u : 0u);
         if (!(want & open)) continue;
-        const unsigned room = (*(volatile unsigned *)&L.cnt[1] <= L.cap ? 1u : 0u) | (*(volatile unsigned *)&L.cnt[2] <= L.cap ? 2u : 0u);
-        open &= __shfl_sync(FULL, room, 0);
+        if (i) {   // (the first task, often the only one, waits for no count)
+            const unsigned room = (*(volatile unsigned *)&L.cnt[1] <= L.cap ? 1u : 0u) | (*(volatile unsigned *)&L.cnt[2] <= L.cap ? 2u : 0u);
+            open &= __shfl_sync(FULL, room, 0);
+        }
         const bool mn = want & open & 1u, mx = want & open & 2u;   // the same for the whole warp
         if (!mn && !mx) continue;
         const int x0 = (int)xs * OA_X, y0 = (int)(t2 % nys) * OA_Y, zs = (int)(t2 / nys) * zrun, ze = min(zs + zrun, nz);
@@ -952,11 +965,33 @@ __global__ void __launch_bounds__(256) k_od_scan(const float *__restrict__ out, 
                 const int x = x0 + 32 * (k & 1) + lane, y = y0 + (k >> 1);
                 v[k] = x < nx && y < ny ? out[(size_t)z * nxy + (size_t)y * nx + x] : NAN;
             }
+            const unsigned j0 = (unsigned)((size_t)z * nxy + (size_t)y0 * nx + x0 + lane);
+            // a plateau shows in the middle row (votes for every row would cost the usual few candidates 1 us)
+            if (mn && __all_sync(FULL, !(__fsub_rd(v[OA_Y], t.z) > umin))) {
+                unsigned m = 0u;
 #pragma unroll
-            for (int k = 0; k < 2 * OA_Y; k++) {   // a NaN is in neither list
-                const unsigned j = (unsigned)((size_t)z * nxy + (size_t)(y0 + (k >> 1)) * nx + x0 + 32 * (k & 1) + lane);
-                if (mn) put(__fsub_rd(v[k], t.z) <= umin, j, &L.cnt[1], L.cmin);
-                if (mx) put(__fadd_ru(v[k], t.z) >= lmax, j, &L.cnt[2], L.cmax);
+                for (int k = 0; k < 2 * OA_Y; k++) m |= (__fsub_rd(v[k], t.z) <= umin ? 1u : 0u) << k;
+                put(m, j0, &L.cnt[1], L.cmin);
+            } else if (mn) {
+#pragma unroll
+                for (int k = 0; k < 2 * OA_Y; k++)   // a NaN is in neither list
+                    if (__fsub_rd(v[k], t.z) <= umin) {
+                        const unsigned q = atomicAdd(&L.cnt[1], 1u);
+                        if (q < L.cap) L.cmin[q] = j0 + (unsigned)((k >> 1) * nx + 32 * (k & 1));
+                    }
+            }
+            if (mx && __all_sync(FULL, !(__fadd_ru(v[OA_Y], t.z) < lmax))) {
+                unsigned m = 0u;
+#pragma unroll
+                for (int k = 0; k < 2 * OA_Y; k++) m |= (__fadd_ru(v[k], t.z) >= lmax ? 1u : 0u) << k;
+                put(m, j0, &L.cnt[2], L.cmax);
+            } else if (mx) {
+#pragma unroll
+                for (int k = 0; k < 2 * OA_Y; k++)
+                    if (__fadd_ru(v[k], t.z) >= lmax) {
+                        const unsigned q = atomicAdd(&L.cnt[2], 1u);
+                        if (q < L.cap) L.cmax[q] = j0 + (unsigned)((k >> 1) * nx + 32 * (k & 1));
+                    }
             }
         }
     }
@@ -967,7 +1002,7 @@ __global__ void __launch_bounds__(256) k_od_scan(const float *__restrict__ out, 
 // it depends on, nor above tap^k(M).  Its other axes leave it in their face layers (0, 1, n - 2,
 // n - 1), and everything it depends on in the same ones, so m and M are the extremes of the raw
 // voxels in the face layers of at least 3 - k axes: r[c], c = 3 - k.
-__device__ __noinline__ void raw_extremes(const float *__restrict__ in, int nx, int ny, int nz, OdStats *st) {
+__device__ __forceinline__ void raw_extremes(const float *__restrict__ in, int nx, int ny, int nz, OdStats *st) {
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     float lo[4], hi[4];   // of the voxels in the face layers of at least c axes
@@ -1026,7 +1061,7 @@ __device__ __noinline__ void raw_extremes(const float *__restrict__ in, int nx, 
     }
 }
 // whether the extremes found among some of the candidates are the bounds above, which makes them the volume's
-__device__ __noinline__ bool plateau_holds(const OdStats *st, bool low, bool high) {
+__device__ __forceinline__ bool plateau_holds(const OdStats *st, bool low, bool high) {
     float mn = INFINITY, mx = -INFINITY;
     for (int c = 0; c < 4; c++) {
         float l = ord2f(*(volatile const int *)&st->rlo[c]), h = ord2f(*(volatile const int *)&st->rhi[c]);
@@ -1046,8 +1081,8 @@ __device__ __noinline__ bool plateau_holds(const OdStats *st, bool low, bool hig
 // is the bound that the raw volume gives (plateau_holds): so for a constant background
 // or a saturated region, which has voxels whose whole window is that value.  Else the caller
 // falls back.  The constant background of a skull-stripped head or of a padded CT fell back on
-// every call without this: 181 x 217 x 181 head 337 -> 294 us (604 -> 416 labelled),
-// 511 x 512 x 300 CT 1619 -> 1100 (2330 -> 1273).  A warp per
+// every call without this: 181 x 217 x 181 head 337 -> 284 us (604 -> 414 labelled),
+// 511 x 512 x 300 CT 1619 -> 1079 (2330 -> 1258).  A warp per
 // voxel: 25 lanes take one row's x tap each, five the y taps, then the z tap, all in
 // the reference's double sequence (a thread per voxel walked the 31 taps one after
 // another: 29 us for the 512^3 CT volume's few thousand voxels).
@@ -1057,7 +1092,8 @@ __global__ void __launch_bounds__(256) k_od_resolve(const float *__restrict__ in
     const unsigned FULL = 0xffffffffu;
     const bool low = st->cnt[1] > L.cap, high = st->cnt[2] > L.cap;   // lists that do not hold every candidate
     const unsigned nu = st->cnt[0], nmin = low ? OD_SAMPLE : st->cnt[1], nmax = high ? OD_SAMPLE : st->cnt[2], n = nu + nmin + nmax;
-    if (st->flags || nu > L.cap || !nmin || !nmax) {   // the caller falls back
+    const unsigned flags = st->flags;
+    if (flags || nu > L.cap || !nmin || !nmax) {   // the caller falls back
         if (blockIdx.x == 0 && threadIdx.x == 0) od_flag(st, OD_FALLBACK);
         return;
     }
