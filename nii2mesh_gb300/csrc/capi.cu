@@ -1,14 +1,19 @@
 // capi.cu — host orchestration of the meshify pipeline and the C ABI.
 //
 // meshify (src/meshify.c:286-389) on the GPU, stage by stage:
-//   1. pre-smooth fused with range + bbox (smooth.cu), or a range/bbox pass
-//   2. one readback: range, isolevel fallback, non-finite check
-//   3. optional clustering (label.cu), range/bbox recomputed afterwards
-//   4. marching cubes count pass + scan (mc.cu / oldcubes.cu), readback of
-//      the vertex/triangle totals, emit pass straight into vec3d/vec3i
-//   5. weld: the few near-grid-point candidates are read back and grouped on
+//   1. pre-smooth with range + bbox (smooth.cu), or a range/bbox pass
+//   2. optional clustering (label.cu), queued before anything is read back
+//   3. one readback: range, isolevel fallback, non-finite check, the bbox after
+//      clustering; what was queued on an isolevel or a smoothing that does not
+//      hold is done again
+//   4. marching cubes count pass + scan (mc.cu / oldcubes.cu), the emit straight into
+//      vec3d/vec3i in the buffers of earlier calls, and 6., queued behind one another;
+//      then the readback of totals, weld candidates and kept triangles (a mesh that
+//      does not fit is emitted again)
+//   5. weld: the few near-grid-point candidates are grouped on
 //      the host with the reference's greedy rule; merges applied on device
-//   6. degenerate-triangle removal and compaction (mesh.cu)
+//   6. degenerate-triangle removal and compaction (mesh.cu), after the weld if
+//      there were candidates
 // Edge darkening is applied on the fly by the marching-cubes value fetch.
 #include <stdarg.h>
 #include <stdint.h>

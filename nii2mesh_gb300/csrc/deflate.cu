@@ -41,7 +41,7 @@ constexpr int DF_HBITS = 10, DF_HSIZE = 1 << DF_HBITS;   // hash buckets per chu
 // CTAs fill the SMs unevenly: a 92 MB mesh took 1934 us with 16, 1836 with 8, 1802 with 4, and with fewer
 // instructions per tile 1778, 1711 and 1744.
 constexpr int LZ_WARPS = 8;
-constexpr int LZ_SLOTS = 48;                     // chunks per SM that the chunk size aims at
+constexpr int LZ_SLOTS = 48;                     // chunks that an SM of a GB300 holds; the chunk size aims at one wave of them
 constexpr int DF_WARPS = 4;                      // chunks per CTA of k_huff
 constexpr int BITS_WARPS = 8;                    // chunks per CTA of k_bits
 constexpr int DF_MAXLEN = 258;

@@ -12,6 +12,9 @@
 
 #define N2M_FLT_EPS 1.19209290e-07f
 
+// Grids are bounded by multiples of 152, the SMs of a GB300 (and LZ_SLOTS in deflate.cu is what one
+// of them holds): on another number of SMs the kernels are correct, their grids no longer fit it.
+
 // ---- error plumbing ---------------------------------------------------------
 void n2m_set_error(const char *fmt, ...);
 #define CK(call)                                                                          \
@@ -38,8 +41,8 @@ extern std::atomic<long long> g_n2m_launches;
 // releases its successor earlier, so two kernels' blocks never run side by side), and
 // grid_wait() returns once everything before it in the stream is complete and visible.
 // A call is a chain of 30 to 45 kernels of a few microseconds, and the gap between two of
-// them counts: 64^3 spheres 437 -> 371 us, brain with Otsu level 835 -> 741, 128^3 fit
-// 1318 -> 1178, HC drop-in 924 -> 842.  Letting successors start as soon as all blocks of
+// them counts: 64^3 spheres 423 -> 382 us, brain with Otsu level 808 -> 755, 128^3 fit
+// 1328 -> 1198, HC drop-in 933 -> 842.  Letting successors start as soon as all blocks of
 // a kernel run was slower (brain 776, HC 1000 us: waiting blocks take slots).
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
@@ -195,7 +198,7 @@ n2m_status launch_stats(const float *vol, int nx, int ny, int nz, float iso, boo
                         cudaStream_t s, int z0 = 0);
 void stats_init_host(VolStats *h);
 
-// scan.cu: exclusive scan of uint4 (component-wise) in place; total -> *d_total
+// scan.cu: exclusive scan in place; total -> *d_total
 struct ScanWork {
     DevBuf part;
 };
