@@ -36,17 +36,14 @@ sys.path.insert(0, str(ROOT))
 METRIC = "Gvox/s smooth+MC+weld at 512³; atlas meshes/s batched vs loop; fwd+bwd ms @128³"
 WORKLOAD = "ct512: 512^3 f32 CT-like, iso 300, -p 1 -l 0 -b 0 -o 0 -r 1 -s 0 (Lewiner MC33)"
 ISO = 300.0
-# DRAM bytes (read + write) per step of each stage on this workload: one ncu capture of
-# `bench.py --profile 384` (dram__bytes_read.sum + dram__bytes_write.sum of the stage's kernels),
-# scaled by the voxel count to 512^3: smooth = pass A + pass B, count = sign words, marks, exact
-# passes on marked voxels, tests, numbering, emit = k_emit, weld, degenerate
-SCALE_384 = (512 / 384) ** 3
-NCU_TRAFFIC = {"smooth": 431.2e6 * SCALE_384, "count": 333.7e6 * SCALE_384, "emit": 107.3e6 * SCALE_384,
-               "weld": 37.0e6 * SCALE_384, "degenerate": 77.7e6 * SCALE_384}
-PASS_A_TRAFFIC = 430.9e6 * SCALE_384   # k_od_approx alone
+# DRAM bytes (read + write) per step of each stage on this workload: dram__bytes_read.sum + dram__bytes_write.sum of
+# the stage's kernels in one ncu capture of the 512^3 call (profiles/kernels_by_workload.md): smooth = pass A + pass B,
+# count = sign words, marks, exact passes on marked voxels, tests, numbering, emit = k_emit, weld, degenerate
+NCU_TRAFFIC = {"smooth": 1094.3e6, "count": 992.8e6, "emit": 318.7e6, "weld": 118.8e6, "degenerate": 236.9e6}
+PASS_A_TRAFFIC = 1093.8e6   # k_od_approx alone
 # what bounds each stage (measured)
-STAGE_BOUND = {"smooth": "FP32 instruction issue in pass A (53 % of the slots, 38 instructions per voxel; registers allow "
-                         "12 warps per SM); DRAM 7.6 B/voxel, no re-reads",
+STAGE_BOUND = {"smooth": "pass A: dependent FP32 chains and half-rate min/max and shifts at 12 warps per SM (registers), 53 % "
+                         "of the issue slots; DRAM 8.15 B/voxel, no re-reads",
                "count": "the exact passes on the ~10 % marked voxels (gathers' latency and issue) and the word passes",
                "emit": "issue and value loads"}
 STAGE_NAMES = ("smooth", "cluster", "count", "emit", "weld", "degenerate", "hc")
@@ -752,9 +749,9 @@ def main():
     roof = {"bound": "hbm", "kernel": "k_od_approx (pre-smooth pass A)", "achieved": round(pa_gbs, 1) if pa_gbs else None,
             "peak": peak, "unit": "GB/s", "frac": round(pa_gbs / peak, 4) if pa_gbs else None, "peak_source": peak_kind,
             "kernel_ms": round(pa_ms, 4), "algorithmic_bytes": pa_bytes, "traffic": PASS_A_TRAFFIC,
-            "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one k_od_approx launch at 384^3, "
-                              "scaled by the voxel count",
-            "limited_by": "FP32 instruction issue (53 % of the slots, 12 warps per SM); memory 4.1 TB/s",
+            "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one k_od_approx launch of this workload",
+            "limited_by": "latency of dependent FP32 chains and half-rate ALU work at register-limited occupancy (12 warps "
+                          "per SM, 53 % of the issue slots)",
             "whole_path": {"bytes": whole, "achieved": round(whole_gbs, 1), "frac": round(whole_gbs / peak, 4),
                            "formula": "(4 N_vox + 24 N_vert + 12 N_tri) / ms_per_step / peak",
                            "dram_bytes": round(sum(NCU_TRAFFIC.values())),

@@ -27,9 +27,9 @@
 // triangle corner finds its vertex id with one 16-byte load.  Inactive words have
 // no record: nothing refers to them.
 //
-// Measured on the 512^3 CT volume (7.1 M triangles, 4.5 M words, cold caches): masks,
+// Measured on a 512^3 CT volume (7.6 M triangles, 4.5 M words, cold caches): masks,
 // marks, counts, scan and active list 290 -> 150 us (k_words 85: a block scan per 256
-// words had cost 120, waiting for the block's fullest warp); emit 474 -> 211 us
+// words had cost 120, waiting for the block's fullest warp); emit 474 -> 207 us
 // against one lane per word listing its cubes for the warp, with separate mask and
 // offset arrays and the ambiguous tests repeated.  Two emit kernels (vertices,
 // triangles) took 255, two vertices per lane in flight 250.  On the brain volume

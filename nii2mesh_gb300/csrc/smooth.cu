@@ -595,7 +595,7 @@ __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.
 // number of polls (flag OD_TIMEOUT), after waiting, also bounded, for the warp's
 // copies still in flight.
 //
-// 512^3: 1.09 GB (8.1 bytes a voxel) in 268 us = 4.1 TB/s, 38 instructions a voxel at
+// 512^3: 1.09 GB (8.15 bytes a voxel) in 255 us = 4.3 TB/s, 38 instructions a voxel at
 // 53 % of the issue slots: the register ring allows 12 warps per SM, and their
 // dependent FP32 chains and the half-rate min/max and shifts bound it.  With one column
 // and 8 rows per lane (x pass first, five shared-memory loads per row, 92
